@@ -7,6 +7,7 @@ prepare(c, s)    what the program holds before the call: plan or weights, inputs
 run(state)       one pass through the public entry points
 work(c)          bytes and floating-point operations one pass cannot do without
 tolerance(c)     how far another correct single-precision implementation may be off
+exact(c, s)      what run returns, from plain torch in double precision
 """
 import math
 
@@ -164,3 +165,69 @@ def tolerance(case):
     # Single-precision transforms and channel sums.  Against the same layer in double precision every
     # case shows a relative error of at most 1.1e-6 and a largest one of 5e-6 of the rms value.
     return {"rel": 4e-6, "max": 2e-5}
+
+
+def exact(case, seed):
+    st = prepare(case, seed)
+    reference = case["layout"] == "reference"
+    rank = 2 if case["DX"] else 1
+    dims = (-2, -1)[-rank:]
+    x, w = st["x"].detach(), st["w"].detach().to(torch.complex128)
+    if reference:
+        x, w = x.transpose(0, 1), w.transpose(0, 1)
+    gy = st.get("grad_y")
+    grad_w = torch.zeros_like(w)
+    ys, gxs = [], []
+    # kept modes: 0..63 of every axis, or -32..31 of the first of two
+    shift = MODES // 2 if case["centered"] else 0
+    step = max(1, 2 ** 26 // (max(x.shape[1], w.shape[1]) * x[0, 0].numel()))
+    for b in range(0, x.shape[0], step):
+        xb = x[b:b + step].to(torch.float64 if st["kind"].startswith("real") else torch.complex128)
+        y, back = _exact_layer(xb, w, dims, shift, None if gy is None else gy[b:b + step])
+        ys.append(y)
+        if back is not None:
+            gxs.append(back[0])
+            grad_w += back[1]
+    y = torch.cat(ys)
+    if gy is not None:
+        return {"y": y, "grad_x": torch.cat(gxs), "grad_w": grad_w}
+    return y.transpose(0, 1).contiguous() if reference else y
+
+
+def _exact_layer(x, w, dims, shift, gy):
+    length = math.prod(x.shape[2:])
+    real = not x.is_complex()
+    L = "xy"[-len(dims):]
+
+    def spectrum(t):
+        s = torch.fft.fftn(t, dim=dims)
+        if shift:
+            s = s.roll(shift, dims=-2)
+        return s[(Ellipsis,) + (slice(0, MODES),) * len(dims)]
+
+    def field(s):
+        full = s.new_zeros(s.shape[:2] + x.shape[2:])
+        full[(Ellipsis,) + (slice(0, MODES),) * len(dims)] = s
+        if shift:
+            full = full.roll(-shift, dims=-2)
+        return torch.fft.ifftn(full, dim=dims)
+
+    def mix(spec, mats, sub):
+        if mats.dim() == 2:
+            sub = sub.replace("%", "")
+        return torch.einsum(sub.replace("%", L).replace("#", L), spec, mats)
+
+    # a real field: the kept half spectrum enters the inverse once (ky = 0) or with its mirror image (ky > 0)
+    half = torch.ones(MODES, dtype=torch.float64, device=w.device)
+    if real:
+        half[0] = 0.5
+    xs = spectrum(x)
+    y = field(mix(xs * half, w, "bk#,kn%->bn#"))
+    if real:
+        y = 2.0 * y.real
+    if gy is None:
+        return y, None
+    gs = spectrum(gy.to(x.dtype)) * half * (2.0 if real else 1.0)
+    grad_x = field(mix(gs, w.conj(), "bn#,kn%->bk#"))
+    grad_w = torch.einsum("bk#,bn#->kn%".replace("%", L if w.dim() > 2 else "").replace("#", L), xs.conj(), gs) / length
+    return y, (grad_x.real if real else grad_x, grad_w)
