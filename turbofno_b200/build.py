@@ -55,11 +55,17 @@ def build_library(force=False, verbose=False):
     srcs = _lib_sources()
     if not force and not _newer(LIB, srcs):
         return LIB
+    # one object per translation unit, compiled side by side
     cus = [s for s in srcs if s.endswith(".cu")]
-    cmd = ["nvcc"] + NVCC_FLAGS + ["-shared"] + cus + ["-o", LIB, "-lcufft", "-lcublas"]
-    if verbose:
-        cmd += ["-Xptxas", "-v"]
-    subprocess.check_call(cmd)
+    objs = [os.path.splitext(s)[0] + ".o" for s in cus]
+    flags = NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else [])
+    jobs = [subprocess.Popen(["nvcc"] + flags + ["-c", s, "-o", o]) for s, o in zip(cus, objs)]
+    for job in jobs:
+        job.wait()
+    for s, job in zip(cus, jobs):
+        if job.returncode:
+            raise subprocess.CalledProcessError(job.returncode, "nvcc -c " + s)
+    subprocess.check_call(["nvcc"] + NVCC_FLAGS + ["-shared"] + objs + ["-o", LIB, "-lcufft", "-lcublas"])
     _stamp(LIB, srcs)
     return LIB
 

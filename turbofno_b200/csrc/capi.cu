@@ -337,6 +337,17 @@ size_t tfno_workspace_bytes(const tfno_plan* plan) { return plan ? plan->ws_byte
 
 }  // extern "C"
 
+// C[n, b, m] = alpha sum_k A[k, b, m] W[k, n, m] on compact spectra A[(k*B + b)*modes + m]
+static PerModeParams permode_layer(const tfno_problem& p, long long B, long long modes, const float2* A, const float2* w, float2* C, float2 alpha) {
+    PerModeParams q{};
+    q.I = (int)B; q.J = p.N; q.red = p.K; q.modes = modes;
+    q.p = A; q.p_sr = B * modes; q.p_si = modes;
+    q.q = w; q.q_sr = p.w_stride_k; q.q_sj = p.w_stride_n; q.q_sm = p.w_stride_m;
+    q.o = C; q.o_si = modes; q.o_sj = B * modes; q.o_sm = 1;
+    q.alpha = q.alpha0 = alpha;
+    return q;
+}
+
 // The dispatch of one layer.  With dev.record set it is a dry run: every launcher appends the
 // name of the kernel it would launch and nothing touches the device.
 static int exec_impl(const tfno_plan* plan, const DeviceInfo& dev, const void* x, const void* w, void* y, void* workspace,
@@ -378,11 +389,7 @@ static int exec_impl(const tfno_plan* plan, const DeviceInfo& dev, const void* x
         if (plan->per_mode) {
             rc = launch_fft_rows(dev, p.DY, fr, st);
             if (rc) return rc;
-            PerModeParams pm{};
-            pm.rows = B; pm.modes = kModes; pm.K = p.K; pm.N = p.N;
-            pm.a = A; pm.w = win; pm.w_sk = p.w_stride_k; pm.w_sn = p.w_stride_n; pm.w_sm = p.w_stride_m;
-            pm.c = C; pm.alpha = alpha;
-            rc = launch_permode(dev, pm, st);
+            rc = launch_permode(dev, permode_layer(p, B, kModes, A, win, C, alpha), PERMODE_APPLY, st);
             if (rc) return rc;
             return launch_ifft_rows(dev, p.DY, ir, st);
         }
@@ -434,11 +441,7 @@ static int exec_impl(const tfno_plan* plan, const DeviceInfo& dev, const void* x
         if (plan->per_mode) {
             rc = launch_fft2d(dev, p.DX, p.DY, fi, false, st);
             if (rc) return rc;
-            PerModeParams pm{};
-            pm.rows = B; pm.modes = (long long)kModes * kModes; pm.K = p.K; pm.N = p.N;
-            pm.a = A; pm.w = win; pm.w_sk = p.w_stride_k; pm.w_sn = p.w_stride_n; pm.w_sm = p.w_stride_m;
-            pm.c = C; pm.alpha = alpha;
-            rc = launch_permode(dev, pm, st);
+            rc = launch_permode(dev, permode_layer(p, B, (long long)kModes * kModes, A, win, C, alpha), PERMODE_APPLY, st);
             if (rc) return rc;
             return launch_fft2d(dev, p.DX, p.DY, ii, true, st);
         }
@@ -862,7 +865,7 @@ int tfno_spectral_conv2d_static(long long bs, int DX, int DY, int K, int N, cons
     int rc = static_device_setup(device, &sd);
     if (rc != TFNO_OK) return rc;
     // every launch of this call must fit before the first one is enqueued: a refused call does nothing
-    if ((long long)image_smem_bytes(DX, DY) > sd->dev.max_smem_optin ||
+    if (!fft2d_fits(sd->dev, DX, DY) ||
         (long long)tile_smem_bytes(2, false, false, K, N > 128 ? 128 : N) > sd->dev.max_smem_optin)
         return TFNO_ERR_UNSUPPORTED;
     cudaStream_t st = static_cast<cudaStream_t>(stream);

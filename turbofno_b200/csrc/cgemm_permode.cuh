@@ -1,128 +1,208 @@
-// Channel contraction of compact spectra with PER-MODE weights (what an FNO layer trains):
+// Channel contractions of compact spectra, one product per retained mode, and the gradients of the
+// weights.  All of them are
 //
-//     C[(n*rows + b)*modes + m] = alpha * sum_k W[k, n, m] * A[(k*rows + b)*modes + m]
+//     O[i, j, m] = scale * sum_r  P[r, i, m] * conj?(Q[r, j, m])          (or the conjugate of it)
+//
+//   layer        C[n, b, m]  = alpha sum_k A[k, b, m] W[k, n, m]              i = b, j = n, r = k
+//   grad of x    Gx[k, b, m] = alpha sum_n G[n, b, m] conj(W[k, n, m])        i = b, j = k, r = n
+//   grad of W    dW[k, n, m] = s     sum_b conj(X[k, b, m]) G[n, b, m]        i = k, j = n, r = b
+//   the same for weights shared by all modes: the sum also runs over m.  (b, m / 8) is then the index r
+//                of a problem of eight modes, whose results are added at the end.
 //
 // The reference contracts with one K x N matrix shared by all modes
-// (fusion_variants/1D_E_baseline/cgemm.cuh:42-43, B[k + n*K]); this is the extension its README
-// names as the FNO use case, with the reference's compact-spectrum layouts on both sides.  It is
-// 64 (1D) or 4096 (2D) independent [rows x K] x [K x N] products whose operands are interleaved
-// mode-fastest in memory, so a CTA takes FOUR adjacent modes (one 32-byte sector per (row, channel)
-// on the A and C side), keeps their weights W[4][K][64 outputs] in shared memory for as long as it
-// stays on those modes, and streams row tiles of 32 past them.  FP32 SIMT: each thread owns one mode,
-// four rows and four output channels.
+// (fusion_variants/1D_E_baseline/cgemm.cuh:42-43, B[k + n*K]); per-mode matrices are the extension its
+// README names as the FNO use case.  The operands are interleaved mode-fastest in memory, so the modes go
+// on the LANES: a CTA takes eight adjacent modes (64 contiguous bytes of every row of P, Q and O), a warp
+// 8 modes x 4 groups of TI rows i, and 8 columns j; eight warps cover 64 columns and WI sets of eight warps
+// WI * 4 * TI rows.  Slabs of P and Q for four r travel by 16-byte asynchronous copies through a ring
+// of kPmStages.  FP32 FMA; a thread keeps TI x 8 complex sums, and per r its warp reads TI * 256 + 8 * 64 bytes
+// of shared memory for TI * 32 FMA instructions.
 #pragma once
 #include <cuda_runtime.h>
+#include <cstdint>
+#include "common.cuh"
 
 namespace tfno {
 
-constexpr int kPmThreads = 512;        // 4 modes x 8 row groups x 16 output groups
-constexpr int kPmModes = 4;            // adjacent modes per CTA
-constexpr int kPmRowTile = 32;         // rows per tile: 8 row groups of 4
-constexpr int kPmNB = 64;              // output channels per pass
+constexpr int kPmModes = 8;            // adjacent modes per CTA
+constexpr int kPmCols = 64;            // columns j per CTA: eight warps of 8
+constexpr int kPmSlab = 4;             // values of r per ring stage
+constexpr int kPmStages = 4;
 
 struct PerModeParams {
-    long long rows;                    // B (1D: bs*dimX, 2D: bs)
-    long long modes;                   // 64 (1D) or 4096 (2D); a multiple of 4
-    int K, N;
-    const float2* a;                   // A[(k*rows + b)*modes + m]
-    const float2* w;                   // W[k*w_sk + n*w_sn + m*w_sm]
-    long long w_sk, w_sn, w_sm;
-    float2* c;                         // C[(n*rows + b)*modes + m]
+    int I, J;                          // J a multiple of 64
+    long long red, modes;              // terms of the sum; modes: a multiple of 8
+    const float2* p; long long p_sr, p_si;                 // P[r*p_sr + i*p_si + m]
+    const float2* q; long long q_sr, q_sj, q_sm;           // Q[r*q_sr + j*q_sj + m*q_sm]
+    float2* o; long long o_si, o_sj, o_sm;                 // O[i*o_si + j*o_sj + m*o_sm]
+    float2* partial;                   // [splits][I][J][modes] (sum_modes: [splits][I][J]) when splits > 1 or sum_modes
     float2 alpha;
-    int splits;                        // row tiles of a mode group are dealt to this many CTAs
-    int stage_a;                       // 1: the A tile goes through shared memory
+    float2 alpha0;                     // factor of the modes m % 64 == 0 (real fields: the ky = 0 column)
+    int splits;                        // r is dealt to this many CTAs in runs of split_len
+    long long split_len;
+    int q_vec;                         // Q may be copied 16 bytes (two modes) at a time
 };
 
-// weights of one mode in shared memory: [K][64] complex, plus 32 bytes so that the four modes a
-// warp reads in one instruction fall into different banks
-__host__ __device__ inline size_t pm_mode_stride_bytes(int K) { return (size_t)K * kPmNB * sizeof(float2) + 32; }
-// A tile of 32 rows x K channels x 4 modes, staged in shared memory when it fits next to the weights
-// (K <= 64): all 16 warps of a CTA read the same A values, and reading them from global memory
-// through L1 costs the load/store unit 2.4x what the arithmetic costs the FMA pipe.
-__host__ __device__ inline size_t pm_atile_bytes(int K) { return (size_t)K * kPmRowTile * kPmModes * sizeof(float2); }
-inline bool pm_stage_a(int K, int max_smem) { return (long long)(kPmModes * pm_mode_stride_bytes(K) + pm_atile_bytes(K)) <= max_smem; }
-inline size_t pm_smem_bytes(int K, bool stage_a) { return kPmModes * pm_mode_stride_bytes(K) + (stage_a ? pm_atile_bytes(K) : 0); }
+// The launches (permode.cu).  `partial` must hold permode_partial_bytes() when that is not zero.
+enum PermodeKind { PERMODE_APPLY, PERMODE_APPLY_CONJ, PERMODE_GRAD, PERMODE_GRAD_SHARED };
+size_t permode_partial_bytes(const DeviceInfo& dev, const PerModeParams& p, PermodeKind kind);
+int launch_permode(const DeviceInfo& dev, PerModeParams p, PermodeKind kind, cudaStream_t st);
+// dst[k*N + n] = conj(w[k*sk + n*sn])
+int launch_conjugate(const DeviceInfo& dev, const float2* w, long long sk, long long sn, int K, int N, float2* dst, cudaStream_t st);
 
-__global__ void __launch_bounds__(kPmThreads, 1) cgemm_permode_kernel(PerModeParams p) {
+template <int TI, int WI> __host__ __device__ constexpr size_t pm_stage_elems() { return (size_t)kPmSlab * (4 * TI * WI + kPmCols) * kPmModes; }
+template <int TI, int WI> __host__ __device__ constexpr size_t pm_smem_bytes() { return kPmStages * pm_stage_elems<TI, WI>() * sizeof(float2); }
+
+#if defined(__CUDACC__)
+// copies `bytes` (16 or 8), or zeros when !live (the source is not read then)
+__device__ __forceinline__ void pm_copy16(uint32_t dst, const void* src, bool live) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void pm_copy8(uint32_t dst, const void* src, bool live) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(live ? 8 : 0) : "memory");
+}
+
+// CONJ_Q: Q enters conjugated.  CONJ_O: the sum is conjugated before it is scaled (conj(P) Q = conj(P conj(Q))).
+// SUM_MODES: the eight modes are added up; results go to `partial`.
+template <int TI, int WI, bool CONJ_Q, bool CONJ_O, bool SUM_MODES>
+__global__ void __launch_bounds__(256 * WI, 2 / WI) cgemm_permode_kernel(PerModeParams p) {
+    constexpr int THREADS = 256 * WI, ROWS = 4 * TI * WI, LINES = ROWS + kPmCols;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int tid = threadIdx.x;
-    const int j = tid & 3;                       // mode inside the group
-    const int rg = (tid >> 2) & 7;               // rows 4*rg .. 4*rg+3 of the tile
-    const int nb = tid >> 5;                     // outputs 4*nb .. 4*nb+3 of the pass (warp-uniform)
-    const size_t mode_stride = pm_mode_stride_bytes(p.K);
-    const long long groups = p.modes / kPmModes;
-    const long long tiles = (p.rows + kPmRowTile - 1) / kPmRowTile;
-    const int passes = p.N / kPmNB;
-    // work item = (mode group, output pass, split): consecutive CTAs take consecutive splits of the
-    // same weights, so a weight slice is fetched from DRAM once and then served by the L2
-    const long long items = groups * passes * p.splits;
-    for (long long item = blockIdx.x; item < items; item += gridDim.x) {
-        const int split = (int)(item % p.splits);
-        const int pass = (int)((item / p.splits) % passes);
-        const long long mg = item / ((long long)p.splits * passes);
-        const long long m0 = mg * kPmModes;
-        const int n_base = pass * kPmNB;
-        __syncthreads();                         // the previous item's weights are no longer read
-        for (int i = tid; i < kPmModes * p.K * kPmNB; i += kPmThreads) {
-            const int jj = i & 3, n = (i >> 2) & (kPmNB - 1), k = i >> 8;      // mode fastest: one sector per (k, n)
-            const float2 wv = __ldg(p.w + (long long)k * p.w_sk + (long long)(n_base + n) * p.w_sn + (m0 + jj) * p.w_sm);
-            *reinterpret_cast<float2*>(smem_raw + jj * mode_stride + ((size_t)k * kPmNB + n) * sizeof(float2)) = wv;
-        }
-        __syncthreads();
-        const float2* wj = reinterpret_cast<const float2*>(smem_raw + j * mode_stride) + 4 * nb;
-        // staged A tile: sA[k][r][rg][mode] (the 32 lanes of a warp read 256 contiguous bytes)
-        float2* sA = reinterpret_cast<float2*>(smem_raw + kPmModes * mode_stride);
-        for (long long tile = split; tile < tiles; tile += p.splits) {
-            const long long b0 = tile * kPmRowTile + 4 * rg;
-            float2 acc[4][4];
+    float2* ring = reinterpret_cast<float2*>(smem_raw);          // [stage][slab][ROWS + 64][8 modes]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m = lane & 7, ig = lane >> 3;
+    const int wi = warp / 8, wj = warp % 8;
+    // CTAs that differ only in their rows i are neighbours: they read the same Q, which is then served by the L2
+    const int iblocks = (p.I + ROWS - 1) / ROWS, jblocks = p.J / kPmCols;
+    long long item = blockIdx.x;
+    const int i0 = (int)(item % iblocks) * ROWS; item /= iblocks;
+    const int j0 = (int)(item % jblocks) * kPmCols; item /= jblocks;
+    const int split = (int)(item % p.splits); item /= p.splits;
+    const long long m0 = item * kPmModes;
+    const long long r0 = split * p.split_len;
+    const long long r1 = (r0 + p.split_len < p.red) ? r0 + p.split_len : p.red;
+    const int slabs = r1 > r0 ? (int)((r1 - r0 + kPmSlab - 1) / kPmSlab) : 0;
+    const uint32_t ring0 = (uint32_t)__cvta_generic_to_shared(ring);
+
+    // A slab is 4 terms x (ROWS + 64) lines of four 16-byte pieces (two modes each).  Every thread keeps its
+    // piece and line for good and one pointer per operand that moves on by a slab: the address arithmetic of a
+    // fresh decomposition per copy took as many issue slots as the FMAs.
+    const int piece = tid & 3;
+    const int p_line = (tid >> 2) % ROWS, p_rr = (tid >> 2) / ROWS;         // p_rr < kPmSlab for tid < 16 * ROWS <= THREADS
+    const bool p_row = p_rr < kPmSlab && i0 + p_line < p.I;
+    const float2* p_src = p.p + (p_row ? (r0 + p_rr) * p.p_sr + (long long)(i0 + p_line) * p.p_si + m0 + 2 * piece : 0);
+    const uint32_t p_dst = ring0 + (uint32_t)((p_rr * LINES + p_line) * kPmModes + 2 * piece) * 8u;
+    const int q_line = (tid >> 2) % kPmCols, q_rr = (tid >> 2) / kPmCols;   // and q_rr + WI, + 2 WI ..
+    const float2* q_src = p.q + (r0 + q_rr) * p.q_sr + (long long)(j0 + q_line) * p.q_sj + m0 + 2 * piece;
+    const uint32_t q_dst = ring0 + (uint32_t)((q_rr * LINES + ROWS + q_line) * kPmModes + 2 * piece) * 8u;
+    constexpr uint32_t STAGE = (uint32_t)(pm_stage_elems<TI, WI>() * sizeof(float2));
+    auto fetch = [&](int slab) {
+        if (slab < slabs) {
+            const uint32_t stage = (uint32_t)(slab % kPmStages) * STAGE;
+            const int left = (int)(r1 - r0) - slab * kPmSlab;               // terms from this slab on
+            if (p_rr < kPmSlab) pm_copy16(p_dst + stage, p_row && p_rr < left ? p_src : p.p, p_row && p_rr < left);
+            p_src += p_row ? kPmSlab * p.p_sr : 0;
+            if (p.q_vec) {
 #pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int n = 0; n < 4; ++n) acc[r][n] = make_float2(0.f, 0.f);
-            // rows beyond the batch are clamped for the loads and dropped at the store
-            long long rowoff[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) rowoff[r] = ((b0 + r < p.rows) ? b0 + r : p.rows - 1) * p.modes + m0 + j;
-            if (p.stage_a) {
-                __syncthreads();                 // the previous tile is no longer read
-                // one 16-byte load = two modes of one (channel, row): 2 * 32 * K of them
-                for (int i = tid; i < 2 * kPmRowTile * p.K; i += kPmThreads) {
-                    const int half = i & 1, row = (i >> 1) & (kPmRowTile - 1), k = i >> 6;
-                    long long b = tile * kPmRowTile + row;
-                    if (b >= p.rows) b = p.rows - 1;
-                    const float4 q = __ldg(reinterpret_cast<const float4*>(p.a + ((long long)k * p.rows + b) * p.modes + m0) + half);
-                    *reinterpret_cast<float4*>(sA + (((size_t)k * 4 + (row & 3)) * 8 + (row >> 2)) * kPmModes + 2 * half) = q;
+                for (int it = 0; it < kPmSlab; it += WI) {
+                    const bool live = q_rr + it < left;
+                    pm_copy16(q_dst + stage + (uint32_t)(it * LINES * kPmModes) * 8u, live ? q_src + it * p.q_sr : p.q, live);
                 }
-                __syncthreads();
+                q_src += kPmSlab * p.q_sr;
+            } else {
+                const long long rs = r0 + (long long)slab * kPmSlab;
+#pragma unroll 1
+                for (int i = tid; i < kPmSlab * kPmCols * 8; i += THREADS) {
+                    const int mode = i & 7, line = (i >> 3) % kPmCols, rr = (i >> 3) / kPmCols;
+                    const bool live = rr < left;
+                    const float2* src = live ? p.q + (rs + rr) * p.q_sr + (long long)(j0 + line) * p.q_sj + (m0 + mode) * p.q_sm : p.q;
+                    pm_copy8(ring0 + stage + (uint32_t)((rr * LINES + ROWS + line) * kPmModes + mode) * 8u, src, live);
+                }
             }
-#pragma unroll 4
-            for (int k = 0; k < p.K; ++k) {
-                const float4 w01 = *reinterpret_cast<const float4*>(wj + (size_t)k * kPmNB);
-                const float4 w23 = *reinterpret_cast<const float4*>(wj + (size_t)k * kPmNB + 2);
-                const float2 wv[4] = {make_float2(w01.x, w01.y), make_float2(w01.z, w01.w), make_float2(w23.x, w23.y), make_float2(w23.z, w23.w)};
-                const float2* ak = p.a + (long long)k * p.rows * p.modes;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    float2 acc[TI][8];
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const float2 av = p.stage_a ? sA[(((size_t)k * 4 + r) * 8 + rg) * kPmModes + j] : __ldg(ak + rowoff[r]);
+    for (int t = 0; t < TI; ++t)
 #pragma unroll
-                    for (int n = 0; n < 4; ++n) {
-                        acc[r][n].x = fmaf(av.x, wv[n].x, fmaf(-av.y, wv[n].y, acc[r][n].x));
-                        acc[r][n].y = fmaf(av.x, wv[n].y, fmaf(av.y, wv[n].x, acc[r][n].y));
+        for (int j = 0; j < 8; ++j) acc[t][j] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int s = 0; s < kPmStages - 1; ++s) fetch(s);
+    for (int slab = 0; slab < slabs; ++slab) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kPmStages - 2) : "memory");
+        __syncthreads();                          // this slab has arrived; everybody has left the stage refilled next
+        fetch(slab + kPmStages - 1);
+        const float2* st = ring + (slab % kPmStages) * pm_stage_elems<TI, WI>();
+#pragma unroll
+        for (int rr = 0; rr < kPmSlab; ++rr) {
+            const float2* line = st + rr * LINES * kPmModes + m;
+            float2 pv[TI];
+#pragma unroll
+            for (int t = 0; t < TI; ++t) pv[t] = line[(wi * 4 * TI + t * 4 + ig) * kPmModes];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float2 qv = line[(ROWS + wj * 8 + j) * kPmModes];
+#pragma unroll
+                for (int t = 0; t < TI; ++t) {
+                    float2& a = acc[t][j];
+                    if (CONJ_Q) {
+                        a.x = fmaf(pv[t].x, qv.x, fmaf(pv[t].y, qv.y, a.x));
+                        a.y = fmaf(pv[t].y, qv.x, fmaf(-pv[t].x, qv.y, a.y));
+                    } else {
+                        a.x = fmaf(pv[t].x, qv.x, fmaf(-pv[t].y, qv.y, a.x));
+                        a.y = fmaf(pv[t].x, qv.y, fmaf(pv[t].y, qv.x, a.y));
                     }
                 }
             }
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                if (b0 + r >= p.rows) continue;
+    for (int t = 0; t < TI; ++t) {
+        const int i = i0 + wi * 4 * TI + t * 4 + ig;
 #pragma unroll
-                for (int n = 0; n < 4; ++n) {
-                    const float2 v = acc[r][n];
-                    p.c[((long long)(n_base + 4 * nb + n) * p.rows + b0 + r) * p.modes + m0 + j] =
-                        make_float2(p.alpha.x * v.x - p.alpha.y * v.y, p.alpha.x * v.y + p.alpha.y * v.x);
+        for (int j = 0; j < 8; ++j) {
+            float2 v = acc[t][j];
+            if (CONJ_O) v.y = -v.y;
+            if (SUM_MODES) {
+#pragma unroll
+                for (int d = 1; d < 8; d <<= 1) {
+                    v.x += __shfl_xor_sync(0xffffffffu, v.x, d);
+                    v.y += __shfl_xor_sync(0xffffffffu, v.y, d);
+                }
+                if (m == 0 && i < p.I) p.partial[((long long)split * p.I + i) * p.J + j0 + wj * 8 + j] = v;
+            } else if (i < p.I) {
+                if (p.splits > 1) p.partial[(((long long)split * p.I + i) * p.J + j0 + wj * 8 + j) * p.modes + m0 + m] = v;
+                else {
+                    const float2 s = ((m0 + m) & 63) ? p.alpha : p.alpha0;
+                    p.o[(long long)i * p.o_si + (long long)(j0 + wj * 8 + j) * p.o_sj + (m0 + m) * p.o_sm] =
+                        make_float2(s.x * v.x - s.y * v.y, s.x * v.y + s.y * v.x);
                 }
             }
         }
     }
 }
+
+// adds the partial sums of the splits, in their order, and scales
+template <bool SUM_MODES>
+__global__ void __launch_bounds__(256) permode_reduce_kernel(PerModeParams p) {
+    const long long per = (long long)p.I * p.J * (SUM_MODES ? 1 : p.modes);
+    for (long long e = blockIdx.x * 256LL + threadIdx.x; e < per; e += gridDim.x * 256LL) {
+        float2 v = make_float2(0.f, 0.f);
+#pragma unroll 4
+        for (int s = 0; s < p.splits; ++s) {
+            const float2 t = p.partial[s * per + e];
+            v.x += t.x; v.y += t.y;
+        }
+        const long long m = SUM_MODES ? 1 : e % p.modes, ij = SUM_MODES ? e : e / p.modes;
+        const float2 s = (m & 63) ? p.alpha : p.alpha0;
+        p.o[(ij / p.J) * p.o_si + (ij % p.J) * p.o_sj + (SUM_MODES ? 0 : m * p.o_sm)] = make_float2(s.x * v.x - s.y * v.y, s.x * v.y + s.y * v.x);
+    }
+}
+
+#endif
 
 }  // namespace tfno

@@ -1,0 +1,139 @@
+// Shared by the translation units of the library: device description, launch set-up cache, and the
+// parameters of the image transforms and per-mode contractions with their launch functions.
+#pragma once
+#include <cuda_runtime.h>
+#include <cstdio>
+#include <cstring>
+#include <mutex>
+#include "../../include/turbofno_b200.h"
+
+namespace tfno {
+
+constexpr int kThreads = 256;      // threads per CTA of the row-tile and stand-alone transform kernels
+constexpr int kModes = 64;         // retained modes per transformed axis
+
+struct DeviceInfo {
+    int device = 0;
+    int sms = 0;
+    int max_smem_optin = 0;
+    bool use_tensor_cores = true;   // tcgen05 fused kernel where its shape limits allow
+    int* status = nullptr;          // device word written by kernels whose bounded waits ran out
+    // Dry run: when set, every launcher appends the name of the kernel it would launch (separated
+    // by ';') and launches nothing.  tfno_plan_kernels reports a plan's kernels this way, from
+    // the same dispatch code tfno_exec runs.
+    char* record = nullptr;
+    size_t record_cap = 0;
+};
+
+inline int log2_exact(long long v) {
+    int l = 0;
+    while ((1LL << l) < v) ++l;
+    return ((1LL << l) == v) ? l : -1;
+}
+inline bool supported_len(int len) { return len == 128 || len == 256 || len == 512 || len == 1024; }
+
+// Appends "name" (printf-style) to the record buffer; true when the caller is a dry run.
+inline bool record_launch(const DeviceInfo& dev, const char* fmt, int a = 0, int b = 0, int c = 0, int d = 0) {
+    if (!dev.record) return false;
+    const size_t used = std::strlen(dev.record);
+    if (used + 2 < dev.record_cap) {
+        int n = 0;
+        if (used) n = std::snprintf(dev.record + used, dev.record_cap - used, ";");
+        std::snprintf(dev.record + used + n, dev.record_cap - used - n, fmt, a, b, c, d);
+    }
+    return true;
+}
+
+// Per-kernel launch set-up, done once per (kernel, device, block size, shared-memory size) and
+// remembered: the opt-in to more than 48 KB of dynamic shared memory and the resident blocks per
+// SM.  A fixed table, no heap: the allocation-free entry point goes through here too.
+struct KernelSetupEntry {
+    const void* func;
+    int device, threads;
+    size_t smem;
+    int occ;
+};
+constexpr int kKernelSetupSlots = 512;
+inline KernelSetupEntry* kernel_setup_table() {
+    static KernelSetupEntry table[kKernelSetupSlots];
+    return table;
+}
+inline std::mutex& kernel_setup_mutex() {
+    static std::mutex m;
+    return m;
+}
+inline int kernel_setup_count(int add = 0) {
+    static int n = 0;
+    n += add;
+    return n;
+}
+
+inline int prepare_kernel_cached(const void* func, int threads, size_t smem, const DeviceInfo& dev, int* blocks_per_sm) {
+    if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
+    std::lock_guard<std::mutex> lock(kernel_setup_mutex());
+    KernelSetupEntry* table = kernel_setup_table();
+    const int n = kernel_setup_count();
+    size_t opted_in = 48 * 1024;        // largest dynamic shared-memory size this kernel has been opted in to so far
+    for (int i = 0; i < n; ++i) {
+        if (table[i].func != func || table[i].device != dev.device) continue;
+        if (table[i].threads == threads && table[i].smem == smem) {
+            *blocks_per_sm = table[i].occ;
+            return TFNO_OK;
+        }
+        if (table[i].smem > opted_in) opted_in = table[i].smem;
+    }
+    // the attribute is one value per kernel: only ever raise it, or a launch that was set up
+    // earlier with a larger size would be refused
+    if (smem > opted_in) {
+        if (cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+            cudaGetLastError();
+            return TFNO_ERR_CUDA;
+        }
+    }
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, func, threads, smem) != cudaSuccess || occ < 1) {
+        cudaGetLastError();
+        return TFNO_ERR_CUDA;
+    }
+    if (n < kKernelSetupSlots) {
+        table[n] = KernelSetupEntry{func, dev.device, threads, smem, occ};
+        kernel_setup_count(1);
+    }
+    *blocks_per_sm = occ;
+    return TFNO_OK;
+}
+
+template <typename Kernel>
+inline int prepare_kernel(Kernel kernel, size_t smem, const DeviceInfo& dev, int* blocks_per_sm, int threads = kThreads) {
+    return prepare_kernel_cached(reinterpret_cast<const void*>(kernel), threads, smem, dev, blocks_per_sm);
+}
+
+inline int launch_status() { return cudaGetLastError() == cudaSuccess ? TFNO_OK : TFNO_ERR_CUDA; }
+
+// ----------------------------------------------------------------------------------------------
+// Whole-image 2-D transforms (spectral_image.cuh, image.cu)
+// ----------------------------------------------------------------------------------------------
+struct ImageParams {
+    long long nimg;
+    long long per_k;                   // images per channel: image i -> channel i / per_k, batch i % per_k
+    const float2* in;
+    float2* out;
+    long long stride_b, stride_k;      // strides of the full-size side
+    float2 gain;
+    int conj_inverse;
+    int real;                          // the full-size side holds float samples (strides in samples)
+    int centered_x;                    // kept X modes are -32..31 (row kx + 32 of the 64 x 64 block) instead of 0..63
+};
+// DX, DY in {128, 256}; full-size side: 16-byte aligned base, even strides
+int launch_fft2d(const DeviceInfo& dev, int DX, int DY, const ImageParams& p, bool inverse, cudaStream_t st);
+bool fft2d_fits(const DeviceInfo& dev, int DX, int DY);      // the launches above need no more shared memory than the device gives
+
+#if defined(__CUDACC__)
+// Ask the L2 for `bytes` of contiguous global memory, one 128-byte line per thread and round.
+__device__ __forceinline__ void prefetch_l2_block(const void* base, int bytes, int tid, int nthreads) {
+    const char* b = static_cast<const char*>(base);
+    for (int off = tid * 128; off < bytes; off += nthreads * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(b + off));
+}
+#endif
+
+}  // namespace tfno

@@ -1,0 +1,117 @@
+// Launches of the whole-image transforms (kernels: spectral_image.cuh).
+#include "spectral_image.cuh"
+
+namespace tfno {
+namespace {
+
+template <int RX, int RY, int C, bool REAL>
+int launch_forward(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st) {
+    constexpr int THREADS = 64 * RX / C;
+    auto kernel = fft2d_trunc_kernel<RX, RY, C, REAL>;
+    const size_t smem = fwd_image_smem_bytes<RX, RY, C>();
+    if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
+    if (RX == 8 ? record_launch(dev, REAL ? "fft2d_trunc32_kernel<%d,%d,real>" : "fft2d_trunc32_kernel<%d,%d>", RX, RY)
+                : record_launch(dev, REAL ? "fft2d_trunc_kernel<%d,%d,real,%d>" : "fft2d_trunc_kernel<%d,%d,paired,%d>", RX / 2, RY / 2, THREADS))
+        return TFNO_OK;
+    int occ = 0;
+    const int rc = prepare_kernel(kernel, smem, dev, &occ, THREADS);
+    if (rc != TFNO_OK) return rc;
+    // one cluster per image, as many as are resident together
+    long long clusters = (long long)dev.sms * occ / C;
+    if (clusters > p.nimg) clusters = p.nimg;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(clusters * C));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = C > 1 ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, kernel, p) != cudaSuccess) {
+        cudaGetLastError();
+        return TFNO_ERR_CUDA;
+    }
+    return launch_status();
+}
+template <int RX, int RY, bool REAL>
+int launch_forward_split(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st) {
+    // Few images: a cluster of CTAs of 64 rows per image (8 images of 128 x 256: 8.4 us against 10.9 with one CTA
+    // each, 16 of 256 x 256: 9.4 against 17.3).  With more than two such CTAs per SM the exchange through
+    // distributed shared memory costs more than the parallelism gives (512 images of 256 x 256: 98 against 73 us).
+    if (p.nimg * (RX / 2) <= 2LL * dev.sms) return launch_forward<RX, RY, RX / 2, REAL>(dev, p, st);
+    return launch_forward<RX, RY, 1, REAL>(dev, p, st);
+}
+
+template <int RX, int RY, int CLS, bool INVERSE, bool REAL>
+int launch_inverse(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st) {
+    constexpr int PARTS = RX / CLS, THREADS = 64 * CLS;
+    auto kernel = ifft2d_pad_kernel<RX, RY, CLS, INVERSE, REAL>;
+    const size_t smem = inv_image_smem_bytes<RY, CLS>();
+    if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
+    if (RX == 8 && RY == 4 ? record_launch(dev, REAL ? "ifft2d_pad32_kernel<%d,%d,real>" : "ifft2d_pad32_kernel<%d,%d,%d>", RX, RY, INVERSE)
+                           : record_launch(dev, REAL ? "ifft2d_pad_kernel<%d,%d,real,%d>" : "ifft2d_pad_kernel<%d,%d,paired,%d>", RX / 2, RY / 2, THREADS))
+        return TFNO_OK;
+    int occ = 0;
+    const int rc = prepare_kernel(kernel, smem, dev, &occ, THREADS);
+    if (rc != TFNO_OK) return rc;
+    long long images = (long long)dev.sms * occ / PARTS;
+    if (images > p.nimg) images = p.nimg;
+    kernel<<<(unsigned)(images * PARTS), THREADS, smem, st>>>(p);
+    return launch_status();
+}
+
+template <int RX, bool CENTERED_X>
+int launch_inverse64(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st) {        // DX = 64 RX, DY = 256
+    constexpr int CLS = 2, PARTS = RX / CLS, THREADS = 64 * CLS;
+    auto kernel = ifft2d_pad64_kernel<RX, 4, CLS, CENTERED_X>;
+    const size_t smem = inv64_image_smem_bytes<4, CLS>();
+    if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
+    if (record_launch(dev, "ifft2d_pad_kernel<%d,%d,paired,%d>", RX, 4, THREADS * PARTS)) return TFNO_OK;
+    int occ = 0;
+    const int rc = prepare_kernel(kernel, smem, dev, &occ, THREADS);
+    if (rc != TFNO_OK) return rc;
+    long long images = (long long)dev.sms * occ / PARTS;
+    if (images > p.nimg) images = p.nimg;
+    kernel<<<(unsigned)(images * PARTS), THREADS, smem, st>>>(p);
+    return launch_status();
+}
+
+template <int RX, int RY, int CLS>
+int launch_image(const DeviceInfo& dev, const ImageParams& p, bool inverse, cudaStream_t st) {
+    if (!inverse) return p.real ? launch_forward_split<RX, RY, true>(dev, p, st) : launch_forward_split<RX, RY, false>(dev, p, st);
+    if (p.real) return launch_inverse<RX, RY, CLS, true, true>(dev, p, st);
+    if constexpr (RY == 8) {
+        // More CTAs than the 64-point kernel has resident (two per SM, RX/4 per image): its throughput decides
+        // (8192 images of 256 x 256: 880 against 993 us).  Fewer: the smaller parts of the 32-point kernel.
+        if (p.nimg * (RX / 4) > 2LL * dev.sms)
+            return p.centered_x && p.conj_inverse ? launch_inverse64<RX / 2, true>(dev, p, st) : launch_inverse64<RX / 2, false>(dev, p, st);
+    }
+    return p.conj_inverse ? launch_inverse<RX, RY, CLS, true, false>(dev, p, st) : launch_inverse<RX, RY, CLS, false, false>(dev, p, st);
+}
+
+}  // namespace
+
+bool fft2d_fits(const DeviceInfo& dev, int DX, int DY) {
+    (void)DX; (void)DY;
+    return (long long)fwd_image_smem_bytes<8, 8, 1>() <= dev.max_smem_optin;      // the largest of the instances below
+}
+
+// Residue classes per inverse CTA: two (128 threads) except at 256 x 256, where four (256 threads, half as many
+// reads of the spectrum) take 993 against 1013 us for 8192 images; at 256 x 128 two take 307 against 333 us for 4096,
+// and all eight in one CTA of 512 threads take 1173 and 380 us.
+int launch_fft2d(const DeviceInfo& dev, int DX, int DY, const ImageParams& p, bool inverse, cudaStream_t st) {
+    if (p.nimg <= 0) return TFNO_OK;
+    const void* full = inverse ? (const void*)p.out : (const void*)p.in;
+    if ((reinterpret_cast<uintptr_t>(full) & 15) != 0 || (p.stride_b & 1) != 0 || (p.stride_k & 1) != 0) return TFNO_ERR_UNSUPPORTED;
+    if (p.real && inverse && !p.conj_inverse) return TFNO_ERR_UNSUPPORTED;
+    if (DX == 128 && DY == 128) return launch_image<4, 4, 2>(dev, p, inverse, st);
+    if (DX == 128 && DY == 256) return launch_image<4, 8, 2>(dev, p, inverse, st);
+    if (DX == 256 && DY == 128) return launch_image<8, 4, 2>(dev, p, inverse, st);
+    if (DX == 256 && DY == 256) return launch_image<8, 8, 4>(dev, p, inverse, st);
+    return TFNO_ERR_UNSUPPORTED;
+}
+
+}  // namespace tfno

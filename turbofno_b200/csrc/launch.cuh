@@ -2,120 +2,19 @@
 // signal R, output channels -> accumulator blocks NB), shared-memory sizing and persistent grids.
 #pragma once
 #include <cuda_runtime.h>
-#include <cstdio>
-#include <cstring>
-#include <mutex>
 #ifdef TFNO_TC_TRACE
 #include <vector>
 #endif
-#include "../../include/turbofno_b200.h"
+#include "common.cuh"
 #include "spectral_kernels.cuh"
 #include "spectral_tc.cuh"
 #include "cgemm_tc.cuh"
 #include "cgemm_permode.cuh"
-#include "spectral_image32.cuh"
 
 namespace tfno {
 
-struct DeviceInfo {
-    int device = 0;
-    int sms = 0;
-    int max_smem_optin = 0;
-    bool use_tensor_cores = true;   // tcgen05 fused kernel where its shape limits allow
-    int* status = nullptr;          // device word written by kernels whose bounded waits ran out
-    // Dry run: when set, every launcher appends the name of the kernel it would launch (separated
-    // by ';') and launches nothing.  tfno_plan_kernels reports a plan's kernels this way, from
-    // the same dispatch code tfno_exec runs.
-    char* record = nullptr;
-    size_t record_cap = 0;
-};
-
-inline int log2_exact(long long v) {
-    int l = 0;
-    while ((1LL << l) < v) ++l;
-    return ((1LL << l) == v) ? l : -1;
-}
-inline bool supported_len(int len) { return len == 128 || len == 256 || len == 512 || len == 1024; }
-
-// Appends "name" (printf-style) to the record buffer; true when the caller is a dry run.
-inline bool record_launch(const DeviceInfo& dev, const char* fmt, int a = 0, int b = 0, int c = 0, int d = 0) {
-    if (!dev.record) return false;
-    const size_t used = std::strlen(dev.record);
-    if (used + 2 < dev.record_cap) {
-        int n = 0;
-        if (used) n = std::snprintf(dev.record + used, dev.record_cap - used, ";");
-        std::snprintf(dev.record + used + n, dev.record_cap - used - n, fmt, a, b, c, d);
-    }
-    return true;
-}
-
-// Per-kernel launch set-up, done once per (kernel, device, block size, shared-memory size) and
-// remembered: the opt-in to more than 48 KB of dynamic shared memory and the resident blocks per
-// SM.  A fixed table, no heap: the allocation-free entry point goes through here too.
-struct KernelSetupEntry {
-    const void* func;
-    int device, threads;
-    size_t smem;
-    int occ;
-};
-constexpr int kKernelSetupSlots = 512;
-inline KernelSetupEntry* kernel_setup_table() {
-    static KernelSetupEntry table[kKernelSetupSlots];
-    return table;
-}
-inline std::mutex& kernel_setup_mutex() {
-    static std::mutex m;
-    return m;
-}
-inline int kernel_setup_count(int add = 0) {
-    static int n = 0;
-    n += add;
-    return n;
-}
-
-inline int prepare_kernel_cached(const void* func, int threads, size_t smem, const DeviceInfo& dev, int* blocks_per_sm) {
-    if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
-    std::lock_guard<std::mutex> lock(kernel_setup_mutex());
-    KernelSetupEntry* table = kernel_setup_table();
-    const int n = kernel_setup_count();
-    size_t opted_in = 48 * 1024;        // largest dynamic shared-memory size this kernel has been opted in to so far
-    for (int i = 0; i < n; ++i) {
-        if (table[i].func != func || table[i].device != dev.device) continue;
-        if (table[i].threads == threads && table[i].smem == smem) {
-            *blocks_per_sm = table[i].occ;
-            return TFNO_OK;
-        }
-        if (table[i].smem > opted_in) opted_in = table[i].smem;
-    }
-    // the attribute is one value per kernel: only ever raise it, or a launch that was set up
-    // earlier with a larger size would be refused
-    if (smem > opted_in) {
-        if (cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-            cudaGetLastError();
-            return TFNO_ERR_CUDA;
-        }
-    }
-    int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, func, threads, smem) != cudaSuccess || occ < 1) {
-        cudaGetLastError();
-        return TFNO_ERR_CUDA;
-    }
-    if (n < kKernelSetupSlots) {
-        table[n] = KernelSetupEntry{func, dev.device, threads, smem, occ};
-        kernel_setup_count(1);
-    }
-    *blocks_per_sm = occ;
-    return TFNO_OK;
-}
-
-template <typename Kernel>
-inline int prepare_kernel(Kernel kernel, size_t smem, const DeviceInfo& dev, int* blocks_per_sm, int threads = kThreads) {
-    return prepare_kernel_cached(reinterpret_cast<const void*>(kernel), threads, smem, dev, blocks_per_sm);
-}
-
 #include "tc_trace.cuh"
 
-inline int launch_status() { return cudaGetLastError() == cudaSuccess ? TFNO_OK : TFNO_ERR_CUDA; }
 
 inline size_t tile_smem_bytes(int R, bool fwd, bool inv, int K, int N) {
     size_t elems = (size_t)K * kModes + (inv ? (size_t)N * kModes : 0) + 2 * (size_t)kSlabK * (N + kWPad) +
@@ -420,29 +319,6 @@ inline int launch_tile(const DeviceInfo& dev, int len, TileParams p, cudaStream_
     return TFNO_OK;
 }
 
-// Per-mode weights: persistent CTAs over (group of four modes, block of 64 outputs, split of the rows).
-inline int launch_permode(const DeviceInfo& dev, PerModeParams p, cudaStream_t st) {
-    if (p.rows <= 0) return TFNO_OK;
-    if (p.K <= 0 || p.N % kPmNB != 0 || p.modes % kPmModes != 0) return TFNO_ERR_UNSUPPORTED;
-    p.stage_a = pm_stage_a(p.K, dev.max_smem_optin) && (p.modes % 2 == 0) ? 1 : 0;
-    const size_t smem = pm_smem_bytes(p.K, p.stage_a != 0);
-    if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
-    if (record_launch(dev, "cgemm_permode_kernel")) return TFNO_OK;
-    int occ = 0;
-    int rc = prepare_kernel(cgemm_permode_kernel, smem, dev, &occ, kPmThreads);
-    if (rc != TFNO_OK) return rc;
-    // enough work items for two per SM, but never more splits than row tiles
-    const long long groups = p.modes / kPmModes, passes = p.N / kPmNB, tiles = (p.rows + kPmRowTile - 1) / kPmRowTile;
-    long long splits = (2LL * dev.sms + groups * passes - 1) / (groups * passes);
-    if (splits > tiles) splits = tiles;
-    if (splits < 1) splits = 1;
-    p.splits = (int)splits;
-    long long grid = groups * passes * splits;
-    if (grid > (long long)dev.sms * occ) grid = (long long)dev.sms * occ;
-    cgemm_permode_kernel<<<(unsigned)grid, kPmThreads, smem, st>>>(p);
-    return launch_status();
-}
-
 template <typename Params, typename Kernel>
 inline int launch_persistent(const DeviceInfo& dev, Kernel kernel, size_t smem, long long work_blocks,
                              const Params& p, cudaStream_t st, const char* name, int R) {
@@ -498,92 +374,6 @@ inline int launch_ifft_cols(const DeviceInfo& dev, int len, const ColsParams& p,
         case 4: return launch_persistent(dev, ifft_cols_pad_kernel<4>, 0, blocks, p, st, "ifft_cols_pad_kernel<%d>", 4);
         case 8: return launch_persistent(dev, ifft_cols_pad_kernel<8>, 0, blocks, p, st, "ifft_cols_pad_kernel<%d>", 8);
         case 16: return launch_persistent(dev, ifft_cols_pad_kernel<16>, 0, blocks, p, st, "ifft_cols_pad_kernel<%d>", 16);
-    }
-    return TFNO_ERR_UNSUPPORTED;
-}
-
-inline size_t image_smem_bytes(int DX, int DY) {
-    return ((size_t)DX * kModes + (DX / 64) * 64 + (DY / 64) * 64) * sizeof(float2);
-}
-// 16-byte loads and stores of sample pairs need 16-byte aligned rows
-inline bool image_rows_aligned(const ImageParams& p, bool inverse) {
-    const void* full = inverse ? (const void*)p.out : (const void*)p.in;
-    return (reinterpret_cast<uintptr_t>(full) & 15) == 0 && (p.stride_b & 1) == 0 && (p.stride_k & 1) == 0;
-}
-// threads of the whole-image kernels: 8 warps at up to 255 registers; 12 warps at 168 registers were
-// slower (2D layer bs=64, K=N=64, 256x256: 1.21 against 1.10 ms)
-constexpr int kImageThreads = 256;
-template <int THREADS, typename Kernel>
-inline int launch_image(const DeviceInfo& dev, Kernel kernel, size_t smem, const ImageParams& p, cudaStream_t st,
-                        const char* name, int RX, int RY) {
-    if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
-    if (record_launch(dev, name, RX, RY, THREADS)) return TFNO_OK;
-    int occ = 0;
-    int rc = prepare_kernel(kernel, smem, dev, &occ, THREADS);
-    if (rc != TFNO_OK) return rc;
-    long long grid = (long long)dev.sms * occ;
-    if (grid > p.nimg) grid = p.nimg;
-    kernel<<<(unsigned)grid, THREADS, smem, st>>>(p);
-    return launch_status();
-}
-// DX = 128: the 64 KB intermediate leaves room for two CTAs per SM if each has 4 warps (255
-// registers per thread); the two then overlap one's X pass (half the warps idle) with the other's Y pass.
-template <int RX> struct ImageThreads { static constexpr int value = (RX == 2) ? 128 : kImageThreads; };
-template <int RX>
-inline int launch_fft2d_rx(const DeviceInfo& dev, int RY, const ImageParams& p, bool inverse, cudaStream_t st) {
-    const size_t smem = image_smem_bytes(64 * RX, 64 * RY);
-    const bool paired = image_rows_aligned(p, inverse);
-#define TFNO_IMG(RYV)                                                                                                  \
-    case RYV:                                                                                                          \
-        if (paired && inverse && p.centered_x)                                                                         \
-            return launch_image<ImageThreads<RX>::value>(dev, ifft2d_pad_kernel<RX, RYV, true, ImageThreads<RX>::value, true>, smem, p, st, "ifft2d_pad_kernel<%d,%d,paired,%d,centered>", RX, RYV);  \
-        if (paired)                                                                                                    \
-            return inverse ? launch_image<ImageThreads<RX>::value>(dev, ifft2d_pad_kernel<RX, RYV, true, ImageThreads<RX>::value>, smem, p, st, "ifft2d_pad_kernel<%d,%d,paired,%d>", RX, RYV)   \
-                           : launch_image<ImageThreads<RX>::value>(dev, fft2d_trunc_kernel<RX, RYV, true, ImageThreads<RX>::value>, smem, p, st, "fft2d_trunc_kernel<%d,%d,paired,%d>", RX, RYV); \
-        if (p.centered_x) return TFNO_ERR_UNSUPPORTED;      /* centered modes only with 16-byte aligned rows */             \
-        return inverse ? launch_image<kThreads>(dev, ifft2d_pad_kernel<RX, RYV, false, kThreads>, smem, p, st, "ifft2d_pad_kernel<%d,%d,scalar,%d>", RX, RYV)         \
-                       : launch_image<kThreads>(dev, fft2d_trunc_kernel<RX, RYV, false, kThreads>, smem, p, st, "fft2d_trunc_kernel<%d,%d,scalar,%d>", RX, RYV);
-    switch (RY) { TFNO_IMG(2) TFNO_IMG(4) }
-#undef TFNO_IMG
-    return TFNO_ERR_UNSUPPORTED;
-}
-// DX = 256: image kernels on the 32-point transform, 16 warps per CTA
-template <typename Kernel>
-inline int launch_image32(const DeviceInfo& dev, Kernel kernel, int DX, int DY, const ImageParams& p, cudaStream_t st, const char* name,
-                          int a, int b, int c = 0) {
-    const size_t smem = image32_smem_bytes(DX, DY);
-    if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
-    if (record_launch(dev, name, a, b, c)) return TFNO_OK;
-    int occ = 0;
-    int rc = prepare_kernel(kernel, smem, dev, &occ, kImage32Threads);
-    if (rc != TFNO_OK) return rc;
-    long long grid = (long long)dev.sms * occ;
-    if (grid > p.nimg) grid = p.nimg;
-    kernel<<<(unsigned)grid, kImage32Threads, smem, st>>>(p);
-    return launch_status();
-}
-inline int launch_fft2d_32(const DeviceInfo& dev, int DY, const ImageParams& p, bool inverse, cudaStream_t st) {
-    const bool conj = p.conj_inverse != 0;
-    if (DY == 256) {
-        if (!inverse) return launch_image32(dev, fft2d_trunc32_kernel<8, 8>, 256, 256, p, st, "fft2d_trunc32_kernel<%d,%d>", 8, 8);
-        return conj ? launch_image32(dev, ifft2d_pad32_kernel<8, 8, true>, 256, 256, p, st, "ifft2d_pad32_kernel<%d,%d,%d>", 8, 8, 1)
-                    : launch_image32(dev, ifft2d_pad32_kernel<8, 8, false>, 256, 256, p, st, "ifft2d_pad32_kernel<%d,%d,%d>", 8, 8, 0);
-    }
-    if (!inverse) return launch_image32(dev, fft2d_trunc32_kernel<8, 4>, 256, 128, p, st, "fft2d_trunc32_kernel<%d,%d>", 8, 4);
-    return conj ? launch_image32(dev, ifft2d_pad32_kernel<8, 4, true>, 256, 128, p, st, "ifft2d_pad32_kernel<%d,%d,%d>", 8, 4, 1)
-                : launch_image32(dev, ifft2d_pad32_kernel<8, 4, false>, 256, 128, p, st, "ifft2d_pad32_kernel<%d,%d,%d>", 8, 4, 0);
-}
-
-// whole-image kernels exist for DX, DY in {128, 256} (a 512-row intermediate would need 256 KB)
-inline int launch_fft2d(const DeviceInfo& dev, int DX, int DY, const ImageParams& p, bool inverse, cudaStream_t st) {
-    if (p.nimg <= 0) return TFNO_OK;
-    // DX = 256: the forward image kernel on the 32-point transform (16 warps) is faster at both row
-    // lengths (bs=64 K=N=64 256x256: 0.528 -> 0.480 ms), the inverse one only at DY = 128 (at
-    // DY = 256 it takes 0.596 ms against 0.528 for the 64-point kernel) -- measured, kernel by kernel.
-    if (DX == 256 && (DY == 128 || (DY == 256 && !inverse))) return launch_fft2d_32(dev, DY, p, inverse, st);
-    switch (DX / 64) {
-        case 2: return launch_fft2d_rx<2>(dev, DY / 64, p, inverse, st);
-        case 4: return launch_fft2d_rx<4>(dev, DY / 64, p, inverse, st);
     }
     return TFNO_ERR_UNSUPPORTED;
 }

@@ -1,0 +1,411 @@
+// Whole-image 2-D transforms on the 32-point register FFT (fft32.cuh): the image is cut into parts of
+// 64 rows that small CTAs of 128 threads (or two parts, 256 threads) work on, so that four (two) CTAs
+// share an SM and one's DRAM phase overlaps the others' arithmetic, and a single image still occupies
+// several SMs.  No counterpart in the reference, which round-trips the X-transformed image through
+// global memory (fusion_variants/2D_D_exp_fused_fft_cgemm_ifft/fused_trunc_2D.cu:188-192).
+//
+//   forward  a cluster of DX/64 CTAs per image.  Each transforms 64 rows along Y and scatters the kept
+//            columns through distributed shared memory: CTA c of the cluster collects columns
+//            c*64/C .. of ALL rows (32 KB), then transforms them along X.  One cluster barrier
+//            between the passes, a second, split one (arrive after the last read, wait before the
+//            next image's first remote store) that the next image's loads and row transforms hide.
+//   inverse  no exchange at all: lane j1 of the zero-padded X transform produces exactly the image
+//            rows RX*j2 + j1, so a CTA takes CLS of the RX residue classes, transforms the 64 columns
+//            for those rows only (every part re-reads the 32 KB spectrum, from the L2), then its rows.
+//
+// REAL: the full-size side holds real samples.  Two rows share one complex 32-point transform
+// (z = a + i b); the forward kernel separates them lane by lane (A[k] = (Z[k] + conj Z[-k])/2) before the
+// lanes are combined, the inverse kernel gives the folded 32-point input its Hermitian mirror image:
+// 2 Re(ifft2(Z')) with the ky = 0 column entering once.
+#pragma once
+#include "fft32.cuh"
+#include <type_traits>
+#include "common.cuh"
+
+namespace tfno {
+
+// ---- shared-memory tiles ----
+// inverse: [rows][64] complex, 512-byte rows of 32 16-byte chunks, low three bits XOR-ed with `key`, the number of
+// the row (of the pair of rows): the groups of a warp read adjacent rows (pairs) at the same chunk.  Local row i is
+// image row RX*(i/CLS) + part*CLS + i%CLS, so that a round writes runs of adjacent image rows.
+TFNO_HD int rtile_chunk(int key, int c) { return (c & ~7) | ((c ^ key) & 7); }
+// forward: [DX rows][64/C columns] complex, rows of 32/C 16-byte chunks, low three bits XOR-ed with a number
+// of the row and (C = 1) of the chunk's group of eight.  The X pass reads RX adjacent rows at one pair (RX = 8)
+// or quadruple (RX = 4) of chunks: the plain row number spreads the former over the banks, the row number
+// rotated by one bit the latter.
+template <int RX, int C>
+TFNO_HD int xtile_index(int row, int col) {
+    const int c = col >> 1;
+    const int s = ((RX == 8) ? (row & 7) : (((row & 1) << 2) | ((row >> 1) & 3))) ^ (C == 1 ? (c >> 3) & 3 : 0);
+    return row * (64 / C) + (((c & ~7) | ((c ^ s) & 7)) << 1) + (col & 1);
+}
+template <int RX, int RY, int C> inline constexpr size_t fwd_image_smem_bytes() {
+    return (size_t)(32 * RX * (64 / C) + RX * 32 + RY * 32) * sizeof(float2);
+}
+template <int RY, int CLS> inline constexpr size_t inv64_image_smem_bytes() {
+    return (size_t)(64 * CLS * kModes + RY * 64 + CLS * 64) * sizeof(float2);
+}
+template <int RY, int CLS> inline constexpr size_t inv_image_smem_bytes() {
+    return (size_t)(32 * CLS * kModes + RY * 32 + CLS * 32) * sizeof(float2);
+}
+
+#if defined(__CUDACC__)
+TFNO_D uint32_t shared_address(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+TFNO_D uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+TFNO_D uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    return a;
+}
+TFNO_D void store_cluster16(uint32_t addr, float2 a, float2 b) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y) : "memory");
+}
+TFNO_D void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+TFNO_D void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// ---- two real rows through one complex transform ----
+template <int R, int LEN>
+TFNO_D void exchange_tail(float2 (&v)[16], int mask, bool up) {          // exchange_round_32 on 2*LEN live entries
+    float2 got[LEN];
+#pragma unroll
+    for (int j = 0; j < LEN; ++j) {
+        const float2 lo = v[j], hi = v[LEN + j];
+        v[j] = up ? hi : lo;
+        got[j] = shfl_xor2(up ? lo : hi, mask);
+    }
+#pragma unroll
+    for (int j = 0; j < LEN; ++j) v[j] = cadd(v[j], got[j]);
+}
+// z[n] = (a, b) sample R*n + r of two real signals.  On return lane r holds modes 64/R*r + j of a in va[j]
+// and of b in vb[j].  twF is the forward table times 1/2.  Slots s and -s of the 32-point result are
+// separated together with s + 16 and 16 - s, which rounds 1 and 2 reduce to two values per signal: a closed
+// set of four registers in, four out (the pairing s <-> -s also holds on rotated lanes: 16 = -16).
+template <int R>
+TFNO_D void forward_trunc32_real2(float2 (&z)[32], const float2* __restrict__ twF, int r, float2 coef, float2 (&va)[16], float2 (&vb)[16]) {
+    fft32<-1>(z, lane_rotated32<R>(r) ? -1.0f : 1.0f);
+    auto table = [&](int s) { return twF[tw_index<R>(r, s)]; };
+#pragma unroll
+    for (int j = 0; j <= 8; ++j) {
+        constexpr int M = 4;
+        const int s[M] = {j, 16 - j, 16 + j, (32 - j) & 31};             // slot pairs: s[0] <-> s[3], s[1] <-> s[2]
+        float2 w[2][M], g[2][M];
+#pragma unroll
+        for (int i = 0; i < M; ++i) {
+            const float2 a = z[slot32(s[i])], b = z[slot32((32 - s[i]) & 31)], t = table(s[i]);
+            w[0][i] = cmul(make_float2(a.x + b.x, a.y - b.y), t);
+            w[1][i] = cmul(make_float2(a.y + b.y, b.x - a.x), t);
+        }
+        // j = 0: s = {0, 16, 16, 0}; j = 8: s = {8, 8, 24, 24}: one value per signal
+        const bool one = j == 0 || j == 8;
+        const int keep = one ? 1 : 2;                                    // kept slots s[0] (and s[1])
+        const int send0 = 2, send1 = 3;                                  // s[2] = s[0] + 16, s[3] = s[1] + 16
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int i = 0; i < M; ++i) {
+                if (one && (i == 1 || i == 3)) continue;
+                g[q][i] = shfl_xor2(w[q][i], R >> 1);
+            }
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int i = 0; i < M; ++i) {
+                if (one && (i == 1 || i == 3)) continue;
+                w[q][i] = cmadd(w[q][i], coef, g[q][i]);
+            }
+        float2 k[2][2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            k[q][0] = shfl_xor2(w[q][send0], R >> 2);
+            if (keep == 2) k[q][1] = shfl_xor2(w[q][send1], R >> 2);
+        }
+        va[j] = cadd(w[0][0], k[0][0]);
+        vb[j] = cadd(w[1][0], k[1][0]);
+        if (keep == 2) {
+            va[16 - j] = cadd(w[0][1], k[0][1]);
+            vb[16 - j] = cadd(w[1][1], k[1][1]);
+        }
+    }
+    if constexpr (R >= 8) {
+        exchange_tail<R, 8>(va, R >> 3, (r & (R >> 3)) != 0);
+        exchange_tail<R, 8>(vb, R >> 3, (r & (R >> 3)) != 0);
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// [image][DX][DY] -> [image][64][64]      RX = DX/32, RY = DY/32 (4 or 8 each)
+// ------------------------------------------------------------------------------------------
+template <int RX, int RY, int C, bool REAL>
+__global__ void __launch_bounds__(64 * RX / C, 8 * C / RX) fft2d_trunc_kernel(ImageParams p) {
+    constexpr int T = 64 * RX / C, COLS = 64 / C, DX = 32 * RX, DY = 32 * RY, ROWS = DX / C, PERY = 64 / RY, PERX = 64 / RX;
+    using Sample = typename std::conditional<REAL, float, float2>::type;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2* sX = reinterpret_cast<float2*>(smem_raw);           // [DX][COLS] swizzled: this CTA's columns
+    float2* twY = sX + DX * COLS;                                // [RY][32]
+    float2* twX = twY + RY * 32;                                 // [RX][32]
+    const int tid = threadIdx.x;
+    const int rank = C > 1 ? (int)cluster_rank() : 0;
+    fill_forward_table32<RY>(twY, tid, T);
+    fill_forward_table32<RX>(twX, tid, T, p.centered_x != 0);
+    __syncthreads();
+    if constexpr (REAL) {
+        for (int i = tid; i < RY * 32; i += T) twY[i] = make_float2(0.5f * twY[i].x, 0.5f * twY[i].y);
+        __syncthreads();
+    }
+    const int g = tid / RY, r = tid % RY;
+    const float2 coefY = round1_coef32<RY>(r);
+    const int col = tid / RX, rx = tid % RX;
+    const float2 coefX = round1_coef32<RX>(rx);
+    // lane r's modes PERY*r .. belong to one CTA of the cluster
+    uint32_t remote = 0;
+    const int dst_col = PERY * r % COLS;
+    if constexpr (C > 1) remote = map_to_rank(shared_address(sX), (uint32_t)(PERY * r / COLS));
+    auto put = [&](int row, int j, float2 a, float2 b) {
+        const int at = xtile_index<RX, C>(row, dst_col + j);
+        if constexpr (C > 1) store_cluster16(remote + 8u * (uint32_t)at, a, b);
+        else *reinterpret_cast<float4*>(sX + at) = make_float4(a.x, a.y, b.x, b.y);
+    };
+    constexpr int GROUPS = T / RY, LINES = REAL ? 2 : 1, STEP = GROUPS * LINES, ROUNDS = ROWS / STEP;
+    static_assert(ROUNDS >= 1, "a round of row transforms fits the CTA's rows");
+    const long long step = gridDim.x / C;
+    auto rows_of = [&](long long img) {
+        return reinterpret_cast<const Sample*>(p.in) + (img % p.per_k) * p.stride_b + (img / p.per_k) * p.stride_k + (long long)rank * ROWS * DY;
+    };
+    if constexpr (C > 1) cluster_arrive();                       // the peers run: their shared memory may be written
+    for (long long img = blockIdx.x / C; img < p.nimg; img += step) {
+        const Sample* src = rows_of(img);
+        const Sample* next = img + step < p.nimg ? rows_of(img + step) : nullptr;
+#pragma unroll 1
+        for (int i0 = 0; i0 < ROUNDS; ++i0) {
+            const int x = i0 * STEP + g * LINES;
+            const Sample* row = src + (long long)x * DY + r;
+            float2 v[32];
+            if constexpr (REAL) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) v[i] = make_float2(__ldg(row + RY * i), __ldg(row + DY + RY * i));
+            } else {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) v[i] = __ldg(row + RY * i);
+            }
+            // The rows of the next round (this image's or the next one's) travel to the L2 meanwhile.  Two rounds
+            // ahead is slower: 913 against 880 us for 8192 images of 256 x 256.
+            const Sample* ahead = i0 + 1 < ROUNDS ? src + (long long)(i0 + 1) * STEP * DY : next;
+            if (ahead) prefetch_l2_block(ahead, STEP * DY * (int)sizeof(Sample), tid, T);
+            const int gx = rank * ROWS + x;
+            if constexpr (REAL) {
+                float2 va[16], vb[16];
+                forward_trunc32_real2<RY>(v, twY, r, coefY, va, vb);
+                if (C > 1 && i0 == 0) cluster_wait();
+#pragma unroll
+                for (int j = 0; j < PERY; j += 2) {
+                    put(gx, j, va[j], va[j + 1]);
+                    put(gx + 1, j, vb[j], vb[j + 1]);
+                }
+            } else {
+                forward_trunc32<RY>(v, twY, r, 1, coefY);
+                if (C > 1 && i0 == 0) cluster_wait();
+#pragma unroll
+                for (int j = 0; j < PERY; j += 2) put(gx, j, v[slot32(j)], v[slot32(j + 1)]);
+            }
+        }
+        if constexpr (C > 1) { cluster_arrive(); cluster_wait(); }
+        else __syncthreads();
+        {
+            float2 v[32];
+#pragma unroll
+            for (int n = 0; n < 32; ++n) v[n] = sX[xtile_index<RX, C>(RX * n + rx, col)];
+            // columns read: the next image may be stored
+            if constexpr (C > 1) { if (next) cluster_arrive(); }
+            else __syncthreads();
+            forward_trunc32<RX>(v, twX, rx, 1, coefX);
+            float2* dst = p.out + img * (long long)(kModes * kModes) + rank * COLS + col;
+#pragma unroll
+            for (int j = 0; j < PERX; ++j) dst[(PERX * rx + j) * kModes] = v[slot32(j)];
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// [image][64][64] -> zero-pad -> inverse along X into shared memory -> inverse along Y -> [image][DX][DY]
+// INVERSE: true inverse or a second forward transform.
+// ------------------------------------------------------------------------------------------
+template <int RX, int RY, int CLS, bool INVERSE, bool REAL>
+__global__ void __launch_bounds__(64 * CLS, 8 / CLS) ifft2d_pad_kernel(ImageParams p) {
+    static_assert(INVERSE || !REAL, "a real field has a true inverse only");
+    constexpr int T = 64 * CLS, ROWS = 32 * CLS, PARTS = RX / CLS, DY = 32 * RY, SIGN = INVERSE ? 1 : -1;
+    constexpr int GROUPS = T / RY, LINES = REAL ? 2 : 1;
+    using Sample = typename std::conditional<REAL, float, float2>::type;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2* sY = reinterpret_cast<float2*>(smem_raw);           // [ROWS][64] swizzled
+    float2* twY = sY + ROWS * kModes;                            // [RY][32]
+    float2* twX = twY + RY * 32;                                 // [CLS][32]
+    const int tid = threadIdx.x;
+    const int part = blockIdx.x % PARTS;                         // the grid is a multiple of PARTS
+    fill_inverse_table32_folded<RY>(twY, tid, T, make_float2(1.f, 0.f), INVERSE);
+    for (int i = tid; i < CLS * 32; i += T) {                    // rows part*CLS .. of fill_inverse_table32_folded<RX>
+        const int j1 = part * CLS + (i >> 5), m = i & 31;
+        const int e = (INVERSE && p.centered_x) ? (j1 * m - 32 * j1) & (32 * RX - 1) : (j1 * m) & (32 * RX - 1);
+        twX[i] = cmul(p.gain, unit_root(e, 32 * RX, INVERSE ? 1.0f : -1.0f));
+    }
+    __syncthreads();
+    const int ky = tid & 63, jl = tid >> 6;
+    const float2 coefX = inverse_fold_coef32<RX>(part * CLS + jl, INVERSE);
+    const int g = tid / RY, j1 = tid % RY;
+    const float2 coefY = inverse_fold_coef32<RY>(j1, INVERSE);
+    const bool odd = (j1 & 1) != 0;
+    for (long long img = blockIdx.x / PARTS; img < p.nimg; img += gridDim.x / PARTS) {
+        const float2* src = p.in + img * (long long)(kModes * kModes) + ky;
+        Sample* dst = reinterpret_cast<Sample*>(p.out) + (img % p.per_k) * p.stride_b + (img / p.per_k) * p.stride_k;
+        {
+            float2 v[32];
+#pragma unroll
+            for (int m = 0; m < 32; m += 2) {
+                const float4 t = *reinterpret_cast<const float4*>(twX + jl * 32 + m);
+                v[m] = cmul(cmadd(__ldg(src + m * kModes), coefX, __ldg(src + (m + 32) * kModes)), make_float2(t.x, t.y));
+                v[m + 1] = cmul(cmadd(__ldg(src + (m + 1) * kModes), coefX, __ldg(src + (m + 33) * kModes)), make_float2(t.z, t.w));
+            }
+            fft32<SIGN>(v);
+#pragma unroll
+            for (int j2 = 0; j2 < 32; ++j2) {
+                const int row = j2 * CLS + jl;
+                sY[row * kModes + rtile_chunk(row / LINES, ky >> 1) * 2 + (ky & 1)] = v[slot32(j2)];
+            }
+        }
+        __syncthreads();
+        // folded input of lane j1, modes 2c and 2c + 1: u[m] = T[m] (C[m] + coef C[m + 32])
+        auto folded = [&](const float2* line, int key, int c, float2& u0, float2& u1) {
+            float4 lo = *reinterpret_cast<const float4*>(line + rtile_chunk(key, c) * 2);
+            const float4 hi = *reinterpret_cast<const float4*>(line + rtile_chunk(key, c + 16) * 2);
+            const float4 t = *reinterpret_cast<const float4*>(twY + tw_index<RY>(j1, 2 * c));
+            if (REAL && c == 0) { lo.x *= 0.5f; lo.y *= 0.5f; }          // ky = 0 has no mirror image
+            u0 = cmul(cmadd(make_float2(lo.x, lo.y), coefY, make_float2(hi.x, hi.y)), make_float2(t.x, t.y));
+            u1 = cmul(cmadd(make_float2(lo.z, lo.w), coefY, make_float2(hi.z, hi.w)), make_float2(t.z, t.w));
+        };
+#pragma unroll 1
+        for (int x0 = 0; x0 < ROWS; x0 += GROUPS * LINES) {
+            const int lr = x0 + g * LINES;
+            const int x = RX * (lr / CLS) + part * CLS + lr % CLS;       // image row of local row lr (REAL: the next one is x + 1)
+            const int key = lr / LINES;
+            float2 v[32];
+            if constexpr (REAL) {
+                // Hermitian sums h[m] = u[m] + conj(u[32 - m]) of row a, m <= 16; then v[m] = h + i h',
+                // v[32 - m] = conj(h) + i conj(h') with h' the same of row b.  Chunks c and 15 - c hold modes
+                // 2c, 2c + 1, 30 - 2c, 31 - 2c; mode 32 - 2c comes from the step before.
+                float2 h[17];
+#pragma unroll
+                for (int l = 0; l < 2; ++l) {
+                    const float2* line = sY + (lr + l) * kModes;
+                    auto put = [&](int m, float2 a, float2 b) {          // a = u[m], b = u[(32 - m) % 32]
+                        const float2 s = make_float2(a.x + b.x, a.y - b.y);
+                        if (l == 0) h[m] = s;
+                        else {
+                            v[m] = make_float2(h[m].x - s.y, h[m].y + s.x);
+                            if (m != 0 && m != 16) v[32 - m] = make_float2(h[m].x + s.y, s.x - h[m].y);
+                        }
+                    };
+                    float2 carried = make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        float2 u0, u1, w0, w1;
+                        folded(line, key, c, u0, u1);
+                        folded(line, key, 15 - c, w0, w1);            // modes 30 - 2c, 31 - 2c
+                        if (c == 0) put(0, u0, u0);
+                        else put(2 * c, u0, carried);
+                        put(2 * c + 1, u1, w1);
+                        carried = w0;
+                        if (c == 7) put(16, w0, w0);
+                    }
+                }
+            } else {
+                const float2* line = sY + lr * kModes;
+#pragma unroll
+                for (int c = 0; c < 16; ++c) folded(line, key, c, v[2 * c], v[2 * c + 1]);
+            }
+            fft32<SIGN>(v);
+            if constexpr (REAL) {
+                // even lanes write two samples of row a, odd lanes two of row b
+                float* row = reinterpret_cast<float*>(dst) + (long long)(x + (odd ? 1 : 0)) * DY + (j1 & ~1);
+#pragma unroll
+                for (int j2 = 0; j2 < 32; ++j2) {
+                    const float2 o = v[slot32(j2)];
+                    const float got = __shfl_xor_sync(0xffffffffu, odd ? o.x : o.y, 1);
+                    *reinterpret_cast<float2*>(row + RY * j2) = odd ? make_float2(got, o.y) : make_float2(o.x, got);
+                }
+            } else {
+                // Lanes j1 and j1 ^ 1 own samples that alternate in memory: each stores 16 bytes (its own
+                // sample and the neighbour's) for every second j2 and they swap the foreign halves with a
+                // shuffle, so that a group writes a whole 128-byte line per instruction.
+                float2* row = reinterpret_cast<float2*>(dst) + (long long)x * DY + (odd ? RY : 0) + (j1 & ~1);
+#pragma unroll
+                for (int n2 = 0; n2 < 16; ++n2) {
+                    const float2 ev = v[slot32(2 * n2)], od = v[slot32(2 * n2 + 1)];
+                    const float2 got = shfl_xor2(odd ? ev : od, 1);
+                    *reinterpret_cast<float4*>(row + 2 * RY * n2) =
+                        odd ? make_float4(got.x, got.y, od.x, od.y) : make_float4(ev.x, ev.y, got.x, got.y);
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// The same on the 64-point transform (DX = 64 RX, DY = 64 RY): a thread holds a whole column or 64 samples of a
+// row, so half as many lanes read each row's 64 modes from shared memory, at 255 registers and eight warps per SM.
+// Two CTAs of 128 threads (CLS = 2 residue classes of 64 rows) share an SM.  The direction is a run-time branch on
+// purpose: it keeps the compiler from moving the loads of the modes into the arithmetic, which costs 50 registers
+// and spills (246 against 233 us for 4096 images of 128 x 256).
+template <int RX, int RY, int CLS, bool CENTERED_X>
+__global__ void __launch_bounds__(64 * CLS, 1) ifft2d_pad64_kernel(ImageParams p) {
+    constexpr int T = 64 * CLS, ROWS = 64 * CLS, PARTS = RX / CLS, DX = 64 * RX, DY = 64 * RY;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2* sY = reinterpret_cast<float2*>(smem_raw);           // [ROWS][64] swizzled
+    float2* twY = sY + ROWS * kModes;                            // [RY][64]
+    float2* twX = twY + RY * 64;                                 // [CLS][64]
+    const int tid = threadIdx.x;
+    const int part = PARTS == 1 ? 0 : (int)(blockIdx.x % PARTS);     // the grid is a multiple of PARTS
+    fill_inverse_table<RY>(twY, tid, T, make_float2(1.f, 0.f), p.conj_inverse != 0);
+    for (int i = tid; i < CLS * 64; i += T) {                    // rows part*CLS .. of fill_inverse_table<RX>
+        const int jl = i >> 6, m = i & 63, j1 = part * CLS + jl;
+        const int e = CENTERED_X ? (j1 * m - 32 * j1) & (DX - 1) : (j1 * m) & (DX - 1);
+        twX[tw_index<CLS>(jl, m)] = cmul(p.gain, unit_root(e, DX, p.conj_inverse ? 1.0f : -1.0f));
+    }
+    __syncthreads();
+    const int ky = tid & 63, jl = tid >> 6;
+    const int g = tid / RY, j1 = tid % RY;
+    for (long long img = blockIdx.x / PARTS; img < p.nimg; img += gridDim.x / PARTS) {
+        {
+            const float2* src = p.in + img * (long long)(kModes * kModes) + ky;
+            float2 v[64];
+#pragma unroll
+            for (int m = 0; m < 64; ++m) v[m] = __ldg(src + m * kModes);
+            if (p.conj_inverse) inverse_pad_lane<+1, CLS, CENTERED_X>(v, twX, jl);
+            else inverse_pad_lane<-1, CLS>(v, twX, jl);
+#pragma unroll
+            for (int j2 = 0; j2 < 64; ++j2) {
+                const int row = j2 * CLS + jl;
+                sY[row * kModes + rtile_chunk(row, ky >> 1) * 2 + (ky & 1)] = v[slot(j2)];
+            }
+        }
+        __syncthreads();
+        float2* dst = p.out + (img % p.per_k) * p.stride_b + (img / p.per_k) * p.stride_k + (long long)(part * CLS) * DY;
+#pragma unroll 1
+        for (int x0 = 0; x0 < ROWS; x0 += T / RY) {
+            const int lr = x0 + g;
+            const float2* line = sY + lr * kModes;
+            float2 v[64];
+#pragma unroll
+            for (int c = 0; c < 32; ++c) {
+                const float4 q = *reinterpret_cast<const float4*>(line + rtile_chunk(lr, c) * 2);
+                v[2 * c] = make_float2(q.x, q.y);
+                v[2 * c + 1] = make_float2(q.z, q.w);
+            }
+            if (p.conj_inverse) inverse_pad_lane<+1, RY>(v, twY, j1);
+            else inverse_pad_lane<-1, RY>(v, twY, j1);
+            store_decimated_paired<RY>(v, dst + (RX * (lr / CLS) + lr % CLS) * DY, j1);
+        }
+        __syncthreads();
+    }
+}
+#endif
+
+}  // namespace tfno

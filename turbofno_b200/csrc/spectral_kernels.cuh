@@ -10,19 +10,15 @@
 //        (fft_N_stride_DY / ifft_N_stride_DY, launches at fusion_variants/1D_A_exp_fft+cgemm+ifft/fused.cu:187-203)
 //   fft_cols_trunc_kernel<R>, ifft_cols_pad_kernel<R>     strided-axis transforms
 //        (fft_N_stride / ifft_N_stride, launches at fusion_variants/2D_D_exp_fused_fft_cgemm_ifft/fused_trunc_2D.cu:153-170)
-//   fft2d_trunc_kernel<RX,RY>, ifft2d_pad_kernel<RX,RY>   whole-image 2-D transforms with the
-//        DX x 64 intermediate kept in shared memory (no counterpart in the reference, which
-//        round-trips the X-transformed image through global memory)
 //
 // Unlike the reference's fused kernel, one CTA produces ALL N output channels of its row, so the
 // forward transform of a row is never recomputed per N-tile (grid.y = N/64 in the reference).
 #pragma once
+#include "common.cuh"
 #include "fft64.cuh"
 
 namespace tfno {
 
-constexpr int kThreads = 256;      // threads per CTA for every kernel in this file
-constexpr int kModes = 64;         // retained modes per transformed axis
 constexpr int kSlabK = 8;          // channels per weight slab in the GEMM main loop
 constexpr int kWPad = 2;           // row padding of the weight slab (bank spread for k-fastest fills)
 
@@ -56,60 +52,6 @@ struct TileParams {
     float2 inv_gain;         // alpha * scale folded into the inverse twiddles (INV)
     int conj_inverse;        // 1: true inverse, 0: second forward transform
 };
-
-// ----------------------------------------------------------------------------------------------
-// lane-level load / store of one decimated signal
-// ----------------------------------------------------------------------------------------------
-template <int R>
-TFNO_D void load_decimated(float2 (&v)[64], const float2* __restrict__ sig, long long elem_stride, int r) {
-#pragma unroll
-    for (int n = 0; n < 64; ++n) v[n] = __ldg(sig + (long long)(R * n + r) * elem_stride);
-}
-
-template <int R>
-TFNO_D void store_decimated(const float2 (&v)[64], float2* __restrict__ sig, long long elem_stride, int j1) {
-#pragma unroll
-    for (int j2 = 0; j2 < 64; ++j2) sig[(long long)(R * j2 + j1) * elem_stride] = v[slot(j2)];
-}
-
-// The same for contiguous, 16-byte aligned signals whose R lanes are ADJACENT lanes of a warp: a
-// lane and its neighbour (lane ^ 1) want samples that alternate in memory (R*n + r and
-// R*n + r + 1), so each of them moves 16 bytes (two samples, one its own and one the
-// neighbour's) for every second n and they swap the foreign halves with one shuffle.  Half as
-// many load / store instructions, each touching 64 instead of 32 contiguous bytes per signal.
-template <int R>
-TFNO_D void load_decimated_paired(float2 (&v)[64], const float2* __restrict__ sig, int r) {
-    const bool odd = (r & 1) != 0;
-    const float2* base = sig + (odd ? R : 0) + (r & ~1);
-#pragma unroll
-    for (int n2 = 0; n2 < 32; ++n2) {
-        const float4 q = __ldg(reinterpret_cast<const float4*>(base + 2 * R * n2));   // samples R*(2*n2 + odd) + (r & ~1), +1
-        const float2 mine = odd ? make_float2(q.z, q.w) : make_float2(q.x, q.y);
-        const float2 send = odd ? make_float2(q.x, q.y) : make_float2(q.z, q.w);
-        float2 got;
-        got.x = __shfl_xor_sync(0xffffffffu, send.x, 1);
-        got.y = __shfl_xor_sync(0xffffffffu, send.y, 1);
-        v[2 * n2] = odd ? got : mine;          // even lane: its sample of n = 2*n2; odd lane: received
-        v[2 * n2 + 1] = odd ? mine : got;
-    }
-}
-
-template <int R>
-TFNO_D void store_decimated_paired(const float2 (&v)[64], float2* __restrict__ sig, int j1, bool live = true) {
-    const bool odd = (j1 & 1) != 0;
-    float2* base = sig + (odd ? R : 0) + (j1 & ~1);
-#pragma unroll
-    for (int n2 = 0; n2 < 32; ++n2) {
-        const float2 even_j2 = v[slot(2 * n2)], odd_j2 = v[slot(2 * n2 + 1)];
-        // an even lane writes (own, neighbour's) of j2 = 2*n2, an odd lane (neighbour's, own) of j2 = 2*n2 + 1
-        const float2 send = odd ? even_j2 : odd_j2;
-        float2 got;
-        got.x = __shfl_xor_sync(0xffffffffu, send.x, 1);
-        got.y = __shfl_xor_sync(0xffffffffu, send.y, 1);
-        const float4 q = odd ? make_float4(got.x, got.y, odd_j2.x, odd_j2.y) : make_float4(even_j2.x, even_j2.y, got.x, got.y);
-        if (live) *reinterpret_cast<float4*>(base + 2 * R * n2) = q;
-    }
-}
 
 // After forward_trunc<R>: lane r holds modes 64/R*r + j in v[slot(j)].  Write them as 16-byte
 // chunks into a swizzled tile row.
@@ -430,142 +372,6 @@ __global__ void __launch_bounds__(kThreads, 1) ifft_cols_pad_kernel(ColsParams p
         if (p.conj_inverse) inverse_pad_lane<+1, R>(v, twI, j1);
         else inverse_pad_lane<-1, R>(v, twI, j1);
         store_decimated<R>(v, p.out + (img % p.per_k) * p.stride_b + (img / p.per_k) * p.stride_k + col, p.DY, j1);
-    }
-}
-
-// ----------------------------------------------------------------------------------------------
-// Whole-image 2-D transforms (one CTA per image, DX x 64 intermediate in shared memory)
-// ----------------------------------------------------------------------------------------------
-struct ImageParams {
-    long long nimg;
-    long long per_k;                   // images per channel: image i -> channel i / per_k, batch i % per_k
-    const float2* in;
-    float2* out;
-    long long stride_b, stride_k;      // strides of the full-size side
-    float2 gain;
-    int conj_inverse;
-    int centered_x;                    // kept X modes are -32..31 (row kx + 32 of the 64 x 64 block) instead of 0..63
-};
-
-// [image][DX][DY] -> [image][64][64]: Y transform of every row (kept modes only) into shared
-// memory, then X transform of the 64 kept columns.
-// Ask the L2 for `bytes` of contiguous global memory, one 128-byte line per thread and round.
-__device__ __forceinline__ void prefetch_l2_block(const void* base, int bytes, int tid, int nthreads) {
-    const char* b = static_cast<const char*>(base);
-    for (int off = tid * 128; off < bytes; off += nthreads * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(b + off));
-}
-
-template <int RX, int RY, bool PAIRED, int THREADS>
-__global__ void __launch_bounds__(THREADS, 1) fft2d_trunc_kernel(ImageParams p) {
-    constexpr int DX = 64 * RX, DY = 64 * RY;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2* sY = reinterpret_cast<float2*>(smem_raw);          // [DX][64] swizzled
-    float2* twY = sY + DX * kModes;                             // [RY][64]
-    float2* twX = twY + RY * 64;                                // [RX][64]
-    const int tid = threadIdx.x;
-    fill_forward_table<RY>(twY, tid, THREADS);
-    fill_forward_table<RX>(twX, tid, THREADS, p.centered_x != 0);
-    __syncthreads();
-    for (long long img = blockIdx.x; img < p.nimg; img += gridDim.x) {
-        const float2* src = p.in + (img % p.per_k) * p.stride_b + (img / p.per_k) * p.stride_k;
-        {
-            constexpr int GROUPS = THREADS / RY;
-            const int g = tid / RY, r = tid % RY;
-#pragma unroll 1
-            for (int x0 = 0; x0 < DX; x0 += GROUPS) {
-                const int x = x0 + g;
-                if (x >= DX) continue;          // last round of a thread count that does not divide DX; whole warps
-                float2 v[64];
-                if constexpr (PAIRED) load_decimated_paired<RY>(v, src + (long long)x * DY, r);
-                else load_decimated<RY>(v, src + (long long)x * DY, 1, r);
-                // While these rows are transformed, the rows of the next round (or the first rows
-                // of this CTA's next image) travel from DRAM to the L2: a warp has no other loads
-                // in flight while it computes, and only two warps share a scheduler.
-                if (x0 + GROUPS < DX) {
-                    const int next_rows = (DX - (x0 + GROUPS) < GROUPS) ? DX - (x0 + GROUPS) : GROUPS;      // stay inside the image
-                    prefetch_l2_block(src + (long long)(x0 + GROUPS) * DY, next_rows * DY * 8, tid, THREADS);
-                } else if (img + gridDim.x < p.nimg) {
-                    const long long nx = img + gridDim.x;
-                    prefetch_l2_block(p.in + (nx % p.per_k) * p.stride_b + (nx / p.per_k) * p.stride_k, GROUPS * DY * 8, tid, THREADS);
-                }
-                forward_trunc<RY>(v, twY, r);
-                store_modes_to_tile<RY>(v, sY, x, r);
-            }
-        }
-        __syncthreads();
-        {
-            constexpr int GROUPS = THREADS / RX, PER = 64 / RX;
-            const int g = tid / RX, r = tid % RX;
-            float2* dst = p.out + img * (long long)(kModes * kModes);
-#pragma unroll 1
-            for (int c0 = 0; c0 < kModes; c0 += GROUPS) {
-                const int ky = c0 + g;
-                if (ky >= kModes) continue;      // whole warps only (32/RX groups per warp divides 64)
-                float2 v[64];
-#pragma unroll
-                for (int n = 0; n < 64; ++n) v[n] = sY[tile_index(RX * n + r, ky)];
-                forward_trunc<RX>(v, twX, r, p.centered_x != 0);
-#pragma unroll
-                for (int j = 0; j < PER; ++j) dst[(PER * r + j) * kModes + ky] = v[slot(j)];
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// [image][64][64] -> zero-pad -> inverse along X into shared memory -> inverse along Y -> [image][DX][DY]
-template <int RX, int RY, bool PAIRED, int THREADS, bool CENTERED_X = false>
-__global__ void __launch_bounds__(THREADS, 1) ifft2d_pad_kernel(ImageParams p) {
-    constexpr int DX = 64 * RX, DY = 64 * RY;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2* sY = reinterpret_cast<float2*>(smem_raw);          // [DX][64] swizzled
-    float2* twY = sY + DX * kModes;
-    float2* twX = twY + RY * 64;
-    const int tid = threadIdx.x;
-    fill_inverse_table<RY>(twY, tid, THREADS, make_float2(1.f, 0.f), p.conj_inverse != 0);
-    fill_inverse_table<RX>(twX, tid, THREADS, p.gain, p.conj_inverse != 0, CENTERED_X);
-    __syncthreads();
-    for (long long img = blockIdx.x; img < p.nimg; img += gridDim.x) {
-        const float2* src = p.in + img * (long long)(kModes * kModes);
-        float2* dst = p.out + (img % p.per_k) * p.stride_b + (img / p.per_k) * p.stride_k;
-        {
-            constexpr int GROUPS = THREADS / RX;
-            const int g = tid / RX, j1 = tid % RX;
-#pragma unroll 1
-            for (int c0 = 0; c0 < kModes; c0 += GROUPS) {
-                const int ky = c0 + g;
-                if (ky >= kModes) continue;
-                float2 v[64];
-#pragma unroll
-                for (int m = 0; m < 64; ++m) v[m] = __ldg(src + m * kModes + ky);
-                if (p.conj_inverse) inverse_pad_lane<+1, RX, CENTERED_X>(v, twX, j1);
-                else inverse_pad_lane<-1, RX>(v, twX, j1);
-#pragma unroll
-                for (int j2 = 0; j2 < 64; ++j2) sY[tile_index(RX * j2 + j1, ky)] = v[slot(j2)];
-            }
-        }
-        __syncthreads();
-        {
-            constexpr int GROUPS = THREADS / RY;
-            const int g = tid / RY, j1 = tid % RY;
-#pragma unroll 1
-            for (int x0 = 0; x0 < DX; x0 += GROUPS) {
-                const int x = x0 + g;
-                if (x >= DX) continue;          // whole warps, as in the forward kernel
-                float2 v[64];
-#pragma unroll
-                for (int c = 0; c < 32; ++c) {
-                    float4 q = *reinterpret_cast<const float4*>(sY + x * kModes + swz_chunk(x, c) * 2);
-                    v[2 * c] = make_float2(q.x, q.y);
-                    v[2 * c + 1] = make_float2(q.z, q.w);
-                }
-                if (p.conj_inverse) inverse_pad_lane<+1, RY>(v, twY, j1);
-                else inverse_pad_lane<-1, RY>(v, twY, j1);
-                if constexpr (PAIRED) store_decimated_paired<RY>(v, dst + (long long)x * DY, j1);
-                else store_decimated<RY>(v, dst + (long long)x * DY, 1, j1);
-            }
-        }
-        __syncthreads();
     }
 }
 
