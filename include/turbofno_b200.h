@@ -133,6 +133,18 @@ size_t tfno_workspace_bytes(const tfno_plan* plan);
 int tfno_exec(const tfno_plan* plan, const void* x, const void* w, void* y,
               void* workspace, void* stream);
 
+/* The same layer of REAL fields: x and y hold float samples (strides of the plan in samples), w complex per-mode
+ * weights.  2D variant D plans with per-mode weights; the field's spectrum carries ky = 0..63 and the layer is
+ * 2 Re(ifft2) of the contracted spectrum with the ky = 0 column halved (rfft2 -> weights -> irfft2). */
+int tfno_exec_real(const tfno_plan* plan, const void* x, const void* w, void* y, void* workspace, void* stream);
+
+/* Gradients of a variant D plan (true inverse, beta = 0) at input x and weights w for the output gradient grad_y:
+ * grad_x (layout of x) and grad_w (layout of w), either of which may be null.  grad_x needs K a multiple of 64.
+ * real_field: x, grad_y and grad_x hold float samples, as for tfno_exec_real. */
+size_t tfno_backward_workspace_bytes(const tfno_plan* plan);
+int tfno_backward(const tfno_plan* plan, int real_field, const void* x, const void* w, const void* grad_y,
+                  void* grad_x, void* grad_w, void* workspace, void* stream);
+
 /* Same layer with HOST buffers: copies x and w to the device, runs tfno_exec, copies y back,
  * pipelined over batch chunks on internal streams; returns when y is complete.  Staging memory
  * is allocated on the first call and kept by the plan (so this entry point is not thread-safe

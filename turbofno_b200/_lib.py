@@ -58,6 +58,9 @@ SYMBOLS = {
     "tfno_plan_destroy": (_i, [_vp]),
     "tfno_workspace_bytes": (ctypes.c_size_t, [_vp]),
     "tfno_exec": (_i, [_vp, _vp, _vp, _vp, _vp, _vp]),
+    "tfno_exec_real": (_i, [_vp, _vp, _vp, _vp, _vp, _vp]),
+    "tfno_backward_workspace_bytes": (ctypes.c_size_t, [_vp]),
+    "tfno_backward": (_i, [_vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "tfno_exec_host": (_i, [_vp, _vp, _vp, _vp]),
     "tfno_plan_set_host_chunk": (_i, [_vp, _ll]),
     "tfno_plan_kernels": (_i, [_vp, ctypes.c_char_p, ctypes.c_size_t]),

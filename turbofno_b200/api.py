@@ -194,6 +194,42 @@ class SpectralConv:
         check(self.lib.tfno_exec(self._plan, _ptr(x), _ptr(w), _ptr(y), _ptr(ws), _stream_ptr(stream, x.device)), "tfno_exec")
         return y
 
+    def exec_real(self, x, w, y=None, stream=None):
+        """The layer of a real field: float32 x and y in the shapes of the plan (tfno_exec_real).  2D variant D plans
+        with per-mode weights."""
+        for name, t, dtype in (("x", x, torch.float32), ("w", w, torch.complex64), ("y", y, torch.float32)):
+            if t is not None and not (t.is_cuda and t.dtype == dtype and t.is_contiguous()):
+                raise TypeError("%s must be a contiguous %s CUDA tensor" % (name, dtype))
+        self._check_call(x, w, y, None)
+        if y is None:
+            y = torch.empty(self.out_shape(), dtype=torch.float32, device=x.device)
+        ws = self._scratch(self.workspace_bytes, x.device, stream)
+        check(self.lib.tfno_exec_real(self._plan, _ptr(x), _ptr(w), _ptr(y), _ptr(ws), _stream_ptr(stream, x.device)), "tfno_exec_real")
+        return y
+
+    def backward(self, x, w, grad_y, grad_x=None, grad_w=None, stream=None):
+        """Gradients of the layer at (x, w) for the output gradient grad_y, into grad_x and / or grad_w (tfno_backward).
+        float32 x, grad_y and grad_x: the layer of a real field."""
+        real = x.dtype == torch.float32
+        for name, t, dtype in (("x", x, x.dtype), ("grad_y", grad_y, x.dtype), ("grad_x", grad_x, x.dtype), ("w", w, torch.complex64), ("grad_w", grad_w, torch.complex64)):
+            if t is not None and not (t.is_cuda and t.dtype == dtype and t.dtype in (torch.float32, torch.complex64) and t.is_contiguous()):
+                raise TypeError("%s must be a contiguous %s CUDA tensor" % (name, dtype))
+        self._check_call(x, w, grad_y, None)
+        if grad_x is not None or grad_w is not None:
+            self._check_call(x if grad_x is None else grad_x, w if grad_w is None else grad_w, None, None)
+        ws = self._scratch(int(self.lib.tfno_backward_workspace_bytes(self._plan)), x.device, stream)
+        check(self.lib.tfno_backward(self._plan, int(real), _ptr(x), _ptr(w), _ptr(grad_y), _ptr(grad_x), _ptr(grad_w), _ptr(ws),
+                                     _stream_ptr(stream, x.device)), "tfno_backward")
+
+    @staticmethod
+    def _scratch(nbytes, device, stream):
+        """Scratch of one call, from the caching allocator's pool of the stream the call runs on: the block may be handed
+        out again as soon as this returns, to work that is ordered behind the call."""
+        if stream is None:
+            return torch.empty(nbytes, dtype=torch.uint8, device=device)
+        with torch.cuda.stream(stream):
+            return torch.empty(nbytes, dtype=torch.uint8, device=device)
+
     def exec_host(self, x_host, w_host, y_host):
         """Host (ideally pinned) complex64 tensors in, host tensor out (tfno_exec_host)."""
         for t in (x_host, w_host, y_host):

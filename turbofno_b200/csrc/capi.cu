@@ -351,7 +351,7 @@ static PerModeParams permode_layer(const tfno_problem& p, long long B, long long
 // The dispatch of one layer.  With dev.record set it is a dry run: every launcher appends the
 // name of the kernel it would launch and nothing touches the device.
 static int exec_impl(const tfno_plan* plan, const DeviceInfo& dev, const void* x, const void* w, void* y, void* workspace,
-                     void* stream) {
+                     void* stream, bool real_field = false) {
     const tfno_problem& p = plan->p;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const Workspace ws = carve(*plan);
@@ -427,6 +427,7 @@ static int exec_impl(const tfno_plan* plan, const DeviceInfo& dev, const void* x
         ii.nimg = p.N * B; ii.per_k = B; ii.in = C; ii.out = yout; ii.stride_b = p.y_stride_b; ii.stride_k = p.y_stride_n;
         ii.gain = f2(scale, 0.f); ii.conj_inverse = conj;
         fi.centered_x = ii.centered_x = p.x_modes_centered ? 1 : 0;
+        fi.real = ii.real = real_field ? 1 : 0;
         ColsParams fc{};   // x -> T1  [K*B][64][DY]
         fc.nimg = p.K * B; fc.per_k = B; fc.DY = p.DY; fc.in = xin; fc.out = T1; fc.stride_b = p.x_stride_b; fc.stride_k = p.x_stride_k;
         ColsParams ic{};   // T2 -> y
@@ -540,6 +541,155 @@ int tfno_exec(const tfno_plan* plan, const void* x, const void* w, void* y, void
     DeviceGuard guard(dev.device);
     if (!guard.ok) return TFNO_ERR_CUDA;
     return exec_impl(plan, dev, x, w, y, workspace, stream);
+}
+
+// A layer of real fields: 2D, per-mode weights (only the image transforms know real samples).
+static bool real_field_plan(const tfno_plan& pl) {
+    return pl.p.rank == 2 && pl.per_mode && pl.p.variant == TFNO_VARIANT_D && !pl.p.second_transform_forward;
+}
+
+int tfno_exec_real(const tfno_plan* plan, const void* x, const void* w, void* y, void* workspace, void* stream) {
+    if (!plan || !x || !w || !y) return TFNO_ERR_INVALID_ARG;
+    if (!aligned16(x) || !aligned16(y) || !aligned16(w) || !aligned16(workspace)) return TFNO_ERR_INVALID_ARG;
+    if (!real_field_plan(*plan)) return TFNO_ERR_UNSUPPORTED;
+    if (!workspace) return TFNO_ERR_WORKSPACE;
+    const DeviceInfo& dev = plan->h->dev;
+    DeviceGuard guard(dev.device);
+    if (!guard.ok) return TFNO_ERR_CUDA;
+    return exec_impl(plan, dev, x, w, y, workspace, stream, true);
+}
+
+// ------------------------------------------------------------------------------------------------
+// Gradients.  The layer is y = alpha A(x) W with A = s F^H P F, s = 1/DY or 1/(DX DY), P the kept modes; A is
+// self-adjoint, so with X = P F x and G = P F grad_y
+//     grad_x = conj(alpha) s F^H P (G W^H),     grad_W = conj(alpha) s X^H G   (per mode, or summed over the modes).
+// Both need G: one transform of grad_y serves the two.  A real field's layer is 2 Re of the complex one with the
+// ky = 0 column halved; its adjoint has the same form, so grad_x runs the same real kernels, and the factors of
+// grad_W are 1 at ky = 0 and 2 elsewhere.
+// ------------------------------------------------------------------------------------------------
+namespace {
+
+struct BackwardWorkspace {
+    size_t offG = 0, offX = 0, offW = 0, offP = 0, total = 0;      // X: first G W^H, then the spectrum of x
+};
+
+PerModeParams weight_gradient(const tfno_plan_s& pl, const float2* X, const float2* G, float2* gw, float2* partial, float2 factor, bool real_field) {
+    const tfno_problem& p = pl.p;
+    const long long modes = (p.rank == 1) ? kModes : (long long)kModes * kModes, S = pl.B * modes;
+    PerModeParams q{};
+    q.I = p.K; q.J = p.N;
+    q.p = X; q.q = G; q.q_sm = 1;
+    q.o = gw; q.o_si = p.w_stride_k; q.o_sj = p.w_stride_n; q.o_sm = p.w_stride_m;
+    q.partial = partial;
+    q.p_si = q.q_sj = S;
+    if (pl.per_mode) { q.red = pl.B; q.modes = modes; q.p_sr = q.q_sr = modes; }
+    else { q.red = S / kPmModes; q.modes = kPmModes; q.p_sr = q.q_sr = kPmModes; }
+    q.alpha = real_field ? cscale(factor, 2.f) : factor;
+    q.alpha0 = factor;
+    return q;
+}
+
+BackwardWorkspace carve_backward(const tfno_plan_s& pl) {
+    const tfno_problem& p = pl.p;
+    const long long modes = (p.rank == 1) ? kModes : (long long)kModes * kModes;
+    BackwardWorkspace w;
+    size_t off = 0;
+    auto take = [&](size_t& slot, size_t bytes) { slot = off; off += align_up(bytes); };
+    take(w.offG, sizeof(float2) * (size_t)(p.N * pl.B * modes));
+    take(w.offX, sizeof(float2) * (size_t)(p.K * pl.B * modes));
+    take(w.offW, pl.per_mode ? 0 : sizeof(float2) * (size_t)p.K * p.N);
+    take(w.offP, permode_partial_bytes(pl.h->dev, weight_gradient(pl, nullptr, nullptr, nullptr, nullptr, f2(1.f, 0.f), false),
+                                       pl.per_mode ? PERMODE_GRAD : PERMODE_GRAD_SHARED));
+    w.total = off;
+    return w;
+}
+
+int backward_supported(const tfno_plan_s& pl, bool real_field, bool need_x) {
+    const tfno_problem& p = pl.p;
+    if (p.variant != TFNO_VARIANT_D || p.second_transform_forward || p.beta_re != 0.f || p.beta_im != 0.f) return TFNO_ERR_UNSUPPORTED;
+    if (real_field && !real_field_plan(pl)) return TFNO_ERR_UNSUPPORTED;
+    // grad_x is the layer with the channel counts swapped: its limits apply
+    if (need_x && (p.K % 64 != 0 || (pl.per_mode && p.N > 96))) return TFNO_ERR_UNSUPPORTED;
+    return TFNO_OK;
+}
+
+// spectrum of a full-size tensor (forward) or the full-size tensor of a spectrum
+int transform(const tfno_plan_s& pl, int channels, const void* in, void* out, long long stride_b, long long stride_c, bool inverse, bool real_field, cudaStream_t st) {
+    const tfno_problem& p = pl.p;
+    const DeviceInfo& dev = pl.h->dev;
+    const float scale = p.scale_inverse ? 1.0f / (p.rank == 1 ? (float)p.DY : (float)p.DX * (float)p.DY) : 1.0f;
+    if (p.rank == 1) {
+        RowsParams r{};
+        r.nsig = channels * pl.B; r.per_k = pl.B; r.in = static_cast<const float2*>(in); r.out = static_cast<float2*>(out);
+        r.stride_row = stride_b; r.stride_k = stride_c; r.gain = f2(scale, 0.f); r.conj_inverse = 1;
+        return inverse ? launch_ifft_rows(dev, p.DY, r, st) : launch_fft_rows(dev, p.DY, r, st);
+    }
+    ImageParams i{};
+    i.nimg = channels * pl.B; i.per_k = pl.B; i.in = static_cast<const float2*>(in); i.out = static_cast<float2*>(out);
+    i.stride_b = stride_b; i.stride_k = stride_c; i.gain = f2(scale, 0.f); i.conj_inverse = 1;
+    i.centered_x = p.x_modes_centered ? 1 : 0; i.real = real_field ? 1 : 0;
+    return launch_fft2d(dev, p.DX, p.DY, i, inverse, st);
+}
+
+}  // namespace
+
+size_t tfno_backward_workspace_bytes(const tfno_plan* plan) { return plan ? carve_backward(*plan).total : 0; }
+
+int tfno_backward(const tfno_plan* plan, int real_field, const void* x, const void* w, const void* grad_y, void* grad_x, void* grad_w,
+                  void* workspace, void* stream) {
+    if (!plan || !x || !w || !grad_y || (!grad_x && !grad_w)) return TFNO_ERR_INVALID_ARG;
+    if (!aligned16(x) || !aligned16(w) || !aligned16(grad_y) || !aligned16(grad_x) || !aligned16(grad_w) || !aligned16(workspace)) return TFNO_ERR_INVALID_ARG;
+    if (!workspace) return TFNO_ERR_WORKSPACE;
+    const tfno_plan_s& pl = *plan;
+    const tfno_problem& p = pl.p;
+    const bool real = real_field != 0;
+    int rc = backward_supported(pl, real, grad_x != nullptr);
+    if (rc != TFNO_OK) return rc;
+    const DeviceInfo& dev = pl.h->dev;
+    DeviceGuard guard(dev.device);
+    if (!guard.ok) return TFNO_ERR_CUDA;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const BackwardWorkspace ws = carve_backward(pl);
+    char* wsb = static_cast<char*>(workspace);
+    float2* G = reinterpret_cast<float2*>(wsb + ws.offG);
+    float2* X = reinterpret_cast<float2*>(wsb + ws.offX);
+    float2* Wc = reinterpret_cast<float2*>(wsb + ws.offW);
+    const float2* win = static_cast<const float2*>(w);
+    const float2 alpha = f2(p.alpha_re, -p.alpha_im);
+    const long long modes = (p.rank == 1) ? kModes : (long long)kModes * kModes;
+
+    rc = transform(pl, p.N, grad_y, G, p.y_stride_b, p.y_stride_n, false, real, st);
+    if (rc != TFNO_OK) return rc;
+    if (grad_x) {
+        if (pl.per_mode) {
+            PerModeParams q{};
+            q.I = (int)pl.B; q.J = p.K; q.red = p.N; q.modes = modes;
+            q.p = G; q.p_sr = pl.B * modes; q.p_si = modes;
+            q.q = win; q.q_sr = p.w_stride_n; q.q_sj = p.w_stride_k; q.q_sm = p.w_stride_m;
+            q.o = X; q.o_si = modes; q.o_sj = pl.B * modes; q.o_sm = 1;
+            q.alpha = q.alpha0 = alpha;
+            rc = launch_permode(dev, q, PERMODE_APPLY_CONJ, st);
+        } else {
+            rc = launch_conjugate(dev, win, p.w_stride_k, p.w_stride_n, p.K, p.N, Wc, st);
+            if (rc != TFNO_OK) return rc;
+            TileParams t{};
+            t.rows = pl.B * (modes / kModes); t.K = p.N; t.N = p.K;
+            t.x = G; t.w = Wc; t.w_stride_k = 1; t.w_stride_n = p.N; t.y = X;
+            t.alpha = alpha; t.beta = f2(0.f, 0.f); t.conj_inverse = 1;
+            rc = launch_tile<false, false>(dev, p.DY, t, st);
+        }
+        if (rc != TFNO_OK) return rc;
+        rc = transform(pl, p.K, X, grad_x, p.x_stride_b, p.x_stride_k, true, real, st);
+        if (rc != TFNO_OK) return rc;
+    }
+    if (grad_w) {
+        rc = transform(pl, p.K, x, X, p.x_stride_b, p.x_stride_k, false, real, st);
+        if (rc != TFNO_OK) return rc;
+        const float scale = p.scale_inverse ? 1.0f / (p.rank == 1 ? (float)p.DY : (float)p.DX * (float)p.DY) : 1.0f;
+        rc = launch_permode(dev, weight_gradient(pl, X, G, static_cast<float2*>(grad_w), reinterpret_cast<float2*>(wsb + ws.offP), cscale(alpha, scale), real),
+                            pl.per_mode ? PERMODE_GRAD : PERMODE_GRAD_SHARED, st);
+    }
+    return rc;
 }
 
 int tfno_plan_kernels(const tfno_plan* plan, char* buf, size_t cap) {

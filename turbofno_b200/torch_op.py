@@ -23,13 +23,12 @@ The operators are registered with torch.library, so they carry a shape function 
 export; they run on the caller's current stream and allocate only their output and, in 2D, the
 plan's workspace through the caching allocator.  Plans are cached per (shape, device).
 
-Both operators have an autograd formula built from the same kernels: the layer is
+The operators have autograd formulas built from the same kernels: the layer is
 y = A(x) W with A = (1/DY) F^H P F (P keeps 64 modes), A is self-adjoint, so
-grad_x = spectral_conv1d(grad_y, W^H) -- which needs the kernel's shape limits for the swapped
+grad_x is the layer of grad_y with W^H -- which needs the kernel's shape limits for the swapped
 channel counts (K a multiple of 64, N a multiple of 8) -- and grad_W = X^H G / DY per mode, summed
-over the batch and (for weights shared by all modes) over the modes, with X, G the truncated spectra of x and grad_y from the stand-alone
-transform kernels (tfno_fft_stride_DY; in 2D tfno_fft_stride along X first).  The same holds for
-spectral_conv2d with 1/(DX*DY).
+over the batch and (for weights shared by all modes) over the modes, with X, G the truncated spectra of
+x and grad_y.  The same holds in two dimensions with 1/(DX*DY).
 """
 import torch
 
@@ -104,6 +103,48 @@ def _truncated_spectrum(t):
     return out
 
 
+# ---- gradients ---------------------------------------------------------------------------------
+# One call of the library computes both (tfno_backward): the spectrum of grad_y serves grad_x and grad_w.  It has no
+# gradient of its own, so a backward pass that is itself recorded (create_graph) takes the formulas below
+# it, whose grad_x is made of the differentiable operators; so do channel counts beyond _NATIVE_CHANNELS.
+_NATIVE_CHANNELS = 192
+
+
+def _aligned(t):
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+@torch.library.custom_op("turbofno_b200::spectral_conv_backward", mutates_args=(), device_types="cuda")
+def spectral_conv_backward(grad_y: torch.Tensor, x: torch.Tensor, w: torch.Tensor, x_modes_centered: bool, need_x: bool,
+                           need_w: bool) -> tuple[torch.Tensor, torch.Tensor]:
+    rank = x.dim() - 2
+    grad_y, x, w = _aligned(grad_y), _aligned(x), _aligned(w)
+    plan = _plan(rank, x.shape[0], x.shape[-1], x.shape[1], w.shape[1], x.shape[2] if rank == 2 else None, x.device.index,
+                 w.dim() > 2, x_modes_centered)
+    grad_x = torch.empty_like(x) if need_x else x.new_empty(0)
+    grad_w = torch.empty_like(w) if need_w else w.new_empty(0)
+    if need_x or need_w:
+        plan.backward(x, w, grad_y, grad_x if need_x else None, grad_w if need_w else None)
+    return grad_x, grad_w
+
+
+@spectral_conv_backward.register_fake
+def _(grad_y, x, w, x_modes_centered, need_x, need_w):
+    return (torch.empty_like(x, memory_format=torch.contiguous_format) if need_x else x.new_empty(0),
+            torch.empty_like(w, memory_format=torch.contiguous_format) if need_w else w.new_empty(0))
+
+
+def _native_backward(ctx, grad_y, centered):
+    """(grad_x, grad_w), or None when the differentiable formulas have to be taken."""
+    x, w = ctx.saved_tensors
+    if torch.is_grad_enabled() or max(w.shape[0], w.shape[1]) > _NATIVE_CHANNELS:
+        return None
+    need_x, need_w = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
+    grad_x, grad_w = torch.ops.turbofno_b200.spectral_conv_backward(grad_y, x, w, centered, need_x, need_w)
+    return (grad_x if need_x else None), (grad_w if need_w else None)
+
+
 def _conv1d_setup_context(ctx, inputs, output):
     x, w = inputs
     ctx.save_for_backward(x, w)
@@ -116,6 +157,9 @@ def _conv2d_setup_context(ctx, inputs, output):
 
 
 def _conv1d_backward(ctx, grad_y):
+    native = _native_backward(ctx, grad_y, False)
+    if native is not None:
+        return native
     x, w = ctx.saved_tensors
     grad_x = grad_w = None
     grad_y = grad_y.contiguous()
@@ -146,6 +190,9 @@ def _truncated_spectrum2d(t, centered=False):
 
 
 def _conv2d_backward(ctx, grad_y):
+    native = _native_backward(ctx, grad_y, ctx.centered)
+    if native is not None:
+        return native + (None,)
     x, w = ctx.saved_tensors
     grad_x = grad_w = None
     grad_y = grad_y.contiguous()
@@ -160,23 +207,66 @@ def _conv2d_backward(ctx, grad_y):
 spectral_conv2d.register_autograd(_conv2d_backward, setup_context=_conv2d_setup_context)
 
 
+@torch.library.custom_op("turbofno_b200::real_spectral_conv2d", mutates_args=(), device_types="cuda")
+def real_spectral_conv2d(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    _check_real(x, w)
+    x, w = _aligned(x), _aligned(w)
+    B, K, DX, DY = x.shape
+    plan = _plan(2, B, DY, K, w.shape[1], DX, x.device.index, True, True)
+    return plan.exec_real(x, w)
+
+
+def _check_real(x, w):
+    if x.dtype != torch.float32 or w.dtype != torch.complex64:
+        raise TypeError("rfft_spectral_conv2d: x must be float32 and w complex64")
+    if x.dim() != 4 or w.shape[0] != x.shape[1] or tuple(w.shape[2:]) != (64, 64):
+        raise ValueError("rfft_spectral_conv2d: expected x[B, K, DX, DY] and w[K, N, 64, 64]")
+
+
+@real_spectral_conv2d.register_fake
+def _(x, w):
+    _check_real(x, w)
+    return x.new_empty((x.shape[0], w.shape[1], x.shape[2], x.shape[3]))
+
+
+def _real_conv2d_setup_context(ctx, inputs, output):
+    x, w = inputs
+    ctx.save_for_backward(x, w)
+
+
+def _real_conv2d_backward(ctx, grad_y):
+    native = _native_backward(ctx, grad_y, True)
+    if native is not None:
+        return native
+    # the layer's adjoint has its own form; grad_w: factors 1 at ky = 0 and 2 elsewhere
+    x, w = ctx.saved_tensors
+    grad_x = grad_w = None
+    if ctx.needs_input_grad[0]:
+        grad_x = real_spectral_conv2d(grad_y, w.conj().transpose(0, 1).contiguous())
+    if ctx.needs_input_grad[1]:
+        X, G = (_truncated_spectrum2d(torch.complex(t, torch.zeros_like(t)), True) for t in (x, grad_y))
+        twice = torch.full((64,), 2.0, dtype=torch.float32, device=w.device)
+        twice[0] = 1.0
+        grad_w = torch.einsum("bkxy,bnxy->knxy", X.conj(), G) * (twice / (x.shape[2] * x.shape[3]))
+    return grad_x, grad_w
+
+
+real_spectral_conv2d.register_autograd(_real_conv2d_backward, setup_context=_real_conv2d_setup_context)
+
+
 def rfft_spectral_conv2d(x, w):
     """The spectral layer of a real-valued field as FNO code writes it,
 
         irfft2(pad(einsum("bkxy,knxy->bnxy", rfft2(x)[:, :, kx, :64], w)), s=(DX, DY)),  kx = -32..31,
 
     for real x[B, K, DX, DY] (float32) and per-mode weights w[K, N, 64, 64] (complex64, X index i is
-    frequency i - 32), through spectral_conv2d: the complex transform of a real field carries the
-    same 64 non-negative Y modes, and the real inverse transform of a half spectrum Z is
-    2 Re(ifft2(Z')) with Z' = Z except for the ky = 0 column, which enters once and is halved.
+    frequency i - 32).  The real inverse transform of a half spectrum Z is 2 Re(ifft2(Z')) with Z' = Z
+    except for the ky = 0 column, which enters once and is halved; the image kernels read and write real
+    samples and transform two rows in one complex transform.
     irfft2 here means the complex inverse along X followed by a real inverse along Y that drops the
     imaginary part of the ky = 0 bin (torch on the CPU); free weights leave a complex value there,
     for which torch's CUDA backend returns something else.
-    Differentiable in x and w.  The complex kernels move twice the bytes a real-input kernel would;
-    real-input (R2C / C2R) kernels are not built."""
+    Differentiable in x and w."""
     if x.is_complex() or w.dim() != 4:
         raise ValueError("rfft_spectral_conv2d: expected real x[B, K, DX, DY] and w[K, N, 64, 64]")
-    half = torch.ones(64, dtype=torch.float32, device=w.device)
-    half[0] = 0.5
-    xc = torch.complex(x.to(torch.float32), torch.zeros_like(x, dtype=torch.float32))
-    return 2.0 * spectral_conv2d(xc, w * half, True).real
+    return real_spectral_conv2d(x.to(torch.float32), w)
