@@ -111,6 +111,21 @@ inline int prepare_kernel(Kernel kernel, size_t smem, const DeviceInfo& dev, int
 inline int launch_status() { return cudaGetLastError() == cudaSuccess ? TFNO_OK : TFNO_ERR_CUDA; }
 
 // ----------------------------------------------------------------------------------------------
+// Transforms of rows (spectral_rows.cuh, rows.cu)
+// ----------------------------------------------------------------------------------------------
+struct RowsParams {
+    long long nsig;            // number of signals
+    long long per_k;           // signals per channel (rows): signal s -> channel s / per_k, row s % per_k
+    const float2* in;
+    float2* out;
+    long long stride_row, stride_k;   // strides of the full-length side (complex elements)
+    float2 gain;
+    int conj_inverse;
+};
+int launch_fft_rows(const DeviceInfo& dev, int len, const RowsParams& p, cudaStream_t st);
+int launch_ifft_rows(const DeviceInfo& dev, int len, const RowsParams& p, cudaStream_t st);
+
+// ----------------------------------------------------------------------------------------------
 // Whole-image 2-D transforms (spectral_image.cuh, image.cu)
 // ----------------------------------------------------------------------------------------------
 struct ImageParams {
@@ -129,6 +144,20 @@ int launch_fft2d(const DeviceInfo& dev, int DX, int DY, const ImageParams& p, bo
 bool fft2d_fits(const DeviceInfo& dev, int DX, int DY);      // the launches above need no more shared memory than the device gives
 
 #if defined(__CUDACC__)
+template <typename Params, typename Kernel>
+inline int launch_persistent(const DeviceInfo& dev, Kernel kernel, size_t smem, long long work_blocks,
+                             const Params& p, cudaStream_t st, const char* name, int R, int threads = kThreads) {
+    if (work_blocks <= 0) return TFNO_OK;
+    if (record_launch(dev, name, R)) return TFNO_OK;
+    int occ = 0;
+    int rc = prepare_kernel(kernel, smem, dev, &occ, threads);
+    if (rc != TFNO_OK) return rc;
+    long long grid = (long long)dev.sms * occ;
+    if (grid > work_blocks) grid = work_blocks;
+    kernel<<<(unsigned)grid, threads, smem, st>>>(p);
+    return launch_status();
+}
+
 // Ask the L2 for `bytes` of contiguous global memory, one 128-byte line per thread and round.
 __device__ __forceinline__ void prefetch_l2_block(const void* base, int bytes, int tid, int nthreads) {
     const char* b = static_cast<const char*>(base);

@@ -319,42 +319,6 @@ inline int launch_tile(const DeviceInfo& dev, int len, TileParams p, cudaStream_
     return TFNO_OK;
 }
 
-template <typename Params, typename Kernel>
-inline int launch_persistent(const DeviceInfo& dev, Kernel kernel, size_t smem, long long work_blocks,
-                             const Params& p, cudaStream_t st, const char* name, int R) {
-    if (work_blocks <= 0) return TFNO_OK;
-    if (record_launch(dev, name, R)) return TFNO_OK;
-    int occ = 0;
-    int rc = prepare_kernel(kernel, smem, dev, &occ);
-    if (rc != TFNO_OK) return rc;
-    long long grid = (long long)dev.sms * occ;
-    if (grid > work_blocks) grid = work_blocks;
-    kernel<<<(unsigned)grid, kThreads, smem, st>>>(p);
-    return launch_status();
-}
-
-inline int launch_fft_rows(const DeviceInfo& dev, int len, const RowsParams& p, cudaStream_t st) {
-    const int R = len / 64;
-    const long long blocks = (p.nsig + kThreads / R - 1) / (kThreads / R);
-    switch (R) {
-        case 2: return launch_persistent(dev, fft_rows_trunc_kernel<2>, 0, blocks, p, st, "fft_rows_trunc_kernel<%d>", 2);
-        case 4: return launch_persistent(dev, fft_rows_trunc_kernel<4>, 0, blocks, p, st, "fft_rows_trunc_kernel<%d>", 4);
-        case 8: return launch_persistent(dev, fft_rows_trunc_kernel<8>, 0, blocks, p, st, "fft_rows_trunc_kernel<%d>", 8);
-        case 16: return launch_persistent(dev, fft_rows_trunc_kernel<16>, 0, blocks, p, st, "fft_rows_trunc_kernel<%d>", 16);
-    }
-    return TFNO_ERR_UNSUPPORTED;
-}
-inline int launch_ifft_rows(const DeviceInfo& dev, int len, const RowsParams& p, cudaStream_t st) {
-    const int R = len / 64;
-    const long long blocks = (p.nsig + kThreads / R - 1) / (kThreads / R);
-    switch (R) {
-        case 2: return launch_persistent(dev, ifft_rows_pad_kernel<2>, 0, blocks, p, st, "ifft_rows_pad_kernel<%d>", 2);
-        case 4: return launch_persistent(dev, ifft_rows_pad_kernel<4>, 0, blocks, p, st, "ifft_rows_pad_kernel<%d>", 4);
-        case 8: return launch_persistent(dev, ifft_rows_pad_kernel<8>, 0, blocks, p, st, "ifft_rows_pad_kernel<%d>", 8);
-        case 16: return launch_persistent(dev, ifft_rows_pad_kernel<16>, 0, blocks, p, st, "ifft_rows_pad_kernel<%d>", 16);
-    }
-    return TFNO_ERR_UNSUPPORTED;
-}
 inline int launch_fft_cols(const DeviceInfo& dev, int len, const ColsParams& p, cudaStream_t st) {
     const int R = len / 64;
     const long long blocks = (p.nimg * p.DY + kThreads / R - 1) / (kThreads / R);

@@ -6,8 +6,6 @@
 //        <R,1,0>  fused FFT+CGEMM        fusion_variants/1D_B_exp_fused_fft_cgemm+ifft/fused_fft_cgemm_7.cuh:8-197
 //        <R,0,1>  fused CGEMM+iFFT       fusion_variants/1D_C_exp_fft+fused_cgemm_ifft/fused_cgemm_ifft_7.cuh:9-222
 //        <R,0,0>  CGEMM                  fusion_variants/1D_E_baseline/cgemm.cuh:4-205
-//   fft_rows_trunc_kernel<R>, ifft_rows_pad_kernel<R>     contiguous-axis transforms
-//        (fft_N_stride_DY / ifft_N_stride_DY, launches at fusion_variants/1D_A_exp_fft+cgemm+ifft/fused.cu:187-203)
 //   fft_cols_trunc_kernel<R>, ifft_cols_pad_kernel<R>     strided-axis transforms
 //        (fft_N_stride / ifft_N_stride, launches at fusion_variants/2D_D_exp_fused_fft_cgemm_ifft/fused_trunc_2D.cu:153-170)
 //
@@ -238,74 +236,6 @@ __global__ void __launch_bounds__(kThreads, 1) spectral_tile_kernel(TileParams p
                 }
             __syncthreads();   // sA is rewritten by the next row
         }
-    }
-}
-
-// ----------------------------------------------------------------------------------------------
-// Stand-alone transforms along the contiguous axis
-// ----------------------------------------------------------------------------------------------
-struct RowsParams {
-    long long nsig;            // number of signals
-    long long per_k;           // signals per channel (rows): signal s -> channel s / per_k, row s % per_k
-    const float2* in;
-    float2* out;
-    long long stride_row, stride_k;   // strides of the full-length side (complex elements)
-    float2 gain;
-    int conj_inverse;
-};
-
-// [signal][DY] -> compact [signal][64]
-template <int R>
-__global__ void __launch_bounds__(kThreads, 1) fft_rows_trunc_kernel(RowsParams p) {
-    __shared__ __align__(16) float2 twF[R * 64];
-    fill_forward_table<R>(twF, threadIdx.x, kThreads);
-    __syncthreads();
-    constexpr int GROUPS = kThreads / R, PER = 64 / R;
-    const int g = threadIdx.x / R, r = threadIdx.x % R;
-    const long long nblk = (p.nsig + GROUPS - 1) / GROUPS;
-    for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
-        // clamp instead of branching so that every lane of a warp takes part in the shuffles
-        long long s = blk * GROUPS + g;
-        const bool live = s < p.nsig;
-        if (!live) s = p.nsig - 1;
-        float2 v[64];
-        load_decimated_paired<R>(v, p.in + (s % p.per_k) * p.stride_row + (s / p.per_k) * p.stride_k, r);
-        forward_trunc<R>(v, twF, r);
-        if (live) {
-            float2* dst = p.out + s * kModes + PER * r;
-#pragma unroll
-            for (int j = 0; j < PER; j += 2)
-                *reinterpret_cast<float4*>(dst + j) =
-                    make_float4(v[slot(j)].x, v[slot(j)].y, v[slot(j + 1)].x, v[slot(j + 1)].y);
-        }
-    }
-}
-
-// compact [signal][64] -> zero-padded inverse -> [signal][DY]
-template <int R>
-__global__ void __launch_bounds__(kThreads, 1) ifft_rows_pad_kernel(RowsParams p) {
-    __shared__ __align__(16) float2 twI[R * 64];
-    fill_inverse_table<R>(twI, threadIdx.x, kThreads, p.gain, p.conj_inverse != 0);
-    __syncthreads();
-    constexpr int GROUPS = kThreads / R;
-    const int g = threadIdx.x / R, j1 = threadIdx.x % R;
-    const long long nblk = (p.nsig + GROUPS - 1) / GROUPS;
-    for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
-        // clamp instead of branching so that every lane of a warp takes part in the store's shuffles
-        long long s = blk * GROUPS + g;
-        const bool live = s < p.nsig;
-        if (!live) s = p.nsig - 1;
-        float2 v[64];
-        const float4* src = reinterpret_cast<const float4*>(p.in + s * kModes);
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-            float4 q = __ldg(src + c);
-            v[2 * c] = make_float2(q.x, q.y);
-            v[2 * c + 1] = make_float2(q.z, q.w);
-        }
-        if (p.conj_inverse) inverse_pad_lane<+1, R>(v, twI, j1);
-        else inverse_pad_lane<-1, R>(v, twI, j1);
-        store_decimated_paired<R>(v, p.out + (s % p.per_k) * p.stride_row + (s / p.per_k) * p.stride_k, j1, live);
     }
 }
 
