@@ -145,6 +145,9 @@ class SpectralConv:
         self._plan = plan
         self.workspace_bytes = int(self.lib.tfno_workspace_bytes(plan))
         self._ws = None
+        # The fused 1D layer itself needs no scratch, so calls of one plan on several streams may overlap; where a wide
+        # layer runs faster with some, every call gets its own (and does without when there is no memory for it).
+        self._optional_ws = self.workspace_bytes > 0 and rank == 1 and variant == "D" and not self.per_mode
 
     def out_shape(self):
         p = self.problem
@@ -178,7 +181,7 @@ class SpectralConv:
         if workspace is not None:
             if not (workspace.is_cuda and workspace.is_contiguous()):
                 raise ValueError("workspace must be a contiguous CUDA tensor")
-            if workspace.numel() * workspace.element_size() < self.workspace_bytes:
+            if workspace.numel() * workspace.element_size() < self.workspace_bytes and not self._optional_ws:
                 raise ValueError("workspace holds %d bytes, the plan needs %d" %
                                  (workspace.numel() * workspace.element_size(), self.workspace_bytes))
 
@@ -190,7 +193,16 @@ class SpectralConv:
         self._check_call(x, w, y, workspace)
         if y is None:
             y = torch.empty(self.out_shape(), dtype=torch.complex64, device=x.device)
-        ws = workspace if workspace is not None else self.workspace(x.device)
+        if workspace is not None:
+            too_small = workspace.numel() * workspace.element_size() < self.workspace_bytes     # only where it is optional
+            ws = None if too_small else workspace
+        elif self._optional_ws:
+            try:
+                ws = self._scratch(self.workspace_bytes, x.device, stream)
+            except torch.OutOfMemoryError:
+                ws = None
+        else:
+            ws = self.workspace(x.device)
         check(self.lib.tfno_exec(self._plan, _ptr(x), _ptr(w), _ptr(y), _ptr(ws), _stream_ptr(stream, x.device)), "tfno_exec")
         return y
 

@@ -36,6 +36,7 @@ struct tfno_plan_s {
     size_t ws_bytes = 0;
     bool default_layout = true;
     bool per_mode = false;              // per-mode weights (w_stride_m != 0)
+    bool wide = false;                  // 1D variant D as transform, contraction, transform when a workspace is given
     // variant E
     cufftHandle fft_fwd = 0, fft_inv = 0;
     bool have_fft = false;
@@ -84,6 +85,7 @@ Workspace carve(const tfno_plan_s& pl) {
     auto take = [&](size_t& slot, size_t sz) { slot = off; off += sz; };
     int v = p.variant;
     if (p.w_stride_m != 0 && p.rank == 1) v = TFNO_VARIANT_A;      // per-mode weights: three kernels, spectra A and C in the workspace
+    if (pl.wide) v = TFNO_VARIANT_A;
     if (p.rank == 1) {
         if (v == TFNO_VARIANT_A || v == TFNO_VARIANT_C || v == TFNO_VARIANT_E) take(w.offA, szA);
         if (v == TFNO_VARIANT_A || v == TFNO_VARIANT_B || v == TFNO_VARIANT_E) take(w.offC, szC);
@@ -98,6 +100,23 @@ Workspace carve(const tfno_plan_s& pl) {
     }
     w.total = off;
     return w;
+}
+
+// The fused 1D kernel makes 64 output channels of at most 96 input channels per launch and reads its rows again in
+// every launch; its long transforms (DY = 512, 1024: chunks of eight and four channels) also use the tensor cores
+// least.  Three kernels over the compact spectra (which are 64/DY of the data) read x once.  Measured, fused against
+// three kernels, us:
+//   DY = 512   K=N=128 at 150 / 600 / 1024 rows 135 / 382 / 531 against 112 / 243 / 355; K=32 N=128 62 / 151 / 204 against 54 / 120 / 177
+//              K=128 N=64 at 600 / 2048 rows 192 / 513 against 161 / 466;  K=N=64 at 1024 rows 142 against 149: stays fused
+//   DY = 1024  K=N=128 at 150 / 1024 rows 191 / 1015 against 140 / 532;  K=N=64 at 600 / 2048 rows 174 / 467 against 153 / 425
+//   DY = 256   K=N=128 at 1024 / 2048 rows 295 / 536 against 274 / 556, K=64 N=128 151 / 269 against 153 / 261: stays fused
+// Below one row per SM (wide) and four rows per SM (64 outputs) a call is short enough that one or two launches
+// without a workspace are kept.
+bool wide_layer(const DeviceInfo& dev, const tfno_problem& p, long long rows) {
+    if (p.rank != 1 || p.variant != TFNO_VARIANT_D || p.w_stride_m != 0 || !dev.use_tensor_cores || !dev.status) return false;
+    if (p.DY < 512 || p.K > 128) return false;
+    if (p.N > 64) return rows >= dev.sms;
+    return rows >= 4LL * dev.sms && (p.K > 96 || (p.DY == 1024 && p.K >= 64));
 }
 
 int validate(const tfno_problem& p) {
@@ -302,6 +321,7 @@ int tfno_plan_create(tfno_handle* h, const tfno_problem* problem, tfno_plan** ou
         delete pl;
         return TFNO_ERR_INVALID_ARG;
     }
+    pl->wide = wide_layer(h->dev, p, pl->B);
     pl->ws_bytes = carve(*pl).total;
 
     if (p.variant == TFNO_VARIANT_E) {
@@ -393,7 +413,9 @@ static int exec_impl(const tfno_plan* plan, const DeviceInfo& dev, const void* x
             if (rc) return rc;
             return launch_ifft_rows(dev, p.DY, ir, st);
         }
-        switch (p.variant) {
+        const bool split = plan->wide && workspace;
+        if (split) t.beta = f2(0.f, 0.f);       // D ignores beta
+        switch (split ? TFNO_VARIANT_A : p.variant) {
             case TFNO_VARIANT_A:
                 rc = launch_fft_rows(dev, p.DY, fr, st);
                 if (rc) return rc;
@@ -536,7 +558,7 @@ extern "C" {
 int tfno_exec(const tfno_plan* plan, const void* x, const void* w, void* y, void* workspace, void* stream) {
     if (!plan || !x || !w || !y) return TFNO_ERR_INVALID_ARG;
     if (!aligned16(x) || !aligned16(y) || !aligned16(w) || !aligned16(workspace)) return TFNO_ERR_INVALID_ARG;
-    if (plan->ws_bytes > 0 && !workspace) return TFNO_ERR_WORKSPACE;
+    if (plan->ws_bytes > 0 && !plan->wide && !workspace) return TFNO_ERR_WORKSPACE;
     const DeviceInfo& dev = plan->h->dev;
     DeviceGuard guard(dev.device);
     if (!guard.ok) return TFNO_ERR_CUDA;
