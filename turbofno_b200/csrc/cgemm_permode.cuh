@@ -13,10 +13,16 @@
 // (fusion_variants/1D_E_baseline/cgemm.cuh:42-43, B[k + n*K]); per-mode matrices are the extension its
 // README names as the FNO use case.  The operands are interleaved mode-fastest in memory, so the modes go
 // on the LANES: a CTA takes eight adjacent modes (64 contiguous bytes of every row of P, Q and O), a warp
-// 8 modes x 4 groups of TI rows i, and 8 columns j; eight warps cover 64 columns and WI sets of eight warps
-// WI * 4 * TI rows.  Slabs of P and Q for four r travel by 16-byte asynchronous copies through a ring
+// 8 modes x 4 groups of TI rows i, and 8 columns j; eight warps cover 64 columns.  Slabs of P and Q for four r travel by 16-byte asynchronous copies through a ring
 // of kPmStages.  FP32 FMA; a thread keeps TI x 8 complex sums, and per r its warp reads TI * 256 + 8 * 64 bytes
 // of shared memory for TI * 32 FMA instructions.
+//
+// What bounds it (2D, 4096 modes, K = N = 64): up to 8 rows the 134 MB of weights (35 us at 1 row, 44 at 8; 20 us at
+// copy speed); beyond that issue slots, 70 % used, 85 % of them FMA (16 rows 71 us, 32 rows 123 us; 30 and 60 us at the
+// full FMA rate).  The four-modes-by-32-rows tile it replaces took 193 us at any batch up to 32.  Two CTAs per SM:
+// one of 512 threads (32 rows) has nothing to cover its first loads and its stores with (137 us at 32 rows, 104
+// against 92 at 20).  Packed two-wide FMAs take the same pipe cycles plus the moves that pair their operands
+// (75 against 72 us at 16 rows).
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -26,6 +32,7 @@ namespace tfno {
 
 constexpr int kPmModes = 8;            // adjacent modes per CTA
 constexpr int kPmCols = 64;            // columns j per CTA: eight warps of 8
+constexpr int kPmThreads = 4 * kPmCols;
 constexpr int kPmSlab = 4;             // values of r per ring stage
 constexpr int kPmStages = 4;
 
@@ -50,8 +57,8 @@ int launch_permode(const DeviceInfo& dev, PerModeParams p, PermodeKind kind, cud
 // dst[k*N + n] = conj(w[k*sk + n*sn])
 int launch_conjugate(const DeviceInfo& dev, const float2* w, long long sk, long long sn, int K, int N, float2* dst, cudaStream_t st);
 
-template <int TI, int WI> __host__ __device__ constexpr size_t pm_stage_elems() { return (size_t)kPmSlab * (4 * TI * WI + kPmCols) * kPmModes; }
-template <int TI, int WI> __host__ __device__ constexpr size_t pm_smem_bytes() { return kPmStages * pm_stage_elems<TI, WI>() * sizeof(float2); }
+template <int TI> __host__ __device__ constexpr size_t pm_stage_elems() { return (size_t)kPmSlab * (4 * TI + kPmCols) * kPmModes; }
+template <int TI> __host__ __device__ constexpr size_t pm_smem_bytes() { return kPmStages * pm_stage_elems<TI>() * sizeof(float2); }
 
 #if defined(__CUDACC__)
 // copies `bytes` (16 or 8), or zeros when !live (the source is not read then)
@@ -64,14 +71,14 @@ __device__ __forceinline__ void pm_copy8(uint32_t dst, const void* src, bool liv
 
 // CONJ_Q: Q enters conjugated.  CONJ_O: the sum is conjugated before it is scaled (conj(P) Q = conj(P conj(Q))).
 // SUM_MODES: the eight modes are added up; results go to `partial`.
-template <int TI, int WI, bool CONJ_Q, bool CONJ_O, bool SUM_MODES>
-__global__ void __launch_bounds__(256 * WI, 2 / WI) cgemm_permode_kernel(PerModeParams p) {
-    constexpr int THREADS = 256 * WI, ROWS = 4 * TI * WI, LINES = ROWS + kPmCols;
+template <int TI, bool CONJ_Q, bool CONJ_O, bool SUM_MODES>
+__global__ void __launch_bounds__(kPmThreads, 2) cgemm_permode_kernel(PerModeParams p) {
+    constexpr int THREADS = kPmThreads, ROWS = 4 * TI, LINES = ROWS + kPmCols;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2* ring = reinterpret_cast<float2*>(smem_raw);          // [stage][slab][ROWS + 64][8 modes]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m = lane & 7, ig = lane >> 3;
-    const int wi = warp / 8, wj = warp % 8;
+    const int wj = warp;
     // CTAs that differ only in their rows i are neighbours: they read the same Q, which is then served by the L2
     const int iblocks = (p.I + ROWS - 1) / ROWS, jblocks = p.J / kPmCols;
     long long item = blockIdx.x;
@@ -92,10 +99,10 @@ __global__ void __launch_bounds__(256 * WI, 2 / WI) cgemm_permode_kernel(PerMode
     const bool p_row = p_rr < kPmSlab && i0 + p_line < p.I;
     const float2* p_src = p.p + (p_row ? (r0 + p_rr) * p.p_sr + (long long)(i0 + p_line) * p.p_si + m0 + 2 * piece : 0);
     const uint32_t p_dst = ring0 + (uint32_t)((p_rr * LINES + p_line) * kPmModes + 2 * piece) * 8u;
-    const int q_line = (tid >> 2) % kPmCols, q_rr = (tid >> 2) / kPmCols;   // and q_rr + WI, + 2 WI ..
-    const float2* q_src = p.q + (r0 + q_rr) * p.q_sr + (long long)(j0 + q_line) * p.q_sj + m0 + 2 * piece;
-    const uint32_t q_dst = ring0 + (uint32_t)((q_rr * LINES + ROWS + q_line) * kPmModes + 2 * piece) * 8u;
-    constexpr uint32_t STAGE = (uint32_t)(pm_stage_elems<TI, WI>() * sizeof(float2));
+    const int q_line = tid >> 2;                                            // of all four terms
+    const float2* q_src = p.q + r0 * p.q_sr + (long long)(j0 + q_line) * p.q_sj + m0 + 2 * piece;
+    const uint32_t q_dst = ring0 + (uint32_t)((ROWS + q_line) * kPmModes + 2 * piece) * 8u;
+    constexpr uint32_t STAGE = (uint32_t)(pm_stage_elems<TI>() * sizeof(float2));
     auto fetch = [&](int slab) {
         if (slab < slabs) {
             const uint32_t stage = (uint32_t)(slab % kPmStages) * STAGE;
@@ -104,8 +111,8 @@ __global__ void __launch_bounds__(256 * WI, 2 / WI) cgemm_permode_kernel(PerMode
             p_src += p_row ? kPmSlab * p.p_sr : 0;
             if (p.q_vec) {
 #pragma unroll
-                for (int it = 0; it < kPmSlab; it += WI) {
-                    const bool live = q_rr + it < left;
+                for (int it = 0; it < kPmSlab; ++it) {
+                    const bool live = it < left;
                     pm_copy16(q_dst + stage + (uint32_t)(it * LINES * kPmModes) * 8u, live ? q_src + it * p.q_sr : p.q, live);
                 }
                 q_src += kPmSlab * p.q_sr;
@@ -134,13 +141,13 @@ __global__ void __launch_bounds__(256 * WI, 2 / WI) cgemm_permode_kernel(PerMode
         asm volatile("cp.async.wait_group %0;" ::"n"(kPmStages - 2) : "memory");
         __syncthreads();                          // this slab has arrived; everybody has left the stage refilled next
         fetch(slab + kPmStages - 1);
-        const float2* st = ring + (slab % kPmStages) * pm_stage_elems<TI, WI>();
+        const float2* st = ring + (slab % kPmStages) * pm_stage_elems<TI>();
 #pragma unroll
         for (int rr = 0; rr < kPmSlab; ++rr) {
             const float2* line = st + rr * LINES * kPmModes + m;
             float2 pv[TI];
 #pragma unroll
-            for (int t = 0; t < TI; ++t) pv[t] = line[(wi * 4 * TI + t * 4 + ig) * kPmModes];
+            for (int t = 0; t < TI; ++t) pv[t] = line[(t * 4 + ig) * kPmModes];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const float2 qv = line[(ROWS + wj * 8 + j) * kPmModes];
@@ -162,7 +169,7 @@ __global__ void __launch_bounds__(256 * WI, 2 / WI) cgemm_permode_kernel(PerMode
 
 #pragma unroll
     for (int t = 0; t < TI; ++t) {
-        const int i = i0 + wi * 4 * TI + t * 4 + ig;
+        const int i = i0 + t * 4 + ig;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             float2 v = acc[t][j];

@@ -14,13 +14,12 @@ __global__ void __launch_bounds__(256) conjugate_kernel(const float2* __restrict
 
 // rows i per CTA: the tile that pads the rows least, the larger one of two equals
 int tile_rows(int I) {
-    const int sizes[] = {4, 8, 12, 16, 24, 32};
-    int best = 32;
-    long long padded = (I + 31LL) / 32 * 32;
-    for (int k = 4; k >= 0; --k) {
-        const long long n = (I + sizes[k] - 1LL) / sizes[k] * sizes[k];
-        // below 24 rows several row blocks would read Q again, for which the tile is too small
-        if (n < padded && (sizes[k] >= 24 || I <= sizes[k])) { padded = n; best = sizes[k]; }
+    int best = 16;
+    long long padded = (I + 15LL) / 16 * 16;
+    for (int rows = 12; rows >= 4; rows -= 4) {
+        const long long n = (I + rows - 1LL) / rows * rows;
+        // several blocks of 4 or 8 rows would read Q again, for which the tile is too small
+        if (n < padded && (rows == 12 || I <= rows)) { padded = n; best = rows; }
     }
     return best;
 }
@@ -39,27 +38,25 @@ int grad_splits(const DeviceInfo& dev, const PerModeParams& p) {
     return splits < 1 ? 1 : (int)splits;
 }
 
-template <int TI, int WI, bool CONJ_Q, bool CONJ_O, bool SUM_MODES>
+template <int TI, bool CONJ_Q, bool CONJ_O, bool SUM_MODES>
 int launch_inst(const DeviceInfo& dev, const PerModeParams& p, cudaStream_t st) {
-    auto kernel = cgemm_permode_kernel<TI, WI, CONJ_Q, CONJ_O, SUM_MODES>;
-    constexpr size_t smem = pm_smem_bytes<TI, WI>();
+    auto kernel = cgemm_permode_kernel<TI, CONJ_Q, CONJ_O, SUM_MODES>;
+    constexpr size_t smem = pm_smem_bytes<TI>();
     int occ = 0;
-    const int rc = prepare_kernel(kernel, smem, dev, &occ, 256 * WI);
+    const int rc = prepare_kernel(kernel, smem, dev, &occ, kPmThreads);
     if (rc != TFNO_OK) return rc;
-    const long long grid = blocks_per_split(p, 4 * TI * WI) * p.splits;
+    const long long grid = blocks_per_split(p, 4 * TI) * p.splits;
     if (grid > 0x7fffffffLL) return TFNO_ERR_UNSUPPORTED;
-    kernel<<<(unsigned)grid, 256 * WI, smem, st>>>(p);
+    kernel<<<(unsigned)grid, kPmThreads, smem, st>>>(p);
     return launch_status();
 }
 template <bool CONJ_Q, bool CONJ_O, bool SUM_MODES>
 int launch_rows(const DeviceInfo& dev, const PerModeParams& p, cudaStream_t st) {
     switch (tile_rows(p.I)) {
-        case 4: return launch_inst<1, 1, CONJ_Q, CONJ_O, SUM_MODES>(dev, p, st);
-        case 8: return launch_inst<2, 1, CONJ_Q, CONJ_O, SUM_MODES>(dev, p, st);
-        case 12: return launch_inst<3, 1, CONJ_Q, CONJ_O, SUM_MODES>(dev, p, st);
-        case 16: return launch_inst<4, 1, CONJ_Q, CONJ_O, SUM_MODES>(dev, p, st);
-        case 24: return launch_inst<3, 2, CONJ_Q, CONJ_O, SUM_MODES>(dev, p, st);
-        default: return launch_inst<4, 2, CONJ_Q, CONJ_O, SUM_MODES>(dev, p, st);
+        case 4: return launch_inst<1, CONJ_Q, CONJ_O, SUM_MODES>(dev, p, st);
+        case 8: return launch_inst<2, CONJ_Q, CONJ_O, SUM_MODES>(dev, p, st);
+        case 12: return launch_inst<3, CONJ_Q, CONJ_O, SUM_MODES>(dev, p, st);
+        default: return launch_inst<4, CONJ_Q, CONJ_O, SUM_MODES>(dev, p, st);
     }
 }
 
