@@ -18,7 +18,7 @@
 // lanes are combined, the inverse kernel gives the folded 32-point input its Hermitian mirror image:
 // 2 Re(ifft2(Z')) with the ky = 0 column entering once.
 #pragma once
-#include "fft32.cuh"
+#include "fft256.cuh"
 #include <type_traits>
 #include "common.cuh"
 
@@ -40,7 +40,7 @@ TFNO_HD int xtile_index(int row, int col) {
     return row * (64 / C) + (((c & ~7) | ((c ^ s) & 7)) << 1) + (col & 1);
 }
 template <int RX, int RY, int C> inline constexpr size_t fwd_image_smem_bytes() {
-    return (size_t)(32 * RX * (64 / C) + RX * 32 + RY * 32) * sizeof(float2);
+    return (size_t)(32 * RX * (64 / C) + RX * 32 + (RY == 8 ? kTable256 + 64 * (8 * RX / C) : RY * 32)) * sizeof(float2);
 }
 template <int RY, int CLS> inline constexpr size_t inv64_image_smem_bytes() {
     return (size_t)(64 * CLS * kModes + RY * 64 + CLS * 64) * sizeof(float2);
@@ -77,7 +77,7 @@ TFNO_D void exchange_tail(float2 (&v)[16], int mask, bool up) {          // exch
     for (int j = 0; j < LEN; ++j) v[j] = cadd(v[j], got[j]);
 }
 // z[n] = (a, b) sample R*n + r of two real signals.  On return lane r holds modes 64/R*r + j of a in va[j]
-// and of b in vb[j].  twF is the forward table times 1/2.  Slots s and -s of the 32-point result are
+// and of b in vb[j], both times 2.  Slots s and -s of the 32-point result are
 // separated together with s + 16 and 16 - s, which rounds 1 and 2 reduce to two values per signal: a closed
 // set of four registers in, four out (the pairing s <-> -s also holds on rotated lanes: 16 = -16).
 template <int R>
@@ -141,28 +141,27 @@ __global__ void __launch_bounds__(64 * RX / C, 8 * C / RX) fft2d_trunc_kernel(Im
     using Sample = typename std::conditional<REAL, float, float2>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2* sX = reinterpret_cast<float2*>(smem_raw);           // [DX][COLS] swizzled: this CTA's columns
-    float2* twY = sX + DX * COLS;                                // [RY][32]
-    float2* twX = twY + RY * 32;                                 // [RX][32]
+    constexpr bool ONCE = RY == 8;                               // rows of 256 samples: one exchange (fft256.cuh)
+    float2* twX = sX + DX * COLS;                                // [RX][32]
+    float2* twY = twX + RX * 32;                                 // [RY][32], or kTable256 entries and 64 elements per group
     const int tid = threadIdx.x;
     const int rank = C > 1 ? (int)cluster_rank() : 0;
-    fill_forward_table32<RY>(twY, tid, T);
+    if constexpr (ONCE) fill_table256(twY, tid, T);
+    else fill_forward_table32<RY>(twY, tid, T);
     fill_forward_table32<RX>(twX, tid, T, p.centered_x != 0);
     __syncthreads();
-    if constexpr (REAL) {
-        for (int i = tid; i < RY * 32; i += T) twY[i] = make_float2(0.5f * twY[i].x, 0.5f * twY[i].y);
+    if constexpr (REAL) {                                        // the 1/2 of the separated rows
+        for (int i = tid; i < RX * 32; i += T) twX[i] = make_float2(0.5f * twX[i].x, 0.5f * twX[i].y);
         __syncthreads();
     }
     const int g = tid / RY, r = tid % RY;
     const float2 coefY = round1_coef32<RY>(r);
     const int col = tid / RX, rx = tid % RX;
     const float2 coefX = round1_coef32<RX>(rx);
-    // lane r's modes PERY*r .. belong to one CTA of the cluster
-    uint32_t remote = 0;
-    const int dst_col = PERY * r % COLS;
-    if constexpr (C > 1) remote = map_to_rank(shared_address(sX), (uint32_t)(PERY * r / COLS));
-    auto put = [&](int row, int j, float2 a, float2 b) {
-        const int at = xtile_index<RX, C>(row, dst_col + j);
-        if constexpr (C > 1) store_cluster16(remote + 8u * (uint32_t)at, a, b);
+    // modes m, m + 1 of image row `row`: to the CTA of the cluster that collects their columns
+    auto put = [&](int row, int m, float2 a, float2 b) {
+        const int at = xtile_index<RX, C>(row, m % COLS);
+        if constexpr (C > 1) store_cluster16(map_to_rank(shared_address(sX), (uint32_t)(m / COLS)) + 8u * (uint32_t)at, a, b);
         else *reinterpret_cast<float4*>(sX + at) = make_float4(a.x, a.y, b.x, b.y);
     };
     constexpr int GROUPS = T / RY, LINES = REAL ? 2 : 1, STEP = GROUPS * LINES, ROUNDS = ROWS / STEP;
@@ -178,34 +177,77 @@ __global__ void __launch_bounds__(64 * RX / C, 8 * C / RX) fft2d_trunc_kernel(Im
 #pragma unroll 1
         for (int i0 = 0; i0 < ROUNDS; ++i0) {
             const int x = i0 * STEP + g * LINES;
-            const Sample* row = src + (long long)x * DY + r;
+            const int gx = rank * ROWS + x;
             float2 v[32];
-            if constexpr (REAL) {
+            float2 (&v0)[16] = *reinterpret_cast<float2(*)[16]>(&v[0]), (&v1)[16] = *reinterpret_cast<float2(*)[16]>(&v[16]);
+            if constexpr (ONCE && REAL) {
+                const float2* row = reinterpret_cast<const float2*>(src + (long long)x * DY) + r;
 #pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = make_float2(__ldg(row + RY * i), __ldg(row + DY + RY * i));
+                for (int i = 0; i < 16; ++i) {
+                    const float2 a = __ldg(row + 8 * i), b = __ldg(row + DY / 2 + 8 * i);
+                    v0[i] = make_float2(a.x, b.x);
+                    v1[i] = make_float2(a.y, b.y);
+                }
+            } else if constexpr (ONCE) {
+                const float4* row = reinterpret_cast<const float4*>(src + (long long)x * DY) + r;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const float4 q = __ldg(row + 8 * i);
+                    v0[i] = make_float2(q.x, q.y);
+                    v1[i] = make_float2(q.z, q.w);
+                }
             } else {
+                const Sample* row = src + (long long)x * DY + r;
 #pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = __ldg(row + RY * i);
+                for (int i = 0; i < 32; ++i) {
+                    if constexpr (REAL) v[i] = make_float2(__ldg(row + RY * i), __ldg(row + DY + RY * i));
+                    else v[i] = __ldg(row + RY * i);
+                }
             }
             // The rows of the next round (this image's or the next one's) travel to the L2 meanwhile.  Two rounds
             // ahead is slower: 913 against 880 us for 8192 images of 256 x 256.
             const Sample* ahead = i0 + 1 < ROUNDS ? src + (long long)(i0 + 1) * STEP * DY : next;
             if (ahead) prefetch_l2_block(ahead, STEP * DY * (int)sizeof(Sample), tid, T);
-            const int gx = rank * ROWS + x;
-            if constexpr (REAL) {
+            if constexpr (ONCE) {
+                fft16<-1>(v0);
+                fft16<-1>(v1);
+                float2* scratch = twY + kTable256 + 64 * g;
+#pragma unroll
+                for (int l = 0; l < LINES; ++l) {
+                    float2 out[2][4];
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        float2 f[16];
+#pragma unroll
+                        for (int q = 0; q < 2; ++q)
+                            exchange256(scratch, r, g & 1, q, f, [&](int d) {
+                                const float2 (&w)[16] = q ? v1 : v0;
+                                const float2 z = w[slot16(2 * d + e)];
+                                if constexpr (!REAL) return z;
+                                // two real rows: 2 A[k] = Z[k] + conj Z[-k], 2 B[k] = -i (Z[k] - conj Z[-k])
+                                const float2 y = w[slot16((16 - 2 * d - e) & 15)];
+                                return l == 0 ? make_float2(z.x + y.x, z.y - y.y) : make_float2(z.y + y.y, y.x - z.x);
+                            });
+                        combine256(f, twY + 6 * (2 * r + e), out[e]);
+                    }
+                    if (C > 1 && i0 == 0 && l == 0) cluster_wait();
+#pragma unroll
+                    for (int k2 = 0; k2 < 4; ++k2) put(gx + l, 2 * r + 16 * k2, out[0][k2], out[1][k2]);
+                }
+            } else if constexpr (REAL) {
                 float2 va[16], vb[16];
                 forward_trunc32_real2<RY>(v, twY, r, coefY, va, vb);
                 if (C > 1 && i0 == 0) cluster_wait();
 #pragma unroll
                 for (int j = 0; j < PERY; j += 2) {
-                    put(gx, j, va[j], va[j + 1]);
-                    put(gx + 1, j, vb[j], vb[j + 1]);
+                    put(gx, PERY * r + j, va[j], va[j + 1]);
+                    put(gx + 1, PERY * r + j, vb[j], vb[j + 1]);
                 }
             } else {
                 forward_trunc32<RY>(v, twY, r, 1, coefY);
                 if (C > 1 && i0 == 0) cluster_wait();
 #pragma unroll
-                for (int j = 0; j < PERY; j += 2) put(gx, j, v[slot32(j)], v[slot32(j + 1)]);
+                for (int j = 0; j < PERY; j += 2) put(gx, PERY * r + j, v[slot32(j)], v[slot32(j + 1)]);
             }
         }
         if constexpr (C > 1) { cluster_arrive(); cluster_wait(); }
