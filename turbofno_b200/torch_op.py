@@ -17,11 +17,11 @@ Beyond the reference, for callers that train an FNO:
     blocks of the non-last axis (rows 32..63 are what FNO code calls weights1, kx = 0..31; rows
     0..31 are weights2, kx = -32..-1);
   * rfft_spectral_conv2d(x_real, w): the rfft2 -> weights -> irfft2 layer of a real-valued field,
-    computed through the complex kernels (see the function).
+    on image kernels that read and write real samples (see the function).
 
 The operators are registered with torch.library, so they carry a shape function for tracing and
-export; they run on the caller's current stream and allocate only their output and, in 2D, the
-plan's workspace through the caching allocator.  Plans are cached per (shape, device).
+export; they run on the caller's current stream and allocate their results and scratch through the
+caching allocator.  Plans are cached per (shape, device).
 
 The operators have autograd formulas built from the same kernels: the layer is
 y = A(x) W with A = (1/DY) F^H P F (P keeps 64 modes), A is self-adjoint, so
