@@ -74,6 +74,7 @@ __device__ __forceinline__ void pm_copy8(uint32_t dst, const void* src, bool liv
 template <int TI, bool CONJ_Q, bool CONJ_O, bool SUM_MODES>
 __global__ void __launch_bounds__(kPmThreads, 2) cgemm_permode_kernel(PerModeParams p) {
     constexpr int THREADS = kPmThreads, ROWS = 4 * TI, LINES = ROWS + kPmCols;
+    static_assert(4 * kPmSlab * ROWS <= THREADS && kPmSlab * kPmCols == THREADS, "a slab is one 16-byte piece of P and kPmSlab of Q per thread");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2* ring = reinterpret_cast<float2*>(smem_raw);          // [stage][slab][ROWS + 64][8 modes]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;

@@ -59,8 +59,24 @@ def _check(x, w, rank):
     return per_mode
 
 
-@torch.library.custom_op("turbofno_b200::spectral_conv1d", mutates_args=(), device_types="cuda")
-def spectral_conv1d(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+# Defined through torch.library's Library: schema, CUDA kernel, shape function and autograd formula, without the checks
+# that custom_op's wrapper makes around every call of the kernel.
+_lib = torch.library.Library("turbofno_b200", "FRAGMENT")
+
+
+def _define(schema, kernel, fake):
+    name = schema[:schema.index("(")]
+    _lib.define(schema, tags=torch.Tag.pt2_compliant_tag)
+    _lib.impl(name, kernel, "CUDA")
+    torch.library.register_fake("turbofno_b200::" + name, fake, lib=_lib)
+    return getattr(torch.ops.turbofno_b200, name).default
+
+
+def _differentiable(name, backward, setup_context):
+    torch.library.register_autograd("turbofno_b200::" + name, backward, setup_context=setup_context, lib=_lib)
+
+
+def _conv1d_cuda(x, w):
     per_mode = _check(x, w, 1)
     x, w = x.contiguous(), w.contiguous()
     B, K, DY = x.shape
@@ -71,14 +87,15 @@ def spectral_conv1d(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     return y
 
 
-@spectral_conv1d.register_fake
-def _(x, w):
+def _conv1d_fake(x, w):
     _check(x, w, 1)
     return x.new_empty((x.shape[0], w.shape[1], x.shape[2]))
 
 
-@torch.library.custom_op("turbofno_b200::spectral_conv2d", mutates_args=(), device_types="cuda")
-def spectral_conv2d(x: torch.Tensor, w: torch.Tensor, x_modes_centered: bool = False) -> torch.Tensor:
+spectral_conv1d = _define("spectral_conv1d(Tensor x, Tensor w) -> Tensor", _conv1d_cuda, _conv1d_fake)
+
+
+def _conv2d_cuda(x, w, x_modes_centered=False):
     per_mode = _check(x, w, 2)
     x, w = x.contiguous(), w.contiguous()
     B, K, DX, DY = x.shape
@@ -89,10 +106,12 @@ def spectral_conv2d(x: torch.Tensor, w: torch.Tensor, x_modes_centered: bool = F
     return y
 
 
-@spectral_conv2d.register_fake
-def _(x, w, x_modes_centered=False):
+def _conv2d_fake(x, w, x_modes_centered=False):
     _check(x, w, 2)
     return x.new_empty((x.shape[0], w.shape[1], x.shape[2], x.shape[3]))
+
+
+spectral_conv2d = _define("spectral_conv2d(Tensor x, Tensor w, bool x_modes_centered=False) -> Tensor", _conv2d_cuda, _conv2d_fake)
 
 
 def _truncated_spectrum(t):
@@ -115,9 +134,7 @@ def _aligned(t):
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
-@torch.library.custom_op("turbofno_b200::spectral_conv_backward", mutates_args=(), device_types="cuda")
-def spectral_conv_backward(grad_y: torch.Tensor, x: torch.Tensor, w: torch.Tensor, x_modes_centered: bool, need_x: bool,
-                           need_w: bool) -> tuple[torch.Tensor, torch.Tensor]:
+def _backward_cuda(grad_y, x, w, x_modes_centered, need_x, need_w):
     rank = x.dim() - 2
     grad_y, x, w = _aligned(grad_y), _aligned(x), _aligned(w)
     plan = _plan(rank, x.shape[0], x.shape[-1], x.shape[1], w.shape[1], x.shape[2] if rank == 2 else None, x.device.index,
@@ -129,10 +146,13 @@ def spectral_conv_backward(grad_y: torch.Tensor, x: torch.Tensor, w: torch.Tenso
     return grad_x, grad_w
 
 
-@spectral_conv_backward.register_fake
-def _(grad_y, x, w, x_modes_centered, need_x, need_w):
+def _backward_fake(grad_y, x, w, x_modes_centered, need_x, need_w):
     return (torch.empty_like(x, memory_format=torch.contiguous_format) if need_x else x.new_empty(0),
             torch.empty_like(w, memory_format=torch.contiguous_format) if need_w else w.new_empty(0))
+
+
+spectral_conv_backward = _define("spectral_conv_backward(Tensor grad_y, Tensor x, Tensor w, bool x_modes_centered, bool need_x, bool need_w) -> (Tensor, Tensor)",
+                                 _backward_cuda, _backward_fake)
 
 
 def _native_backward(ctx, grad_y, centered):
@@ -141,7 +161,7 @@ def _native_backward(ctx, grad_y, centered):
     if torch.is_grad_enabled() or max(w.shape[0], w.shape[1]) > _NATIVE_CHANNELS:
         return None
     need_x, need_w = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
-    grad_x, grad_w = torch.ops.turbofno_b200.spectral_conv_backward(grad_y, x, w, centered, need_x, need_w)
+    grad_x, grad_w = spectral_conv_backward(grad_y, x, w, centered, need_x, need_w)
     return (grad_x if need_x else None), (grad_w if need_w else None)
 
 
@@ -171,7 +191,7 @@ def _conv1d_backward(ctx, grad_y):
     return grad_x, grad_w
 
 
-spectral_conv1d.register_autograd(_conv1d_backward, setup_context=_conv1d_setup_context)
+_differentiable("spectral_conv1d", _conv1d_backward, _conv1d_setup_context)
 
 
 def _truncated_spectrum2d(t, centered=False):
@@ -204,11 +224,10 @@ def _conv2d_backward(ctx, grad_y):
     return grad_x, grad_w, None
 
 
-spectral_conv2d.register_autograd(_conv2d_backward, setup_context=_conv2d_setup_context)
+_differentiable("spectral_conv2d", _conv2d_backward, _conv2d_setup_context)
 
 
-@torch.library.custom_op("turbofno_b200::real_spectral_conv2d", mutates_args=(), device_types="cuda")
-def real_spectral_conv2d(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+def _real_conv2d_cuda(x, w):
     _check_real(x, w)
     x, w = _aligned(x), _aligned(w)
     B, K, DX, DY = x.shape
@@ -223,10 +242,12 @@ def _check_real(x, w):
         raise ValueError("rfft_spectral_conv2d: expected x[B, K, DX, DY] and w[K, N, 64, 64]")
 
 
-@real_spectral_conv2d.register_fake
-def _(x, w):
+def _real_conv2d_fake(x, w):
     _check_real(x, w)
     return x.new_empty((x.shape[0], w.shape[1], x.shape[2], x.shape[3]))
+
+
+real_spectral_conv2d = _define("real_spectral_conv2d(Tensor x, Tensor w) -> Tensor", _real_conv2d_cuda, _real_conv2d_fake)
 
 
 def _real_conv2d_setup_context(ctx, inputs, output):
@@ -251,7 +272,7 @@ def _real_conv2d_backward(ctx, grad_y):
     return grad_x, grad_w
 
 
-real_spectral_conv2d.register_autograd(_real_conv2d_backward, setup_context=_real_conv2d_setup_context)
+_differentiable("real_spectral_conv2d", _real_conv2d_backward, _real_conv2d_setup_context)
 
 
 def rfft_spectral_conv2d(x, w):
