@@ -40,7 +40,8 @@ template <int RX, int RY, bool REAL>
 int launch_forward_split(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st) {
     // Few images: a cluster of CTAs of 64 rows per image (8 images of 128 x 256: 8.4 us against 10.9 with one CTA
     // each, 16 of 256 x 256: 9.4 against 17.3).  With more than two such CTAs per SM the exchange through
-    // distributed shared memory costs more than the parallelism gives (512 images of 256 x 256: 98 against 73 us).
+    // distributed shared memory costs more than the parallelism gives (512 images of 256 x 256: 98 against 73 us;
+    // all four with rows on the 32-point transform).
     if (p.nimg * (RX / 2) <= 2LL * dev.sms) return launch_forward<RX, RY, RX / 2, REAL>(dev, p, st);
     return launch_forward<RX, RY, 1, REAL>(dev, p, st);
 }
