@@ -155,8 +155,8 @@ class SpectralConv:
         return ((p.N, self.B) if self.layout == "reference" else (self.B, p.N)) + tail
 
     def workspace(self, device):
-        """The plan's own scratch buffer (allocated on first use).  It serves ONE stream at a time:
-        callers that run the same plan on several streams concurrently pass their own `workspace`."""
+        """The plan's own scratch buffer (allocated on first use).  It serves ONE stream and one thread at a time:
+        callers that run the same plan from several pass each call a `workspace` (`call_scratch` makes one)."""
         if self.workspace_bytes and (self._ws is None or self._ws.device != device):
             self._ws = torch.empty(self.workspace_bytes, dtype=torch.uint8, device=device)
         return self._ws
@@ -197,10 +197,7 @@ class SpectralConv:
             too_small = workspace.numel() * workspace.element_size() < self.workspace_bytes     # only where it is optional
             ws = None if too_small else workspace
         elif self._optional_ws:
-            try:
-                ws = self._scratch(self.workspace_bytes, x.device, stream)
-            except torch.OutOfMemoryError:
-                ws = None
+            ws = self.call_scratch(x.device, stream)
         else:
             ws = self.workspace(x.device)
         check(self.lib.tfno_exec(self._plan, _ptr(x), _ptr(w), _ptr(y), _ptr(ws), _stream_ptr(stream, x.device)), "tfno_exec")
@@ -232,6 +229,18 @@ class SpectralConv:
         ws = self._scratch(int(self.lib.tfno_backward_workspace_bytes(self._plan)), x.device, stream)
         check(self.lib.tfno_backward(self._plan, int(real), _ptr(x), _ptr(w), _ptr(grad_y), _ptr(grad_x), _ptr(grad_w), _ptr(ws),
                                      _stream_ptr(stream, x.device)), "tfno_backward")
+
+    def call_scratch(self, device, stream=None):
+        """Scratch for one call of the layer on `stream`; None where the plan needs none, or can do without and there is
+        no memory for it."""
+        if not self.workspace_bytes:
+            return None
+        try:
+            return self._scratch(self.workspace_bytes, device, stream)
+        except torch.OutOfMemoryError:
+            if self._optional_ws:
+                return None
+            raise
 
     @staticmethod
     def _scratch(nbytes, device, stream):

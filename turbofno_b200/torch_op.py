@@ -47,6 +47,13 @@ def _plan(rank, bs, DY, K, N, DX, device, per_mode=False, centered=False):
     return plan
 
 
+def _run_layer(plan, x, w, y):
+    """One layer with scratch of its own.  Every caller of a shape shares its plan, on any stream and thread, and the
+    plan's own buffer serves one stream and one thread at a time: two calls in flight would write the same spectra."""
+    plan(x, w, y=y, workspace=plan.call_scratch(x.device))
+    return y
+
+
 def _check(x, w, rank):
     """Returns True when w carries one matrix per mode."""
     if x.dtype != torch.complex64 or w.dtype != torch.complex64:
@@ -82,9 +89,7 @@ def _conv1d_cuda(x, w):
     B, K, DY = x.shape
     N = w.shape[1]
     plan = _plan(1, B, DY, K, N, None, x.device.index, per_mode)
-    y = torch.empty((B, N, DY), dtype=torch.complex64, device=x.device)
-    plan(x, w, y=y)
-    return y
+    return _run_layer(plan, x, w, torch.empty((B, N, DY), dtype=torch.complex64, device=x.device))
 
 
 def _conv1d_fake(x, w):
@@ -101,9 +106,7 @@ def _conv2d_cuda(x, w, x_modes_centered=False):
     B, K, DX, DY = x.shape
     N = w.shape[1]
     plan = _plan(2, B, DY, K, N, DX, x.device.index, per_mode, bool(x_modes_centered))
-    y = torch.empty((B, N, DX, DY), dtype=torch.complex64, device=x.device)
-    plan(x, w, y=y)
-    return y
+    return _run_layer(plan, x, w, torch.empty((B, N, DX, DY), dtype=torch.complex64, device=x.device))
 
 
 def _conv2d_fake(x, w, x_modes_centered=False):
