@@ -20,6 +20,23 @@ def _ptr(t):
     return ctypes.c_void_p(t.data_ptr())
 
 
+def _out_ptr(t):
+    if t is not None and (t.is_conj() or t.is_neg()):
+        raise TypeError("a tensor with a pending conjugation or negation cannot be written: pass the memory it views")
+    return _ptr(t)
+
+
+def _plain(t, stream=None):
+    """An input whose memory holds its values.  w.conj() (and the gradients autograd hands on) is a flag on the memory
+    of w, which the kernels would read as it is; the copy is made on the stream that reads it."""
+    if t is None or not (t.is_conj() or t.is_neg()):
+        return t
+    if stream is None:
+        return t.resolve_conj().resolve_neg()
+    with torch.cuda.stream(stream):
+        return t.resolve_conj().resolve_neg()
+
+
 def _stream_ptr(stream=None, device=None):
     """cudaStream_t of `stream`, or of the current stream of `device` (not of the current device:
     the tensors decide where the work runs)."""
@@ -145,6 +162,7 @@ class SpectralConv:
         self._plan = plan
         self.workspace_bytes = int(self.lib.tfno_workspace_bytes(plan))
         self._ws = None
+        self._device = torch.device("cuda", self.handle.device)
         # The fused 1D layer itself needs no scratch, so calls of one plan on several streams may overlap; where a wide
         # layer runs faster with some, every call gets its own (and does without when there is no memory for it).
         self._optional_ws = self.workspace_bytes > 0 and rank == 1 and variant == "D" and not self.per_mode
@@ -174,7 +192,7 @@ class SpectralConv:
     def _check_call(self, x, w, y, workspace):
         p = self.problem
         check_shapes(self.rank, self.layout, self.B, p.K, p.N, p.DY, p.DX, x.shape, w.shape, None if y is None else y.shape, self.per_mode)
-        dev = torch.device("cuda", self.handle.device)
+        dev = self._device
         for name, t in (("x", x), ("w", w), ("y", y), ("workspace", workspace)):
             if t is not None and t.device != dev:
                 raise ValueError("%s is on %s, the plan's handle on %s" % (name, t.device, dev))
@@ -188,8 +206,12 @@ class SpectralConv:
     def __call__(self, x, w, y=None, workspace=None, stream=None):
         _check_tensor(x, "x")
         _check_tensor(w, "w")
+        if x.is_conj() or w.is_conj():
+            x, w = _plain(x, stream), _plain(w, stream)
         if y is not None:
             _check_tensor(y, "y")
+            if y.is_conj():
+                raise TypeError("y has a pending conjugation: pass the memory it views")
         self._check_call(x, w, y, workspace)
         if y is None:
             y = torch.empty(self.out_shape(), dtype=torch.complex64, device=x.device)
@@ -210,10 +232,11 @@ class SpectralConv:
             if t is not None and not (t.is_cuda and t.dtype == dtype and t.is_contiguous()):
                 raise TypeError("%s must be a contiguous %s CUDA tensor" % (name, dtype))
         self._check_call(x, w, y, None)
+        x, w = _plain(x, stream), _plain(w, stream)
         if y is None:
             y = torch.empty(self.out_shape(), dtype=torch.float32, device=x.device)
         ws = self._scratch(self.workspace_bytes, x.device, stream)
-        check(self.lib.tfno_exec_real(self._plan, _ptr(x), _ptr(w), _ptr(y), _ptr(ws), _stream_ptr(stream, x.device)), "tfno_exec_real")
+        check(self.lib.tfno_exec_real(self._plan, _ptr(x), _ptr(w), _out_ptr(y), _ptr(ws), _stream_ptr(stream, x.device)), "tfno_exec_real")
         return y
 
     def backward(self, x, w, grad_y, grad_x=None, grad_w=None, stream=None):
@@ -226,8 +249,9 @@ class SpectralConv:
         self._check_call(x, w, grad_y, None)
         if grad_x is not None or grad_w is not None:
             self._check_call(x if grad_x is None else grad_x, w if grad_w is None else grad_w, None, None)
+        x, w, grad_y = _plain(x, stream), _plain(w, stream), _plain(grad_y, stream)
         ws = self._scratch(int(self.lib.tfno_backward_workspace_bytes(self._plan)), x.device, stream)
-        check(self.lib.tfno_backward(self._plan, int(real), _ptr(x), _ptr(w), _ptr(grad_y), _ptr(grad_x), _ptr(grad_w), _ptr(ws),
+        check(self.lib.tfno_backward(self._plan, int(real), _ptr(x), _ptr(w), _ptr(grad_y), _out_ptr(grad_x), _out_ptr(grad_w), _ptr(ws),
                                      _stream_ptr(stream, x.device)), "tfno_backward")
 
     def call_scratch(self, device, stream=None):
@@ -256,6 +280,9 @@ class SpectralConv:
         for t in (x_host, w_host, y_host):
             if t.is_cuda or t.dtype != torch.complex64 or not t.is_contiguous():
                 raise TypeError("exec_host needs contiguous complex64 host tensors")
+        if y_host.is_conj():
+            raise TypeError("y_host has a pending conjugation: pass the memory it views")
+        x_host, w_host = _plain(x_host), _plain(w_host)
         p = self.problem
         check_shapes(self.rank, self.layout, self.B, p.K, p.N, p.DY, p.DX, x_host.shape, w_host.shape, y_host.shape, self.per_mode)
         check(self.lib.tfno_exec_host(self._plan, ctypes.c_void_p(x_host.data_ptr()), ctypes.c_void_p(w_host.data_ptr()),
@@ -285,58 +312,66 @@ def _log2(n):
 
 
 def fused_fft_cgemm_ifft(M, N, K, FFT_input, B, C, FFT_output, alpha=1 + 0j, beta=0j, DY=128, stream=None):
+    FFT_input, B = _plain(FFT_input, stream), _plain(B, stream)
     h = Handle.get(FFT_input.device.index)
     a, b = complex(alpha), complex(beta)
-    check(h.lib.tfno_fused_fft_cgemm_ifft(h._h, _log2(DY), M, N, K, _ptr(FFT_input), _ptr(B), _ptr(C), _ptr(FFT_output),
+    check(h.lib.tfno_fused_fft_cgemm_ifft(h._h, _log2(DY), M, N, K, _ptr(FFT_input), _ptr(B), _ptr(C), _out_ptr(FFT_output),
                                           a.real, a.imag, b.real, b.imag, _stream_ptr(stream, FFT_input.device)), "tfno_fused_fft_cgemm_ifft")
     return FFT_output
 
 
 def fused_fft_cgemm(M, N, K, FFT_input, B, C, alpha=1 + 0j, beta=0j, DY=128, stream=None):
+    FFT_input, B = _plain(FFT_input, stream), _plain(B, stream)
     h = Handle.get(FFT_input.device.index)
     a, b = complex(alpha), complex(beta)
-    check(h.lib.tfno_fused_fft_cgemm(h._h, _log2(DY), M, N, K, _ptr(FFT_input), _ptr(B), _ptr(C),
+    check(h.lib.tfno_fused_fft_cgemm(h._h, _log2(DY), M, N, K, _ptr(FFT_input), _ptr(B), _out_ptr(C),
                                      a.real, a.imag, b.real, b.imag, _stream_ptr(stream, FFT_input.device)), "tfno_fused_fft_cgemm")
     return C
 
 
 def fused_cgemm_ifft(M, N, K, A, B, C, FFT_output, alpha=1 + 0j, beta=0j, DY=128, stream=None):
+    A, B = _plain(A, stream), _plain(B, stream)
     h = Handle.get(A.device.index)
     a, b = complex(alpha), complex(beta)
-    check(h.lib.tfno_fused_cgemm_ifft(h._h, _log2(DY), M, N, K, _ptr(A), _ptr(B), _ptr(C), _ptr(FFT_output),
+    check(h.lib.tfno_fused_cgemm_ifft(h._h, _log2(DY), M, N, K, _ptr(A), _ptr(B), _ptr(C), _out_ptr(FFT_output),
                                       a.real, a.imag, b.real, b.imag, _stream_ptr(stream, A.device)), "tfno_fused_cgemm_ifft")
     return FFT_output
 
 
 def cgemm(M, N, K, A, B, C, alpha=1 + 0j, beta=0j, stream=None):
+    A, B = _plain(A, stream), _plain(B, stream)
     h = Handle.get(A.device.index)
     a, b = complex(alpha), complex(beta)
-    check(h.lib.tfno_cgemm(h._h, M, N, K, _ptr(A), _ptr(B), _ptr(C), a.real, a.imag, b.real, b.imag,
+    check(h.lib.tfno_cgemm(h._h, M, N, K, _ptr(A), _ptr(B), _out_ptr(C), a.real, a.imag, b.real, b.imag,
                            _stream_ptr(stream, A.device)), "tfno_cgemm")
     return C
 
 
 def fft_stride_DY(inp, out, total_signals, DY, stream=None):
+    inp = _plain(inp, stream)
     h = Handle.get(inp.device.index)
-    check(h.lib.tfno_fft_stride_DY(h._h, _log2(DY), _ptr(inp), _ptr(out), total_signals, _stream_ptr(stream, inp.device)), "tfno_fft_stride_DY")
+    check(h.lib.tfno_fft_stride_DY(h._h, _log2(DY), _ptr(inp), _out_ptr(out), total_signals, _stream_ptr(stream, inp.device)), "tfno_fft_stride_DY")
     return out
 
 
 def ifft_stride_DY(inp, out, total_signals, DY, stream=None):
+    inp = _plain(inp, stream)
     h = Handle.get(inp.device.index)
-    check(h.lib.tfno_ifft_stride_DY(h._h, _log2(DY), _ptr(inp), _ptr(out), total_signals, _stream_ptr(stream, inp.device)), "tfno_ifft_stride_DY")
+    check(h.lib.tfno_ifft_stride_DY(h._h, _log2(DY), _ptr(inp), _out_ptr(out), total_signals, _stream_ptr(stream, inp.device)), "tfno_ifft_stride_DY")
     return out
 
 
 def fft_stride(inp, out, DY, total_columns, DX, stream=None):
+    inp = _plain(inp, stream)
     h = Handle.get(inp.device.index)
-    check(h.lib.tfno_fft_stride(h._h, _log2(DX), _ptr(inp), _ptr(out), DY, total_columns, _stream_ptr(stream, inp.device)), "tfno_fft_stride")
+    check(h.lib.tfno_fft_stride(h._h, _log2(DX), _ptr(inp), _out_ptr(out), DY, total_columns, _stream_ptr(stream, inp.device)), "tfno_fft_stride")
     return out
 
 
 def ifft_stride(inp, out, DY, total_columns, DX, stream=None):
+    inp = _plain(inp, stream)
     h = Handle.get(inp.device.index)
-    check(h.lib.tfno_ifft_stride(h._h, _log2(DX), _ptr(inp), _ptr(out), DY, total_columns, _stream_ptr(stream, inp.device)), "tfno_ifft_stride")
+    check(h.lib.tfno_ifft_stride(h._h, _log2(DX), _ptr(inp), _out_ptr(out), DY, total_columns, _stream_ptr(stream, inp.device)), "tfno_ifft_stride")
     return out
 
 
@@ -348,6 +383,7 @@ def spectral_conv2d_static(x, w, y=None, alpha=1 + 0j, stream=None):
     reference layout; y is allocated here by torch only if the caller does not pass one."""
     _check_tensor(x, "x")
     _check_tensor(w, "w")
+    x, w = _plain(x, stream), _plain(w, stream)
     if x.dim() != 4 or w.dim() != 2:
         raise ValueError("x must be [K, bs, DX, DY] and w [N, K]")
     K, bs, DX, DY = x.shape
@@ -363,6 +399,6 @@ def spectral_conv2d_static(x, w, y=None, alpha=1 + 0j, stream=None):
     lib = _lib.load()
     a = complex(alpha)
     with torch.cuda.device(x.device):
-        check(lib.tfno_spectral_conv2d_static(bs, DX, DY, K, N, _ptr(x), _ptr(w), _ptr(y), a.real, a.imag,
+        check(lib.tfno_spectral_conv2d_static(bs, DX, DY, K, N, _ptr(x), _ptr(w), _out_ptr(y), a.real, a.imag,
                                               _stream_ptr(stream, x.device)), "tfno_spectral_conv2d_static")
     return y
