@@ -125,15 +125,24 @@ int tfno_plan_destroy(tfno_plan* plan);
 
 /* Bytes of caller-provided device scratch tfno_exec needs (intermediates A, C and, for E, the
  * full-size transform buffer -- dA, dC, dFFT_output at fusion_variants/1D_E_baseline/fused.cu:95-100).
- * 0 for the fused 1D variant D, except for wide layers of long signals (more than 64 output or 96 input channels at
- * DY >= 512, large batches): with this much scratch they run as three kernels, about 1.2 to 2 times faster; there
- * alone a null workspace is allowed too and keeps the fused kernel. */
+ * 0 for the fused 1D variant D.  A workspace holds one call at a time: it serves one stream, and calls
+ * from several threads on that stream must not overlap on the host either. */
 size_t tfno_workspace_bytes(const tfno_plan* plan);
 
 /* One spectral-convolution layer.  Replaces the timed body of the drivers
- * (fusion_variants/1D_D_exp_fused_fft_cgemm_ifft/fused.cu:135-139 and the A/B/C/E equivalents). */
+ * (fusion_variants/1D_D_exp_fused_fft_cgemm_ifft/fused.cu:135-139 and the A/B/C/E equivalents).
+ * A plan whose tfno_workspace_bytes is 0 leaves `workspace` alone. */
 int tfno_exec(const tfno_plan* plan, const void* x, const void* w, void* y,
               void* workspace, void* stream);
+
+/* Scratch a plan can do without but runs faster with, or 0.  Not 0 for 1D variant D plans with shared weights, DY >= 512
+ * and K <= 128 whose batch has at least one row (bs*dimX) per SM with N > 64, or four rows per SM with N = 64 and
+ * K > 96 (at DY = 1024: K >= 64): given this much they run as three kernels, 1.1 to 1.9 times faster.
+ * tfno_exec_scratch is tfno_exec with the size of the workspace: it uses the scratch when there is enough (and runs as
+ * tfno_exec when there is less); the rule for one workspace and several streams or threads is the same. */
+size_t tfno_optional_workspace_bytes(const tfno_plan* plan);
+int tfno_exec_scratch(const tfno_plan* plan, const void* x, const void* w, void* y,
+                      void* workspace, size_t workspace_bytes, void* stream);
 
 /* The same layer of REAL fields: x and y hold float samples (strides of the plan in samples), w complex per-mode
  * weights.  2D variant D plans with per-mode weights; the field's spectrum carries ky = 0..63 and the layer is
@@ -160,8 +169,8 @@ int tfno_exec_host(tfno_plan* plan, const void* x_host, const void* w_host, void
  * cudaMemcpy (fusion_variants/1D_D_exp_fused_fft_cgemm_ifft/fused.cu:116). */
 int tfno_plan_set_host_chunk(tfno_plan* plan, long long batch_items);
 
-/* Writes the names of the kernels (and library calls) one tfno_exec of this plan launches, in
- * launch order and separated by ';', e.g. "spectral_tc_kernel<8,1>" or
+/* Writes the names of the kernels (and library calls) one tfno_exec of this plan launches (a plan
+ * with optional scratch: one tfno_exec_scratch that has it), in launch order and separated by ';', e.g. "spectral_tc_kernel<8,1>" or
  * "fft2d_trunc_kernel<4,4,paired,256>;cgemm_tc_kernel<128>;ifft2d_pad_kernel<4,4,paired,256>".
  * It is produced by a dry run of the dispatch code tfno_exec itself executes.  Stands in for reading
  * which table entry a reference driver launches

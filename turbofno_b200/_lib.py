@@ -58,6 +58,8 @@ SYMBOLS = {
     "tfno_plan_destroy": (_i, [_vp]),
     "tfno_workspace_bytes": (ctypes.c_size_t, [_vp]),
     "tfno_exec": (_i, [_vp, _vp, _vp, _vp, _vp, _vp]),
+    "tfno_optional_workspace_bytes": (ctypes.c_size_t, [_vp]),
+    "tfno_exec_scratch": (_i, [_vp, _vp, _vp, _vp, _vp, ctypes.c_size_t, _vp]),
     "tfno_exec_real": (_i, [_vp, _vp, _vp, _vp, _vp, _vp]),
     "tfno_backward_workspace_bytes": (ctypes.c_size_t, [_vp]),
     "tfno_backward": (_i, [_vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),

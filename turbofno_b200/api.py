@@ -160,12 +160,13 @@ class SpectralConv:
         plan = ctypes.c_void_p()
         check(self.lib.tfno_plan_create(self.handle._h, ctypes.byref(p), ctypes.byref(plan)), "tfno_plan_create")
         self._plan = plan
-        self.workspace_bytes = int(self.lib.tfno_workspace_bytes(plan))
+        # The fused 1D layer needs no scratch, so calls of one plan on several streams may overlap; where a wide layer runs
+        # faster with some, every call gets its own (and does without when there is no memory for it).
+        optional = int(self.lib.tfno_optional_workspace_bytes(plan))
+        self._optional_ws = optional > 0
+        self.workspace_bytes = optional or int(self.lib.tfno_workspace_bytes(plan))
         self._ws = None
         self._device = torch.device("cuda", self.handle.device)
-        # The fused 1D layer itself needs no scratch, so calls of one plan on several streams may overlap; where a wide
-        # layer runs faster with some, every call gets its own (and does without when there is no memory for it).
-        self._optional_ws = self.workspace_bytes > 0 and rank == 1 and variant == "D" and not self.per_mode
 
     def out_shape(self):
         p = self.problem
@@ -215,13 +216,12 @@ class SpectralConv:
         self._check_call(x, w, y, workspace)
         if y is None:
             y = torch.empty(self.out_shape(), dtype=torch.complex64, device=x.device)
-        if workspace is not None:
-            too_small = workspace.numel() * workspace.element_size() < self.workspace_bytes     # only where it is optional
-            ws = None if too_small else workspace
-        elif self._optional_ws:
-            ws = self.call_scratch(x.device, stream)
-        else:
-            ws = self.workspace(x.device)
+        if self._optional_ws:
+            ws = workspace if workspace is not None else self.call_scratch(x.device, stream)
+            nbytes = 0 if ws is None else ws.numel() * ws.element_size()
+            check(self.lib.tfno_exec_scratch(self._plan, _ptr(x), _ptr(w), _ptr(y), _ptr(ws), nbytes, _stream_ptr(stream, x.device)), "tfno_exec_scratch")
+            return y
+        ws = workspace if workspace is not None else self.workspace(x.device)
         check(self.lib.tfno_exec(self._plan, _ptr(x), _ptr(w), _ptr(y), _ptr(ws), _stream_ptr(stream, x.device)), "tfno_exec")
         return y
 

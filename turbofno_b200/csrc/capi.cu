@@ -33,10 +33,11 @@ struct tfno_plan_s {
     tfno_handle_s* h = nullptr;
     tfno_problem p{};
     long long B = 0;                    // 1D: bs*dimX rows; 2D: bs images per channel
-    size_t ws_bytes = 0;
+    size_t ws_bytes = 0;                // scratch tfno_exec needs
+    size_t optional_bytes = 0;          // scratch that makes tfno_exec_scratch faster (wide layers)
     bool default_layout = true;
     bool per_mode = false;              // per-mode weights (w_stride_m != 0)
-    bool wide = false;                  // 1D variant D as transform, contraction, transform when a workspace is given
+    bool wide = false;                  // 1D variant D as transform, contraction, transform when tfno_exec_scratch is given the room
     // variant E
     cufftHandle fft_fwd = 0, fft_inv = 0;
     bool have_fft = false;
@@ -111,7 +112,8 @@ Workspace carve(const tfno_plan_s& pl) {
 //   DY = 1024  K=N=128 at 150 / 1024 rows 191 / 1015 against 140 / 532;  K=N=64 at 600 / 2048 rows 174 / 467 against 153 / 425
 //   DY = 256   K=N=128 at 1024 / 2048 rows 295 / 536 against 274 / 556, K=64 N=128 151 / 269 against 153 / 261: stays fused
 // Below one row per SM (wide) and four rows per SM (64 outputs) a call is short enough that one or two launches
-// without a workspace are kept.
+// without a workspace are kept.  The scratch is a separate offer (tfno_exec_scratch, with its size): tfno_exec of these
+// plans needs none and leaves a pointer it is given alone, so a plan may run on several streams at once.
 bool wide_layer(const DeviceInfo& dev, const tfno_problem& p, long long rows) {
     if (p.rank != 1 || p.variant != TFNO_VARIANT_D || p.w_stride_m != 0 || !dev.use_tensor_cores || !dev.status) return false;
     if (p.DY < 512 || p.K > 128) return false;
@@ -322,7 +324,7 @@ int tfno_plan_create(tfno_handle* h, const tfno_problem* problem, tfno_plan** ou
         return TFNO_ERR_INVALID_ARG;
     }
     pl->wide = wide_layer(h->dev, p, pl->B);
-    pl->ws_bytes = carve(*pl).total;
+    (pl->wide ? pl->optional_bytes : pl->ws_bytes) = carve(*pl).total;
 
     if (p.variant == TFNO_VARIANT_E) {
         if (!pl->default_layout) { delete pl; return TFNO_ERR_UNSUPPORTED; }
@@ -354,6 +356,7 @@ int tfno_plan_create(tfno_handle* h, const tfno_problem* problem, tfno_plan** ou
 }
 
 size_t tfno_workspace_bytes(const tfno_plan* plan) { return plan ? plan->ws_bytes : 0; }
+size_t tfno_optional_workspace_bytes(const tfno_plan* plan) { return plan ? plan->optional_bytes : 0; }
 
 }  // extern "C"
 
@@ -370,8 +373,9 @@ static PerModeParams permode_layer(const tfno_problem& p, long long B, long long
 
 // The dispatch of one layer.  With dev.record set it is a dry run: every launcher appends the
 // name of the kernel it would launch and nothing touches the device.
+// split: a wide 1D layer as three kernels (the workspace holds optional_bytes).
 static int exec_impl(const tfno_plan* plan, const DeviceInfo& dev, const void* x, const void* w, void* y, void* workspace,
-                     void* stream, bool real_field = false) {
+                     void* stream, bool split, bool real_field = false) {
     const tfno_problem& p = plan->p;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const Workspace ws = carve(*plan);
@@ -413,7 +417,6 @@ static int exec_impl(const tfno_plan* plan, const DeviceInfo& dev, const void* x
             if (rc) return rc;
             return launch_ifft_rows(dev, p.DY, ir, st);
         }
-        const bool split = plan->wide && workspace;
         if (split) t.beta = f2(0.f, 0.f);       // D ignores beta
         switch (split ? TFNO_VARIANT_A : p.variant) {
             case TFNO_VARIANT_A:
@@ -558,11 +561,24 @@ extern "C" {
 int tfno_exec(const tfno_plan* plan, const void* x, const void* w, void* y, void* workspace, void* stream) {
     if (!plan || !x || !w || !y) return TFNO_ERR_INVALID_ARG;
     if (!aligned16(x) || !aligned16(y) || !aligned16(w) || !aligned16(workspace)) return TFNO_ERR_INVALID_ARG;
-    if (plan->ws_bytes > 0 && !plan->wide && !workspace) return TFNO_ERR_WORKSPACE;
+    if (plan->ws_bytes > 0 && !workspace) return TFNO_ERR_WORKSPACE;
     const DeviceInfo& dev = plan->h->dev;
     DeviceGuard guard(dev.device);
     if (!guard.ok) return TFNO_ERR_CUDA;
-    return exec_impl(plan, dev, x, w, y, workspace, stream);
+    return exec_impl(plan, dev, x, w, y, workspace, stream, false);
+}
+
+int tfno_exec_scratch(const tfno_plan* plan, const void* x, const void* w, void* y, void* workspace, size_t workspace_bytes, void* stream) {
+    if (!plan) return TFNO_ERR_INVALID_ARG;
+    if (!plan->wide || !workspace || workspace_bytes < plan->optional_bytes) {
+        if (plan->ws_bytes > workspace_bytes) return TFNO_ERR_WORKSPACE;
+        return tfno_exec(plan, x, w, y, plan->wide ? nullptr : workspace, stream);
+    }
+    if (!x || !w || !y || !aligned16(x) || !aligned16(y) || !aligned16(w) || !aligned16(workspace)) return TFNO_ERR_INVALID_ARG;
+    const DeviceInfo& dev = plan->h->dev;
+    DeviceGuard guard(dev.device);
+    if (!guard.ok) return TFNO_ERR_CUDA;
+    return exec_impl(plan, dev, x, w, y, workspace, stream, true);
 }
 
 // A layer of real fields: 2D, per-mode weights (only the image transforms know real samples).
@@ -578,7 +594,7 @@ int tfno_exec_real(const tfno_plan* plan, const void* x, const void* w, void* y,
     const DeviceInfo& dev = plan->h->dev;
     DeviceGuard guard(dev.device);
     if (!guard.ok) return TFNO_ERR_CUDA;
-    return exec_impl(plan, dev, x, w, y, workspace, stream, true);
+    return exec_impl(plan, dev, x, w, y, workspace, stream, false, true);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -722,7 +738,7 @@ int tfno_plan_kernels(const tfno_plan* plan, char* buf, size_t cap) {
     dev.record_cap = cap;
     // dry run over stand-in operands: 256-byte aligned, never dereferenced
     char* fake = reinterpret_cast<char*>(static_cast<uintptr_t>(1) << 20);
-    return exec_impl(plan, dev, fake, fake, fake, fake, nullptr);
+    return exec_impl(plan, dev, fake, fake, fake, fake, nullptr, plan->wide);
 }
 
 // ------------------------------------------------------------------------------------------------
