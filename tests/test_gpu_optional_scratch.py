@@ -1,6 +1,8 @@
 """Scratch that wide 1D layers can do without: tfno_exec needs none and leaves a workspace alone, tfno_exec_scratch uses
 what is large enough, and the host-buffer path does not ask for it."""
 import ctypes
+import os
+import subprocess
 
 import pytest
 
@@ -106,3 +108,12 @@ def test_host_path_does_not_ask_for_it(cuda):
     assert ((yh.transpose(0, 1).to(cuda) - ref).norm() / ref.norm()).item() <= REL
     plan.close()
     warm.close()
+
+
+def test_executable_runs_a_wide_layer(cuda):
+    import json
+
+    from test_gpu_drivers import BIN
+
+    out = subprocess.check_output([os.path.join(BIN, "TurboFNO_1D_D"), "300", "1", "1024", "128", "128", "--stream", "--json"], text=True, timeout=120)
+    assert json.loads(out)["time_ms"] > 0, out

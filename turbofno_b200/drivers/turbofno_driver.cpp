@@ -134,9 +134,17 @@ int main(int argc, char** argv) {
             tfno_plan_destroy(plan);
             continue;
         }
+        // scratch the layer can do without: taken where there is room
+        size_t extra = tfno_optional_workspace_bytes(plan);
+        if (xb + yb + wb + wsb + extra + (256u << 20) > free_b) extra = 0;
         float2 *dx = nullptr, *dy = nullptr, *dw = nullptr; void* dws = nullptr;
         bool ok = cuda_ok(cudaMalloc(&dx, xb), "cudaMalloc x") && cuda_ok(cudaMalloc(&dy, yb), "cudaMalloc y") &&
                   cuda_ok(cudaMalloc(&dw, wb), "cudaMalloc w") && (wsb == 0 || cuda_ok(cudaMalloc(&dws, wsb), "cudaMalloc workspace"));
+        if (ok && extra && cudaMalloc(&dws, extra) != cudaSuccess) {
+            cudaGetLastError();
+            dws = nullptr;
+            extra = 0;
+        }
         if (ok) {
             // host fill in slices of at most 64 Mi floats
             const size_t slice = 64u << 20;
@@ -156,9 +164,9 @@ int main(int argc, char** argv) {
         }
         float ms = 0.f;
         if (ok) {
-            rc = tfno_exec(plan, dx, dw, dy, dws, nullptr);          // warm-up, checked
+            rc = tfno_exec_scratch(plan, dx, dw, dy, dws, wsb + extra, nullptr);          // warm-up, checked
             ok = (rc == TFNO_OK) && cuda_ok(cudaDeviceSynchronize(), "warm-up");
-            if (rc) fprintf(stderr, "tfno_exec: %s\n", tfno_status_string(rc));
+            if (rc) fprintf(stderr, "tfno_exec_scratch: %s\n", tfno_status_string(rc));
         }
         if (ok) {
             cudaEvent_t e0, e1;
@@ -166,7 +174,7 @@ int main(int argc, char** argv) {
             const int reps = stream_mode ? 20 : ntest;
             cudaEventRecord(e0);
             for (int i = 0; i < reps && rc == TFNO_OK; ++i) {
-                rc = tfno_exec(plan, dx, dw, dy, dws, nullptr);
+                rc = tfno_exec_scratch(plan, dx, dw, dy, dws, wsb + extra, nullptr);
                 if (!stream_mode) cudaDeviceSynchronize();
             }
             cudaEventRecord(e1);
