@@ -117,3 +117,32 @@ def test_executable_runs_a_wide_layer(cuda):
 
     out = subprocess.check_output([os.path.join(BIN, "TurboFNO_1D_D"), "300", "1", "1024", "128", "128", "--stream", "--json"], text=True, timeout=120)
     assert json.loads(out)["time_ms"] > 0, out
+
+
+def test_a_captured_call_records_no_block_of_the_allocator(cuda):
+    """A graph may be captured by other means than torch.cuda.graph, whose pool would keep the block; with a workspace
+    the graph uses that."""
+    import torch
+    import turbofno_b200 as t
+
+    B, K, N, DY = 160, 16, 128, 512
+    x, w, ref = _inputs(B, K, N, DY)
+    plan = t.SpectralConv(1, B, DY, K, N, layout="batch_major")
+    y = torch.empty(plan.out_shape(), dtype=torch.complex64, device=cuda)
+    ws = torch.empty(plan.workspace_bytes, dtype=torch.uint8, device=cuda)
+    side = torch.cuda.Stream()
+    for kw in ({}, {"workspace": ws}, {"stream": side}):
+        plan(x, w, y=y, **kw)
+        torch.cuda.synchronize()
+        y.zero_()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            before = torch.cuda.memory_stats()["allocation.all.allocated"]
+            plan(x, w, y=y, **kw)
+            allocated = torch.cuda.memory_stats()["allocation.all.allocated"] - before
+        assert allocated == 0, kw
+        graph.replay()
+        torch.cuda.synchronize()
+        assert ((y - ref).norm() / ref.norm()).item() <= REL
+        del graph
+    plan.close()

@@ -44,6 +44,11 @@ def _stream_ptr(stream=None, device=None):
     return ctypes.c_void_p(s.cuda_stream)
 
 
+def _capturing(device, stream=None):
+    with torch.cuda.stream(stream if stream is not None else torch.cuda.current_stream(device)):
+        return torch.cuda.is_current_stream_capturing()
+
+
 def _check_tensor(t, name):
     if not (isinstance(t, torch.Tensor) and t.is_cuda and t.dtype == torch.complex64 and t.is_contiguous()):
         raise TypeError("%s must be a contiguous complex64 CUDA tensor" % name)
@@ -161,7 +166,8 @@ class SpectralConv:
         check(self.lib.tfno_plan_create(self.handle._h, ctypes.byref(p), ctypes.byref(plan)), "tfno_plan_create")
         self._plan = plan
         # The fused 1D layer needs no scratch, so calls of one plan on several streams may overlap; where a wide layer runs
-        # faster with some, every call gets its own (and does without when there is no memory for it).
+        # faster with some, every call gets its own (and does without when there is no memory for it, and while a graph
+        # is captured: the graph would keep the address of a block that goes back to the allocator.  Pass a workspace).
         optional = int(self.lib.tfno_optional_workspace_bytes(plan))
         self._optional_ws = optional > 0
         self.workspace_bytes = optional or int(self.lib.tfno_workspace_bytes(plan))
@@ -217,7 +223,9 @@ class SpectralConv:
         if y is None:
             y = torch.empty(self.out_shape(), dtype=torch.complex64, device=x.device)
         if self._optional_ws:
-            ws = workspace if workspace is not None else self.call_scratch(x.device, stream)
+            ws = workspace
+            if ws is None and not _capturing(x.device, stream):
+                ws = self.call_scratch(x.device, stream)
             nbytes = 0 if ws is None else ws.numel() * ws.element_size()
             check(self.lib.tfno_exec_scratch(self._plan, _ptr(x), _ptr(w), _ptr(y), _ptr(ws), nbytes, _stream_ptr(stream, x.device)), "tfno_exec_scratch")
             return y
@@ -269,7 +277,8 @@ class SpectralConv:
     @staticmethod
     def _scratch(nbytes, device, stream):
         """Scratch of one call, from the caching allocator's pool of the stream the call runs on: the block may be handed
-        out again as soon as this returns, to work that is ordered behind the call."""
+        out again as soon as the call has returned, to work that is ordered behind it.  Calls that take their scratch here are
+        captured through torch.cuda.graph, which keeps such blocks for the graph."""
         if stream is None:
             return torch.empty(nbytes, dtype=torch.uint8, device=device)
         with torch.cuda.stream(stream):
