@@ -171,7 +171,8 @@ int tfno_plan_set_host_chunk(tfno_plan* plan, long long batch_items);
 
 /* Writes the names of the kernels (and library calls) one tfno_exec of this plan launches (a plan
  * with optional scratch: one tfno_exec_scratch that has it), in launch order and separated by ';', e.g. "spectral_tc_kernel<8,1>" or
- * "fft2d_trunc_kernel<4,4,paired,256>;cgemm_tc_kernel<128>;ifft2d_pad_kernel<4,4,paired,256>".
+ * "fft2d_trunc_kernel<8,8,1>;cgemm_tc_kernel<128>;ifft2d_pad64_kernel<4,4,2,0>": kernel and template
+ * arguments (those that tell complex from real fields left out).
  * It is produced by a dry run of the dispatch code tfno_exec itself executes.  Stands in for reading
  * which table entry a reference driver launches
  * (fusion_variants/1D_D_exp_fused_fft_cgemm_ifft/fused.cu:15-16,126). */

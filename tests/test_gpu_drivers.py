@@ -107,11 +107,36 @@ def test_plan_reports_the_kernels_it_launches(cuda):
     assert kernels(1, 300, 256, 64, 64, "A") == ["fft_rows_trunc_kernel<4>", "cgemm_tc_kernel<128>", "ifft_rows_pad_kernel<4>"]
     assert kernels(1, 300, 256, 64, 64, "A", beta=1j)[1] == "spectral_tile_kernel<2,0,0,1>"
     # 2D variant D
-    assert kernels(2, 16, 256, 32, 64, DX=256) == ["fft2d_trunc32_kernel<8,8>", "cgemm_tc_kernel<128>", "ifft2d_pad_kernel<4,4,paired,256>"]
-    assert kernels(2, 16, 128, 32, 64, DX=256) == ["fft2d_trunc32_kernel<8,4>", "cgemm_tc_kernel<128>", "ifft2d_pad32_kernel<8,4,1>"]
-    assert kernels(2, 1, 128, 8, 64, DX=128) == ["fft2d_trunc_kernel<2,2,paired,128>", "cgemm_tc_kernel<64>", "ifft2d_pad_kernel<2,2,paired,128>"]
+    assert kernels(2, 16, 256, 32, 64, DX=256) == ["fft2d_trunc_kernel<8,8,1>", "cgemm_tc_kernel<128>", "ifft2d_pad64_kernel<4,4,2,0>"]
+    assert kernels(2, 16, 128, 32, 64, DX=256) == ["fft2d_trunc_kernel<8,4,1>", "cgemm_tc_kernel<128>", "ifft2d_pad_kernel<8,4,2,1>"]
+    assert kernels(2, 1, 128, 8, 64, DX=128) == ["fft2d_trunc_kernel<4,4,2>", "cgemm_tc_kernel<64>", "ifft2d_pad_kernel<4,4,2,1>"]
     assert kernels(2, 8, 128, 104, 64, DX=128)[1:3] == ["cgemm_tc_kernel<128>", "cgemm_tc_kernel<128>+="]     # 64 + 40 channels
     assert kernels(2, 1, 128, 104, 64, DX=128)[1] == "spectral_tile_kernel<2,0,0,1>"                         # too few rows for two launches
     assert kernels(2, 8, 128, 72, 64, DX=128)[1] == "cgemm_tc_kernel<64>"                                    # 65..96 channels: 64-mode tiles
     # library path
     assert kernels(1, 4, 128, 8, 64, "E") == ["cufftExecC2C", "truncate_rows_kernel", "cublasCgemm", "zero_pad_rows_kernel", "cufftExecC2C"]
+
+
+# bs, DX, DY, options -> image kernels, on both sides of every line of the dispatch (148 SMs; 8 channels in, 64 out)
+@pytest.mark.parametrize("bs,DX,DY,options,forward,inverse", [
+    (9, 256, 256, {}, "fft2d_trunc_kernel<8,8,4>", "ifft2d_pad64_kernel<4,4,2,0>"),      # 72 images in: a cluster of 4 CTAs each
+    (10, 256, 256, {}, "fft2d_trunc_kernel<8,8,1>", "ifft2d_pad64_kernel<4,4,2,0>"),     # 80: one CTA each
+    (2, 256, 256, {}, "fft2d_trunc_kernel<8,8,4>", "ifft2d_pad_kernel<8,8,4,1>"),        # 128 images out
+    (3, 256, 256, {}, "fft2d_trunc_kernel<8,8,4>", "ifft2d_pad64_kernel<4,4,2,0>"),      # 192
+    (18, 128, 256, {}, "fft2d_trunc_kernel<4,8,2>", "ifft2d_pad64_kernel<2,4,2,0>"),     # 144 images in: a cluster of 2 CTAs each
+    (19, 128, 256, {}, "fft2d_trunc_kernel<4,8,1>", "ifft2d_pad64_kernel<2,4,2,0>"),
+    (4, 128, 256, {}, "fft2d_trunc_kernel<4,8,2>", "ifft2d_pad_kernel<4,8,2,1>"),        # 256 images out
+    (5, 128, 256, {}, "fft2d_trunc_kernel<4,8,2>", "ifft2d_pad64_kernel<2,4,2,0>"),      # 320
+    (16, 256, 128, {}, "fft2d_trunc_kernel<8,4,1>", "ifft2d_pad_kernel<8,4,2,1>"),       # rows of 128: the 32-point inverse always
+    (20, 128, 128, {}, "fft2d_trunc_kernel<4,4,1>", "ifft2d_pad_kernel<4,4,2,1>"),
+    (3, 256, 256, {"x_modes_centered": True}, "fft2d_trunc_kernel<8,8,4>", "ifft2d_pad64_kernel<4,4,2,1>"),
+    (3, 256, 256, {"second_transform_forward": True}, "fft2d_trunc_kernel<8,8,4>", "ifft2d_pad64_kernel<4,4,2,0>"),
+    (2, 256, 256, {"second_transform_forward": True}, "fft2d_trunc_kernel<8,8,4>", "ifft2d_pad_kernel<8,8,4,0>")])
+def test_image_kernels_by_the_number_of_images(cuda, bs, DX, DY, options, forward, inverse):
+    import turbofno_b200 as t
+
+    assert t.Handle.get(0).sm_count == 148
+    plan = t.SpectralConv(2, bs, DY, 8, 64, DX=DX, **options)
+    names = plan.kernels()
+    plan.close()
+    assert (names[0], names[-1]) == (forward, inverse)

@@ -10,9 +10,7 @@ int launch_forward(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st)
     auto kernel = fft2d_trunc_kernel<RX, RY, C, REAL>;
     const size_t smem = fwd_image_smem_bytes<RX, RY, C>();
     if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
-    if (RX == 8 ? record_launch(dev, REAL ? "fft2d_trunc32_kernel<%d,%d,real>" : "fft2d_trunc32_kernel<%d,%d>", RX, RY)
-                : record_launch(dev, REAL ? "fft2d_trunc_kernel<%d,%d,real,%d>" : "fft2d_trunc_kernel<%d,%d,paired,%d>", RX / 2, RY / 2, THREADS))
-        return TFNO_OK;
+    if (record_launch(dev, "fft2d_trunc_kernel<%d,%d,%d>", RX, RY, C)) return TFNO_OK;
     int occ = 0;
     const int rc = prepare_kernel(kernel, smem, dev, &occ, THREADS);
     if (rc != TFNO_OK) return rc;
@@ -52,9 +50,7 @@ int launch_inverse(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st)
     auto kernel = ifft2d_pad_kernel<RX, RY, CLS, INVERSE, REAL>;
     const size_t smem = inv_image_smem_bytes<RY, CLS>();
     if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
-    if (RX == 8 && RY == 4 ? record_launch(dev, REAL ? "ifft2d_pad32_kernel<%d,%d,real>" : "ifft2d_pad32_kernel<%d,%d,%d>", RX, RY, INVERSE)
-                           : record_launch(dev, REAL ? "ifft2d_pad_kernel<%d,%d,real,%d>" : "ifft2d_pad_kernel<%d,%d,paired,%d>", RX / 2, RY / 2, THREADS))
-        return TFNO_OK;
+    if (record_launch(dev, "ifft2d_pad_kernel<%d,%d,%d,%d>", RX, RY, CLS, INVERSE)) return TFNO_OK;
     int occ = 0;
     const int rc = prepare_kernel(kernel, smem, dev, &occ, THREADS);
     if (rc != TFNO_OK) return rc;
@@ -70,7 +66,7 @@ int launch_inverse64(const DeviceInfo& dev, const ImageParams& p, cudaStream_t s
     auto kernel = ifft2d_pad64_kernel<RX, 4, CLS, CENTERED_X>;
     const size_t smem = inv64_image_smem_bytes<4, CLS>();
     if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
-    if (record_launch(dev, "ifft2d_pad_kernel<%d,%d,paired,%d>", RX, 4, THREADS * PARTS)) return TFNO_OK;
+    if (record_launch(dev, "ifft2d_pad64_kernel<%d,%d,%d,%d>", RX, 4, CLS, CENTERED_X)) return TFNO_OK;
     int occ = 0;
     const int rc = prepare_kernel(kernel, smem, dev, &occ, THREADS);
     if (rc != TFNO_OK) return rc;

@@ -72,7 +72,7 @@ size_t permode_partial_bytes(const DeviceInfo& dev, const PerModeParams& p, Perm
 int launch_permode(const DeviceInfo& dev, PerModeParams p, PermodeKind kind, cudaStream_t st) {
     if (p.I <= 0 || p.red <= 0) return TFNO_OK;
     if (p.J <= 0 || p.J % kPmCols != 0 || p.modes % kPmModes != 0) return TFNO_ERR_UNSUPPORTED;
-    if (record_launch(dev, is_grad(kind) ? "cgemm_permode_kernel<grad>" : "cgemm_permode_kernel")) return TFNO_OK;
+    if (record_launch(dev, "cgemm_permode_kernel")) return TFNO_OK;
     p.q_vec = (p.q_sm == 1 && ((p.q_sr | p.q_sj) & 1) == 0 && (reinterpret_cast<uintptr_t>(p.q) & 15) == 0) ? 1 : 0;
     p.splits = is_grad(kind) ? grad_splits(dev, p) : 1;
     p.split_len = ((p.red + p.splits - 1) / p.splits + kPmSlab - 1) / kPmSlab * kPmSlab;
@@ -93,7 +93,6 @@ int launch_permode(const DeviceInfo& dev, PerModeParams p, PermodeKind kind, cud
 }
 
 int launch_conjugate(const DeviceInfo& dev, const float2* w, long long sk, long long sn, int K, int N, float2* dst, cudaStream_t st) {
-    if (record_launch(dev, "conjugate_kernel")) return TFNO_OK;
     conjugate_kernel<<<(unsigned)((K * N + 255) / 256), 256, 0, st>>>(w, sk, sn, K, N, dst);
     return launch_status();
 }
