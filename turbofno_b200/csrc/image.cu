@@ -14,9 +14,9 @@ int launch_forward(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st)
     int occ = 0;
     const int rc = prepare_kernel(kernel, smem, dev, &occ, THREADS);
     if (rc != TFNO_OK) return rc;
-    // one cluster per image, as many as are resident together
-    long long clusters = (long long)dev.sms * occ / C;
-    if (clusters > p.nimg) clusters = p.nimg;
+    // a cluster of CTAs per image, or as many CTAs as are resident together
+    long long clusters = p.nimg;
+    if (C == 1 && clusters > (long long)dev.sms * occ) clusters = (long long)dev.sms * occ;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(clusters * C));
     cfg.blockDim = dim3(THREADS);

@@ -6,9 +6,10 @@
 //
 //   forward  a cluster of DX/64 CTAs per image.  Each transforms 64 rows along Y and scatters the kept
 //            columns through distributed shared memory: CTA c of the cluster collects columns
-//            c*64/C .. of ALL rows (32 KB), then transforms them along X.  One cluster barrier
-//            between the passes, a second, split one (arrive after the last read, wait before the
-//            next image's first remote store) that the next image's loads and row transforms hide.
+//            c*64/C .. of ALL rows (32 KB), then transforms them along X.  A cluster takes ONE image: a
+//            cluster barrier says that the peers run before the first remote store (the row loads and
+//            transforms hide it), a second one separates the passes.  With many images (C = 1) a CTA
+//            takes one after the other.
 //   inverse  no exchange at all: lane j1 of the zero-padded X transform produces exactly the image
 //            rows RX*j2 + j1, so a CTA takes CLS of the RX residue classes, transforms the 64 columns
 //            for those rows only (every part re-reads the 32 KB spectrum, from the L2), then its rows.
@@ -166,14 +167,14 @@ __global__ void __launch_bounds__(64 * RX / C, 8 * C / RX) fft2d_trunc_kernel(Im
     };
     constexpr int GROUPS = T / RY, LINES = REAL ? 2 : 1, STEP = GROUPS * LINES, ROUNDS = ROWS / STEP;
     static_assert(ROUNDS >= 1, "a round of row transforms fits the CTA's rows");
-    const long long step = gridDim.x / C;
+    const long long step = C > 1 ? p.nimg : gridDim.x;           // a cluster's only image; there are as many clusters as images
     auto rows_of = [&](long long img) {
         return reinterpret_cast<const Sample*>(p.in) + (img % p.per_k) * p.stride_b + (img / p.per_k) * p.stride_k + (long long)rank * ROWS * DY;
     };
-    if constexpr (C > 1) cluster_arrive();                       // the peers run: their shared memory may be written
+    if constexpr (C > 1) cluster_arrive();                       // this CTA runs: its shared memory may be written
     for (long long img = blockIdx.x / C; img < p.nimg; img += step) {
         const Sample* src = rows_of(img);
-        const Sample* next = img + step < p.nimg ? rows_of(img + step) : nullptr;
+        const Sample* next = C == 1 && img + step < p.nimg ? rows_of(img + step) : nullptr;
 #pragma unroll 1
         for (int i0 = 0; i0 < ROUNDS; ++i0) {
             const int x = i0 * STEP + g * LINES;
@@ -256,9 +257,7 @@ __global__ void __launch_bounds__(64 * RX / C, 8 * C / RX) fft2d_trunc_kernel(Im
             float2 v[32];
 #pragma unroll
             for (int n = 0; n < 32; ++n) v[n] = sX[xtile_index<RX, C>(RX * n + rx, col)];
-            // columns read: the next image may be stored
-            if constexpr (C > 1) { if (next) cluster_arrive(); }
-            else __syncthreads();
+            if constexpr (C == 1) __syncthreads();              // columns read: the next image may be stored
             forward_trunc32<RX>(v, twX, rx, 1, coefX);
             float2* dst = p.out + img * (long long)(kModes * kModes) + rank * COLS + col;
 #pragma unroll
