@@ -1053,7 +1053,7 @@ int tfno_spectral_conv2d_static(long long bs, int DX, int DY, int K, int N, cons
     int rc = static_device_setup(device, &sd);
     if (rc != TFNO_OK) return rc;
     // every launch of this call must fit before the first one is enqueued: a refused call does nothing
-    if (!fft2d_fits(sd->dev, DX, DY) ||
+    if (!fft2d_fits(sd->dev) ||
         (long long)tile_smem_bytes(2, false, false, K, N > 128 ? 128 : N) > sd->dev.max_smem_optin)
         return TFNO_ERR_UNSUPPORTED;
     cudaStream_t st = static_cast<cudaStream_t>(stream);

@@ -141,7 +141,7 @@ struct ImageParams {
 };
 // DX, DY in {128, 256}; full-size side: 16-byte aligned base, even strides
 int launch_fft2d(const DeviceInfo& dev, int DX, int DY, const ImageParams& p, bool inverse, cudaStream_t st);
-bool fft2d_fits(const DeviceInfo& dev, int DX, int DY);      // the launches above need no more shared memory than the device gives
+bool fft2d_fits(const DeviceInfo& dev);      // no launch above needs more shared memory than the device gives
 
 #if defined(__CUDACC__)
 template <typename Params, typename Kernel>

@@ -125,15 +125,12 @@ TFNO_HD void fill_inverse_table32(float2* twI, int tid, int nthreads, float2 g, 
 // Folded form of the inverse table: W_DY^{-j1 (m'+32)} = W_DY^{-j1 m'} W_R^{-j1}, so
 //     C[m'] T[m'] + C[m'+32] T[m'+32] = T[m'] ( C[m'] + c C[m'+32] ),   c = inverse_fold_coef32(j1)
 // and a lane needs 32 table entries (m' < 32) plus one constant.
-// `centered` (true inverse only): the 64 given modes are -32..31; sample R*j2 + j1 of the result is
-// the ordinary one times e^{-2 pi i 32 (R*j2 + j1) / DY} = e^{-2 pi i j1 / R}, a per-lane constant.
 template <int R>
-TFNO_HD void fill_inverse_table32_folded(float2* twI, int tid, int nthreads, float2 g, bool conj, bool centered = false) {
+TFNO_HD void fill_inverse_table32_folded(float2* twI, int tid, int nthreads, float2 g, bool conj) {
     constexpr int DY = 32 * R;
     for (int i = tid; i < R * 32; i += nthreads) {
         const int j1 = i >> 5, m = i & 31;
-        const int e = centered ? (j1 * m - 32 * j1) & (DY - 1) : (j1 * m) & (DY - 1);
-        twI[tw_index<R>(j1, m)] = cmul(g, unit_root(e, DY, conj ? 1.0f : -1.0f));
+        twI[tw_index<R>(j1, m)] = cmul(g, unit_root((j1 * m) & (DY - 1), DY, conj ? 1.0f : -1.0f));
     }
 }
 template <int R>

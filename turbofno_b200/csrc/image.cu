@@ -91,8 +91,7 @@ int launch_image(const DeviceInfo& dev, const ImageParams& p, bool inverse, cuda
 
 }  // namespace
 
-bool fft2d_fits(const DeviceInfo& dev, int DX, int DY) {
-    (void)DX; (void)DY;
+bool fft2d_fits(const DeviceInfo& dev) {
     return (long long)fwd_image_smem_bytes<8, 8, 1>() <= dev.max_smem_optin;      // the largest of the instances below
 }
 

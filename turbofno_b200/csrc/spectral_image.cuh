@@ -65,24 +65,13 @@ TFNO_D void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.alig
 TFNO_D void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 // ---- two real rows through one complex transform ----
-template <int R, int LEN>
-TFNO_D void exchange_tail(float2 (&v)[16], int mask, bool up) {          // exchange_round_32 on 2*LEN live entries
-    float2 got[LEN];
-#pragma unroll
-    for (int j = 0; j < LEN; ++j) {
-        const float2 lo = v[j], hi = v[LEN + j];
-        v[j] = up ? hi : lo;
-        got[j] = shfl_xor2(up ? lo : hi, mask);
-    }
-#pragma unroll
-    for (int j = 0; j < LEN; ++j) v[j] = cadd(v[j], got[j]);
-}
-// z[n] = (a, b) sample R*n + r of two real signals.  On return lane r holds modes 64/R*r + j of a in va[j]
-// and of b in vb[j], both times 2.  Slots s and -s of the 32-point result are
+// Rows of 128 samples (R = 4; those of 256 go through fft256.cuh).  z[n] = (a, b) sample R*n + r of two real signals.
+// On return lane r holds modes 64/R*r + j of a in va[j] and of b in vb[j], both times 2.  Slots s and -s of the 32-point result are
 // separated together with s + 16 and 16 - s, which rounds 1 and 2 reduce to two values per signal: a closed
 // set of four registers in, four out (the pairing s <-> -s also holds on rotated lanes: 16 = -16).
 template <int R>
 TFNO_D void forward_trunc32_real2(float2 (&z)[32], const float2* __restrict__ twF, int r, float2 coef, float2 (&va)[16], float2 (&vb)[16]) {
+    static_assert(R == 4, "two exchange rounds leave sixteen modes of each signal");
     fft32<-1>(z, lane_rotated32<R>(r) ? -1.0f : 1.0f);
     auto table = [&](int s) { return twF[tw_index<R>(r, s)]; };
 #pragma unroll
@@ -126,10 +115,6 @@ TFNO_D void forward_trunc32_real2(float2 (&z)[32], const float2* __restrict__ tw
             va[16 - j] = cadd(w[0][1], k[0][1]);
             vb[16 - j] = cadd(w[1][1], k[1][1]);
         }
-    }
-    if constexpr (R >= 8) {
-        exchange_tail<R, 8>(va, R >> 3, (r & (R >> 3)) != 0);
-        exchange_tail<R, 8>(vb, R >> 3, (r & (R >> 3)) != 0);
     }
 }
 
@@ -284,7 +269,7 @@ __global__ void __launch_bounds__(64 * CLS, 8 / CLS) ifft2d_pad_kernel(ImagePara
     const int part = blockIdx.x % PARTS;                         // the grid is a multiple of PARTS
     fill_inverse_table32_folded<RY>(twY, tid, T, make_float2(1.f, 0.f), INVERSE);
     for (int i = tid; i < CLS * 32; i += T) {                    // rows part*CLS .. of fill_inverse_table32_folded<RX>
-        const int j1 = part * CLS + (i >> 5), m = i & 31;
+        const int j1 = part * CLS + (i >> 5), m = i & 31;        // modes -32..31: times e^{-2 pi i j1 / RX}
         const int e = (INVERSE && p.centered_x) ? (j1 * m - 32 * j1) & (32 * RX - 1) : (j1 * m) & (32 * RX - 1);
         twX[i] = cmul(p.gain, unit_root(e, 32 * RX, INVERSE ? 1.0f : -1.0f));
     }
