@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(64 * RX / C, 8 * C / RX) fft2d_trunc_kernel(Im
                                 const float2 y = w[slot16((16 - 2 * d - e) & 15)];
                                 return l == 0 ? make_float2(z.x + y.x, z.y - y.y) : make_float2(z.y + y.y, y.x - z.x);
                             });
-                        combine256(f, twY + 6 * (2 * r + e), out[e]);
+                        combine256(f, twY, 2 * r + e, out[e]);
                     }
                     if (C > 1 && i0 == 0 && l == 0) cluster_wait();
 #pragma unroll
