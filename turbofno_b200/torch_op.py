@@ -79,6 +79,38 @@ def _define(schema, kernel, fake):
     return getattr(torch.ops.turbofno_b200, name).default
 
 
+class _Operator:
+    """An operator as callers of this module hold it: called like a function, and open to the registrations that
+    torch.library offers for custom operators."""
+
+    def __init__(self, overload):
+        self._overload = overload
+
+    def __call__(self, *args, **kwargs):
+        return self._overload(*args, **kwargs)
+
+    def __getattr__(self, name):
+        return getattr(self.__dict__["_overload"], name)
+
+    def __repr__(self):
+        return "<operator %s>" % self._overload.name()
+
+    def register_kernel(self, device_types, func=None):
+        return torch.library.register_kernel(self._overload, device_types, func)
+
+    def register_fake(self, func):
+        return torch.library.register_fake(self._overload, func, allow_override=True)
+
+    def register_autocast(self, device_type, cast_inputs):
+        return torch.library.register_autocast(self._overload, device_type, cast_inputs)
+
+    def register_vmap(self, func=None):
+        return torch.library.register_vmap(self._overload, func)
+
+    def register_torch_dispatch(self, torch_dispatch_class, func=None):
+        return torch.library.register_torch_dispatch(self._overload, torch_dispatch_class, func)
+
+
 def _differentiable(name, backward, setup_context):
     torch.library.register_autograd("turbofno_b200::" + name, backward, setup_context=setup_context, lib=_lib)
 
@@ -97,7 +129,7 @@ def _conv1d_fake(x, w):
     return x.new_empty((x.shape[0], w.shape[1], x.shape[2]))
 
 
-spectral_conv1d = _define("spectral_conv1d(Tensor x, Tensor w) -> Tensor", _conv1d_cuda, _conv1d_fake)
+spectral_conv1d = _Operator(_define("spectral_conv1d(Tensor x, Tensor w) -> Tensor", _conv1d_cuda, _conv1d_fake))
 
 
 def _conv2d_cuda(x, w, x_modes_centered=False):
@@ -114,7 +146,7 @@ def _conv2d_fake(x, w, x_modes_centered=False):
     return x.new_empty((x.shape[0], w.shape[1], x.shape[2], x.shape[3]))
 
 
-spectral_conv2d = _define("spectral_conv2d(Tensor x, Tensor w, bool x_modes_centered=False) -> Tensor", _conv2d_cuda, _conv2d_fake)
+spectral_conv2d = _Operator(_define("spectral_conv2d(Tensor x, Tensor w, bool x_modes_centered=False) -> Tensor", _conv2d_cuda, _conv2d_fake))
 
 
 def _truncated_spectrum(t):
