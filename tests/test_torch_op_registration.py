@@ -1,7 +1,10 @@
-"""What callers may do with the operators besides calling them: register further kernels and rules."""
+"""What callers may do with the operators besides calling them: register further kernels and rules, and learn that a
+gradient has no derivative of its own."""
 import os
 import subprocess
 import sys
+
+import pytest
 
 from util import ROOT
 
@@ -37,3 +40,33 @@ print("ok")
 def test_operators_take_further_registrations():
     out = subprocess.run([sys.executable, "-c", PROGRAM], cwd=ROOT, capture_output=True, text=True, timeout=300, env=dict(os.environ, PYTHONPATH=ROOT))
     assert out.stdout.strip() == "ok", out.stderr[-2000:]
+
+
+@pytest.mark.parametrize("which", ["grad_y", "x", "w"])
+def test_backward_operator_refuses_to_be_recorded(which):
+    import torch
+
+    from turbofno_b200 import torch_op
+
+    t = {"grad_y": torch.zeros((1, 64, 128), dtype=torch.complex64), "x": torch.zeros((1, 64, 128), dtype=torch.complex64),
+         "w": torch.zeros((64, 64), dtype=torch.complex64)}
+    t[which].requires_grad_(True)
+    with pytest.raises(RuntimeError, match="no derivative"):
+        torch_op._backward_cuda(t["grad_y"], t["x"], t["w"], False, True, True)
+
+
+@pytest.mark.gpu
+def test_backward_operator_called_directly(cuda):
+    import torch
+
+    from test_gpu_backward import _reference, _tensors
+
+    x, w, gy = _tensors(2, 64, 64, (128,), False, False)
+    op = torch.ops.turbofno_b200.spectral_conv_backward
+    got, want = op(gy, x, w, False, True, True), _reference(x, w, gy, False)[1:]
+    for a, b in zip(got, want):
+        assert ((a - b).norm() / b.norm()).item() <= 4e-6          # as in the gradient tests
+    with pytest.raises(RuntimeError, match="no derivative"):
+        op(gy, x.requires_grad_(True), w, False, True, True)
+    with torch.no_grad():
+        op(gy, x, w, False, True, True)

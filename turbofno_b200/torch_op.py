@@ -170,6 +170,8 @@ def _aligned(t):
 
 
 def _backward_cuda(grad_y, x, w, x_modes_centered, need_x, need_w):
+    if torch.is_grad_enabled() and (grad_y.requires_grad or x.requires_grad or w.requires_grad):
+        raise RuntimeError("spectral_conv_backward has no derivative formula: differentiate the layer with create_graph=True")
     rank = x.dim() - 2
     grad_y, x, w = _aligned(grad_y), _aligned(x), _aligned(w)
     plan = _plan(rank, x.shape[0], x.shape[-1], x.shape[1], w.shape[1], x.shape[2] if rank == 2 else None, x.device.index,
