@@ -10,6 +10,7 @@ from util import ROOT
 
 # in a process of its own: the registrations stay for good
 PROGRAM = """
+import copy
 import torch
 from turbofno_b200 import torch_op
 
@@ -33,6 +34,10 @@ for op, signal in ((torch_op.spectral_conv1d, (128,)), (torch_op.spectral_conv2d
     assert torch.equal(y, torch.stack([layer(a, w) for a in x]))
     op.register_autocast("cpu", torch.complex64)
     assert "spectral_conv" in repr(op) and op._schema.returns
+    # held by a module, copied with it, traced
+    assert copy.deepcopy({"op": op})["op"] is op and torch.equal(copy.copy(op)(x[0], w), y[0])
+    traced = torch.compile(lambda a, b: op(a, b) * 2, backend="eager", fullgraph=True)
+    assert torch.equal(traced(x[0], w), y[0] * 2)
 print("ok")
 """
 
