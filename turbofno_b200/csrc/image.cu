@@ -36,10 +36,12 @@ int launch_forward(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st)
 }
 template <int RX, int RY, bool REAL>
 int launch_forward_split(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st) {
-    // Few images: a cluster of CTAs of 64 rows per image (8 images of 128 x 256: 8.4 us against 10.9 with one CTA
-    // each, 16 of 256 x 256: 9.4 against 17.3).  With more than two such CTAs per SM the exchange through
-    // distributed shared memory costs more than the parallelism gives (512 images of 256 x 256: 98 against 73 us;
-    // all four with rows on the 32-point transform).
+    // Few images: a cluster of CTAs of 64 rows per image, while two such CTAs per SM cover them.  Kernel times of the
+    // cluster against one CTA per image, us: 8 images of 128 x 256 7.3 / 9.2, 16 of 256 x 256 9.2 / 16.7; at the line 72 of
+    // 256 x 256 15.6 / 18.3 and of 256 x 128 14.6 / 15.7, 144 of 128 x 256 13.4 / 13.4 and of 128 x 128 11.9 / 10.9 (real samples
+    // 24 % better to 14 % worse).  Beyond it the exchange through distributed shared memory costs as much as the parallelism
+    // gives: 144 of 256 x 256 27.0 / 23.3, 512 68.8 / 70.2, 512 of 256 x 128 63.2 / 54.1; just above a full wave of one-CTA images
+    // (148 of DX = 256, 296 of DX = 128) the cluster still wins: 152 of 256 x 256 28.6 / 36.9, 304 47.6 / 54.2.
     if (p.nimg * (RX / 2) <= 2LL * dev.sms) return launch_forward<RX, RY, RX / 2, REAL>(dev, p, st);
     return launch_forward<RX, RY, 1, REAL>(dev, p, st);
 }

@@ -12,7 +12,11 @@ __global__ void __launch_bounds__(256) conjugate_kernel(const float2* __restrict
     }
 }
 
-// rows i per CTA: the tile that pads the rows least, the larger one of two equals
+// rows i per CTA: the tile that pads the rows least, the larger one of two equals.  At 4096 modes (64 -> 64 and 32 -> 128
+// channels, 1 to 48 rows, every tile forced in turn) that is the fastest one up to 36 rows: 1 row 33 us (tile of 8: 42), 8 rows 45
+// (4: 54, 12: 54), 12 rows 56 (8: 75, 16: 71), 16 rows 73 (8: 76, 12: 94), 20 rows 94 with 12 (8: 114, 16: 132), 32 rows 125 with 16
+// (12: 144); 48 rows 192 with 16 against 184 with 12.  With the 64 modes of a 1D layer and so few rows the grid is a handful of CTAs
+// and the smallest tile is the fastest (16 rows: 10.8 us with 4, 20.6 with 16); the rule does not know that.
 int tile_rows(int I) {
     int best = 16;
     long long padded = (I + 15LL) / 16 * 16;
