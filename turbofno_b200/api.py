@@ -45,6 +45,8 @@ def _stream_ptr(stream=None, device=None):
 
 
 def _capturing(device, stream=None):
+    if stream is None and device.index == torch.cuda.current_device():
+        return torch.cuda.is_current_stream_capturing()
     with torch.cuda.stream(stream if stream is not None else torch.cuda.current_stream(device)):
         return torch.cuda.is_current_stream_capturing()
 
