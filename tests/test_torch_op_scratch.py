@@ -12,8 +12,9 @@ class _RecordingPlan:
         self._scratch = SpectralConv._scratch
         self.call_scratch = lambda device, stream=None: SpectralConv.call_scratch(self, device, stream)
 
-    def __call__(self, x, w, y=None, workspace=None, stream=None):
+    def _launch(self, x, w, y, workspace, stream=None):
         self.calls.append((y, workspace))
+        return y
 
 
 @pytest.mark.parametrize("kernel,x_shape,w_shape", [("_conv1d_cuda", (2, 8, 128), (8, 64, 64)), ("_conv2d_cuda", (2, 8, 128, 128), (8, 64))])
@@ -33,6 +34,16 @@ def test_every_operator_call_brings_its_own_scratch(monkeypatch, kernel, x_shape
     plan.workspace_bytes = 0
     getattr(torch_op, kernel)(x, w)
     assert plan.calls[-1][1] is None
+
+
+def test_operands_on_different_devices_are_refused(monkeypatch):
+    import torch
+
+    from turbofno_b200 import torch_op
+
+    monkeypatch.setattr(torch_op, "_plan", lambda *a, **k: _RecordingPlan(0))
+    with pytest.raises(ValueError):
+        torch_op._conv1d_cuda(torch.zeros((1, 8, 128), dtype=torch.complex64), torch.zeros((8, 64), dtype=torch.complex64, device="meta"))
 
 
 @pytest.mark.gpu

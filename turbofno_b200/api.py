@@ -224,15 +224,22 @@ class SpectralConv:
         self._check_call(x, w, y, workspace)
         if y is None:
             y = torch.empty(self.out_shape(), dtype=torch.complex64, device=x.device)
-        if self._optional_ws:
-            ws = workspace
-            if ws is None and not _capturing(x.device, stream):
+        ws = workspace
+        if ws is None:
+            if not self._optional_ws:
+                ws = self.workspace(x.device)
+            elif not _capturing(x.device, stream):
                 ws = self.call_scratch(x.device, stream)
+        return self._launch(x, w, y, ws, stream)
+
+    def _launch(self, x, w, y, ws, stream=None):
+        """The call itself, on operands that fit the plan (scratch that need not be there may be None or short)."""
+        st = _stream_ptr(stream, x.device)
+        if self._optional_ws:
             nbytes = 0 if ws is None else ws.numel() * ws.element_size()
-            check(self.lib.tfno_exec_scratch(self._plan, _ptr(x), _ptr(w), _ptr(y), _ptr(ws), nbytes, _stream_ptr(stream, x.device)), "tfno_exec_scratch")
-            return y
-        ws = workspace if workspace is not None else self.workspace(x.device)
-        check(self.lib.tfno_exec(self._plan, _ptr(x), _ptr(w), _ptr(y), _ptr(ws), _stream_ptr(stream, x.device)), "tfno_exec")
+            check(self.lib.tfno_exec_scratch(self._plan, _ptr(x), _ptr(w), _ptr(y), _ptr(ws), nbytes, st), "tfno_exec_scratch")
+        else:
+            check(self.lib.tfno_exec(self._plan, _ptr(x), _ptr(w), _ptr(y), _ptr(ws), st), "tfno_exec")
         return y
 
     def exec_real(self, x, w, y=None, stream=None):

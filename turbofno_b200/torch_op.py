@@ -49,9 +49,11 @@ def _plan(rank, bs, DY, K, N, DX, device, per_mode=False, centered=False):
 
 def _run_layer(plan, x, w, y):
     """One layer with scratch of its own.  Every caller of a shape shares its plan, on any stream and thread, and the
-    plan's own buffer serves one stream and one thread at a time: two calls in flight would write the same spectra."""
-    plan(x, w, y=y, workspace=plan.call_scratch(x.device))
-    return y
+    plan's own buffer serves one stream and one thread at a time: two calls in flight would write the same spectra.
+    The plan is made from the shapes of x and w, whose types the operator has checked."""
+    if w.device != x.device:
+        raise ValueError("w is on %s, x on %s" % (w.device, x.device))
+    return plan._launch(x, w, y, plan.call_scratch(x.device))
 
 
 def _check(x, w, rank):
