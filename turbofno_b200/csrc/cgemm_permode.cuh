@@ -11,18 +11,21 @@
 //
 // The reference contracts with one K x N matrix shared by all modes
 // (fusion_variants/1D_E_baseline/cgemm.cuh:42-43, B[k + n*K]); per-mode matrices are the extension its
-// README names as the FNO use case.  The operands are interleaved mode-fastest in memory, so the modes go
-// on the LANES: a CTA takes eight adjacent modes (64 contiguous bytes of every row of P, Q and O), a warp
-// 8 modes x 4 groups of TI rows i, and 8 columns j; eight warps cover 64 columns.  Slabs of P and Q for four r travel by 16-byte asynchronous copies through a ring
-// of kPmStages.  FP32 FMA; a thread keeps TI x 8 complex sums, and per r its warp reads TI * 256 + 8 * 64 bytes
-// of shared memory for TI * 32 FMA instructions.
+// README names as the FNO use case.
 //
-// What bounds it (2D, 4096 modes, K = N = 64): up to 8 rows the 134 MB of weights (35 us at 1 row, 44 at 8; 20 us at
-// copy speed); beyond that issue slots, 70 % used, 85 % of them FMA (16 rows 71 us, 32 rows 123 us; 30 and 60 us at the
-// full FMA rate).  The four-modes-by-32-rows tile it replaces took 193 us at any batch up to 32.  Two CTAs per SM:
-// one of 512 threads (32 rows) has nothing to cover its first loads and its stores with (137 us at 32 rows, 104
-// against 92 at 20).  Packed two-wide FMAs take the same pipe cycles plus the moves that pair their operands
-// (75 against 72 us at 16 rows).
+// On the tensor cores through mma.sync m16n8k8 (tf32), every FP32 value split into two tf32 parts and three products
+// kept (hi*hi + lo*hi + hi*lo).  Fragments live in registers, so the operands are split on the way from the ring to the
+// multiplier, each value once; tcgen05 would want both parts of every matrix written back to shared memory, one mode
+// at a time, for products of 64 x 64 x (a few rows) each.  The tensor cores truncate when they accumulate, so a chain
+// covers the eight terms of one step only and the steps are added in FP32: closer to the exact sums than the chains
+// of FP32 FMAs this replaces (whole layer against 64-bit results: 1D training step 2.4e-7 -> 2.1e-7, real 2D field 2.9e-7 -> 2.5e-7).
+//
+// What bounds it (2D, 4096 modes, K = N = 64; us, with the FP32 kernel before it): layer of 1 row 36 (36), 16 rows 51 (73), 20
+// rows 66 (94), 64 rows 172 (242); gradient of W at 16 rows 63 (84), 20 rows 78 (97).  1D, 64 modes: 16 rows 7 (21), 512 rows
+// 28 (37).  Up to 8 rows the 134 MB of weights (20 us at copy speed); beyond that the multiplier, 55 % busy (20 rows: 33 us at
+// 512 multiply-adds a cycle), with the latencies of a step (load, split, chain of six) behind four warps per scheduler.
+// Tried: persistent CTAs whose ring runs on across tiles (79 us at 20 rows: 3.5 tiles per CTA are dealt worse than by the
+// hardware), tiles of 16 columns with three CTAs per SM (71), all loads of a step ahead of its products (68).
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -30,37 +33,18 @@
 
 namespace tfno {
 
-constexpr int kPmModes = 8;            // adjacent modes per CTA
-constexpr int kPmCols = 64;            // columns j per CTA: eight warps of 8
-constexpr int kPmThreads = 4 * kPmCols;
-constexpr int kPmSlab = 4;             // values of r per ring stage
-constexpr int kPmStages = 4;
+constexpr int kPmCols = 32;            // columns j per CTA
+constexpr int kPmThreads = 256;
+constexpr int kPmTerms = 8;            // values of r per ring stage = depth of a matrix instruction
+constexpr int kPmStages = 3;
+constexpr int kPmSumTile = 64;         // gradient of shared weights: rows i and columns j per CTA
+constexpr int kPmSumTerms = 4;         // and r per ring stage (each eight modes deep)
 
-struct PerModeParams {
-    int I, J;                          // J a multiple of 64
-    long long red, modes;              // terms of the sum; modes: a multiple of 8
-    const float2* p; long long p_sr, p_si;                 // P[r*p_sr + i*p_si + m]
-    const float2* q; long long q_sr, q_sj, q_sm;           // Q[r*q_sr + j*q_sj + m*q_sm]
-    float2* o; long long o_si, o_sj, o_sm;                 // O[i*o_si + j*o_sj + m*o_sm]
-    float2* partial;                   // [splits][I][J][modes] (sum_modes: [splits][I][J]) when splits > 1 or sum_modes
-    float2 alpha;
-    float2 alpha0;                     // factor of the modes m % 64 == 0 (real fields: the ky = 0 column)
-    int splits;                        // r is dealt to this many CTAs in runs of split_len
-    long long split_len;
-    int q_vec;                         // Q may be copied 16 bytes (two modes) at a time
-};
+template <int NT> __host__ __device__ constexpr int pm_stage_bytes() { return kPmTerms * (8 * NT + kPmCols) * kPmModes * 8; }
+template <int NT> __host__ __device__ constexpr int pm_smem_bytes() { return kPmStages * pm_stage_bytes<NT>(); }
+constexpr int kPmSumStageBytes = 2 * kPmSumTile * kPmSumTerms * kPmModes * 8;
+constexpr int kPmSumSmemBytes = kPmStages * kPmSumStageBytes;
 
-// The launches (permode.cu).  `partial` must hold permode_partial_bytes() when that is not zero.
-enum PermodeKind { PERMODE_APPLY, PERMODE_APPLY_CONJ, PERMODE_GRAD, PERMODE_GRAD_SHARED };
-size_t permode_partial_bytes(const DeviceInfo& dev, const PerModeParams& p, PermodeKind kind);
-int launch_permode(const DeviceInfo& dev, PerModeParams p, PermodeKind kind, cudaStream_t st);
-// dst[k*N + n] = conj(w[k*sk + n*sn])
-int launch_conjugate(const DeviceInfo& dev, const float2* w, long long sk, long long sn, int K, int N, float2* dst, cudaStream_t st);
-
-template <int TI> __host__ __device__ constexpr size_t pm_stage_elems() { return (size_t)kPmSlab * (4 * TI + kPmCols) * kPmModes; }
-template <int TI> __host__ __device__ constexpr size_t pm_smem_bytes() { return kPmStages * pm_stage_elems<TI>() * sizeof(float2); }
-
-#if defined(__CUDACC__)
 // copies `bytes` (16 or 8), or zeros when !live (the source is not read then)
 __device__ __forceinline__ void pm_copy16(uint32_t dst, const void* src, bool live) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
@@ -68,19 +52,74 @@ __device__ __forceinline__ void pm_copy16(uint32_t dst, const void* src, bool li
 __device__ __forceinline__ void pm_copy8(uint32_t dst, const void* src, bool live) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(live ? 8 : 0) : "memory");
 }
+__device__ __forceinline__ float4 pm_load16(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ float2 pm_load8(uint32_t addr) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
+    return v;
+}
+// v = hi + lo, hi rounded to tf32 (cvt.rna.tf32 is five instructions here, for the sake of infinities and NaNs, which this
+// passes on as infinities and NaNs in hi or lo).  The multiplier drops the low 13 bits of an operand: at most the last of
+// lo's 12 bits.
+__device__ __forceinline__ void pm_split(float v, uint32_t& hi, uint32_t& lo) {
+    hi = (__float_as_uint(v) + 0x1000u) & 0xffffe000u;
+    lo = __float_as_uint(v - __uint_as_float(hi));
+}
+__device__ __forceinline__ void pm_mma(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+__device__ __forceinline__ void pm_mma_first(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {      // d = a b
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(0.f));
+}
+// The two parts of a fragment of one matrix (real or imaginary).  Q is the 16-row operand: lane 4 g + t holds rows g, g + 8 at
+// terms t, t + 4; P the 8-column one: column g at terms t, t + 4.
+struct PmFragQ { uint32_t hi[4], lo[4]; };
+struct PmFragP { uint32_t hi[2], lo[2]; };
+__device__ __forceinline__ PmFragP pm_negated(const PmFragP& f) {
+    PmFragP n;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) { n.hi[i] = f.hi[i] ^ 0x80000000u; n.lo[i] = f.lo[i] ^ 0x80000000u; }
+    return n;
+}
+// sum += P conj?(Q) over eight terms, the small products first
+struct PmSum { float2 re[2], im[2]; };             // a fragment of results: lane 4 g + t holds columns 2 t, 2 t + 1 of rows g, g + 8
+template <bool CONJ_Q>
+__device__ __forceinline__ void pm_step(PmSum& sum, const PmFragQ& qr, const PmFragQ& qi, const PmFragP& pr, const PmFragP& pi, const PmFragP& n) {
+    // Q: re = Pr Qr - Pi Qi, im = Pi Qr + Pr Qi, n = -Pi;  conj(Q): re = Pr Qr + Pi Qi, im = Pi Qr - Pr Qi, n = -Pr
+    const PmFragP &re2 = CONJ_Q ? pi : n, &im2 = CONJ_Q ? n : pr;
+    float a[4], b[4];
+    pm_mma_first(a, qr.lo, pr.hi);  pm_mma_first(b, qr.lo, pi.hi);
+    pm_mma(a, qi.lo, re2.hi); pm_mma(b, qi.lo, im2.hi);
+    pm_mma(a, qr.hi, pr.lo);  pm_mma(b, qr.hi, pi.lo);
+    pm_mma(a, qi.hi, re2.lo); pm_mma(b, qi.hi, im2.lo);
+    pm_mma(a, qr.hi, pr.hi);  pm_mma(b, qr.hi, pi.hi);
+    pm_mma(a, qi.hi, re2.hi); pm_mma(b, qi.hi, im2.hi);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        sum.re[h] = __fadd2_rn(sum.re[h], make_float2(a[2 * h], a[2 * h + 1]));
+        sum.im[h] = __fadd2_rn(sum.im[h], make_float2(b[2 * h], b[2 * h + 1]));
+    }
+}
 
+// ---- one product per mode ----
+// A CTA takes eight adjacent modes, 32 columns j and 8 NT rows i, a warp one mode of them.  Stages of eight r travel by
+// 16-byte asynchronous copies through a ring of kPmStages; the 16-byte pieces of a line are permuted by r % 4, so that the
+// sixteen lanes of a half-warp (four lines, four r) meet two by two.  The results leave through shared memory, as whole
+// 64-byte lines.
 // CONJ_Q: Q enters conjugated.  CONJ_O: the sum is conjugated before it is scaled (conj(P) Q = conj(P conj(Q))).
-// SUM_MODES: the eight modes are added up; results go to `partial`.
-template <int TI, bool CONJ_Q, bool CONJ_O, bool SUM_MODES>
-__global__ void __launch_bounds__(kPmThreads, 2) cgemm_permode_kernel(PerModeParams p) {
-    constexpr int THREADS = kPmThreads, ROWS = 4 * TI, LINES = ROWS + kPmCols;
-    static_assert(4 * kPmSlab * ROWS <= THREADS && kPmSlab * kPmCols == THREADS, "a slab is one 16-byte piece of P and kPmSlab of Q per thread");
+template <int NT, bool CONJ_Q, bool CONJ_O>
+__global__ void __launch_bounds__(kPmThreads, NT == 1 ? 3 : 2) cgemm_permode_kernel(PerModeParams p) {
+    constexpr int ROWS = 8 * NT, LINES = ROWS + kPmCols, STAGE = pm_stage_bytes<NT>(), MT = kPmCols / 16;
+    static_assert(ROWS * kPmCols * 64 <= pm_smem_bytes<NT>(), "the results pass through the ring");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2* ring = reinterpret_cast<float2*>(smem_raw);          // [stage][slab][ROWS + 64][8 modes]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m = lane & 7, ig = lane >> 3;
-    const int wj = warp;
-    // CTAs that differ only in their rows i are neighbours: they read the same Q, which is then served by the L2
+    // CTAs that differ only in their rows i or columns j are neighbours: they share Q or P, which the L2 then serves
     const int iblocks = (p.I + ROWS - 1) / ROWS, jblocks = p.J / kPmCols;
     long long item = blockIdx.x;
     const int i0 = (int)(item % iblocks) * ROWS; item /= iblocks;
@@ -89,115 +128,206 @@ __global__ void __launch_bounds__(kPmThreads, 2) cgemm_permode_kernel(PerModePar
     const long long m0 = item * kPmModes;
     const long long r0 = split * p.split_len;
     const long long r1 = (r0 + p.split_len < p.red) ? r0 + p.split_len : p.red;
-    const int slabs = r1 > r0 ? (int)((r1 - r0 + kPmSlab - 1) / kPmSlab) : 0;
-    const uint32_t ring0 = (uint32_t)__cvta_generic_to_shared(ring);
+    const int terms = r1 > r0 ? (int)(r1 - r0) : 0, steps = (terms + kPmTerms - 1) / kPmTerms;
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem_raw);
 
-    // A slab is 4 terms x (ROWS + 64) lines of four 16-byte pieces (two modes each).  Every thread keeps its
-    // piece and line for good and one pointer per operand that moves on by a slab: the address arithmetic of a
-    // fresh decomposition per copy took as many issue slots as the FMAs.
-    const int piece = tid & 3;
-    const int p_line = (tid >> 2) % ROWS, p_rr = (tid >> 2) / ROWS;         // p_rr < kPmSlab for tid < 16 * ROWS <= THREADS
-    const bool p_row = p_rr < kPmSlab && i0 + p_line < p.I;
-    const float2* p_src = p.p + (p_row ? (r0 + p_rr) * p.p_sr + (long long)(i0 + p_line) * p.p_si + m0 + 2 * piece : 0);
-    const uint32_t p_dst = ring0 + (uint32_t)((p_rr * LINES + p_line) * kPmModes + 2 * piece) * 8u;
-    const int q_line = tid >> 2;                                            // of all four terms
-    const float2* q_src = p.q + r0 * p.q_sr + (long long)(j0 + q_line) * p.q_sj + m0 + 2 * piece;
-    const uint32_t q_dst = ring0 + (uint32_t)((ROWS + q_line) * kPmModes + 2 * piece) * 8u;
-    constexpr uint32_t STAGE = (uint32_t)(pm_stage_elems<TI>() * sizeof(float2));
-    auto fetch = [&](int slab) {
-        if (slab < slabs) {
-            const uint32_t stage = (uint32_t)(slab % kPmStages) * STAGE;
-            const int left = (int)(r1 - r0) - slab * kPmSlab;               // terms from this slab on
-            if (p_rr < kPmSlab) pm_copy16(p_dst + stage, p_row && p_rr < left ? p_src : p.p, p_row && p_rr < left);
-            p_src += p_row ? kPmSlab * p.p_sr : 0;
+    // copies: warp w brings the lines of term w of a stage, eight lines (512 bytes) at a time.  A copy of no bytes (rows
+    // past I, terms past the end) fills with zeros and does not look at its source.
+    const int c_line = lane >> 2, c_piece = lane & 3;
+    const uint32_t c_dst = ring + (uint32_t)((warp * LINES + c_line) * 64 + ((c_piece ^ (warp & 3)) << 4));
+    const float2* p_src = p.p + (r0 + warp) * p.p_sr + (long long)(i0 + c_line) * p.p_si + m0 + 2 * c_piece;
+    const float2* q_src = p.q + (r0 + warp) * p.q_sr + (long long)(j0 + c_line) * p.q_sj + m0 + 2 * c_piece;
+    auto fetch = [&](int step) {
+        if (step < steps) {
+            const uint32_t stage = (uint32_t)(step % kPmStages) * STAGE, dst = c_dst + stage;
+            const bool live = step * kPmTerms + warp < terms;
+#pragma unroll
+            for (int l = 0; l < NT; ++l) pm_copy16(dst + l * 512, p_src + 8 * l * p.p_si, live && i0 + 8 * l + c_line < p.I);
             if (p.q_vec) {
 #pragma unroll
-                for (int it = 0; it < kPmSlab; ++it) {
-                    const bool live = it < left;
-                    pm_copy16(q_dst + stage + (uint32_t)(it * LINES * kPmModes) * 8u, live ? q_src + it * p.q_sr : p.q, live);
-                }
-                q_src += kPmSlab * p.q_sr;
+                for (int l = 0; l < kPmCols / 8; ++l) pm_copy16(dst + (ROWS + 8 * l) * 64, q_src + 8 * l * p.q_sj, live);
             } else {
-                const long long rs = r0 + (long long)slab * kPmSlab;
+                // modes that are not adjacent, or lines on odd addresses: eight bytes at a time
+                const float2* term = p.q + (r0 + (long long)step * kPmTerms + warp) * p.q_sr;
 #pragma unroll 1
-                for (int i = tid; i < kPmSlab * kPmCols * 8; i += THREADS) {
-                    const int mode = i & 7, line = (i >> 3) % kPmCols, rr = (i >> 3) / kPmCols;
-                    const bool live = rr < left;
-                    const float2* src = live ? p.q + (rs + rr) * p.q_sr + (long long)(j0 + line) * p.q_sj + (m0 + mode) * p.q_sm : p.q;
-                    pm_copy8(ring0 + stage + (uint32_t)((rr * LINES + ROWS + line) * kPmModes + mode) * 8u, src, live);
+                for (int i = lane; i < kPmCols * 8; i += 32) {
+                    const int mode = i & 7, line = i >> 3;
+                    const uint32_t at = (uint32_t)((warp * LINES + ROWS + line) * 64 + (((mode >> 1) ^ (warp & 3)) << 4) + (mode & 1) * 8);
+                    pm_copy8(ring + stage + at, term + (long long)(j0 + line) * p.q_sj + (m0 + mode) * p.q_sm, live);
                 }
             }
+            p_src += kPmTerms * p.p_sr;
+            q_src += kPmTerms * p.q_sr;
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
 
-    float2 acc[TI][8];
+    const int g = lane >> 2, t = lane & 3;
+    const uint32_t frag = ring + (uint32_t)((t * LINES + g) * 64 + (((warp >> 1) ^ t) << 4) + (warp & 1) * 8);
+    constexpr uint32_t HALF = 4 * LINES * 64;                    // terms t + 4
+    PmSum acc[NT][MT];
 #pragma unroll
-    for (int t = 0; t < TI; ++t)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[t][j] = make_float2(0.f, 0.f);
+    for (int i = 0; i < NT * MT; ++i) (&acc[0][0])[i] = PmSum{};
 #pragma unroll
     for (int s = 0; s < kPmStages - 1; ++s) fetch(s);
-    for (int slab = 0; slab < slabs; ++slab) {
+#pragma unroll 1
+    for (int step = 0; step < steps; ++step) {
         asm volatile("cp.async.wait_group %0;" ::"n"(kPmStages - 2) : "memory");
-        __syncthreads();                          // this slab has arrived; everybody has left the stage refilled next
-        fetch(slab + kPmStages - 1);
-        const float2* st = ring + (slab % kPmStages) * pm_stage_elems<TI>();
+        __syncthreads();                          // this stage has arrived; everybody has left the one refilled next
+        fetch(step + kPmStages - 1);
+        const uint32_t st = frag + (uint32_t)(step % kPmStages) * STAGE;
+        PmFragQ qr[MT], qi[MT];
 #pragma unroll
-        for (int rr = 0; rr < kPmSlab; ++rr) {
-            const float2* line = st + rr * LINES * kPmModes + m;
-            float2 pv[TI];
+        for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-            for (int t = 0; t < TI; ++t) pv[t] = line[(t * 4 + ig) * kPmModes];
+            for (int i = 0; i < 4; ++i) {
+                const float2 v = pm_load8(st + (ROWS + 16 * mt + 8 * (i & 1)) * 64 + (i >> 1) * HALF);
+                pm_split(v.x, qr[mt].hi[i], qr[mt].lo[i]);
+                pm_split(v.y, qi[mt].hi[i], qi[mt].lo[i]);
+            }
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float2 qv = line[(ROWS + wj * 8 + j) * kPmModes];
+        for (int nt = 0; nt < NT; ++nt) {
+            PmFragP pr, pi;
 #pragma unroll
-                for (int t = 0; t < TI; ++t) {
-                    float2& a = acc[t][j];
-                    if (CONJ_Q) {
-                        a.x = fmaf(pv[t].x, qv.x, fmaf(pv[t].y, qv.y, a.x));
-                        a.y = fmaf(pv[t].y, qv.x, fmaf(-pv[t].x, qv.y, a.y));
-                    } else {
-                        a.x = fmaf(pv[t].x, qv.x, fmaf(-pv[t].y, qv.y, a.x));
-                        a.y = fmaf(pv[t].x, qv.y, fmaf(pv[t].y, qv.x, a.y));
-                    }
-                }
+            for (int i = 0; i < 2; ++i) {
+                const float2 v = pm_load8(st + nt * 512 + i * HALF);
+                pm_split(v.x, pr.hi[i], pr.lo[i]);
+                pm_split(v.y, pi.hi[i], pi.lo[i]);
+            }
+            const PmFragP n = pm_negated(CONJ_Q ? pr : pi);
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) pm_step<CONJ_Q>(acc[nt][mt], qr[mt], qi[mt], pr, pi, n);
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+
+    // results: line (i, j) of eight modes, the 8-byte modes permuted by a key of the line so that a half-warp (four j, four
+    // pairs of i) covers all banks
+    auto key = [](int i, int j) { return ((j >> 1) & 1) | (((i >> 1) & 3) << 1); };
+    float2* out = reinterpret_cast<float2*>(smem_raw);
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int i = 8 * nt + 2 * t + (e & 1), j = 16 * mt + g + 8 * (e >> 1);
+                const PmSum& s = acc[nt][mt];
+                const float re = (e & 1) ? s.re[e >> 1].y : s.re[e >> 1].x, im = (e & 1) ? s.im[e >> 1].y : s.im[e >> 1].x;
+                out[(i * kPmCols + j) * kPmModes + (warp ^ key(i, j))] = make_float2(re, CONJ_O ? -im : im);
+            }
+    __syncthreads();
+    const long long m = m0 + 2 * (tid & 3);
+    const float2 s0 = (m & 63) ? p.alpha : p.alpha0, s1 = p.alpha;       // m is even: m + 1 is no multiple of 64
+#pragma unroll 2
+    for (int line = tid >> 2; line < ROWS * kPmCols; line += kPmThreads / 4) {
+        const int i = line / kPmCols, j = line % kPmCols, k = key(i, j);
+        if (i0 + i >= p.I) break;
+        const float4 v = *reinterpret_cast<const float4*>(out + line * kPmModes + 2 * ((tid & 3) ^ (k >> 1)));
+        float2 a = (k & 1) ? make_float2(v.z, v.w) : make_float2(v.x, v.y), b = (k & 1) ? make_float2(v.x, v.y) : make_float2(v.z, v.w);
+        if (p.splits > 1) {
+            *reinterpret_cast<float4*>(p.partial + (((long long)split * p.I + i0 + i) * p.J + j0 + j) * p.modes + m) = make_float4(a.x, a.y, b.x, b.y);
+            continue;
+        }
+        a = make_float2(s0.x * a.x - s0.y * a.y, s0.x * a.y + s0.y * a.x);
+        b = make_float2(s1.x * b.x - s1.y * b.y, s1.x * b.y + s1.y * b.x);
+        float2* o = p.o + (long long)(i0 + i) * p.o_si + (long long)(j0 + j) * p.o_sj + m * p.o_sm;
+        if (p.o_vec) *reinterpret_cast<float4*>(o) = make_float4(a.x, a.y, b.x, b.y);
+        else { o[0] = a; o[p.o_sm] = b; }
+    }
+}
+
+// ---- gradient of weights that all modes share ----
+//     partial[split, i, j] = conj( sum_r sum_m P[r, i, m] conj(Q[r, j, m]) ),  r = (b, m / 8)
+// Here the sum runs along memory, so a matrix instruction is eight modes deep: lane 4 g + t takes modes 2 t and 2 t + 1 of
+// its line (any assignment of modes to terms serves, as long as P and Q share it).  64 x 64 results per CTA, a warp
+// 16 columns j by 32 rows i; the 64-byte pieces of odd lines change places in pairs, so that two adjacent lines at
+// the same r cover all banks.
+__global__ void __launch_bounds__(kPmThreads, 2) cgemm_modesum_kernel(PerModeParams p) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int iblocks = (p.I + kPmSumTile - 1) / kPmSumTile, jblocks = p.J / kPmSumTile;
+    int item = blockIdx.x;
+    const int i0 = (item % iblocks) * kPmSumTile; item /= iblocks;
+    const int j0 = (item % jblocks) * kPmSumTile; item /= jblocks;
+    const int split = item;
+    const long long r0 = split * p.split_len;
+    const long long r1 = (r0 + p.split_len < p.red) ? r0 + p.split_len : p.red;
+    const int terms = r1 > r0 ? (int)(r1 - r0) : 0, steps = (terms + kPmSumTerms - 1) / kPmSumTerms;
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem_raw);
+
+    // copies: sixteen lanes bring the four terms of a line (256 bytes where the r are adjacent)
+    const int c_line = tid >> 4, c_r = (tid >> 2) & 3, c_piece = tid & 3;
+    const uint32_t c_dst = ring + (uint32_t)(c_line * 256 + ((c_r ^ (c_line & 1)) << 6) + (c_piece << 4));
+    const float2* p_src = p.p + (r0 + c_r) * p.p_sr + (long long)(i0 + c_line) * p.p_si + 2 * c_piece;
+    const float2* q_src = p.q + (r0 + c_r) * p.q_sr + (long long)(j0 + c_line) * p.q_sj + 2 * c_piece;
+    auto fetch = [&](int step) {
+        if (step < steps) {
+            const uint32_t dst = c_dst + (uint32_t)(step % kPmStages) * kPmSumStageBytes;
+            const bool live = step * kPmSumTerms + c_r < terms;
+#pragma unroll
+            for (int l = 0; l < kPmSumTile / 16; ++l) {
+                const bool row = live && i0 + 16 * l + c_line < p.I;
+                pm_copy16(dst + l * 4096, p_src + 16 * l * p.p_si, row);
+                pm_copy16(dst + kPmSumTile * 256 + l * 4096, q_src + 16 * l * p.q_sj, live);
+            }
+            p_src += kPmSumTerms * p.p_sr;
+            q_src += kPmSumTerms * p.q_sr;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    const int g = lane >> 2, t = lane & 3, iw = (warp & 1) * 32, jw = (warp >> 1) * 16;
+    PmSum acc[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[i] = PmSum{};
+#pragma unroll
+    for (int s = 0; s < kPmStages - 1; ++s) fetch(s);
+#pragma unroll 1
+    for (int step = 0; step < steps; ++step) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kPmStages - 2) : "memory");
+        __syncthreads();
+        fetch(step + kPmStages - 1);
+        const uint32_t st = ring + (uint32_t)(step % kPmStages) * kPmSumStageBytes + (uint32_t)(g * 256 + (t << 4));
+#pragma unroll 2
+        for (int r = 0; r < kPmSumTerms; ++r) {
+            const uint32_t at = st + ((r ^ (g & 1)) << 6);
+            const float4 q[2] = {pm_load16(at + (kPmSumTile + jw) * 256), pm_load16(at + (kPmSumTile + jw + 8) * 256)};
+            PmFragQ qr, qi;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                pm_split(q[h].x, qr.hi[h], qr.lo[h]);
+                pm_split(q[h].y, qi.hi[h], qi.lo[h]);
+                pm_split(q[h].z, qr.hi[h + 2], qr.lo[h + 2]);
+                pm_split(q[h].w, qi.hi[h + 2], qi.lo[h + 2]);
+            }
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                const float4 v = pm_load16(at + (iw + 8 * nt) * 256);
+                PmFragP pr, pi;
+                pm_split(v.x, pr.hi[0], pr.lo[0]);
+                pm_split(v.y, pi.hi[0], pi.lo[0]);
+                pm_split(v.z, pr.hi[1], pr.lo[1]);
+                pm_split(v.w, pi.hi[1], pi.lo[1]);
+                pm_step<true>(acc[nt], qr, qi, pr, pi, pm_negated(pr));
             }
         }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-
 #pragma unroll
-    for (int t = 0; t < TI; ++t) {
-        const int i = i0 + t * 4 + ig;
+    for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            float2 v = acc[t][j];
-            if (CONJ_O) v.y = -v.y;
-            if (SUM_MODES) {
-#pragma unroll
-                for (int d = 1; d < 8; d <<= 1) {
-                    v.x += __shfl_xor_sync(0xffffffffu, v.x, d);
-                    v.y += __shfl_xor_sync(0xffffffffu, v.y, d);
-                }
-                if (m == 0 && i < p.I) p.partial[((long long)split * p.I + i) * p.J + j0 + wj * 8 + j] = v;
-            } else if (i < p.I) {
-                if (p.splits > 1) p.partial[(((long long)split * p.I + i) * p.J + j0 + wj * 8 + j) * p.modes + m0 + m] = v;
-                else {
-                    const float2 s = ((m0 + m) & 63) ? p.alpha : p.alpha0;
-                    p.o[(long long)i * p.o_si + (long long)(j0 + wj * 8 + j) * p.o_sj + (m0 + m) * p.o_sm] =
-                        make_float2(s.x * v.x - s.y * v.y, s.x * v.y + s.y * v.x);
-                }
-            }
+        for (int e = 0; e < 4; ++e) {
+            const int i = i0 + iw + 8 * nt + 2 * t + (e & 1), j = j0 + jw + g + 8 * (e >> 1);
+            const float2 re = acc[nt].re[e >> 1], im = acc[nt].im[e >> 1];
+            if (i < p.I) p.partial[((long long)split * p.I + i) * p.J + j] = make_float2((e & 1) ? re.y : re.x, (e & 1) ? -im.y : -im.x);
         }
-    }
 }
 
 // adds the partial sums of the splits, in their order, and scales
-template <bool SUM_MODES>
 __global__ void __launch_bounds__(256) permode_reduce_kernel(PerModeParams p) {
-    const long long per = (long long)p.I * p.J * (SUM_MODES ? 1 : p.modes);
+    const long long per = (long long)p.I * p.J * p.modes;
     for (long long e = blockIdx.x * 256LL + threadIdx.x; e < per; e += gridDim.x * 256LL) {
         float2 v = make_float2(0.f, 0.f);
 #pragma unroll 4
@@ -205,12 +335,33 @@ __global__ void __launch_bounds__(256) permode_reduce_kernel(PerModeParams p) {
             const float2 t = p.partial[s * per + e];
             v.x += t.x; v.y += t.y;
         }
-        const long long m = SUM_MODES ? 1 : e % p.modes, ij = SUM_MODES ? e : e / p.modes;
+        const long long m = e % p.modes, ij = e / p.modes;
         const float2 s = (m & 63) ? p.alpha : p.alpha0;
-        p.o[(ij / p.J) * p.o_si + (ij % p.J) * p.o_sj + (SUM_MODES ? 0 : m * p.o_sm)] = make_float2(s.x * v.x - s.y * v.y, s.x * v.y + s.y * v.x);
+        p.o[(ij / p.J) * p.o_si + (ij % p.J) * p.o_sj + m * p.o_sm] = make_float2(s.x * v.x - s.y * v.y, s.x * v.y + s.y * v.x);
     }
 }
-
-#endif
+// The same for shared weights: few results (K x N) of many splits, so eight threads share a result (a fixed order again).
+constexpr int kPmSumReducers = 32;
+__global__ void __launch_bounds__(32 * kPmSumReducers) modesum_reduce_kernel(PerModeParams p) {
+    __shared__ float2 part[kPmSumReducers][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, per = p.I * p.J;
+    const int e = blockIdx.x * 32 + lane;
+    float2 v = make_float2(0.f, 0.f);
+    if (e < per) {
+#pragma unroll 8
+        for (int s = w; s < p.splits; s += kPmSumReducers) {
+            const float2 t = p.partial[(long long)s * per + e];
+            v.x += t.x; v.y += t.y;
+        }
+    }
+    part[w][lane] = v;
+    __syncthreads();
+    if (w == 0 && e < per) {
+#pragma unroll
+        for (int i = 1; i < kPmSumReducers; ++i) { v.x += part[i][lane].x; v.y += part[i][lane].y; }
+        p.o[(e / p.J) * p.o_si + (e % p.J) * p.o_sj] =
+            make_float2(p.alpha.x * v.x - p.alpha.y * v.y, p.alpha.x * v.y + p.alpha.y * v.x);
+    }
+}
 
 }  // namespace tfno

@@ -143,6 +143,33 @@ struct ImageParams {
 int launch_fft2d(const DeviceInfo& dev, int DX, int DY, const ImageParams& p, bool inverse, cudaStream_t st);
 bool fft2d_fits(const DeviceInfo& dev);      // no launch above needs more shared memory than the device gives
 
+// ----------------------------------------------------------------------------------------------
+// Per-mode contractions and weight gradients (cgemm_permode.cuh, permode.cu)
+// ----------------------------------------------------------------------------------------------
+constexpr int kPmModes = 8;            // adjacent modes per CTA: 64 contiguous bytes of every row of P, Q and O
+
+struct PerModeParams {
+    int I, J;                          // J a multiple of 64
+    long long red, modes;              // terms of the sum; modes: a multiple of 8
+    const float2* p; long long p_sr, p_si;                 // P[r*p_sr + i*p_si + m]
+    const float2* q; long long q_sr, q_sj, q_sm;           // Q[r*q_sr + j*q_sj + m*q_sm]
+    float2* o; long long o_si, o_sj, o_sm;                 // O[i*o_si + j*o_sj + m*o_sm]
+    float2* partial;                   // [splits][I][J][modes] (sum over modes: [splits][I][J]) when splits > 1 or the modes are summed
+    float2 alpha;
+    float2 alpha0;                     // factor of the modes m % 64 == 0 (real fields: the ky = 0 column)
+    int splits;                        // r is dealt to this many CTAs in runs of split_len
+    long long split_len;
+    int q_vec;                         // Q may be copied 16 bytes (two modes) at a time
+    int o_vec;                         // O may be written 16 bytes (two modes) at a time
+};
+
+// The launches (permode.cu).  `partial` must hold permode_partial_bytes() when that is not zero.
+enum PermodeKind { PERMODE_APPLY, PERMODE_APPLY_CONJ, PERMODE_GRAD, PERMODE_GRAD_SHARED };
+size_t permode_partial_bytes(const DeviceInfo& dev, const PerModeParams& p, PermodeKind kind);
+int launch_permode(const DeviceInfo& dev, PerModeParams p, PermodeKind kind, cudaStream_t st);
+// dst[k*N + n] = conj(w[k*sk + n*sn])
+int launch_conjugate(const DeviceInfo& dev, const float2* w, long long sk, long long sn, int K, int N, float2* dst, cudaStream_t st);
+
 #if defined(__CUDACC__)
 template <typename Params, typename Kernel>
 inline int launch_persistent(const DeviceInfo& dev, Kernel kernel, size_t smem, long long work_blocks,

@@ -9,7 +9,6 @@
 #include "spectral_kernels.cuh"
 #include "spectral_tc.cuh"
 #include "cgemm_tc.cuh"
-#include "cgemm_permode.cuh"
 
 namespace tfno {
 
