@@ -246,10 +246,9 @@ __device__ __forceinline__ uint64_t make_kmajor_desc(uint32_t addr, uint32_t lbo
 __device__ __forceinline__ uint32_t make_idesc_tf32(int n) {
     return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
+// nearest tf32 by an add and a mask; cvt.rna.tf32 takes five instructions here, which only differ for NaNs (whose rest is NaN either way)
 __device__ __forceinline__ float tf32_hi(float v) {
-    uint32_t u;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(v));
-    return __uint_as_float(u);
+    return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u);
 }
 
 #define TFNO_TMEM_ST8(taddr, r)                                                                            \
