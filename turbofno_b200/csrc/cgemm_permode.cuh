@@ -168,6 +168,8 @@ __global__ void __launch_bounds__(kPmThreads, NT == 1 ? 3 : 2) cgemm_permode_ker
     PmSum acc[NT][MT];
 #pragma unroll
     for (int i = 0; i < NT * MT; ++i) (&acc[0][0])[i] = PmSum{};
+    follow_previous_kernel();
+    admit_next_kernel();
 #pragma unroll
     for (int s = 0; s < kPmStages - 1; ++s) fetch(s);
 #pragma unroll 1
@@ -282,6 +284,8 @@ __global__ void __launch_bounds__(kPmThreads, 2) cgemm_modesum_kernel(PerModePar
     PmSum acc[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i] = PmSum{};
+    follow_previous_kernel();
+    admit_next_kernel();
 #pragma unroll
     for (int s = 0; s < kPmStages - 1; ++s) fetch(s);
 #pragma unroll 1
@@ -328,6 +332,8 @@ __global__ void __launch_bounds__(kPmThreads, 2) cgemm_modesum_kernel(PerModePar
 // adds the partial sums of the splits, in their order, and scales
 __global__ void __launch_bounds__(256) permode_reduce_kernel(PerModeParams p) {
     const long long per = (long long)p.I * p.J * p.modes;
+    follow_previous_kernel();
+    admit_next_kernel();
     for (long long e = blockIdx.x * 256LL + threadIdx.x; e < per; e += gridDim.x * 256LL) {
         float2 v = make_float2(0.f, 0.f);
 #pragma unroll 4
@@ -347,6 +353,8 @@ __global__ void __launch_bounds__(32 * kPmSumReducers) modesum_reduce_kernel(Per
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, per = p.I * p.J;
     const int e = blockIdx.x * 32 + lane;
     float2 v = make_float2(0.f, 0.f);
+    follow_previous_kernel();
+    admit_next_kernel();
     if (e < per) {
 #pragma unroll 8
         for (int s = w; s < p.splits; s += kPmSumReducers) {

@@ -113,6 +113,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) cgemm_tc_kernel(CgemmTcParams
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const uint32_t TM_WHI = 0, TM_WLO = 2 * Kp, TM_ACC = 4 * Kp;
+    follow_previous_kernel();
+    admit_next_kernel();
 
     const long long first = blockIdx.x;
     const int n_it = first < p.tiles ? (int)((p.tiles - first + gridDim.x - 1) / gridDim.x) : 0;

@@ -338,13 +338,30 @@ TFNO_HD void inverse_pad_lane(float2 (&v)[64], const float2* __restrict__ twI, i
 }
 
 #if defined(__CUDACC__)
+// Loads of what the previous kernel wrote: not through the read-only path (__ldg), whose data may not change while the kernel
+// runs, and it runs already when follow_previous_kernel() returns.  In their order, ahead of the arithmetic.
+__device__ __forceinline__ float4 load_global(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float2 load_global(const float2* p) {
+    float2 v;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float load_global(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
 // ----------------------------------------------------------------------------------------------
 // lane-level load / store of one decimated signal
 // ----------------------------------------------------------------------------------------------
 template <int R>
 TFNO_D void load_decimated(float2 (&v)[64], const float2* __restrict__ sig, long long elem_stride, int r) {
 #pragma unroll
-    for (int n = 0; n < 64; ++n) v[n] = __ldg(sig + (long long)(R * n + r) * elem_stride);
+    for (int n = 0; n < 64; ++n) v[n] = load_global(sig + (long long)(R * n + r) * elem_stride);
 }
 
 template <int R>
@@ -364,7 +381,7 @@ TFNO_D void load_decimated_paired(float2 (&v)[64], const float2* __restrict__ si
     const float2* base = sig + (odd ? R : 0) + (r & ~1);
 #pragma unroll
     for (int n2 = 0; n2 < 32; ++n2) {
-        const float4 q = __ldg(reinterpret_cast<const float4*>(base + 2 * R * n2));   // samples R*(2*n2 + odd) + (r & ~1), +1
+        const float4 q = load_global(reinterpret_cast<const float4*>(base + 2 * R * n2));   // samples R*(2*n2 + odd) + (r & ~1), +1
         const float2 mine = odd ? make_float2(q.z, q.w) : make_float2(q.x, q.y);
         const float2 send = odd ? make_float2(q.x, q.y) : make_float2(q.z, q.w);
         float2 got;

@@ -17,22 +17,7 @@ int launch_forward(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st)
     // a cluster of CTAs per image, or as many CTAs as are resident together
     long long clusters = p.nimg;
     if (C == 1 && clusters > (long long)dev.sms * occ) clusters = (long long)dev.sms * occ;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(clusters * C));
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = C;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = C > 1 ? 1 : 0;
-    if (cudaLaunchKernelEx(&cfg, kernel, p) != cudaSuccess) {
-        cudaGetLastError();
-        return TFNO_ERR_CUDA;
-    }
-    return launch_status();
+    return launch_chained(kernel, dim3((unsigned)(clusters * C)), THREADS, smem, st, clusters == p.nimg, C, p);
 }
 template <int RX, int RY, bool REAL>
 int launch_forward_split(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st) {
@@ -58,8 +43,7 @@ int launch_inverse(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st)
     if (rc != TFNO_OK) return rc;
     long long images = (long long)dev.sms * occ / PARTS;
     if (images > p.nimg) images = p.nimg;
-    kernel<<<(unsigned)(images * PARTS), THREADS, smem, st>>>(p);
-    return launch_status();
+    return launch_chained(kernel, dim3((unsigned)(images * PARTS)), THREADS, smem, st, images == p.nimg, 1, p);
 }
 
 template <int RX, bool CENTERED_X>
@@ -74,8 +58,7 @@ int launch_inverse64(const DeviceInfo& dev, const ImageParams& p, cudaStream_t s
     if (rc != TFNO_OK) return rc;
     long long images = (long long)dev.sms * occ / PARTS;
     if (images > p.nimg) images = p.nimg;
-    kernel<<<(unsigned)(images * PARTS), THREADS, smem, st>>>(p);
-    return launch_status();
+    return launch_chained(kernel, dim3((unsigned)(images * PARTS)), THREADS, smem, st, images == p.nimg, 1, p);
 }
 
 template <int RX, int RY, int CLS>

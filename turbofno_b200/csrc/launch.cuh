@@ -32,8 +32,7 @@ inline int launch_tile_inst(const DeviceInfo& dev, const TileParams& p, cudaStre
     if (rc != TFNO_OK) return rc;
     long long grid = (long long)dev.sms * occ;
     if (grid > p.rows) grid = p.rows;
-    kernel<<<dim3((unsigned)grid, (unsigned)n_blocks), kThreads, smem, st>>>(p);    // p.N channels per block of blockIdx.y
-    return launch_status();
+    return launch_chained(kernel, dim3((unsigned)grid, (unsigned)n_blocks), kThreads, smem, st, grid == p.rows, 1, p);    // p.N channels per block of blockIdx.y
 }
 
 template <bool FWD, bool INV, int NB>
@@ -172,32 +171,12 @@ inline int launch_tc_inst(const DeviceInfo& dev, const TileParams& p, cudaStream
 #ifdef TFNO_TC_TRACE
     q.trace = tc_trace_buffer(dev, true);
 #endif
-#ifndef TFNO_NO_PDL
-    {
-        // launched so that its set-up may overlap the tail of the previous kernel in the stream
-        // (the kernel orders itself behind that kernel with griddepcontrol.wait)
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned)grid);
-        cfg.blockDim = dim3(tc::kTcThreads);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        if (cudaLaunchKernelEx(&cfg, kernel, q) != cudaSuccess) {
-            cudaGetLastError();
-            return TFNO_ERR_CUDA;
-        }
-    }
-#else
-    kernel<<<(unsigned)grid, tc::kTcThreads, smem, st>>>(q);
-#endif
+    rc = launch_chained(kernel, dim3((unsigned)grid), tc::kTcThreads, smem, st, true, 1, q);
+    if (rc != TFNO_OK) return rc;
 #ifdef TFNO_TC_TRACE
     tc_trace_report(dev, (int)grid);
 #endif
-    return launch_status();
+    return TFNO_OK;
 }
 
 // Tensor-core contraction of compact spectra: N a multiple of 64 (64 per launch), K a multiple of 16 up to 64, beta = 0.
@@ -232,8 +211,7 @@ inline int launch_cgemm_tc_inst(const DeviceInfo& dev, const TileParams& p, cuda
     q.accumulate = accumulate ? 1 : 0;
     long long grid = dev.sms;
     if (grid > q.tiles) grid = q.tiles;
-    kernel<<<(unsigned)grid, tcg::kGemmThreads, smem, st>>>(q);
-    return launch_status();
+    return launch_chained(kernel, dim3((unsigned)grid), tcg::kGemmThreads, smem, st, grid == q.tiles, 1, q);
 }
 // 128-mode tiles when M allows it and there are enough of them to fill the device
 inline int launch_cgemm_tc(const DeviceInfo& dev, const TileParams& p, cudaStream_t st) {

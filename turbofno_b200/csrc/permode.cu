@@ -5,7 +5,9 @@ namespace tfno {
 namespace {
 
 // dst[k*N + n] = conj(w[k, n])
-__global__ void __launch_bounds__(256) conjugate_kernel(const float2* __restrict__ w, long long sk, long long sn, int K, int N, float2* __restrict__ dst) {
+__global__ void __launch_bounds__(256) conjugate_kernel(const float2* w, long long sk, long long sn, int K, int N, float2* dst) {
+    follow_previous_kernel();
+    admit_next_kernel();
     for (int e = blockIdx.x * 256 + threadIdx.x; e < K * N; e += gridDim.x * 256) {
         const float2 v = w[(e / N) * sk + (e % N) * sn];
         dst[e] = make_float2(v.x, -v.y);
@@ -53,8 +55,7 @@ int launch_inst(const DeviceInfo& dev, const PerModeParams& p, cudaStream_t st) 
     if (rc != TFNO_OK) return rc;
     const long long grid = blocks_per_split(p, NT) * p.splits;
     if (grid > 0x7fffffffLL) return TFNO_ERR_UNSUPPORTED;
-    kernel<<<(unsigned)grid, kPmThreads, smem, st>>>(p);
-    return launch_status();
+    return launch_chained(kernel, dim3((unsigned)grid), kPmThreads, smem, st, true, 1, p);
 }
 template <bool CONJ_Q, bool CONJ_O>
 int launch_rows(const DeviceInfo& dev, const PerModeParams& p, PermodeKind kind, cudaStream_t st) {
@@ -71,8 +72,7 @@ int launch_modesum(const DeviceInfo& dev, const PerModeParams& p, cudaStream_t s
     const int rc = prepare_kernel(cgemm_modesum_kernel, kPmSumSmemBytes, dev, &occ, kPmThreads);
     if (rc != TFNO_OK) return rc;
     const unsigned grid = (unsigned)((p.I + kPmSumTile - 1) / kPmSumTile) * (unsigned)(p.J / kPmSumTile) * (unsigned)p.splits;
-    cgemm_modesum_kernel<<<grid, kPmThreads, kPmSumSmemBytes, st>>>(p);
-    return launch_status();
+    return launch_chained(cgemm_modesum_kernel, dim3(grid), kPmThreads, kPmSumSmemBytes, st, true, 1, p);
 }
 
 }  // namespace
@@ -101,20 +101,16 @@ int launch_permode(const DeviceInfo& dev, PerModeParams p, PermodeKind kind, cud
         case PERMODE_GRAD_SHARED: rc = launch_modesum(dev, p, st); break;
     }
     if (rc != TFNO_OK || (kind == PERMODE_GRAD && p.splits == 1)) return rc;
-    if (kind == PERMODE_GRAD_SHARED) {
-        modesum_reduce_kernel<<<(unsigned)((p.I * p.J + 31) / 32), 32 * kPmSumReducers, 0, st>>>(p);
-        return launch_status();
-    }
+    if (kind == PERMODE_GRAD_SHARED)
+        return launch_chained(modesum_reduce_kernel, dim3((unsigned)((p.I * p.J + 31) / 32)), 32 * kPmSumReducers, 0, st, true, 1, p);
     const long long sums = (long long)p.I * p.J * p.modes;
     long long grid = (sums + 255) / 256;
     if (grid > 8LL * dev.sms) grid = 8LL * dev.sms;
-    permode_reduce_kernel<<<(unsigned)grid, 256, 0, st>>>(p);
-    return launch_status();
+    return launch_chained(permode_reduce_kernel, dim3((unsigned)grid), 256, 0, st, true, 1, p);
 }
 
 int launch_conjugate(const DeviceInfo& dev, const float2* w, long long sk, long long sn, int K, int N, float2* dst, cudaStream_t st) {
-    conjugate_kernel<<<(unsigned)((K * N + 255) / 256), 256, 0, st>>>(w, sk, sn, K, N, dst);
-    return launch_status();
+    return launch_chained(conjugate_kernel, dim3((unsigned)((K * N + 255) / 256)), 256, 0, st, true, 1, w, sk, sn, K, N, dst);
 }
 
 }  // namespace tfno

@@ -157,7 +157,9 @@ __global__ void __launch_bounds__(64 * RX / C, 8 * C / RX) fft2d_trunc_kernel(Im
         return reinterpret_cast<const Sample*>(p.in) + (img % p.per_k) * p.stride_b + (img / p.per_k) * p.stride_k + (long long)rank * ROWS * DY;
     };
     if constexpr (C > 1) cluster_arrive();                       // this CTA runs: its shared memory may be written
+    follow_previous_kernel();
     for (long long img = blockIdx.x / C; img < p.nimg; img += step) {
+        if (step >= p.nimg) admit_next_kernel();
         const Sample* src = rows_of(img);
         const Sample* next = C == 1 && img + step < p.nimg ? rows_of(img + step) : nullptr;
 #pragma unroll 1
@@ -170,7 +172,7 @@ __global__ void __launch_bounds__(64 * RX / C, 8 * C / RX) fft2d_trunc_kernel(Im
                 const float2* row = reinterpret_cast<const float2*>(src + (long long)x * DY) + r;
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    const float2 a = __ldg(row + 8 * i), b = __ldg(row + DY / 2 + 8 * i);
+                    const float2 a = load_global(row + 8 * i), b = load_global(row + DY / 2 + 8 * i);
                     v0[i] = make_float2(a.x, b.x);
                     v1[i] = make_float2(a.y, b.y);
                 }
@@ -178,7 +180,7 @@ __global__ void __launch_bounds__(64 * RX / C, 8 * C / RX) fft2d_trunc_kernel(Im
                 const float4* row = reinterpret_cast<const float4*>(src + (long long)x * DY) + r;
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    const float4 q = __ldg(row + 8 * i);
+                    const float4 q = load_global(row + 8 * i);
                     v0[i] = make_float2(q.x, q.y);
                     v1[i] = make_float2(q.z, q.w);
                 }
@@ -186,8 +188,8 @@ __global__ void __launch_bounds__(64 * RX / C, 8 * C / RX) fft2d_trunc_kernel(Im
                 const Sample* row = src + (long long)x * DY + r;
 #pragma unroll
                 for (int i = 0; i < 32; ++i) {
-                    if constexpr (REAL) v[i] = make_float2(__ldg(row + RY * i), __ldg(row + DY + RY * i));
-                    else v[i] = __ldg(row + RY * i);
+                    if constexpr (REAL) v[i] = make_float2(load_global(row + RY * i), load_global(row + DY + RY * i));
+                    else v[i] = load_global(row + RY * i);
                 }
             }
             // The rows of the next round (this image's or the next one's) travel to the L2 meanwhile.  Two rounds
@@ -279,7 +281,9 @@ __global__ void __launch_bounds__(64 * CLS, 8 / CLS) ifft2d_pad_kernel(ImagePara
     const int g = tid / RY, j1 = tid % RY;
     const float2 coefY = inverse_fold_coef32<RY>(j1, INVERSE);
     const bool odd = (j1 & 1) != 0;
+    follow_previous_kernel();
     for (long long img = blockIdx.x / PARTS; img < p.nimg; img += gridDim.x / PARTS) {
+        if (gridDim.x / PARTS >= p.nimg) admit_next_kernel();
         const float2* src = p.in + img * (long long)(kModes * kModes) + ky;
         Sample* dst = reinterpret_cast<Sample*>(p.out) + (img % p.per_k) * p.stride_b + (img / p.per_k) * p.stride_k;
         {
@@ -287,8 +291,8 @@ __global__ void __launch_bounds__(64 * CLS, 8 / CLS) ifft2d_pad_kernel(ImagePara
 #pragma unroll
             for (int m = 0; m < 32; m += 2) {
                 const float4 t = *reinterpret_cast<const float4*>(twX + jl * 32 + m);
-                v[m] = cmul(cmadd(__ldg(src + m * kModes), coefX, __ldg(src + (m + 32) * kModes)), make_float2(t.x, t.y));
-                v[m + 1] = cmul(cmadd(__ldg(src + (m + 1) * kModes), coefX, __ldg(src + (m + 33) * kModes)), make_float2(t.z, t.w));
+                v[m] = cmul(cmadd(load_global(src + m * kModes), coefX, load_global(src + (m + 32) * kModes)), make_float2(t.x, t.y));
+                v[m + 1] = cmul(cmadd(load_global(src + (m + 1) * kModes), coefX, load_global(src + (m + 33) * kModes)), make_float2(t.z, t.w));
             }
             fft32<SIGN>(v);
 #pragma unroll
@@ -398,12 +402,14 @@ __global__ void __launch_bounds__(64 * CLS, 1) ifft2d_pad64_kernel(ImageParams p
     __syncthreads();
     const int ky = tid & 63, jl = tid >> 6;
     const int g = tid / RY, j1 = tid % RY;
+    follow_previous_kernel();
     for (long long img = blockIdx.x / PARTS; img < p.nimg; img += gridDim.x / PARTS) {
+        if (gridDim.x / PARTS >= p.nimg) admit_next_kernel();
         {
             const float2* src = p.in + img * (long long)(kModes * kModes) + ky;
             float2 v[64];
 #pragma unroll
-            for (int m = 0; m < 64; ++m) v[m] = __ldg(src + m * kModes);
+            for (int m = 0; m < 64; ++m) v[m] = load_global(src + m * kModes);
             if (p.conj_inverse) inverse_pad_lane<+1, CLS, CENTERED_X>(v, twX, jl);
             else inverse_pad_lane<-1, CLS>(v, twX, jl);
 #pragma unroll

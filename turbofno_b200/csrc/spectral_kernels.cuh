@@ -89,7 +89,9 @@ __global__ void __launch_bounds__(kThreads, 1) spectral_tile_kernel(TileParams p
     const float2* wbase = p.w + (long long)blockIdx.y * N * p.w_stride_n;
     float2* ybase = p.y + (long long)blockIdx.y * N * (INV ? p.y_stride_n : M);
 
+    follow_previous_kernel();
     for (long long row = blockIdx.x; row < p.rows; row += gridDim.x) {
+        if (gridDim.x >= p.rows) admit_next_kernel();
         // ---------------- stage 1: spectrum tile sA[k][m] ----------------
         if (FWD) {
             constexpr int GROUPS = kThreads / R;
@@ -110,7 +112,7 @@ __global__ void __launch_bounds__(kThreads, 1) spectral_tile_kernel(TileParams p
             // compact spectrum: 64 consecutive m per channel
             for (int i = tid; i < K * 32; i += kThreads) {
                 int k = i >> 5, c = i & 31;
-                float4 q = __ldg(reinterpret_cast<const float4*>(p.x + row * kModes + (long long)k * M) + c);
+                float4 q = load_global(reinterpret_cast<const float4*>(p.x + row * kModes + (long long)k * M) + c);
                 *reinterpret_cast<float4*>(sA + k * kModes + swz_chunk(k, c) * 2) = q;
             }
         }
@@ -132,7 +134,7 @@ __global__ void __launch_bounds__(kThreads, 1) spectral_tile_kernel(TileParams p
                 int e = tid + i * kThreads;
                 int kk, n;
                 if (p.w_stride_n == 1) { n = e % N; kk = e / N; } else { kk = e % kSlabK; n = e / kSlabK; }
-                wreg[i] = __ldg(wbase + (long long)(k0 + kk) * p.w_stride_k + (long long)n * p.w_stride_n);
+                wreg[i] = load_global(wbase + (long long)(k0 + kk) * p.w_stride_k + (long long)n * p.w_stride_n);
             }
         };
         auto stash_slab = [&](int buf) {
@@ -263,7 +265,9 @@ __global__ void __launch_bounds__(kThreads, 1) fft_cols_trunc_kernel(ColsParams 
     const int g = threadIdx.x / R, r = threadIdx.x % R;
     const long long ncol = p.nimg * p.DY;
     const long long nblk = (ncol + GROUPS - 1) / GROUPS;
+    follow_previous_kernel();
     for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
+        if (gridDim.x >= nblk) admit_next_kernel();
         long long c = blk * GROUPS + g;
         const bool live = c < ncol;
         if (!live) c = ncol - 1;
@@ -290,7 +294,9 @@ __global__ void __launch_bounds__(kThreads, 1) ifft_cols_pad_kernel(ColsParams p
     const int g = threadIdx.x / R, j1 = threadIdx.x % R;
     const long long ncol = p.nimg * p.DY;
     const long long nblk = (ncol + GROUPS - 1) / GROUPS;
+    follow_previous_kernel();
     for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
+        if (gridDim.x >= nblk) admit_next_kernel();
         long long c = blk * GROUPS + g;
         if (c >= ncol) continue;
         const long long img = c / p.DY;
@@ -298,7 +304,7 @@ __global__ void __launch_bounds__(kThreads, 1) ifft_cols_pad_kernel(ColsParams p
         float2 v[64];
         const float2* src = p.in + img * (long long)kModes * p.DY + col;
 #pragma unroll
-        for (int m = 0; m < 64; ++m) v[m] = __ldg(src + (long long)m * p.DY);
+        for (int m = 0; m < 64; ++m) v[m] = load_global(src + (long long)m * p.DY);
         if (p.conj_inverse) inverse_pad_lane<+1, R>(v, twI, j1);
         else inverse_pad_lane<-1, R>(v, twI, j1);
         store_decimated<R>(v, p.out + (img % p.per_k) * p.stride_b + (img / p.per_k) * p.stride_k + col, p.DY, j1);

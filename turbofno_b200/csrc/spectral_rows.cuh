@@ -28,7 +28,9 @@ __global__ void __launch_bounds__(kThreads, 2) fft_rows_trunc_kernel(RowsParams 
     const int g = threadIdx.x / R, r = threadIdx.x % R;
     const float2 coef = round1_coef32<R>(r);
     const long long nblk = (p.nsig + GROUPS - 1) / GROUPS;
+    follow_previous_kernel();
     for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
+        if (gridDim.x >= nblk) admit_next_kernel();
         // clamp instead of branching so that every lane of a warp takes part in the shuffles
         long long s = blk * GROUPS + g;
         const bool live = s < p.nsig;
@@ -36,7 +38,7 @@ __global__ void __launch_bounds__(kThreads, 2) fft_rows_trunc_kernel(RowsParams 
         const float2* row = p.in + row_offset(p, s) + r;
         float2 v[32];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = __ldg(row + R * i);
+        for (int i = 0; i < 32; ++i) v[i] = load_global(row + R * i);
         forward_trunc32<R>(v, twF, r, 1, coef);
         if (live) {
             float2* dst = p.out + s * kModes + PER * r;
@@ -59,7 +61,9 @@ __global__ void __launch_bounds__(kIfftRowsThreads, 1) ifft_rows_pad_kernel(Rows
     constexpr int GROUPS = kIfftRowsThreads / R;
     const int g = threadIdx.x / R, j1 = threadIdx.x % R;
     const long long nblk = (p.nsig + GROUPS - 1) / GROUPS;
+    follow_previous_kernel();
     for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
+        if (gridDim.x >= nblk) admit_next_kernel();
         // clamp instead of branching so that every lane of a warp takes part in the store's shuffles
         long long s = blk * GROUPS + g;
         const bool live = s < p.nsig;
@@ -68,7 +72,7 @@ __global__ void __launch_bounds__(kIfftRowsThreads, 1) ifft_rows_pad_kernel(Rows
         const float4* src = reinterpret_cast<const float4*>(p.in + s * kModes);
 #pragma unroll
         for (int c = 0; c < 32; ++c) {
-            float4 q = __ldg(src + c);
+            const float4 q = load_global(src + c);
             v[2 * c] = make_float2(q.x, q.y);
             v[2 * c + 1] = make_float2(q.z, q.w);
         }

@@ -48,6 +48,7 @@
 #include <cstdint>
 #include <type_traits>
 #include <cuda.h>          // CUtensorMap (types only: the encoder is fetched from the runtime)
+#include "common.cuh"
 #include "fft32.cuh"
 
 namespace tfno {
@@ -360,14 +361,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) spectral_tc_kernel(const __grid
     const uint32_t tmem = *tmem_slot;
     const uint32_t TM_WHI = 0, TM_WLO = 2 * Kp, TM_ACC = 4 * Kp;      // column offsets; accumulators 2 x 64 columns
 
-#ifndef TFNO_NO_PDL
-    // Programmatic dependent launch: everything above touched only this CTA's shared and tensor
-    // memory, so it may run while the previous kernel of the stream is still finishing on other
-    // SMs.  From here on global memory is read and written: wait for the previous kernel to
-    // complete, then let the next launch begin its own set-up as SMs become free.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-#endif
+    // everything above touched only this CTA's shared and tensor memory
+    follow_previous_kernel();
+    admit_next_kernel();
 #ifdef TFNO_TC_TRACE
     tr_dep = clock64();
 #endif
