@@ -8,7 +8,7 @@ template <int RX, int RY, int C, bool REAL>
 int launch_forward(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st) {
     constexpr int THREADS = 64 * RX / C;
     auto kernel = fft2d_trunc_kernel<RX, RY, C, REAL>;
-    const size_t smem = fwd_image_smem_bytes<RX, RY, C>();
+    const size_t smem = fwd_image_smem_bytes<RX, RY, C, REAL>();
     if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
     if (record_launch(dev, "fft2d_trunc_kernel<%d,%d,%d>", RX, RY, C)) return TFNO_OK;
     int occ = 0;
@@ -35,7 +35,7 @@ template <int RX, int RY, int CLS, bool INVERSE, bool REAL>
 int launch_inverse(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st) {
     constexpr int PARTS = RX / CLS, THREADS = 64 * CLS;
     auto kernel = ifft2d_pad_kernel<RX, RY, CLS, INVERSE, REAL>;
-    const size_t smem = inv_image_smem_bytes<RY, CLS>();
+    const size_t smem = inv_image_smem_bytes<RY, CLS, REAL>();
     if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
     if (record_launch(dev, "ifft2d_pad_kernel<%d,%d,%d,%d>", RX, RY, CLS, INVERSE)) return TFNO_OK;
     int occ = 0;
@@ -77,7 +77,7 @@ int launch_image(const DeviceInfo& dev, const ImageParams& p, bool inverse, cuda
 }  // namespace
 
 bool fft2d_fits(const DeviceInfo& dev) {
-    return (long long)fwd_image_smem_bytes<8, 8, 1>() <= dev.max_smem_optin;      // the largest of the instances below
+    return (long long)fwd_image_smem_bytes<8, 8, 1, true>() <= dev.max_smem_optin;      // the largest of the instances below
 }
 
 // Residue classes per inverse CTA: two (128 threads) except at 256 x 256, where four (256 threads, half as many

@@ -14,12 +14,10 @@
 //            rows RX*j2 + j1, so a CTA takes CLS of the RX residue classes, transforms the 64 columns
 //            for those rows only (every part re-reads the 32 KB spectrum, from the L2), then its rows.
 //
-// REAL: the full-size side holds real samples.  Two rows share one complex 32-point transform
-// (z = a + i b); the forward kernel separates them lane by lane (A[k] = (Z[k] + conj Z[-k])/2) before the
-// lanes are combined, the inverse kernel gives the folded 32-point input its Hermitian mirror image:
-// 2 Re(ifft2(Z')) with the ky = 0 column entering once.
+// REAL: the full-size side holds real samples.  Two rows share one complex transform (fft_real.cuh), whose lanes own each kept
+// mode together with its mirror image: 2 Re(ifft2(Z')) with the ky = 0 column entering once.
 #pragma once
-#include "fft256.cuh"
+#include "fft_real.cuh"
 #include <type_traits>
 #include "common.cuh"
 
@@ -33,21 +31,24 @@ TFNO_HD int rtile_chunk(int key, int c) { return (c & ~7) | ((c ^ key) & 7); }
 // forward: [DX rows][64/C columns] complex, rows of 32/C 16-byte chunks, low three bits XOR-ed with a number
 // of the row and (C = 1) of the chunk's group of eight.  The X pass reads RX adjacent rows at one pair (RX = 8)
 // or quadruple (RX = 4) of chunks: the plain row number spreads the former over the banks, the row number
-// rotated by one bit the latter.
-template <int RX, int C>
+// rotated by one bit the latter.  REAL and RX = 4: the lanes store two or four adjacent chunks of every second row.
+template <int RX, int C, bool REAL>
 TFNO_HD int xtile_index(int row, int col) {
     const int c = col >> 1;
-    const int s = ((RX == 8) ? (row & 7) : (((row & 1) << 2) | ((row >> 1) & 3))) ^ (C == 1 ? (c >> 3) & 3 : 0);
+    const int s = ((RX == 8) ? (row & 7) : REAL ? ((((row >> 2) ^ row) & 1) << 2) | (row & 2) : (((row & 1) << 2) | ((row >> 1) & 3))) ^
+                  (C == 1 ? (c >> 3) & 3 : 0);
     return row * (64 / C) + (((c & ~7) | ((c ^ s) & 7)) << 1) + (col & 1);
 }
-template <int RX, int RY, int C> inline constexpr size_t fwd_image_smem_bytes() {
-    return (size_t)(32 * RX * (64 / C) + RX * 32 + (RY == 8 ? kTable256 + 64 * (8 * RX / C) : RY * 32)) * sizeof(float2);
+// REAL: the inverse reads two or four adjacent chunks of every second row
+TFNO_HD int rtile_pair_key(int pair) { return ((pair & 1) << 2) | (pair & 2) | ((pair >> 2) & 1); }
+template <int RX, int RY, int C, bool REAL> inline constexpr size_t fwd_image_smem_bytes() {
+    return (size_t)(32 * RX * (64 / C) + RX * 32 + (REAL ? RY * 32 + 8 * (64 * RX / C) : RY == 8 ? kTable256 + 64 * (8 * RX / C) : RY * 32)) * sizeof(float2);
 }
 template <int RY, int CLS> inline constexpr size_t inv64_image_smem_bytes() {
     return (size_t)(64 * CLS * kModes + RY * 64 + CLS * 64) * sizeof(float2);
 }
-template <int RY, int CLS> inline constexpr size_t inv_image_smem_bytes() {
-    return (size_t)(32 * CLS * kModes + RY * 32 + CLS * 32) * sizeof(float2);
+template <int RY, int CLS, bool REAL> inline constexpr size_t inv_image_smem_bytes() {
+    return (size_t)(32 * CLS * kModes + RY * 32 + CLS * 32 + (REAL ? 8 * (64 * CLS) : 0)) * sizeof(float2);
 }
 
 #if defined(__CUDACC__)
@@ -61,62 +62,9 @@ TFNO_D uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
 TFNO_D void store_cluster16(uint32_t addr, float2 a, float2 b) {
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y) : "memory");
 }
+TFNO_D void store_cluster8(uint32_t addr, float2 a) { asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(a.x), "f"(a.y) : "memory"); }
 TFNO_D void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 TFNO_D void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-
-// ---- two real rows through one complex transform ----
-// Rows of 128 samples (R = 4; those of 256 go through fft256.cuh).  z[n] = (a, b) sample R*n + r of two real signals.
-// On return lane r holds modes 64/R*r + j of a in va[j] and of b in vb[j], both times 2.  Slots s and -s of the 32-point result are
-// separated together with s + 16 and 16 - s, which rounds 1 and 2 reduce to two values per signal: a closed
-// set of four registers in, four out (the pairing s <-> -s also holds on rotated lanes: 16 = -16).
-template <int R>
-TFNO_D void forward_trunc32_real2(float2 (&z)[32], const float2* __restrict__ twF, int r, float2 coef, float2 (&va)[16], float2 (&vb)[16]) {
-    static_assert(R == 4, "two exchange rounds leave sixteen modes of each signal");
-    fft32<-1>(z, lane_rotated32<R>(r) ? -1.0f : 1.0f);
-    auto table = [&](int s) { return twF[tw_index<R>(r, s)]; };
-#pragma unroll
-    for (int j = 0; j <= 8; ++j) {
-        constexpr int M = 4;
-        const int s[M] = {j, 16 - j, 16 + j, (32 - j) & 31};             // slot pairs: s[0] <-> s[3], s[1] <-> s[2]
-        float2 w[2][M], g[2][M];
-#pragma unroll
-        for (int i = 0; i < M; ++i) {
-            const float2 a = z[slot32(s[i])], b = z[slot32((32 - s[i]) & 31)], t = table(s[i]);
-            w[0][i] = cmul(make_float2(a.x + b.x, a.y - b.y), t);
-            w[1][i] = cmul(make_float2(a.y + b.y, b.x - a.x), t);
-        }
-        // j = 0: s = {0, 16, 16, 0}; j = 8: s = {8, 8, 24, 24}: one value per signal
-        const bool one = j == 0 || j == 8;
-        const int keep = one ? 1 : 2;                                    // kept slots s[0] (and s[1])
-        const int send0 = 2, send1 = 3;                                  // s[2] = s[0] + 16, s[3] = s[1] + 16
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-#pragma unroll
-            for (int i = 0; i < M; ++i) {
-                if (one && (i == 1 || i == 3)) continue;
-                g[q][i] = shfl_xor2(w[q][i], R >> 1);
-            }
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-#pragma unroll
-            for (int i = 0; i < M; ++i) {
-                if (one && (i == 1 || i == 3)) continue;
-                w[q][i] = cmadd(w[q][i], coef, g[q][i]);
-            }
-        float2 k[2][2];
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            k[q][0] = shfl_xor2(w[q][send0], R >> 2);
-            if (keep == 2) k[q][1] = shfl_xor2(w[q][send1], R >> 2);
-        }
-        va[j] = cadd(w[0][0], k[0][0]);
-        vb[j] = cadd(w[1][0], k[1][0]);
-        if (keep == 2) {
-            va[16 - j] = cadd(w[0][1], k[0][1]);
-            vb[16 - j] = cadd(w[1][1], k[1][1]);
-        }
-    }
-}
 
 // ------------------------------------------------------------------------------------------
 // [image][DX][DY] -> [image][64][64]      RX = DX/32, RY = DY/32 (4 or 8 each)
@@ -129,10 +77,11 @@ __global__ void __launch_bounds__(64 * RX / C, 8 * C / RX) fft2d_trunc_kernel(Im
     float2* sX = reinterpret_cast<float2*>(smem_raw);           // [DX][COLS] swizzled: this CTA's columns
     constexpr bool ONCE = RY == 8;                               // rows of 256 samples: one exchange (fft256.cuh)
     float2* twX = sX + DX * COLS;                                // [RX][32]
-    float2* twY = twX + RX * 32;                                 // [RY][32], or kTable256 entries and 64 elements per group
+    float2* twY = twX + RX * 32;                                 // factors of the rows, then the exchanged values of the groups of lanes
     const int tid = threadIdx.x;
     const int rank = C > 1 ? (int)cluster_rank() : 0;
-    if constexpr (ONCE) fill_table256(twY, tid, T);
+    if constexpr (REAL) fill_real_table<DY>(twY, tid, T);
+    else if constexpr (ONCE) fill_table256(twY, tid, T);
     else fill_forward_table32<RY>(twY, tid, T);
     fill_forward_table32<RX>(twX, tid, T, p.centered_x != 0);
     __syncthreads();
@@ -144,11 +93,16 @@ __global__ void __launch_bounds__(64 * RX / C, 8 * C / RX) fft2d_trunc_kernel(Im
     const float2 coefY = round1_coef32<RY>(r);
     const int col = tid / RX, rx = tid % RX;
     const float2 coefX = round1_coef32<RX>(rx);
-    // modes m, m + 1 of image row `row`: to the CTA of the cluster that collects their columns
+    // modes m, m + 1 (or m alone) of image row `row`: to the CTA of the cluster that collects their columns
     auto put = [&](int row, int m, float2 a, float2 b) {
-        const int at = xtile_index<RX, C>(row, m % COLS);
+        const int at = xtile_index<RX, C, REAL>(row, m % COLS);
         if constexpr (C > 1) store_cluster16(map_to_rank(shared_address(sX), (uint32_t)(m / COLS)) + 8u * (uint32_t)at, a, b);
         else *reinterpret_cast<float4*>(sX + at) = make_float4(a.x, a.y, b.x, b.y);
+    };
+    auto put1 = [&](int row, int m, float2 a) {
+        const int at = xtile_index<RX, C, REAL>(row, m % COLS);
+        if constexpr (C > 1) store_cluster8(map_to_rank(shared_address(sX), (uint32_t)(m / COLS)) + 8u * (uint32_t)at, a);
+        else sX[at] = a;
     };
     constexpr int GROUPS = T / RY, LINES = REAL ? 2 : 1, STEP = GROUPS * LINES, ROUNDS = ROWS / STEP;
     static_assert(ROUNDS >= 1, "a round of row transforms fits the CTA's rows");
@@ -164,17 +118,27 @@ __global__ void __launch_bounds__(64 * RX / C, 8 * C / RX) fft2d_trunc_kernel(Im
         const Sample* next = C == 1 && img + step < p.nimg ? rows_of(img + step) : nullptr;
 #pragma unroll 1
         for (int i0 = 0; i0 < ROUNDS; ++i0) {
-            const int x = i0 * STEP + g * LINES;
+            // REAL, four groups to a warp: the two of a half-warp take pairs of rows that lie two apart (bank conflicts of put1)
+            const int x = i0 * STEP + (REAL && RY == 8 ? (g & ~3) | ((g & 1) << 1) | ((g >> 1) & 1) : g) * LINES;
             const int gx = rank * ROWS + x;
             float2 v[32];
             float2 (&v0)[16] = *reinterpret_cast<float2(*)[16]>(&v[0]), (&v1)[16] = *reinterpret_cast<float2(*)[16]>(&v[16]);
-            if constexpr (ONCE && REAL) {
-                const float2* row = reinterpret_cast<const float2*>(src + (long long)x * DY) + r;
+            if constexpr (REAL) {
+                constexpr int Q = RealRows<DY>::Q, K1 = RealRows<DY>::K1;
+                const Sample* row = src + (long long)x * DY + Q * r;
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const float2 a = load_global(row + 8 * i), b = load_global(row + DY / 2 + 8 * i);
-                    v0[i] = make_float2(a.x, b.x);
-                    v1[i] = make_float2(a.y, b.y);
+                for (int j = 0; j < K1; ++j) {
+                    if constexpr (Q == 2) {
+                        const float2 a = load_global(reinterpret_cast<const float2*>(row + 16 * j)), b = load_global(reinterpret_cast<const float2*>(row + DY + 16 * j));
+                        v[j] = make_float2(a.x, b.x);
+                        v[K1 + j] = make_float2(a.y, b.y);
+                    } else {
+                        const float4 a = load_global(reinterpret_cast<const float4*>(row + 16 * j)), b = load_global(reinterpret_cast<const float4*>(row + DY + 16 * j));
+                        v[j] = make_float2(a.x, b.x);
+                        v[K1 + j] = make_float2(a.y, b.y);
+                        v[2 * K1 + j] = make_float2(a.z, b.z);
+                        v[3 * K1 + j] = make_float2(a.w, b.w);
+                    }
                 }
             } else if constexpr (ONCE) {
                 const float4* row = reinterpret_cast<const float4*>(src + (long long)x * DY) + r;
@@ -187,50 +151,42 @@ __global__ void __launch_bounds__(64 * RX / C, 8 * C / RX) fft2d_trunc_kernel(Im
             } else {
                 const Sample* row = src + (long long)x * DY + r;
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    if constexpr (REAL) v[i] = make_float2(load_global(row + RY * i), load_global(row + DY + RY * i));
-                    else v[i] = load_global(row + RY * i);
-                }
+                for (int i = 0; i < 32; ++i) v[i] = load_global(row + RY * i);
             }
             // The rows of the next round (this image's or the next one's) travel to the L2 meanwhile.  Two rounds
             // ahead is slower: 913 against 880 us for 8192 images of 256 x 256 (rows on the 32-point transform).
             const Sample* ahead = i0 + 1 < ROUNDS ? src + (long long)(i0 + 1) * STEP * DY : next;
             if (ahead) prefetch_l2_block(ahead, STEP * DY * (int)sizeof(Sample), tid, T);
-            if constexpr (ONCE) {
+            if constexpr (REAL) {
+                constexpr int N = DY, Q = RealRows<N>::Q, K1 = RealRows<N>::K1, M = RealRows<N>::M;
+                float2 fa[16], fb[16];
+                real_forward<N>(*reinterpret_cast<float2(*)[Q][K1]>(&v[0]), twY, twY + N + RealRows<N>::SCRATCH * g, r, g & 1, fa, fb);
+                if (C > 1 && i0 == 0) cluster_wait();
+                const int kb = real_mode<N>(1, r);
+#pragma unroll
+                for (int k2 = 0; k2 < M; ++k2)
+#pragma unroll
+                    for (int part = 0; part < 2; ++part) {
+                        float2 a, b;
+                        real_separate<N>(fa, fb, part, r == 0, k2, a, b);
+                        put1(gx, (part ? kb : r) + K1 * k2, a);
+                        put1(gx + 1, (part ? kb : r) + K1 * k2, b);
+                    }
+            } else if constexpr (ONCE) {
                 fft16<-1>(v0);
                 fft16<-1>(v1);
                 float2* scratch = twY + kTable256 + 64 * g;
+                float2 out[2][4];
 #pragma unroll
-                for (int l = 0; l < LINES; ++l) {
-                    float2 out[2][4];
+                for (int e = 0; e < 2; ++e) {
+                    float2 f[16];
 #pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        float2 f[16];
-#pragma unroll
-                        for (int q = 0; q < 2; ++q)
-                            exchange256(scratch, r, g & 1, q, f, [&](int d) {
-                                const float2 (&w)[16] = q ? v1 : v0;
-                                const float2 z = w[slot16(2 * d + e)];
-                                if constexpr (!REAL) return z;
-                                // two real rows: 2 A[k] = Z[k] + conj Z[-k], 2 B[k] = -i (Z[k] - conj Z[-k])
-                                const float2 y = w[slot16((16 - 2 * d - e) & 15)];
-                                return l == 0 ? make_float2(z.x + y.x, z.y - y.y) : make_float2(z.y + y.y, y.x - z.x);
-                            });
-                        combine256(f, twY, 2 * r + e, out[e]);
-                    }
-                    if (C > 1 && i0 == 0 && l == 0) cluster_wait();
-#pragma unroll
-                    for (int k2 = 0; k2 < 4; ++k2) put(gx + l, 2 * r + 16 * k2, out[0][k2], out[1][k2]);
+                    for (int q = 0; q < 2; ++q) exchange256(scratch, r, g & 1, q, f, [&](int d) { return (q ? v1 : v0)[slot16(2 * d + e)]; });
+                    combine256(f, twY, 2 * r + e, out[e]);
                 }
-            } else if constexpr (REAL) {
-                float2 va[16], vb[16];
-                forward_trunc32_real2<RY>(v, twY, r, coefY, va, vb);
                 if (C > 1 && i0 == 0) cluster_wait();
 #pragma unroll
-                for (int j = 0; j < PERY; j += 2) {
-                    put(gx, PERY * r + j, va[j], va[j + 1]);
-                    put(gx + 1, PERY * r + j, vb[j], vb[j + 1]);
-                }
+                for (int k2 = 0; k2 < 4; ++k2) put(gx, 2 * r + 16 * k2, out[0][k2], out[1][k2]);
             } else {
                 forward_trunc32<RY>(v, twY, r, 1, coefY);
                 if (C > 1 && i0 == 0) cluster_wait();
@@ -243,7 +199,7 @@ __global__ void __launch_bounds__(64 * RX / C, 8 * C / RX) fft2d_trunc_kernel(Im
         {
             float2 v[32];
 #pragma unroll
-            for (int n = 0; n < 32; ++n) v[n] = sX[xtile_index<RX, C>(RX * n + rx, col)];
+            for (int n = 0; n < 32; ++n) v[n] = sX[xtile_index<RX, C, REAL>(RX * n + rx, col)];
             if constexpr (C == 1) __syncthreads();              // columns read: the next image may be stored
             forward_trunc32<RX>(v, twX, rx, 1, coefX);
             float2* dst = p.out + img * (long long)(kModes * kModes) + rank * COLS + col;
@@ -266,10 +222,11 @@ __global__ void __launch_bounds__(64 * CLS, 8 / CLS) ifft2d_pad_kernel(ImagePara
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2* sY = reinterpret_cast<float2*>(smem_raw);           // [ROWS][64] swizzled
     float2* twY = sY + ROWS * kModes;                            // [RY][32]
-    float2* twX = twY + RY * 32;                                 // [CLS][32]
+    float2* twX = twY + RY * 32;                                 // [CLS][32]; REAL: then the exchanged values of the groups of lanes
     const int tid = threadIdx.x;
     const int part = blockIdx.x % PARTS;                         // the grid is a multiple of PARTS
-    fill_inverse_table32_folded<RY>(twY, tid, T, make_float2(1.f, 0.f), INVERSE);
+    if constexpr (REAL) fill_real_table<DY>(twY, tid, T);
+    else fill_inverse_table32_folded<RY>(twY, tid, T, make_float2(1.f, 0.f), INVERSE);
     for (int i = tid; i < CLS * 32; i += T) {                    // rows part*CLS .. of fill_inverse_table32_folded<RX>
         const int j1 = part * CLS + (i >> 5), m = i & 31;        // modes -32..31: times e^{-2 pi i j1 / RX}
         const int e = (INVERSE && p.centered_x) ? (j1 * m - 32 * j1) & (32 * RX - 1) : (j1 * m) & (32 * RX - 1);
@@ -298,16 +255,15 @@ __global__ void __launch_bounds__(64 * CLS, 8 / CLS) ifft2d_pad_kernel(ImagePara
 #pragma unroll
             for (int j2 = 0; j2 < 32; ++j2) {
                 const int row = j2 * CLS + jl;
-                sY[row * kModes + rtile_chunk(row / LINES, ky >> 1) * 2 + (ky & 1)] = v[slot32(j2)];
+                sY[row * kModes + rtile_chunk(REAL ? rtile_pair_key(row / 2) : row, ky >> 1) * 2 + (ky & 1)] = v[slot32(j2)];
             }
         }
         __syncthreads();
         // folded input of lane j1, modes 2c and 2c + 1: u[m] = T[m] (C[m] + coef C[m + 32])
         auto folded = [&](const float2* line, int key, int c, float2& u0, float2& u1) {
-            float4 lo = *reinterpret_cast<const float4*>(line + rtile_chunk(key, c) * 2);
+            const float4 lo = *reinterpret_cast<const float4*>(line + rtile_chunk(key, c) * 2);
             const float4 hi = *reinterpret_cast<const float4*>(line + rtile_chunk(key, c + 16) * 2);
             const float4 t = *reinterpret_cast<const float4*>(twY + tw_index<RY>(j1, 2 * c));
-            if (REAL && c == 0) { lo.x *= 0.5f; lo.y *= 0.5f; }          // ky = 0 has no mirror image
             u0 = cmul(cmadd(make_float2(lo.x, lo.y), coefY, make_float2(hi.x, hi.y)), make_float2(t.x, t.y));
             u1 = cmul(cmadd(make_float2(lo.z, lo.w), coefY, make_float2(hi.z, hi.w)), make_float2(t.z, t.w));
         };
@@ -315,53 +271,38 @@ __global__ void __launch_bounds__(64 * CLS, 8 / CLS) ifft2d_pad_kernel(ImagePara
         for (int x0 = 0; x0 < ROWS; x0 += GROUPS * LINES) {
             const int lr = x0 + g * LINES;
             const int x = RX * (lr / CLS) + part * CLS + lr % CLS;       // image row of local row lr (REAL: the next one is x + 1)
-            const int key = lr / LINES;
-            float2 v[32];
             if constexpr (REAL) {
-                // Hermitian sums h[m] = u[m] + conj(u[32 - m]) of row a, m <= 16; then v[m] = h + i h',
-                // v[32 - m] = conj(h) + i conj(h') with h' the same of row b.  Chunks c and 15 - c hold modes
-                // 2c, 2c + 1, 30 - 2c, 31 - 2c; mode 32 - 2c comes from the step before.
-                float2 h[17];
+                constexpr int N = DY, Q = RealRows<N>::Q, K1 = RealRows<N>::K1, M = RealRows<N>::M;
+                const int key = rtile_pair_key(lr / 2), kb = real_mode<N>(1, j1);
+                const float2 *la = sY + lr * kModes, *lb = la + kModes;
+                float2 aA[M], bA[M], aB[M], bB[M], fa[16], fb[16], v[Q][K1];
 #pragma unroll
-                for (int l = 0; l < 2; ++l) {
-                    const float2* line = sY + (lr + l) * kModes;
-                    auto put = [&](int m, float2 a, float2 b) {          // a = u[m], b = u[(32 - m) % 32]
-                        const float2 s = make_float2(a.x + b.x, a.y - b.y);
-                        if (l == 0) h[m] = s;
-                        else {
-                            v[m] = make_float2(h[m].x - s.y, h[m].y + s.x);
-                            if (m != 0 && m != 16) v[32 - m] = make_float2(h[m].x + s.y, s.x - h[m].y);
-                        }
-                    };
-                    float2 carried = make_float2(0.f, 0.f);
+                for (int k2 = 0; k2 < M; ++k2) {
+                    const int ka = j1 + K1 * k2, kk = kb + K1 * k2;
+                    const int atA = rtile_chunk(key, ka >> 1) * 2 + (ka & 1), atB = rtile_chunk(key, kk >> 1) * 2 + (kk & 1);
+                    aA[k2] = la[atA]; bA[k2] = lb[atA];
+                    aB[k2] = la[atB]; bB[k2] = lb[atB];
+                }
+                real_join<N>(fa, fb, aA, bA, aB, bB, j1 == 0);
+                real_inverse<N>(fa, fb, twY, twX + CLS * 32 + RealRows<N>::SCRATCH * g, j1, g & 1, v);
+                float* row = reinterpret_cast<float*>(dst) + (long long)x * DY + Q * j1;
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        float2 u0, u1, w0, w1;
-                        folded(line, key, c, u0, u1);
-                        folded(line, key, 15 - c, w0, w1);            // modes 30 - 2c, 31 - 2c
-                        if (c == 0) put(0, u0, u0);
-                        else put(2 * c, u0, carried);
-                        put(2 * c + 1, u1, w1);
-                        carried = w0;
-                        if (c == 7) put(16, w0, w0);
+                for (int j = 0; j < K1; ++j) {
+                    const int at = real_slot<N>(j);
+                    if constexpr (Q == 2) {
+                        *reinterpret_cast<float2*>(row + 16 * j) = make_float2(v[0][at].x, v[1][at].x);
+                        *reinterpret_cast<float2*>(row + DY + 16 * j) = make_float2(v[0][at].y, v[1][at].y);
+                    } else {
+                        *reinterpret_cast<float4*>(row + 16 * j) = make_float4(v[0][at].x, v[1][at].x, v[2][at].x, v[3][at].x);
+                        *reinterpret_cast<float4*>(row + DY + 16 * j) = make_float4(v[0][at].y, v[1][at].y, v[2][at].y, v[3][at].y);
                     }
                 }
             } else {
+                float2 v[32];
                 const float2* line = sY + lr * kModes;
 #pragma unroll
-                for (int c = 0; c < 16; ++c) folded(line, key, c, v[2 * c], v[2 * c + 1]);
-            }
-            fft32<SIGN>(v);
-            if constexpr (REAL) {
-                // even lanes write two samples of row a, odd lanes two of row b
-                float* row = reinterpret_cast<float*>(dst) + (long long)(x + (odd ? 1 : 0)) * DY + (j1 & ~1);
-#pragma unroll
-                for (int j2 = 0; j2 < 32; ++j2) {
-                    const float2 o = v[slot32(j2)];
-                    const float got = __shfl_xor_sync(0xffffffffu, odd ? o.x : o.y, 1);
-                    *reinterpret_cast<float2*>(row + RY * j2) = odd ? make_float2(got, o.y) : make_float2(o.x, got);
-                }
-            } else {
+                for (int c = 0; c < 16; ++c) folded(line, lr, c, v[2 * c], v[2 * c + 1]);
+                fft32<SIGN>(v);
                 // Lanes j1 and j1 ^ 1 own samples that alternate in memory: each stores 16 bytes (its own
                 // sample and the neighbour's) for every second j2 and they swap the foreign halves with a
                 // shuffle, so that a group writes a whole 128-byte line per instruction.
