@@ -179,11 +179,10 @@ inline int launch_tc_inst(const DeviceInfo& dev, const TileParams& p, cudaStream
     return TFNO_OK;
 }
 
-// Tensor-core contraction of compact spectra: N a multiple of 64 (64 per launch), K a multiple of 16 up to 64, beta = 0.
+// Tensor-core contraction of compact spectra: N a multiple of 64 (64 per launch), K a multiple of 8 up to 128, beta = 0.
 inline bool cgemm_tc_eligible(const DeviceInfo& dev, const TileParams& p) {
     if (!dev.use_tensor_cores || !dev.status) return false;
-    // K a multiple of 8 (a last chunk of 8 channels is padded with zero weights), at most 96 per
-    // launch (tensor memory) and 128 in two launches, the second adding to C
+    // K a multiple of 8, at most 96 per launch (tensor memory) and 128 in two launches, the second adding to C
     if (p.N % 64 != 0 || p.K < 8 || p.K > 128 || p.K % 8 != 0) return false;
     // several launches (per block of 64 output channels, per half of K > 64), each re-reading its
     // spectra: worth it only when the launches are long
