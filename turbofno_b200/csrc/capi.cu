@@ -608,7 +608,7 @@ int tfno_exec_real(const tfno_plan* plan, const void* x, const void* w, void* y,
 namespace {
 
 struct BackwardWorkspace {
-    size_t offG = 0, offX = 0, offW = 0, offP = 0, total = 0;      // X: first G W^H, then the spectrum of x
+    size_t offG = 0, offX = 0, offP = 0, total = 0;      // X: first G W^H, then the spectrum of x
 };
 
 PerModeParams weight_gradient(const tfno_plan_s& pl, const float2* X, const float2* G, float2* gw, float2* partial, float2 factor, bool real_field) {
@@ -635,7 +635,6 @@ BackwardWorkspace carve_backward(const tfno_plan_s& pl) {
     auto take = [&](size_t& slot, size_t bytes) { slot = off; off += align_up(bytes); };
     take(w.offG, sizeof(float2) * (size_t)(p.N * pl.B * modes));
     take(w.offX, sizeof(float2) * (size_t)(p.K * pl.B * modes));
-    take(w.offW, pl.per_mode ? 0 : sizeof(float2) * (size_t)p.K * p.N);
     take(w.offP, permode_partial_bytes(pl.h->dev, weight_gradient(pl, nullptr, nullptr, nullptr, nullptr, f2(1.f, 0.f), false),
                                        pl.per_mode ? PERMODE_GRAD : PERMODE_GRAD_SHARED));
     w.total = off;
@@ -691,7 +690,6 @@ int tfno_backward(const tfno_plan* plan, int real_field, const void* x, const vo
     char* wsb = static_cast<char*>(workspace);
     float2* G = reinterpret_cast<float2*>(wsb + ws.offG);
     float2* X = reinterpret_cast<float2*>(wsb + ws.offX);
-    float2* Wc = reinterpret_cast<float2*>(wsb + ws.offW);
     const float2* win = static_cast<const float2*>(w);
     const float2 alpha = f2(p.alpha_re, -p.alpha_im);
     const long long modes = (p.rank == 1) ? kModes : (long long)kModes * kModes;
@@ -708,11 +706,9 @@ int tfno_backward(const tfno_plan* plan, int real_field, const void* x, const vo
             q.alpha = q.alpha0 = alpha;
             rc = launch_permode(dev, q, PERMODE_APPLY_CONJ, st);
         } else {
-            rc = launch_conjugate(dev, win, p.w_stride_k, p.w_stride_n, p.K, p.N, Wc, st);
-            if (rc != TFNO_OK) return rc;
             TileParams t{};
             t.rows = pl.B * (modes / kModes); t.K = p.N; t.N = p.K;
-            t.x = G; t.w = Wc; t.w_stride_k = 1; t.w_stride_n = p.N; t.y = X;
+            t.x = G; t.w = win; t.w_stride_k = p.w_stride_n; t.w_stride_n = p.w_stride_k; t.conj_w = 1; t.y = X;
             t.alpha = alpha; t.beta = f2(0.f, 0.f); t.conj_inverse = 1;
             rc = launch_tile<false, false>(dev, p.DY, t, st);
         }

@@ -61,6 +61,7 @@ struct CgemmTcParams {
     const float2* w; long long w_stride_k, w_stride_n;
     float2* c; long long c_stride_n;             // C[m + n * c_stride_n]
     float2 alpha;
+    int conj_w;                          // the weights enter conjugated
     int accumulate;                      // 1: C += alpha A W (the second of two launches over the halves of the channels)
     int* status;
 };
@@ -170,7 +171,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) cgemm_tc_kernel(CgemmTcParams
                     uint32_t hi[8], lo[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const float2 w1 = cmul(*reinterpret_cast<const float2*>(wst + n * wrow + (8 * c + j) * 8), p.alpha);
+                        float2 w1 = *reinterpret_cast<const float2*>(wst + n * wrow + (8 * c + j) * 8);
+                        if (p.conj_w) w1.y = -w1.y;
+                        w1 = cmul(w1, p.alpha);
                         // Re row: [ Wr | -Wi ],  Im row: [ Wi | Wr ]  against  S = [ Ar ; Ai ]
                         const float x = im_row ? (part ? w1.x : w1.y) : (part ? -w1.y : w1.x);
                         const float h = tf32_hi(x);

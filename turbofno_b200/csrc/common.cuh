@@ -167,8 +167,6 @@ struct PerModeParams {
 enum PermodeKind { PERMODE_APPLY, PERMODE_APPLY_CONJ, PERMODE_GRAD, PERMODE_GRAD_SHARED };
 size_t permode_partial_bytes(const DeviceInfo& dev, const PerModeParams& p, PermodeKind kind);
 int launch_permode(const DeviceInfo& dev, PerModeParams p, PermodeKind kind, cudaStream_t st);
-// dst[k*N + n] = conj(w[k*sk + n*sn])
-int launch_conjugate(const DeviceInfo& dev, const float2* w, long long sk, long long sn, int K, int N, float2* dst, cudaStream_t st);
 
 #if defined(__CUDACC__)
 // Programmatic dependent launch.  A kernel launched `early` may have CTAs resident while the previous kernel of the stream

@@ -206,7 +206,7 @@ inline int launch_cgemm_tc_inst(const DeviceInfo& dev, const TileParams& p, cuda
     q.a = p.x; q.a_stride_k = M;
     q.w = p.w; q.w_stride_k = p.w_stride_k; q.w_stride_n = p.w_stride_n;
     q.c = p.y; q.c_stride_n = M;
-    q.alpha = p.alpha; q.status = dev.status;
+    q.alpha = p.alpha; q.conj_w = p.conj_w; q.status = dev.status;
     q.accumulate = accumulate ? 1 : 0;
     long long grid = dev.sms;
     if (grid > q.tiles) grid = q.tiles;

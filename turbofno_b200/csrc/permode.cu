@@ -4,16 +4,6 @@
 namespace tfno {
 namespace {
 
-// dst[k*N + n] = conj(w[k, n])
-__global__ void __launch_bounds__(256) conjugate_kernel(const float2* w, long long sk, long long sn, int K, int N, float2* dst) {
-    follow_previous_kernel();
-    admit_next_kernel();
-    for (int e = blockIdx.x * 256 + threadIdx.x; e < K * N; e += gridDim.x * 256) {
-        const float2 v = w[(e / N) * sk + (e % N) * sn];
-        dst[e] = make_float2(v.x, -v.y);
-    }
-}
-
 bool is_grad(PermodeKind kind) { return kind == PERMODE_GRAD || kind == PERMODE_GRAD_SHARED; }
 
 long long blocks_per_split(const PerModeParams& p, int nt) {
@@ -107,10 +97,6 @@ int launch_permode(const DeviceInfo& dev, PerModeParams p, PermodeKind kind, cud
     long long grid = (sums + 255) / 256;
     if (grid > 8LL * dev.sms) grid = 8LL * dev.sms;
     return launch_chained(permode_reduce_kernel, dim3((unsigned)grid), 256, 0, st, true, 1, p);
-}
-
-int launch_conjugate(const DeviceInfo& dev, const float2* w, long long sk, long long sn, int K, int N, float2* dst, cudaStream_t st) {
-    return launch_chained(conjugate_kernel, dim3((unsigned)((K * N + 255) / 256)), 256, 0, st, true, 1, w, sk, sn, K, N, dst);
 }
 
 }  // namespace tfno

@@ -49,6 +49,7 @@ struct TileParams {
     float2 alpha, beta;      // beta only read when !INV
     float2 inv_gain;         // alpha * scale folded into the inverse twiddles (INV)
     int conj_inverse;        // 1: true inverse, 0: second forward transform
+    int conj_w;              // !FWD && !INV: the weights enter conjugated
 };
 
 // After forward_trunc<R>: lane r holds modes 64/R*r + j in v[slot(j)].  Write them as 16-byte
@@ -135,6 +136,7 @@ __global__ void __launch_bounds__(kThreads, 1) spectral_tile_kernel(TileParams p
                 int kk, n;
                 if (p.w_stride_n == 1) { n = e % N; kk = e / N; } else { kk = e % kSlabK; n = e / kSlabK; }
                 wreg[i] = load_global(wbase + (long long)(k0 + kk) * p.w_stride_k + (long long)n * p.w_stride_n);
+                if (!FWD && !INV && p.conj_w) wreg[i].y = -wreg[i].y;
             }
         };
         auto stash_slab = [&](int buf) {
