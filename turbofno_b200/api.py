@@ -15,9 +15,7 @@ from ._lib import Problem, VARIANT, check
 
 
 def _ptr(t):
-    if t is None:
-        return None
-    return ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def _out_ptr(t):
@@ -40,8 +38,10 @@ def _plain(t, stream=None):
 def _stream_ptr(stream=None, device=None):
     """cudaStream_t of `stream`, or of the current stream of `device` (not of the current device:
     the tensors decide where the work runs)."""
-    s = stream if stream is not None else torch.cuda.current_stream(device)
-    return ctypes.c_void_p(s.cuda_stream)
+    if stream is not None:
+        return stream.cuda_stream
+    index = None if device is None else device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def _capturing(device, stream=None):
@@ -175,6 +175,8 @@ class SpectralConv:
         self.workspace_bytes = optional or int(self.lib.tfno_workspace_bytes(plan))
         self._ws = None
         self._device = torch.device("cuda", self.handle.device)
+        self._shapes = expected_shapes(rank, layout, self.B, p.K, p.N, p.DY, p.DX, self.per_mode)
+        self._backward_bytes = None
 
     def out_shape(self):
         p = self.problem
@@ -199,12 +201,16 @@ class SpectralConv:
         check(self.lib.tfno_plan_set_host_chunk(self._plan, int(batch_items)), "tfno_plan_set_host_chunk")
 
     def _check_call(self, x, w, y, workspace):
-        p = self.problem
-        check_shapes(self.rank, self.layout, self.B, p.K, p.N, p.DY, p.DX, x.shape, w.shape, None if y is None else y.shape, self.per_mode)
-        dev = self._device
-        for name, t in (("x", x), ("w", w), ("y", y), ("workspace", workspace)):
-            if t is not None and t.device != dev:
-                raise ValueError("%s is on %s, the plan's handle on %s" % (name, t.device, dev))
+        # an eager call of a small layer is as long as these checks: the shapes and the device number are the plan's own
+        ex, ew, ey = self._shapes
+        if x.shape != ex or w.shape != ew or (y is not None and y.shape != ey):
+            p = self.problem
+            check_shapes(self.rank, self.layout, self.B, p.K, p.N, p.DY, p.DX, x.shape, w.shape, None if y is None else y.shape, self.per_mode)
+        dev = self.handle.device
+        for t in (x, w, y, workspace):
+            if t is not None and t.get_device() != dev:
+                name = "x" if t is x else "w" if t is w else "y" if t is y else "workspace"
+                raise ValueError("%s is on %s, the plan's handle on %s" % (name, t.device, self._device))
         if workspace is not None:
             if not (workspace.is_cuda and workspace.is_contiguous()):
                 raise ValueError("workspace must be a contiguous CUDA tensor")
@@ -227,19 +233,21 @@ class SpectralConv:
         ws = workspace
         if ws is None:
             if not self._optional_ws:
-                ws = self.workspace(x.device)
+                ws = self.workspace(self._device) if self.workspace_bytes else None
             elif not _capturing(x.device, stream):
                 ws = self.call_scratch(x.device, stream)
         return self._launch(x, w, y, ws, stream)
 
     def _launch(self, x, w, y, ws, stream=None):
         """The call itself, on operands that fit the plan (scratch that need not be there may be None or short)."""
-        st = _stream_ptr(stream, x.device)
+        st = _stream_ptr(stream, self._device)
         if self._optional_ws:
             nbytes = 0 if ws is None else ws.numel() * ws.element_size()
-            check(self.lib.tfno_exec_scratch(self._plan, _ptr(x), _ptr(w), _ptr(y), _ptr(ws), nbytes, st), "tfno_exec_scratch")
+            check(self.lib.tfno_exec_scratch(self._plan, x.data_ptr(), w.data_ptr(), y.data_ptr(), _ptr(ws), nbytes, st), "tfno_exec_scratch")
         else:
-            check(self.lib.tfno_exec(self._plan, _ptr(x), _ptr(w), _ptr(y), _ptr(ws), st), "tfno_exec")
+            status = self.lib.tfno_exec(self._plan, x.data_ptr(), w.data_ptr(), y.data_ptr(), _ptr(ws), st)
+            if status:
+                check(status, "tfno_exec")
         return y
 
     def exec_real(self, x, w, y=None, stream=None):
@@ -267,7 +275,9 @@ class SpectralConv:
         if grad_x is not None or grad_w is not None:
             self._check_call(x if grad_x is None else grad_x, w if grad_w is None else grad_w, None, None)
         x, w, grad_y = _plain(x, stream), _plain(w, stream), _plain(grad_y, stream)
-        ws = self._scratch(int(self.lib.tfno_backward_workspace_bytes(self._plan)), x.device, stream)
+        if self._backward_bytes is None:
+            self._backward_bytes = int(self.lib.tfno_backward_workspace_bytes(self._plan))
+        ws = self._scratch(self._backward_bytes, x.device, stream)
         check(self.lib.tfno_backward(self._plan, int(real), _ptr(x), _ptr(w), _ptr(grad_y), _out_ptr(grad_x), _out_ptr(grad_w), _ptr(ws),
                                      _stream_ptr(stream, x.device)), "tfno_backward")
 

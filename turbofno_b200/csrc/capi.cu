@@ -48,11 +48,14 @@ struct tfno_plan_s {
 namespace {
 
 struct DeviceGuard {
-    int prev = -1;
+    int prev = -1;                      // the device to go back to, if another one was current
     bool ok = true;
     explicit DeviceGuard(int dev) {
-        if (cudaGetDevice(&prev) != cudaSuccess) { ok = false; return; }
-        if (prev != dev && cudaSetDevice(dev) != cudaSuccess) ok = false;
+        int current = -1;
+        if (cudaGetDevice(&current) != cudaSuccess) { ok = false; return; }
+        if (current == dev) return;
+        prev = current;
+        if (cudaSetDevice(dev) != cudaSuccess) ok = false;
     }
     ~DeviceGuard() { if (prev >= 0) cudaSetDevice(prev); }
 };
