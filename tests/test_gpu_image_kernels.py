@@ -103,3 +103,25 @@ def test_per_mode_weights_in_other_orders(cuda, order):
     lib.tfno_plan_destroy(plan)
     s = torch.einsum("bkm,knm->bnm", torch.fft.fft(x.to(torch.complex128))[..., :64], w.to(torch.complex128))
     _check(y, torch.fft.ifft(torch.cat([s, s.new_zeros(B, N, DY - 64)], -1)))
+
+
+@pytest.mark.parametrize("DX,DY", [(128, 128), (128, 256), (256, 128), (256, 256)])
+@pytest.mark.parametrize("images", [152, 200, 296, 304, 320])       # just above a wave of images, two thirds of one, a full one
+@pytest.mark.parametrize("real", [False, True])
+def test_forward_images_around_the_waves_of_a_launch(cuda, DX, DY, images, real):
+    """One CTA or a cluster of them per image, by how much of the last wave would stay empty."""
+    import torch
+    import turbofno_b200 as t
+
+    g = torch.Generator(device="cuda").manual_seed(images)
+    K, B = 8, images // 8
+    plan = t.SpectralConv(2, B, DY, K, 64, DX=DX, layout="batch_major", per_mode_weights=real, x_modes_centered=real)
+    if real:
+        x, w = torch.rand((B, K, DX, DY), generator=g, device="cuda") * 2 - 1, _field(g, K, 64, 64, 64)
+        half = torch.ones(64, dtype=torch.float64, device="cuda")
+        half[0] = 0.5
+        _check(plan.exec_real(x, w), 2 * _layer(x, w.to(torch.complex128) * half, True).real)
+    else:
+        x, w = _field(g, B, K, DX, DY), _field(g, K, 64)
+        _check(plan(x, w), _layer(x, w))
+    plan.close()

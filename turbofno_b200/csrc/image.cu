@@ -19,15 +19,25 @@ int launch_forward(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st)
     if (C == 1 && clusters > (long long)dev.sms * occ) clusters = (long long)dev.sms * occ;
     return launch_chained(kernel, dim3((unsigned)(clusters * C)), THREADS, smem, st, clusters == p.nimg, C, p);
 }
+// A cluster of CTAs of 64 rows per image, or one CTA per image.  The cluster takes an image at a time, so its launches have no
+// last wave to speak of, but the exchange through distributed shared memory costs more per image:
+//   - while two such CTAs per SM cover the images: us, cluster / one CTA, 80 images of 128 x 256 11.6 / 11.7, of 256 x 256 16.1 / 18.9,
+//     of 256 x 128 15.4 / 16.2, of 128 x 128 11.0 / 10.9; a few images up to twice as fast (16 of 256 x 256 9.2 / 16.7);
+//   - beyond one wave of images, where one CTA per image would leave more of its last wave empty than the exchange costs (rows of
+//     256 samples 16 %, 20 % for real samples or two images per SM; rows of 128, which shuffle on both sides, 45 %; of 128 x 128 and
+//     real ones never).  256 x 256: 152 images 28.4 / 37.0, 200 33.9 / 37.8, 296 46.2 / 41.6, 448 62.3 / 69.5, 512 68.6 / 71.3, 592 77.6 /
+//     72.5; real 152 21.1 / 27.7, 448 47.0 / 50.9, 512 52.0 / 51.1.  128 x 256: 320 29.1 / 30.0, 448 35.9 / 37.1, 512 39.6 / 38.5.  256 x 128: 152
+//     24.0 / 29.8, 200 28.9 / 30.1, 320 44.0 / 42.7; real 152 21.8 / 21.1.  128 x 128: 320 23.1 / 23.0, 448 29.9 / 29.1.
+template <int RX, int RY, bool REAL>
+bool image_clusters(const DeviceInfo& dev, long long images) {
+    if (images * (RX / 2) <= 2LL * dev.sms) return true;
+    constexpr int COST = RY == 8 ? (REAL || RX == 4 ? 120 : 116) : REAL || RX == 4 ? 0 : 145;      // per cent of one CTA's time per image
+    const long long wave = dev.sms * (RX == 8 ? 1LL : 2LL);
+    return COST && images > wave && images * COST < 100 * ((images + wave - 1) / wave) * wave;
+}
 template <int RX, int RY, bool REAL>
 int launch_forward_split(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st) {
-    // Few images: a cluster of CTAs of 64 rows per image, while two such CTAs per SM cover them.  Kernel times of the
-    // cluster against one CTA per image, us: 8 images of 128 x 256 7.3 / 9.2, 16 of 256 x 256 9.2 / 16.7; at the line 72 of
-    // 256 x 256 15.6 / 18.3 and of 256 x 128 14.6 / 15.7, 144 of 128 x 256 13.4 / 13.4 and of 128 x 128 11.9 / 10.9 (real samples
-    // 24 % better to 14 % worse).  Beyond it the exchange through distributed shared memory costs as much as the parallelism
-    // gives: 144 of 256 x 256 27.0 / 23.3, 512 68.8 / 70.2, 512 of 256 x 128 63.2 / 54.1; just above a full wave of one-CTA images
-    // (148 of DX = 256, 296 of DX = 128) the cluster still wins: 152 of 256 x 256 28.6 / 36.9, 304 47.6 / 54.2.
-    if (p.nimg * (RX / 2) <= 2LL * dev.sms) return launch_forward<RX, RY, RX / 2, REAL>(dev, p, st);
+    if (image_clusters<RX, RY, REAL>(dev, p.nimg)) return launch_forward<RX, RY, RX / 2, REAL>(dev, p, st);
     return launch_forward<RX, RY, 1, REAL>(dev, p, st);
 }
 
