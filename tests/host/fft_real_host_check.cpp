@@ -13,7 +13,7 @@ static double urand() { return 2.0 * rand() / RAND_MAX - 1.0; }
 
 template <int N> static void check() {
     constexpr int L = RealRows<N>::L, K1 = RealRows<N>::K1, Q = RealRows<N>::Q, M = RealRows<N>::M;
-    alignas(16) static float2 tw[N];
+    alignas(16) static float2 tw[N / 2];
     fill_real_table<N>(tw, 0, 1);
     auto part_k1 = [](int part, int d) { return real_mode<N>(part, d); };
     double fe = 0, fr = 0, ie = 0, ir = 0;
@@ -27,12 +27,12 @@ template <int N> static void check() {
                 for (int j = 0; j < K1; ++j) v[r][q][j] = make_float2(a[0][16 * j + Q * r + q], a[1][16 * j + Q * r + q]);
                 real_inner<N, -1>(v[r][q]);
             }
-        for (int d = 0; d < L; ++d)
-            for (int part = 0; part < 2; ++part) {
+        for (int d = 0; d < L; ++d) {
+            for (int part = 0; part < 2; ++part)
                 for (int r = 0; r < L; ++r)
                     for (int q = 0; q < Q; ++q) f[d][part][Q * r + q] = v[r][q][real_slot<N>(part_k1(part, d))];
-                real_combine<N>(f[d][part], tw, part, d);
-            }
+            real_combine<N>(f[d][0], f[d][1], tw, d);
+        }
         for (int d = 0; d < L; ++d)
             for (int part = 0; part < 2; ++part)
                 for (int k2 = 0; k2 < M; ++k2) {
@@ -56,8 +56,7 @@ template <int N> static void check() {
             for (auto& e : f[d][0]) e = make_float2(NAN, NAN);   // inputs that must not be read
             for (auto& e : f[d][1]) e = make_float2(NAN, NAN);
             real_join<N>(f[d][0], f[d][1], m[0][0], m[0][1], m[1][0], m[1][1], d == 0);
-            real_spread<N, 0>(f[d][0], tw, d);
-            real_spread<N, 1>(f[d][1], tw, d);
+            real_spread<N>(f[d][0], f[d][1], tw, d);
         }
         for (int r = 0; r < L; ++r)
             for (int q = 0; q < Q; ++q) {

@@ -29,36 +29,44 @@ template <int N, int S> TFNO_HD void real_inner(float2 (&v)[N / 16]) {
     else fft8<S>(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], make_odd_sign(1.0f));
 }
 
-// Factors of (part, lane, rho); those of rho, rho + 1 of the L lanes are adjacent.  N entries.
-template <int N> TFNO_HD constexpr int real_table_index(int part, int d, int rho) { return ((part * 8 + (rho >> 1)) * RealRows<N>::L + d) * 2 + (rho & 1); }
+// Factors W_N^{rho d} of lane d; those of rho, rho + 1 of the L lanes are adjacent.  N/2 entries.  Part B's are their conjugates;
+// lane 0, whose part A needs none, has those of its part B: W_N^{rho K1/2}.
+template <int N> TFNO_HD constexpr int real_table_index(int d, int rho) { return ((rho >> 1) * RealRows<N>::L + d) * 2 + (rho & 1); }
 template <int N> TFNO_HD void fill_real_table(float2* tw, int tid, int nthreads) {
     constexpr int L = RealRows<N>::L, K1 = RealRows<N>::K1;
-    for (int i = tid; i < N; i += nthreads) {
-        const int part = i / (16 * L), d = (i / 16) % L, rho = i % 16;
-        const int e = part == 0 ? rho * d : -rho * (d ? d : K1 / 2);
-        tw[real_table_index<N>(part, d, rho)] = unit_root(e & (N - 1), N, -1.0f);
+    for (int i = tid; i < N / 2; i += nthreads) {
+        const int d = i / 16, rho = i % 16;
+        tw[real_table_index<N>(d, rho)] = unit_root((rho * (d ? d : K1 / 2)) & (N - 1), N, -1.0f);
     }
+    static_assert(16 * L == N / 2, "sixteen factors per lane");
 }
 // first k of a part
 template <int N> TFNO_HD int real_mode(int part, int d) { return part == 0 ? d : d ? RealRows<N>::K1 - d : RealRows<N>::K1 / 2; }
 
 TFNO_HD float2 cmul_conj(float2 a, float2 b) { return make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y); }
-// f[at(rho)] times the factors of (part, lane), or their conjugates
-template <int N, bool CONJ, typename At>
-TFNO_HD void real_twiddle(float2 (&f)[16], const float2* tw, int part, int d, At at) {
+// the parts' f[at(rho)] times their factors (forward) or the conjugates of them (inverse)
+template <int N, bool INVERSE, typename At>
+TFNO_HD void real_twiddle(float2 (&fa)[16], float2 (&fb)[16], const float2* tw, int d, At at) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        const float4 t = *reinterpret_cast<const float4*>(tw + real_table_index<N>(part, d, 2 * j));
-        const float2 t0 = make_float2(t.x, t.y), t1 = make_float2(t.z, t.w);
-        if (j) f[at(2 * j)] = CONJ ? cmul_conj(f[at(2 * j)], t0) : cmul(f[at(2 * j)], t0);
-        f[at(2 * j + 1)] = CONJ ? cmul_conj(f[at(2 * j + 1)], t1) : cmul(f[at(2 * j + 1)], t1);
+        const float4 t = *reinterpret_cast<const float4*>(tw + real_table_index<N>(d, 2 * j));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (j == 0 && h == 0) continue;
+            const float2 w = h ? make_float2(t.z, t.w) : make_float2(t.x, t.y);
+            const float2 wa = d ? w : make_float2(1.f, 0.f);
+            float2 &a = fa[at(2 * j + h)], &b = fb[at(2 * j + h)];
+            a = INVERSE ? cmul_conj(a, wa) : cmul(a, wa);
+            b = INVERSE ? cmul(b, w) : cmul_conj(b, w);
+        }
     }
 }
 
-// ---- forward, after the exchange: f[rho] of a part -> k2 (part A) or s (part B) at f[slot16(.)] ----
-template <int N> TFNO_HD void real_combine(float2 (&f)[16], const float2* tw, int part, int d) {
-    real_twiddle<N, false>(f, tw, part, d, [](int rho) { return rho; });
-    fft16<-1>(f);
+// ---- forward, after the exchange: f[rho] of the parts -> k2 (part A) and s (part B) at f[slot16(.)] ----
+template <int N> TFNO_HD void real_combine(float2 (&fa)[16], float2 (&fb)[16], const float2* tw, int d) {
+    real_twiddle<N, false>(fa, fb, tw, d, [](int rho) { return rho; });
+    fft16<-1>(fa);
+    fft16<-1>(fb);
 }
 // mode real_mode(part, d) + K1 k2 of rows a and b, both times 2
 template <int N>
@@ -110,10 +118,11 @@ TFNO_HD void real_expand(float2 (&f)[16]) {
         for (int k1 = 0; k1 < 4; ++k1) dft4<1>(f[4 * k1], f[4 * k1 + 1], f[4 * k1 + 2], f[4 * k1 + 3]);
     }
 }
-template <int N, int PART>
-TFNO_HD void real_spread(float2 (&f)[16], const float2* tw, int d) {          // result for rho at f[slot16(rho)]
-    real_expand<N, PART>(f);
-    real_twiddle<N, true>(f, tw, PART, d, [](int rho) { return slot16(rho); });
+template <int N>
+TFNO_HD void real_spread(float2 (&fa)[16], float2 (&fb)[16], const float2* tw, int d) {          // result for rho at f[slot16(rho)]
+    real_expand<N, 0>(fa);
+    real_expand<N, 1>(fb);
+    real_twiddle<N, true>(fa, fb, tw, d, [](int rho) { return slot16(rho); });
 }
 
 #if defined(__CUDACC__)
@@ -167,15 +176,14 @@ TFNO_D void real_forward(float2 (&v)[RealRows<N>::Q][N / 16], const float2* tw, 
             else
                 real_exchange128(scratch, r, odd_group, [&](int e, int h) { return v[q + h][real_slot<N>(k1(e))]; }, [&](int c, int h, float2 x) { f[4 * c + q + h] = x; });
         }
-        real_combine<N>(f, tw, part, r);
     }
+    real_combine<N>(fa, fb, tw, r);
 }
 // Inputs of the parts (consumed) -> samples of rho = Q r + q: j at v[q][real_slot<N>(j)]
 template <int N>
 TFNO_D void real_inverse(float2 (&fa)[16], float2 (&fb)[16], const float2* tw, float2* scratch, int r, int odd_group, float2 (&v)[RealRows<N>::Q][N / 16]) {
     constexpr int K1 = RealRows<N>::K1, Q = RealRows<N>::Q;
-    real_spread<N, 0>(fa, tw, r);
-    real_spread<N, 1>(fb, tw, r);
+    real_spread<N>(fa, fb, tw, r);
 #pragma unroll
     for (int part = 0; part < 2; ++part) {
         const float2 (&f)[16] = part ? fb : fa;

@@ -42,7 +42,7 @@ TFNO_HD int xtile_index(int row, int col) {
 // REAL: the inverse reads two or four adjacent chunks of every second row
 TFNO_HD int rtile_pair_key(int pair) { return ((pair & 1) << 2) | (pair & 2) | ((pair >> 2) & 1); }
 template <int RX, int RY, int C, bool REAL> inline constexpr size_t fwd_image_smem_bytes() {
-    return (size_t)(32 * RX * (64 / C) + RX * 32 + (REAL ? RY * 32 + 8 * (64 * RX / C) : RY == 8 ? kTable256 + 64 * (8 * RX / C) : RY * 32)) * sizeof(float2);
+    return (size_t)(32 * RX * (64 / C) + RX * 32 + (REAL ? RY * 16 + 8 * (64 * RX / C) : RY == 8 ? kTable256 + 64 * (8 * RX / C) : RY * 32)) * sizeof(float2);
 }
 template <int RY, int CLS> inline constexpr size_t inv64_image_smem_bytes() {
     return (size_t)(64 * CLS * kModes + RY * 64 + CLS * 64) * sizeof(float2);
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(64 * RX / C, 8 * C / RX) fft2d_trunc_kernel(Im
             if constexpr (REAL) {
                 constexpr int N = DY, Q = RealRows<N>::Q, K1 = RealRows<N>::K1, M = RealRows<N>::M;
                 float2 fa[16], fb[16];
-                real_forward<N>(*reinterpret_cast<float2(*)[Q][K1]>(&v[0]), twY, twY + N + RealRows<N>::SCRATCH * g, r, g & 1, fa, fb);
+                real_forward<N>(*reinterpret_cast<float2(*)[Q][K1]>(&v[0]), twY, twY + N / 2 + RealRows<N>::SCRATCH * g, r, g & 1, fa, fb);
                 if (C > 1 && i0 == 0) cluster_wait();
                 const int kb = real_mode<N>(1, r);
 #pragma unroll
