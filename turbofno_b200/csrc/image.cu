@@ -87,7 +87,7 @@ int launch_image(const DeviceInfo& dev, const ImageParams& p, bool inverse, cuda
 }  // namespace
 
 bool fft2d_fits(const DeviceInfo& dev) {
-    return (long long)fwd_image_smem_bytes<8, 8, 1, true>() <= dev.max_smem_optin;      // the largest of the instances below
+    return (long long)fwd_image_smem_bytes<8, 8, 1, false>() <= dev.max_smem_optin;      // the largest of the instances below
 }
 
 // Residue classes per inverse CTA: two (128 threads) except at 256 x 256, where four (256 threads, half as many
