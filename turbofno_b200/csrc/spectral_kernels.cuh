@@ -13,7 +13,7 @@
 // forward transform of a row is never recomputed per N-tile (grid.y = N/64 in the reference).
 #pragma once
 #include "common.cuh"
-#include "fft64.cuh"
+#include "fft32.cuh"
 
 namespace tfno {
 
@@ -52,15 +52,15 @@ struct TileParams {
     int conj_w;              // !FWD && !INV: the weights enter conjugated
 };
 
-// After forward_trunc<R>: lane r holds modes 64/R*r + j in v[slot(j)].  Write them as 16-byte
+// After forward_trunc32<R>: lane r holds modes 64/R*r + j in v[slot32(j)].  Write them as 16-byte
 // chunks into a swizzled tile row.
 template <int R>
-TFNO_D void store_modes_to_tile(const float2 (&v)[64], float2* tile, int row, int r) {
+TFNO_D void store_modes_to_tile(const float2 (&v)[32], float2* tile, int row, int r) {
     constexpr int PER = 64 / R;
 #pragma unroll
     for (int j = 0; j < PER; j += 2) {
         int m = PER * r + j;
-        float4 q = make_float4(v[slot(j)].x, v[slot(j)].y, v[slot(j + 1)].x, v[slot(j + 1)].y);
+        float4 q = make_float4(v[slot32(j)].x, v[slot32(j)].y, v[slot32(j + 1)].x, v[slot32(j + 1)].y);
         *reinterpret_cast<float4*>(tile + row * kModes + swz_chunk(row, m >> 1) * 2) = q;
     }
 }
@@ -68,18 +68,25 @@ TFNO_D void store_modes_to_tile(const float2 (&v)[64], float2* tile, int row, in
 // ----------------------------------------------------------------------------------------------
 // The row-tile kernel
 // ----------------------------------------------------------------------------------------------
+// The forward transform runs on the 32-point register FFT, L = 2 R = DY/32 lanes per signal: what counts here is the chain of
+// one row, and a signal on twice the lanes is transformed in half the time while there are lanes to spare (8 channels of 128
+// samples keep 32 of them busy, 32 channels of 256 all 256).  The inverse has N signals and stays on 64 samples per lane:
+// its table for twice the lanes would take shared memory from the widest layers.  The first weights travel beside the
+// forward transforms.  Calls back to back, us, with 64 samples per lane and now: 64 rows, 32 -> 128 channels, 256 samples 12.7 -> 12.0;
+// 64 x 16 -> 64 of 1024 24.7 -> 24.3; 140 x 72 -> 64 of 256 22.6 -> 19.4; 1200 x 200 -> 128 659 -> 610.
 template <int R, bool FWD, bool INV, int NB>   // NB = N / 64
 __global__ void __launch_bounds__(kThreads, 1) spectral_tile_kernel(TileParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2* sA = reinterpret_cast<float2*>(smem_raw);                 // [K][64] swizzled
     float2* sC = sA + (size_t)p.K * kModes;                            // [N][64] swizzled (INV only)
     float2* sW = sC + (INV ? (size_t)p.N * kModes : 0);                // [2][kSlabK][N]
-    float2* twF = sW + 2 * kSlabK * (p.N + kWPad);                               // [R][64]
-    float2* twI = twF + (FWD ? R * 64 : 0);                            // [R][64]
+    constexpr int L = 2 * R;                                           // lanes per signal, forward
+    float2* twF = sW + 2 * kSlabK * (p.N + kWPad);                               // [L][32]
+    float2* twI = twF + (FWD ? L * 32 : 0);                            // [R][64]
 
     const int tid = threadIdx.x;
     const int K = p.K, N = p.N;
-    if (FWD) fill_forward_table<R>(twF, tid, kThreads);
+    if (FWD) fill_forward_table32<L>(twF, tid, kThreads);
     if (INV) fill_inverse_table<R>(twI, tid, kThreads, p.inv_gain, p.conj_inverse != 0);
     __syncthreads();
 
@@ -90,24 +97,49 @@ __global__ void __launch_bounds__(kThreads, 1) spectral_tile_kernel(TileParams p
     const float2* wbase = p.w + (long long)blockIdx.y * N * p.w_stride_n;
     float2* ybase = p.y + (long long)blockIdx.y * N * (INV ? p.y_stride_n : M);
 
+    constexpr int WPT = kSlabK * 64 * NB / kThreads;     // weight elements per thread per slab
+    float2 wreg[WPT];
+    auto fetch_slab = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < WPT; ++i) {
+            int e = tid + i * kThreads;
+            int kk, n;
+            if (p.w_stride_n == 1) { n = e % N; kk = e / N; } else { kk = e % kSlabK; n = e / kSlabK; }
+            wreg[i] = load_global(wbase + (long long)(k0 + kk) * p.w_stride_k + (long long)n * p.w_stride_n);
+            if (!FWD && !INV && p.conj_w) wreg[i].y = -wreg[i].y;
+        }
+    };
+    auto stash_slab = [&](int buf) {
+#pragma unroll
+        for (int i = 0; i < WPT; ++i) {
+            int e = tid + i * kThreads;
+            int kk, n;
+            if (p.w_stride_n == 1) { n = e % N; kk = e / N; } else { kk = e % kSlabK; n = e / kSlabK; }
+            sW[(buf * kSlabK + kk) * (N + kWPad) + n] = wreg[i];
+        }
+    };
     follow_previous_kernel();
     for (long long row = blockIdx.x; row < p.rows; row += gridDim.x) {
         if (gridDim.x >= p.rows) admit_next_kernel();
+        fetch_slab(0);                                  // arrives beside the transforms
         // ---------------- stage 1: spectrum tile sA[k][m] ----------------
         if (FWD) {
-            constexpr int GROUPS = kThreads / R;
-            const int g = tid / R, r = tid % R;
-            const int warp_g0 = (tid & ~31) / R;        // first group of this warp
+            constexpr int GROUPS = kThreads / L;
+            const int g = tid / L, r = tid % L;
+            const int warp_g0 = (tid & ~31) / L;        // first group of this warp
+            const float2 coef = round1_coef32<L>(r);
             for (int k0 = 0; k0 < K; k0 += GROUPS) {
                 // Whole warps beyond K skip; inside a partly filled warp the spare lanes redo
-                // channel K-1 so that every lane takes part in the shuffles of forward_trunc.
+                // channel K-1 so that every lane takes part in the shuffles of forward_trunc32.
                 if (k0 + warp_g0 >= K) continue;
                 const bool live = k0 + g < K;
                 const int k = live ? k0 + g : K - 1;
-                float2 v[64];
-                load_decimated_paired<R>(v, p.x + row * p.x_stride_row + (long long)k * p.x_stride_k, r);
-                forward_trunc<R>(v, twF, r);
-                if (live) store_modes_to_tile<R>(v, sA, k, r);
+                const float2* sig = p.x + row * p.x_stride_row + (long long)k * p.x_stride_k + r;
+                float2 v[32];
+#pragma unroll
+                for (int i = 0; i < 32; ++i) v[i] = load_global(sig + L * i);
+                forward_trunc32<L>(v, twF, r, 1, coef);
+                if (live) store_modes_to_tile<L>(v, sA, k, r);
             }
         } else {
             // compact spectrum: 64 consecutive m per channel
@@ -127,28 +159,6 @@ __global__ void __launch_bounds__(kThreads, 1) spectral_tile_kernel(TileParams p
 #pragma unroll
                 for (int j = 0; j < 4; ++j) acc[b][i][j] = make_float2(0.f, 0.f);
 
-        constexpr int WPT = kSlabK * 64 * NB / kThreads;     // weight elements per thread per slab
-        float2 wreg[WPT];
-        auto fetch_slab = [&](int k0) {
-#pragma unroll
-            for (int i = 0; i < WPT; ++i) {
-                int e = tid + i * kThreads;
-                int kk, n;
-                if (p.w_stride_n == 1) { n = e % N; kk = e / N; } else { kk = e % kSlabK; n = e / kSlabK; }
-                wreg[i] = load_global(wbase + (long long)(k0 + kk) * p.w_stride_k + (long long)n * p.w_stride_n);
-                if (!FWD && !INV && p.conj_w) wreg[i].y = -wreg[i].y;
-            }
-        };
-        auto stash_slab = [&](int buf) {
-#pragma unroll
-            for (int i = 0; i < WPT; ++i) {
-                int e = tid + i * kThreads;
-                int kk, n;
-                if (p.w_stride_n == 1) { n = e % N; kk = e / N; } else { kk = e % kSlabK; n = e / kSlabK; }
-                sW[(buf * kSlabK + kk) * (N + kWPad) + n] = wreg[i];
-            }
-        };
-        fetch_slab(0);
         stash_slab(0);
         __syncthreads();   // sA complete, slab 0 visible
 
