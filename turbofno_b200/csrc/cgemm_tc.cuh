@@ -18,7 +18,7 @@
 //
 // Against the form it replaces (four convert warps with 4-byte stores of one chunk per half-team, results through Re/Im planes of
 // 64 KB): 64 channels, 28672 modes 17.2 -> 16.0 us, 65536 25.5 -> 24.2, 524288 133 -> 122 (2D layer of 128 x 64 images 129 -> 117; 82 at copy
-// speed), one image of 8 channels 6.9 -> 6.7.  Bound by the MMA thread: an instruction of this shape takes it 80 cycles (48 a
+// speed).  Bound by the MMA thread: an instruction of this shape takes it 80 cycles (48 a
 // tile), a chunk another 450 for its barriers and commit; so 16 channels per chunk and not 8 (144 us).  Tried: stores straight
 // from the accumulator rows, 32 bytes of sixteen channels each (202 us), landing buffers in registers (146) and private rings
 // of 16-byte asynchronous copies (124).

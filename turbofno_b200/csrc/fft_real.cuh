@@ -10,8 +10,8 @@
 //
 // Against separating the rows before the exchange: half the exchanged values, and one combination of sixteen residues
 // per k1 instead of one for each row.  The inverse, which took the 64 modes into every lane, reads each mode once.  1024
-// images (1280 of 128 x 128), us, before and now: 256 x 256 forward 104 -> 86, inverse 115 -> 82 (46 at copy speed); 128 x 256 61 -> 50
-// and 60 -> 41; 256 x 128 87 -> 66 and 77 -> 54; 128 x 128 57 -> 41 and 50 -> 35 (19).  Bound by issue slots and the load/store unit.
+// images (1280 of 128 x 128), us, before and now: 256 x 256 forward 104 -> 85, inverse 115 -> 81 (46 at copy speed); 128 x 256 61 -> 49
+// and 60 -> 40; 256 x 128 87 -> 64 and 77 -> 53; 128 x 128 57 -> 41 and 50 -> 34 (19).  Bound by issue slots and the load/store unit.
 #pragma once
 #include "fft256.cuh"
 

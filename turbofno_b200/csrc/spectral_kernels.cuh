@@ -73,7 +73,7 @@ TFNO_D void store_modes_to_tile(const float2 (&v)[32], float2* tile, int row, in
 // samples keep 32 of them busy, 32 channels of 256 all 256).  The inverse has N signals and stays on 64 samples per lane:
 // its table for twice the lanes would take shared memory from the widest layers.  The first weights travel beside the
 // forward transforms.  Calls back to back, us, with 64 samples per lane and now: 64 rows, 32 -> 128 channels, 256 samples 12.7 -> 12.0;
-// 64 x 16 -> 64 of 1024 24.7 -> 24.3; 140 x 72 -> 64 of 256 22.6 -> 19.4; 1200 x 200 -> 128 659 -> 610.
+// together with launches that start beside the previous one's tail: 140 rows, 72 -> 64 channels 22.6 -> 19.4, 1200 rows, 200 -> 128 659 -> 610.
 template <int R, bool FWD, bool INV, int NB>   // NB = N / 64
 __global__ void __launch_bounds__(kThreads, 1) spectral_tile_kernel(TileParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
