@@ -22,7 +22,7 @@ int tile_eights(const DeviceInfo& dev, const PerModeParams& p, PermodeKind kind)
     return nt;
 }
 int grad_splits(const DeviceInfo& dev, const PerModeParams& p, PermodeKind kind) {
-    // two CTAs for every SM
+    // two CTAs for every SM and no more: a few in a second wave would double the time
     long long blocks, most;
     if (kind == PERMODE_GRAD_SHARED) {
         blocks = (long long)((p.I + kPmSumTile - 1) / kPmSumTile) * (p.J / kPmSumTile);
@@ -31,7 +31,7 @@ int grad_splits(const DeviceInfo& dev, const PerModeParams& p, PermodeKind kind)
         blocks = blocks_per_split(p, tile_eights(dev, p, kind));
         most = most_splits(p, kind);
     }
-    long long splits = (2LL * dev.sms + blocks - 1) / blocks;
+    long long splits = 2LL * dev.sms / blocks;
     if (splits > most) splits = most;
     return splits < 1 ? 1 : (int)splits;
 }
