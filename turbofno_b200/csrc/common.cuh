@@ -175,7 +175,8 @@ int launch_permode(const DeviceInfo& dev, PerModeParams p, PermodeKind kind, cud
 // its writes are visible, so whoever waits for a kernel of the chain waits for all before it.  Only then may the next one be
 // prepared: admit_next_kernel() allows that once every CTA has called it or ended.
 //
-// Launches of one wave go early and admit others early, as do the fused kernel and the per-mode contractions at any length (their
+// Launches of one wave admit others early, and go early where no SM gets two of their CTAs (those that start as SMs become free
+// are stacked on the first of them: contraction of 64 x 128 CTAs that fit twice 53 -> 60 us for a whole 2D layer of 128 -> 128 channels), as do the fused kernel and the per-mode contractions at any length (their
 // operands bypass the L1 cache; training step of 7 x 64 images of 128 x 128 194 against 201 us).  Longer launches of the
 // transforms read through that cache and lose more than they gain when they start beside a kernel that has the shared
 // memory: an SM that never drains keeps the division of the two.  1D layer of 1024 x 128 signals of 512 samples as three
@@ -218,7 +219,7 @@ inline int launch_persistent(const DeviceInfo& dev, Kernel kernel, size_t smem, 
     if (rc != TFNO_OK) return rc;
     long long grid = (long long)dev.sms * occ;
     if (grid > work_blocks) grid = work_blocks;
-    return launch_chained(kernel, dim3((unsigned)grid), threads, smem, st, grid == work_blocks, 1, p);
+    return launch_chained(kernel, dim3((unsigned)grid), threads, smem, st, grid == work_blocks && grid <= dev.sms, 1, p);
 }
 
 // Ask the L2 for `bytes` of contiguous global memory, one 128-byte line per thread and round.

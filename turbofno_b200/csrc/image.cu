@@ -17,7 +17,7 @@ int launch_forward(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st)
     // a cluster of CTAs per image, or as many CTAs as are resident together
     long long clusters = p.nimg;
     if (C == 1 && clusters > (long long)dev.sms * occ) clusters = (long long)dev.sms * occ;
-    return launch_chained(kernel, dim3((unsigned)(clusters * C)), THREADS, smem, st, clusters == p.nimg, C, p);
+    return launch_chained(kernel, dim3((unsigned)(clusters * C)), THREADS, smem, st, clusters == p.nimg && clusters * C <= dev.sms, C, p);
 }
 // A cluster of CTAs of 64 rows per image, or one CTA per image.  The cluster takes an image at a time, so its launches have no
 // last wave to speak of, but the exchange through distributed shared memory costs more per image:
@@ -53,7 +53,7 @@ int launch_inverse(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st)
     if (rc != TFNO_OK) return rc;
     long long images = (long long)dev.sms * occ / PARTS;
     if (images > p.nimg) images = p.nimg;
-    return launch_chained(kernel, dim3((unsigned)(images * PARTS)), THREADS, smem, st, images == p.nimg, 1, p);
+    return launch_chained(kernel, dim3((unsigned)(images * PARTS)), THREADS, smem, st, images == p.nimg && images * PARTS <= dev.sms, 1, p);
 }
 
 template <int RX, bool CENTERED_X>
@@ -68,7 +68,7 @@ int launch_inverse64(const DeviceInfo& dev, const ImageParams& p, cudaStream_t s
     if (rc != TFNO_OK) return rc;
     long long images = (long long)dev.sms * occ / PARTS;
     if (images > p.nimg) images = p.nimg;
-    return launch_chained(kernel, dim3((unsigned)(images * PARTS)), THREADS, smem, st, images == p.nimg, 1, p);
+    return launch_chained(kernel, dim3((unsigned)(images * PARTS)), THREADS, smem, st, images == p.nimg && images * PARTS <= dev.sms, 1, p);
 }
 
 template <int RX, int RY, int CLS>

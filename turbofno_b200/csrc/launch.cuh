@@ -32,7 +32,7 @@ inline int launch_tile_inst(const DeviceInfo& dev, const TileParams& p, cudaStre
     if (rc != TFNO_OK) return rc;
     long long grid = (long long)dev.sms * occ;
     if (grid > p.rows) grid = p.rows;
-    return launch_chained(kernel, dim3((unsigned)grid, (unsigned)n_blocks), kThreads, smem, st, grid == p.rows, 1, p);    // p.N channels per block of blockIdx.y
+    return launch_chained(kernel, dim3((unsigned)grid, (unsigned)n_blocks), kThreads, smem, st, grid == p.rows && grid * n_blocks <= dev.sms && occ == 1, 1, p);    // p.N channels per block of blockIdx.y
 }
 
 template <bool FWD, bool INV, int NB>

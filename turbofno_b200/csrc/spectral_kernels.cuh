@@ -142,11 +142,20 @@ __global__ void __launch_bounds__(kThreads, 1) spectral_tile_kernel(TileParams p
                 if (live) store_modes_to_tile<L>(v, sA, k, r);
             }
         } else {
-            // compact spectrum: 64 consecutive m per channel
-            for (int i = tid; i < K * 32; i += kThreads) {
-                int k = i >> 5, c = i & 31;
-                float4 q = load_global(reinterpret_cast<const float4*>(p.x + row * kModes + (long long)k * M) + c);
-                *reinterpret_cast<float4*>(sA + k * kModes + swz_chunk(k, c) * 2) = q;
+            // compact spectrum: 64 consecutive m per channel; four loads on their way at a time (eight take the
+            // registers of the second CTA of an SM)
+            for (int i0 = tid; i0 < K * 32; i0 += 4 * kThreads) {
+                float4 q[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int i = i0 + j * kThreads;
+                    if (i < K * 32) q[j] = load_global(reinterpret_cast<const float4*>(p.x + row * kModes + (long long)(i >> 5) * M) + (i & 31));
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int i = i0 + j * kThreads, k = i >> 5;
+                    if (i < K * 32) *reinterpret_cast<float4*>(sA + k * kModes + swz_chunk(k, i & 31) * 2) = q[j];
+                }
             }
         }
 
