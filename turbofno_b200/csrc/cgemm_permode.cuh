@@ -62,9 +62,8 @@ __device__ __forceinline__ float2 pm_load8(uint32_t addr) {
     asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
     return v;
 }
-// v = hi + lo, hi rounded to tf32 (cvt.rna.tf32 is five instructions here, for the sake of infinities and NaNs, which this
-// passes on as infinities and NaNs in hi or lo).  The multiplier drops the low 13 bits of an operand: at most the last of
-// lo's 12 bits.
+// v = hi + lo, hi rounded to tf32 by an add and a mask; infinities and NaNs are passed on as infinities and NaNs in hi or
+// lo.  The multiplier drops the low 13 bits of an operand: at most the last of lo's 12 bits.
 __device__ __forceinline__ void pm_split(float v, uint32_t& hi, uint32_t& lo) {
     hi = (__float_as_uint(v) + 0x1000u) & 0xffffe000u;
     lo = __float_as_uint(v - __uint_as_float(hi));
