@@ -53,3 +53,47 @@ def test_values_that_are_not_finite_stay_in_their_mode_and_output(cuda, value):
     keep = [n for n in range(N) if n != 5]
     assert torch.equal(y[:, keep], clean[:, keep])
     plan.close()
+
+
+def _not_a_number(kind):
+    """On the GPU: a NaN from the host has the payload 0x400000, one that arithmetic made there all bits."""
+    import torch
+
+    inf = torch.full((), float("inf"), device="cuda")
+    return {"host": torch.full((), float("nan"), device="cuda"), "arithmetic": inf * 0, "negative": -(inf * 0), "inf": inf}[kind]
+
+
+@pytest.mark.parametrize("kind", ["host", "arithmetic", "negative", "inf"])
+@pytest.mark.parametrize("part", [0, 1])
+@pytest.mark.parametrize("path", ["fused", "wide", "2d", "grad_x"])
+def test_shared_weights_that_are_not_finite_spoil_their_output(cuda, path, part, kind):
+    """A shared weight that is no number must not pass for zero on the tensor cores."""
+    import torch
+    import turbofno_b200 as t
+
+    rank, B, K, N, DY = {"fused": (1, 300, 64, 64, 256), "wide": (1, 300, 64, 128, 512), "2d": (2, 2, 32, 64, 128), "grad_x": (2, 2, 64, 64, 128)}[path]
+    sig = (DY,) * rank
+    plan = t.SpectralConv(rank, B, DY, K, N, layout="batch_major")
+    kernel = "spectral_tc_kernel" if path == "fused" else "cgemm_tc_kernel"
+    assert any(k.startswith(kernel) for k in plan.kernels())
+    g = torch.Generator(device="cuda").manual_seed(2)
+    x, w = _field(g, B, K, *sig), _field(g, K, N)
+    if path == "grad_x":
+        gy, out, own = _field(g, B, N, *sig), 3, K
+
+        def call():
+            gx = torch.empty_like(x)
+            plan.backward(x, w, gy, gx, None)
+            return gx
+    else:
+        out, own = 5, N
+
+        def call():
+            return plan(x, w)
+    clean = call()
+    torch.view_as_real(w)[3, 5, part] = _not_a_number(kind)
+    y = call()
+    assert not torch.isfinite(torch.view_as_real(y[:, out])).any()
+    keep = [n for n in range(own) if n != out]
+    assert torch.equal(y[:, keep], clean[:, keep])
+    plan.close()

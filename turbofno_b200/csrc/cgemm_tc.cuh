@@ -176,9 +176,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) cgemm_tc_kernel(CgemmTcParams
                         w1 = cmul(w1, p.alpha);
                         // Re row: [ Wr | -Wi ],  Im row: [ Wi | Wr ]  against  S = [ Ar ; Ai ]
                         const float x = im_row ? (part ? w1.x : w1.y) : (part ? -w1.y : w1.x);
-                        const float h = tf32_hi(x);
-                        hi[j] = __float_as_uint(h);
-                        lo[j] = __float_as_uint(tf32_hi(x - h));
+                        tf32_parts(x, hi[j], lo[j]);
                     }
                     const uint32_t col = (uint32_t)(16 * c + 8 * part);
                     TFNO_TMEM_ST8(trow + TM_WHI + col, hi);
