@@ -144,9 +144,10 @@ size_t tfno_optional_workspace_bytes(const tfno_plan* plan);
 int tfno_exec_scratch(const tfno_plan* plan, const void* x, const void* w, void* y,
                       void* workspace, size_t workspace_bytes, void* stream);
 
-/* The same layer of REAL fields: x and y hold float samples (strides of the plan in samples), w complex per-mode
- * weights.  2D variant D plans with per-mode weights; the field's spectrum carries ky = 0..63 and the layer is
- * 2 Re(ifft2) of the contracted spectrum with the ky = 0 column halved (rfft2 -> weights -> irfft2). */
+/* The same layer of REAL fields: x and y hold float samples (strides of the plan in samples, even as for every plan; rows
+ * of 128 samples move in wider accesses when the strides are multiples of four), w complex per-mode weights.  2D variant D
+ * plans with per-mode weights; the field's spectrum carries ky = 0..63 and the layer is 2 Re(ifft2) of the contracted
+ * spectrum with the ky = 0 column halved (rfft2 -> weights -> irfft2). */
 int tfno_exec_real(const tfno_plan* plan, const void* x, const void* w, void* y, void* workspace, void* stream);
 
 /* Gradients of a variant D plan (true inverse, beta = 0) at input x and weights w for the output gradient grad_y:

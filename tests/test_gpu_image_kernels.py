@@ -125,3 +125,56 @@ def test_forward_images_around_the_waves_of_a_launch(cuda, DX, DY, images, real)
         x, w = _field(g, B, K, DX, DY), _field(g, K, 64)
         _check(plan(x, w), _layer(x, w))
     plan.close()
+
+
+@pytest.mark.parametrize("DX,DY", [(128, 128), (256, 128), (256, 256)])
+@pytest.mark.parametrize("B", [1, 5])                # a cluster and one CTA per image
+@pytest.mark.parametrize("pad_channel,pad_batch", [(2, 0), (0, 2), (6, 4), (4, 0)])
+def test_real_images_apart_by_any_even_number_of_samples(cuda, DX, DY, B, pad_channel, pad_batch):
+    """Layer and gradients of real images with gaps between them: those that start on 8-byte boundaries only, too.  Bit for bit
+    the results of dense images, and the gaps stay as they are."""
+    import torch
+    import turbofno_b200 as t
+    from turbofno_b200._lib import Problem, check, load
+
+    K = N = 64
+    g = torch.Generator(device="cuda").manual_seed(3)
+    real = lambda: torch.rand((B, K, DX, DY), generator=g, device="cuda") * 2 - 1
+    x, gy, w = real(), real(), _field(g, K, N, 64, 64)
+    dense = t.SpectralConv(2, B, DY, K, N, DX=DX, layout="batch_major", per_mode_weights=True, x_modes_centered=True)
+    want = [dense.exec_real(x, w), torch.empty_like(x), torch.empty_like(w)]
+    dense.backward(x, w, gy, want[1], want[2])
+    dense.close()
+
+    stride_k = DX * DY + pad_channel
+    stride_b = K * stride_k + pad_batch
+
+    def apart(values=None):
+        mem = torch.full((B * stride_b,), 7.0, device=cuda)
+        view = mem.as_strided((B, K, DX, DY), (stride_b, stride_k, DY, 1))
+        if values is not None:
+            view.copy_(values)
+        return mem, view
+
+    lib, handle = load(), t.Handle.get(0)
+    p = Problem()
+    check(lib.tfno_problem_init(ctypes.byref(p), 2))
+    p.bs, p.DX, p.DY, p.K, p.N, p.x_modes_centered = B, DX, DY, K, N, 1
+    p.x_stride_b = p.y_stride_b = stride_b
+    p.x_stride_k = p.y_stride_n = stride_k
+    p.w_stride_k, p.w_stride_n, p.w_stride_m = N * 4096, 4096, 1
+    plan = ctypes.c_void_p()
+    check(lib.tfno_plan_create(handle._h, ctypes.byref(p), ctypes.byref(plan)))
+    ws = torch.empty(max(lib.tfno_workspace_bytes(plan), lib.tfno_backward_workspace_bytes(plan)), dtype=torch.uint8, device=cuda)
+    (xm, _), (gym, _), (ym, y), (gxm, gx) = apart(x), apart(gy), apart(), apart()
+    gw = torch.empty_like(w)
+    stream = torch.cuda.current_stream().cuda_stream
+    check(lib.tfno_exec_real(plan, xm.data_ptr(), w.data_ptr(), ym.data_ptr(), ws.data_ptr(), stream))
+    check(lib.tfno_backward(plan, 1, xm.data_ptr(), w.data_ptr(), gym.data_ptr(), gxm.data_ptr(), gw.data_ptr(), ws.data_ptr(), stream))
+    torch.cuda.synchronize()
+    lib.tfno_plan_destroy(plan)
+    for got, ref in ((y, want[0]), (gx, want[1]), (gw, want[2])):
+        assert torch.equal(got, ref)
+    for mem, view in ((ym, y), (gxm, gx)):
+        view.fill_(7.0)
+        assert (mem == 7.0).all()

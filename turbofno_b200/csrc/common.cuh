@@ -137,6 +137,7 @@ struct ImageParams {
     float2 gain;
     int conj_inverse;
     int real;                          // the full-size side holds float samples (strides in samples)
+    int rows16;                        // real rows of 128 samples: images start on 16-byte boundaries, else on 8-byte ones (set by the launch)
     int centered_x;                    // kept X modes are -32..31 (row kx + 32 of the 64 x 64 block) instead of 0..63
 };
 // DX, DY in {128, 256}; full-size side: 16-byte aligned base, even strides

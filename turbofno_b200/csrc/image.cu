@@ -93,11 +93,13 @@ bool fft2d_fits(const DeviceInfo& dev) {
 // Residue classes per inverse CTA: two (128 threads) except at 256 x 256, where four (256 threads, half as many
 // reads of the spectrum) take 993 against 1013 us for 8192 images; at 256 x 128 two take 307 against 333 us for 4096,
 // and all eight in one CTA of 512 threads take 1173 and 380 us.
-int launch_fft2d(const DeviceInfo& dev, int DX, int DY, const ImageParams& p, bool inverse, cudaStream_t st) {
+int launch_fft2d(const DeviceInfo& dev, int DX, int DY, const ImageParams& params, bool inverse, cudaStream_t st) {
+    ImageParams p = params;
     if (p.nimg <= 0) return TFNO_OK;
     const void* full = inverse ? (const void*)p.out : (const void*)p.in;
     if ((reinterpret_cast<uintptr_t>(full) & 15) != 0 || (p.stride_b & 1) != 0 || (p.stride_k & 1) != 0) return TFNO_ERR_UNSUPPORTED;
     if (p.real && inverse && !p.conj_inverse) return TFNO_ERR_UNSUPPORTED;
+    p.rows16 = p.real && ((p.stride_b | p.stride_k) & 3) == 0 ? 1 : 0;       // even strides are 16 bytes of complex samples, 8 of real ones
     if (DX == 128 && DY == 128) return launch_image<4, 4, 2>(dev, p, inverse, st);
     if (DX == 128 && DY == 256) return launch_image<4, 8, 2>(dev, p, inverse, st);
     if (DX == 256 && DY == 128) return launch_image<8, 4, 2>(dev, p, inverse, st);

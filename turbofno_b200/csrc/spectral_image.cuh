@@ -126,13 +126,19 @@ __global__ void __launch_bounds__(64 * RX / C, 8 * C / RX) fft2d_trunc_kernel(Im
             if constexpr (REAL) {
                 constexpr int Q = RealRows<DY>::Q, K1 = RealRows<DY>::K1;
                 const Sample* row = src + (long long)x * DY + Q * r;
+                auto load2 = [&](int q, int j) {                       // samples q, q + 1 of both rows
+                    const float2 a = load_global(reinterpret_cast<const float2*>(row + 16 * j + q)), b = load_global(reinterpret_cast<const float2*>(row + DY + 16 * j + q));
+                    v[q * K1 + j] = make_float2(a.x, b.x);
+                    v[(q + 1) * K1 + j] = make_float2(a.y, b.y);
+                };
+                if (Q == 2 || !p.rows16) {
 #pragma unroll
-                for (int j = 0; j < K1; ++j) {
-                    if constexpr (Q == 2) {
-                        const float2 a = load_global(reinterpret_cast<const float2*>(row + 16 * j)), b = load_global(reinterpret_cast<const float2*>(row + DY + 16 * j));
-                        v[j] = make_float2(a.x, b.x);
-                        v[K1 + j] = make_float2(a.y, b.y);
-                    } else {
+                    for (int j = 0; j < K1; ++j)
+#pragma unroll
+                        for (int q = 0; q < Q; q += 2) load2(q, j);
+                } else if constexpr (Q == 4) {
+#pragma unroll
+                    for (int j = 0; j < K1; ++j) {
                         const float4 a = load_global(reinterpret_cast<const float4*>(row + 16 * j)), b = load_global(reinterpret_cast<const float4*>(row + DY + 16 * j));
                         v[j] = make_float2(a.x, b.x);
                         v[K1 + j] = make_float2(a.y, b.y);
@@ -286,13 +292,19 @@ __global__ void __launch_bounds__(64 * CLS, 8 / CLS) ifft2d_pad_kernel(ImagePara
                 real_join<N>(fa, fb, aA, bA, aB, bB, j1 == 0);
                 real_inverse<N>(fa, fb, twY, twX + CLS * 32 + RealRows<N>::SCRATCH * g, j1, g & 1, v);
                 float* row = reinterpret_cast<float*>(dst) + (long long)x * DY + Q * j1;
+                if (Q == 2 || !p.rows16) {
 #pragma unroll
-                for (int j = 0; j < K1; ++j) {
-                    const int at = real_slot<N>(j);
-                    if constexpr (Q == 2) {
-                        *reinterpret_cast<float2*>(row + 16 * j) = make_float2(v[0][at].x, v[1][at].x);
-                        *reinterpret_cast<float2*>(row + DY + 16 * j) = make_float2(v[0][at].y, v[1][at].y);
-                    } else {
+                    for (int j = 0; j < K1; ++j)
+#pragma unroll
+                        for (int q = 0; q < Q; q += 2) {
+                            const float2 s0 = v[q][real_slot<N>(j)], s1 = v[q + 1][real_slot<N>(j)];
+                            *reinterpret_cast<float2*>(row + 16 * j + q) = make_float2(s0.x, s1.x);
+                            *reinterpret_cast<float2*>(row + DY + 16 * j + q) = make_float2(s0.y, s1.y);
+                        }
+                } else if constexpr (Q == 4) {
+#pragma unroll
+                    for (int j = 0; j < K1; ++j) {
+                        const int at = real_slot<N>(j);
                         *reinterpret_cast<float4*>(row + 16 * j) = make_float4(v[0][at].x, v[1][at].x, v[2][at].x, v[3][at].x);
                         *reinterpret_cast<float4*>(row + DY + 16 * j) = make_float4(v[0][at].y, v[1][at].y, v[2][at].y, v[3][at].y);
                     }
