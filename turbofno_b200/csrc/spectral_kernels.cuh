@@ -74,8 +74,12 @@ TFNO_D void store_modes_to_tile(const float2 (&v)[32], float2* tile, int row, in
 // its table for twice the lanes would take shared memory from the widest layers.  The first weights travel beside the
 // forward transforms.  Calls back to back, us, with 64 samples per lane and now: 64 rows, 32 -> 128 channels, 256 samples 12.7 -> 12.0;
 // together with launches that start beside the previous one's tail: 140 rows, 72 -> 64 channels 22.6 -> 19.4, 1200 rows, 200 -> 128 659 -> 610.
+// The contraction alone (!FWD && !INV) of 64 output channels runs two CTAs per SM, which its 128 registers a thread just allow: 1024
+// rows, 192 -> 64 channels 171 us, with 130 registers and one CTA 227.  Its weights are plain loads, which the compiler places
+// among the multiplications (173 with loads in their order), and are conjugated on their way to shared memory: behind the load
+// every slab waits for memory (256 -> 128 channels, 64 rows 32 against 39 us).
 template <int R, bool FWD, bool INV, int NB>   // NB = N / 64
-__global__ void __launch_bounds__(kThreads, 1) spectral_tile_kernel(TileParams p) {
+__global__ void __launch_bounds__(kThreads, !FWD && !INV && NB == 1 ? 2 : 1) spectral_tile_kernel(TileParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2* sA = reinterpret_cast<float2*>(smem_raw);                 // [K][64] swizzled
     float2* sC = sA + (size_t)p.K * kModes;                            // [N][64] swizzled (INV only)
@@ -105,8 +109,8 @@ __global__ void __launch_bounds__(kThreads, 1) spectral_tile_kernel(TileParams p
             int e = tid + i * kThreads;
             int kk, n;
             if (p.w_stride_n == 1) { n = e % N; kk = e / N; } else { kk = e % kSlabK; n = e / kSlabK; }
-            wreg[i] = load_global(wbase + (long long)(k0 + kk) * p.w_stride_k + (long long)n * p.w_stride_n);
-            if (!FWD && !INV && p.conj_w) wreg[i].y = -wreg[i].y;
+            const float2* src = wbase + (long long)(k0 + kk) * p.w_stride_k + (long long)n * p.w_stride_n;
+            wreg[i] = (FWD || INV) ? load_global(src) : *src;
         }
     };
     auto stash_slab = [&](int buf) {
@@ -115,7 +119,9 @@ __global__ void __launch_bounds__(kThreads, 1) spectral_tile_kernel(TileParams p
             int e = tid + i * kThreads;
             int kk, n;
             if (p.w_stride_n == 1) { n = e % N; kk = e / N; } else { kk = e % kSlabK; n = e / kSlabK; }
-            sW[(buf * kSlabK + kk) * (N + kWPad) + n] = wreg[i];
+            float2 v = wreg[i];
+            if (!FWD && !INV && p.conj_w) v.y = -v.y;      // not in fetch_slab: it would wait for the load there
+            sW[(buf * kSlabK + kk) * (N + kWPad) + n] = v;
         }
     };
     follow_previous_kernel();
@@ -142,8 +148,7 @@ __global__ void __launch_bounds__(kThreads, 1) spectral_tile_kernel(TileParams p
                 if (live) store_modes_to_tile<L>(v, sA, k, r);
             }
         } else {
-            // compact spectrum: 64 consecutive m per channel; four loads on their way at a time (eight take the
-            // registers of the second CTA of an SM)
+            // compact spectrum: 64 consecutive m per channel; four loads on their way at a time
             for (int i0 = tid; i0 < K * 32; i0 += 4 * kThreads) {
                 float4 q[4];
 #pragma unroll
