@@ -97,3 +97,18 @@ def test_shared_weights_that_are_not_finite_spoil_their_output(cuda, path, part,
     keep = [n for n in range(own) if n != out]
     assert torch.equal(y[:, keep], clean[:, keep])
     plan.close()
+
+
+@pytest.mark.parametrize("rows", [296, 297, 298, 592, 600])      # tiles of 128 modes (of 64: 297) one, two and a few more than two per SM
+@pytest.mark.parametrize("K,N", [(104, 64), (128, 128)])
+def test_contraction_in_two_launches_of_which_the_second_adds(cuda, rows, K, N):
+    import torch
+    import turbofno_b200 as t
+
+    M = 64 * rows
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    A, w = _field(g, K, M), _field(g, N, K)
+    C = torch.full((N, M), float("nan"), dtype=torch.complex64, device=cuda)
+    t.api.cgemm(M, N, K, A, w, C)
+    want = w.to(torch.complex128) @ A.to(torch.complex128)
+    assert ((C - want).norm() / want.norm()).item() <= REL

@@ -62,7 +62,6 @@ struct CgemmTcParams {
     float2* c; long long c_stride_n;             // C[m + n * c_stride_n]
     float2 alpha;
     int conj_w;                          // the weights enter conjugated
-    int accumulate;                      // 1: C += alpha A W (the second of two launches over the halves of the channels)
     int* status;
 };
 
@@ -73,7 +72,8 @@ __host__ inline size_t cgemm_tc_smem_bytes() {
     return (size_t)G::S_BUFFERS * 2 * G::PART_BYTES + (size_t)kGemmStages * G::STAGE_BYTES + 4 * kOutBytes + 512 + 1024;
 }
 
-template <int TN>
+// ADD: C += alpha A W (the second of two launches over the halves of the channels)
+template <int TN, bool ADD>
 __global__ void __launch_bounds__(kGemmThreads, 1) cgemm_tc_kernel(CgemmTcParams p) {
     static_assert(TN == 64 || TN == 128, "tile of 64 or 128 modes");
     using G = GemmGeom<TN>;
@@ -197,10 +197,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1) cgemm_tc_kernel(CgemmTcParams
         unsigned char* out = ostage + q * kOutBytes;
         float4* put = reinterpret_cast<float4*>(out + (lane >> 1) * kOutStride + (odd ? 16 : 0));
         const float4* get = reinterpret_cast<const float4*>(out + (lane >> 4) * kOutStride + (lane & 15) * 16);
+        // ADD: C of the next 32 modes is on its way while these are staged (a load right ahead of its sum waits for memory
+        // eight times in a row, behind the stores: 8192 rows, 128 -> 64 channels 661 us)
+        float4 prev[8];
+        auto fetch = [&](const float2* from) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) prev[i] = *reinterpret_cast<const float4*>(from + (long long)(2 * i) * p.c_stride_n);
+        };
         bool ok = true;
         for (int it = 0; it < n_it && ok; ++it) {
             const int buf = it & 1;
             float2* ctile = p.c + (long long)(16 * q + (lane >> 4)) * p.c_stride_n + (first + (long long)it * gridDim.x) * TN + 2 * (lane & 15);
+            if (ADD && it == 0) fetch(ctile);
             ok = __all_sync(0xffffffffu, mbar_wait(bar(B_AFULL + buf), (it >> 1) & 1, abort_flag, p.status, 71, kGemmIdleNs));
             if (!ok) break;
             tc_fence_after();
@@ -229,12 +237,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) cgemm_tc_kernel(CgemmTcParams
                 for (int i = 0; i < 8; ++i) {                // channels 2 i, 2 i + 1 of the warp
                     float4 o = get[i * (2 * kOutStride / 16)];
                     float4* dst = reinterpret_cast<float4*>(ctile + (long long)(2 * i) * p.c_stride_n + c0);
-                    if (p.accumulate) {
-                        const float4 prev = *dst;
-                        o.x += prev.x; o.y += prev.y; o.z += prev.z; o.w += prev.w;
-                    }
+                    if (ADD) { o.x += prev[i].x; o.y += prev[i].y; o.z += prev[i].z; o.w += prev[i].w; }
                     *dst = o;
                 }
+                if (ADD && (c0 + 32 < TN || it + 1 < n_it))
+                    fetch(c0 + 32 < TN ? ctile + c0 + 32 : ctile + (long long)gridDim.x * TN);
             }
         }
     } else if (warp == kMmaWarp && lane == 0) {

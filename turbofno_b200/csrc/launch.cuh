@@ -196,12 +196,12 @@ inline bool cgemm_tc_eligible(const DeviceInfo& dev, const TileParams& p) {
     if (p.beta.x != 0.f || p.beta.y != 0.f) return false;
     return ((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.y)) & 15) == 0;
 }
-template <int TN>
-inline int launch_cgemm_tc_inst(const DeviceInfo& dev, const TileParams& p, cudaStream_t st, bool accumulate) {
-    auto kernel = tcg::cgemm_tc_kernel<TN>;
+template <int TN, bool ADD>
+inline int launch_cgemm_tc_inst(const DeviceInfo& dev, const TileParams& p, cudaStream_t st) {
+    auto kernel = tcg::cgemm_tc_kernel<TN, ADD>;
     const size_t smem = tcg::cgemm_tc_smem_bytes<TN>();
     if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
-    if (record_launch(dev, accumulate ? "cgemm_tc_kernel<%d>+=" : "cgemm_tc_kernel<%d>", TN)) return TFNO_OK;
+    if (record_launch(dev, ADD ? "cgemm_tc_kernel<%d>+=" : "cgemm_tc_kernel<%d>", TN)) return TFNO_OK;
     int occ = 0;
     int rc = prepare_kernel(kernel, smem, dev, &occ, tcg::kGemmThreads);
     if (rc != TFNO_OK) return rc;
@@ -212,7 +212,6 @@ inline int launch_cgemm_tc_inst(const DeviceInfo& dev, const TileParams& p, cuda
     q.w = p.w; q.w_stride_k = p.w_stride_k; q.w_stride_n = p.w_stride_n;
     q.c = p.y; q.c_stride_n = M;
     q.alpha = p.alpha; q.conj_w = p.conj_w; q.status = dev.status;
-    q.accumulate = accumulate ? 1 : 0;
     long long grid = dev.sms;
     if (grid > q.tiles) grid = q.tiles;
     return launch_chained(kernel, dim3((unsigned)grid), tcg::kGemmThreads, smem, st, grid == q.tiles, 1, q);
@@ -232,8 +231,9 @@ inline int launch_cgemm_tc(const DeviceInfo& dev, const TileParams& p, cudaStrea
             q.x = p.x + (long long)k0 * M;                   // A[m + k*M]
             q.w = p.w + (long long)n0 * p.w_stride_n + (long long)k0 * p.w_stride_k;
             q.y = p.y + (long long)n0 * M;
-            const bool acc = k0 != 0;
-            const int rc = (!narrow && p.rows % 2 == 0 && p.rows / 2 >= dev.sms) ? launch_cgemm_tc_inst<128>(dev, q, st, acc) : launch_cgemm_tc_inst<64>(dev, q, st, acc);
+            const bool wide = !narrow && p.rows % 2 == 0 && p.rows / 2 >= dev.sms;
+            const int rc = k0 == 0 ? (wide ? launch_cgemm_tc_inst<128, false>(dev, q, st) : launch_cgemm_tc_inst<64, false>(dev, q, st))
+                                   : (wide ? launch_cgemm_tc_inst<128, true>(dev, q, st) : launch_cgemm_tc_inst<64, true>(dev, q, st));
             if (rc != TFNO_OK) return rc;
         }
     }
