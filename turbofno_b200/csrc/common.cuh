@@ -184,6 +184,13 @@ int launch_permode(const DeviceInfo& dev, PerModeParams p, PermodeKind kind, cud
 // kernels: all early 391 us, none 351; 2D layer of 128 x 64 images 2160 against 2040.  The contraction of shared weights in
 // several waves: 359 against 355.  Gains: three kernels of one image 27.7 -> 24.0 us, a row-tile kernel behind another 14.3 -> 12.7,
 // training step of 512 x 64 signals of 512 samples 256 -> 247.
+// Dynamic shared memory for a launch of `ctas`.  A CTA for every SM or fewer: each asks for more than half of an SM's, so that none
+// share one; launched early they would be stacked on the first SMs that become free.  2D layers of one batch item, us, each
+// launch in order / early and stacked / early and apart: 64 images of 256 x 256 39.0 / 41.0 / 34.9, 64 of 128 x 128 28.8 / 26.2 /
+// 22.9, 16 of 256 x 256 32.8 / 32.6 / 25.6; gradients of 64 images of 128 x 128 with per-mode weights 113 / 118 / 104.
+inline size_t unshared_smem(const DeviceInfo& dev, long long ctas, size_t smem) {
+    return ctas <= dev.sms && (long long)smem <= dev.max_smem_optin / 2 ? dev.max_smem_optin / 2 + 1024 : smem;
+}
 template <typename... Params>
 inline int launch_chained(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, bool early, int cluster, const Params&... args) {
     cudaLaunchConfig_t cfg{};

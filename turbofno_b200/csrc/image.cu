@@ -8,7 +8,7 @@ template <int RX, int RY, int C, bool REAL>
 int launch_forward(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st) {
     constexpr int THREADS = 64 * RX / C;
     auto kernel = fft2d_trunc_kernel<RX, RY, C, REAL>;
-    const size_t smem = fwd_image_smem_bytes<RX, RY, C, REAL>();
+    const size_t smem = unshared_smem(dev, p.nimg * C, fwd_image_smem_bytes<RX, RY, C, REAL>());
     if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
     if (record_launch(dev, "fft2d_trunc_kernel<%d,%d,%d>", RX, RY, C)) return TFNO_OK;
     int occ = 0;
@@ -45,7 +45,7 @@ template <int RX, int RY, int CLS, bool INVERSE, bool REAL>
 int launch_inverse(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st) {
     constexpr int PARTS = RX / CLS, THREADS = 64 * CLS;
     auto kernel = ifft2d_pad_kernel<RX, RY, CLS, INVERSE, REAL>;
-    const size_t smem = inv_image_smem_bytes<RY, CLS, REAL>();
+    const size_t smem = unshared_smem(dev, p.nimg * PARTS, inv_image_smem_bytes<RY, CLS, REAL>());
     if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
     if (record_launch(dev, "ifft2d_pad_kernel<%d,%d,%d,%d>", RX, RY, CLS, INVERSE)) return TFNO_OK;
     int occ = 0;
@@ -60,7 +60,7 @@ template <int RX, bool CENTERED_X>
 int launch_inverse64(const DeviceInfo& dev, const ImageParams& p, cudaStream_t st) {        // DX = 64 RX, DY = 256
     constexpr int CLS = 2, PARTS = RX / CLS, THREADS = 64 * CLS;
     auto kernel = ifft2d_pad64_kernel<RX, 4, CLS, CENTERED_X>;
-    const size_t smem = inv64_image_smem_bytes<4, CLS>();
+    const size_t smem = unshared_smem(dev, p.nimg * PARTS, inv64_image_smem_bytes<4, CLS>());
     if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
     if (record_launch(dev, "ifft2d_pad64_kernel<%d,%d,%d,%d>", RX, 4, CLS, CENTERED_X)) return TFNO_OK;
     int occ = 0;

@@ -26,18 +26,16 @@ inline int launch_tile_inst(const DeviceInfo& dev, const TileParams& p, cudaStre
     auto kernel = spectral_tile_kernel<R, FWD, INV, NB>;
     size_t smem = tile_smem_bytes(R, FWD, INV, p.K, p.N);
     if ((long long)smem > dev.max_smem_optin) return TFNO_ERR_UNSUPPORTED;
-    // A CTA for every SM or fewer: each asks for more than half of the shared memory, so that none share an SM (launched early
-    // they would be stacked on the first SMs that become free).  Transform, contraction, transform of 32 -> 128 channels of 512
-    // samples, 32 rows 18.5 us, launched in order 20.6; one image of 256 x 128, 32 -> 128 channels 30.8 and 32.9.
-    const bool single = p.rows * n_blocks <= dev.sms;
-    if (single && (long long)smem <= dev.max_smem_optin / 2) smem = dev.max_smem_optin / 2 + 1024;
+    // transform, contraction, transform of 32 -> 128 channels of 512 samples: 32 rows 18.5 us, launched in order 20.6; one image of
+    // 256 x 128, 32 -> 128 channels 30.8 and 32.9
+    smem = unshared_smem(dev, p.rows * n_blocks, smem);
     if (record_launch(dev, "spectral_tile_kernel<%d,%d,%d,%d>", R, FWD, INV, NB)) return TFNO_OK;
     int occ = 0;
     int rc = prepare_kernel(kernel, smem, dev, &occ);
     if (rc != TFNO_OK) return rc;
     long long grid = (long long)dev.sms * occ;
     if (grid > p.rows) grid = p.rows;
-    return launch_chained(kernel, dim3((unsigned)grid, (unsigned)n_blocks), kThreads, smem, st, single && occ == 1, 1, p);    // p.N channels per block of blockIdx.y
+    return launch_chained(kernel, dim3((unsigned)grid, (unsigned)n_blocks), kThreads, smem, st, grid == p.rows && grid * n_blocks <= dev.sms, 1, p);    // p.N channels per block of blockIdx.y
 }
 
 template <bool FWD, bool INV, int NB>
