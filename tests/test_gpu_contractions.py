@@ -112,3 +112,37 @@ def test_contraction_in_two_launches_of_which_the_second_adds(cuda, rows, K, N):
     t.api.cgemm(M, N, K, A, w, C)
     want = w.to(torch.complex128) @ A.to(torch.complex128)
     assert ((C - want).norm() / want.norm()).item() <= REL
+
+
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_per_mode_contractions_of_the_largest_floats(cuda, sign):
+    """FLT_MAX as a weight, or in the spectrum of a gradient: finite results where the products are."""
+    import torch
+    import turbofno_b200 as t
+
+    B, K, N, DY = 9, 64, 64, 128
+    top = sign * torch.finfo(torch.float32).max
+    g = torch.Generator(device="cuda").manual_seed(4)
+    small = lambda *s: _field(g, *s) * 2.0 ** -9
+    rel = lambda got, want: ((got.to(torch.complex128) - want).abs().max() / want.abs().max()).item()
+    spectrum = lambda v: torch.fft.fft(v.to(torch.complex128))[..., :64]
+    pad = lambda s: torch.fft.ifft(torch.cat([s, s.new_zeros(*s.shape[:2], DY - 64)], -1))
+    x, gy, w = small(B, K, DY), small(B, N, DY), _field(g, K, N, 64)
+    w[3, 5, 17] = complex(top, -top)
+    plan = t.SpectralConv(1, B, DY, K, N, layout="batch_major", per_mode_weights=True)
+    w2 = w.to(torch.complex128)
+    # one channel in, one mode: each product is within 4 roundings of 2^-24 and two dropped parts of 2^-22, the transforms as above
+    assert rel(plan(x, w)[:, 5], pad(torch.einsum("bkm,knm->bnm", spectrum(x), w2))[:, 5]) <= REL
+    # a pulse has FLT_MAX in every mode
+    x[2, 7] = 0
+    x[2, 7, 0] = top
+    gx, gw = torch.empty_like(x), torch.empty_like(w)
+    plan.backward(x, w, gy, gx, gw)
+    assert rel(gx[:, 3], pad(torch.einsum("bnm,knm->bkm", spectrum(gy), w2.conj()))[:, 3]) <= REL
+    assert rel(gw[7], torch.einsum("bkm,bnm->knm", spectrum(x).conj(), spectrum(gy))[7] / DY) <= REL
+    plan.close()
+    shared = t.SpectralConv(1, B, DY, K, N, layout="batch_major")
+    gw = torch.empty(K, N, dtype=torch.complex64, device=cuda)
+    shared.backward(x, _field(g, K, N), gy, None, gw)
+    assert rel(gw[7], torch.einsum("bkm,bnm->kn", spectrum(x).conj(), spectrum(gy))[7] / DY) <= REL
+    shared.close()

@@ -62,11 +62,15 @@ __device__ __forceinline__ float2 pm_load8(uint32_t addr) {
     asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
     return v;
 }
-// v = hi + lo, hi rounded to tf32 by an add and a mask; infinities and NaNs are passed on as infinities and NaNs in hi or
-// lo.  The multiplier drops the low 13 bits of an operand: at most the last of lo's 12 bits.
+// v = hi + lo, hi rounded to tf32 by an add and a mask and at most the largest finite tf32 (the last values below FLT_MAX would
+// round to infinity, with a rest of minus infinity, and finite products would become NaN); infinities and NaNs are passed on in
+// lo.  The bound costs up to 0.4 us of a small layer (64 signals of 128 samples 19.7 -> 20.1 us, training step of 512 of 512
+// samples 246.0 -> 246.0).  The multiplier drops the low 13 bits of an operand: at most the last of lo's 12 bits.
 __device__ __forceinline__ void pm_split(float v, uint32_t& hi, uint32_t& lo) {
-    hi = (__float_as_uint(v) + 0x1000u) & 0xffffe000u;
-    lo = __float_as_uint(v - __uint_as_float(hi));
+    float h;
+    asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(h) : "f"(__uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u)), "f"(__uint_as_float(0x7f7fe000u)));
+    hi = __float_as_uint(h);
+    lo = __float_as_uint(v - h);
 }
 __device__ __forceinline__ void pm_mma(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
     asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
