@@ -146,3 +146,24 @@ def test_per_mode_contractions_of_the_largest_floats(cuda, sign):
     shared.backward(x, _field(g, K, N), gy, None, gw)
     assert rel(gw[7], torch.einsum("bkm,bnm->kn", spectrum(x).conj(), spectrum(gy))[7] / DY) <= REL
     shared.close()
+
+
+@pytest.mark.parametrize("B", [1, 2, 4, 15, 16, 20, 23, 24])
+@pytest.mark.parametrize("K", [64, 8])
+def test_short_sums_are_as_exact_as_fp32(cuda, B, K):
+    """Gradient of per-mode weights against the exact products of the spectra the library itself makes, so that the error is
+    that of the contraction.  An FP32 chain of 2 B multiply-adds rounds at the sizes of its partial sums: in the norm
+    sqrt(B) times the rms of a rounding, 2.5e-8, and one more at the front.  Two tf32 parts alone make 1.1e-7 of one term."""
+    import torch
+    import turbofno_b200 as t
+
+    N, DY = 64, 256
+    g = torch.Generator(device="cuda").manual_seed(6)
+    x, gy, w = _field(g, B, K, DY), _field(g, B, N, DY), _field(g, K, N, 64)
+    plan = t.SpectralConv(1, B, DY, K, N, layout="batch_major", per_mode_weights=True)
+    gw = torch.empty_like(w)
+    plan.backward(x, w, gy, None, gw)
+    plan.close()
+    X, G = (t.api.fft_stride_DY(v, torch.empty(v.shape[:2] + (64,), dtype=v.dtype, device=cuda), v.shape[0] * v.shape[1], DY).to(torch.complex128) for v in (x, gy))
+    want = torch.einsum("bkm,bnm->knm", X.conj(), G) / DY
+    assert ((gw.to(torch.complex128) - want).norm() / want.norm()).item() <= 2.5e-8 * (B + 1) ** 0.5 * 1.15

@@ -14,15 +14,16 @@
 // README names as the FNO use case.
 //
 // On the tensor cores through mma.sync m16n8k8 (tf32), every FP32 value split into two tf32 parts and three products
-// kept (hi*hi + lo*hi + hi*lo).  Fragments live in registers, so the operands are split on the way from the ring to the
-// multiplier, each value once; tcgen05 would want both parts of every matrix written back to shared memory, one mode
-// at a time, for products of 64 x 64 x (a few rows) each.  The tensor cores truncate when they accumulate, so a chain
-// covers the eight terms of one step only and the steps are added in FP32: closer to the exact sums than the chains
-// of FP32 FMAs this replaces (whole layer against 64-bit results: 1D training step 2.4e-7 -> 2.1e-7, real 2D field 2.9e-7 -> 2.5e-7).
+// kept (hi*hi + lo*hi + hi*lo), but for sums of few terms (PmProducts).  Fragments live in registers, so the operands are
+// split on the way from the ring to the multiplier, each value once; tcgen05 would want both parts of every matrix written
+// back to shared memory, one mode at a time, for products of 64 x 64 x (a few rows) each.  The tensor cores truncate when
+// they accumulate, so a chain covers the eight terms of one step only and the steps are added in FP32: closer to the exact
+// sums than chains of 24 FP32 FMAs and more (whole layer against 64-bit results: 1D training step 2.4e-7 -> 2.1e-7, real 2D
+// field 2.9e-7 -> 2.6e-7).  Operands below 2^-115 lose the last bits of their low parts.
 //
 // What bounds it (2D, 4096 modes, K = N = 64; us, with the FP32 kernel before it): layer of 1 row 36 (36), 16 rows 51 (73), 20
-// rows 66 (94), 64 rows 172 (242); gradient of W at 16 rows 63 (84), 20 rows 78 (97).  1D, 64 modes: 16 rows 7 (21), 512 rows
-// 28 (37).  Up to 8 rows the 134 MB of weights (20 us at copy speed); beyond that the multiplier, 55 % busy (20 rows: 33 us at
+// rows 66 (94), 64 rows 172 (242).  1D, 64 modes: 16 rows 7 (21), 512 rows 28 (37).  Not always ahead: 40 -> 128 channels, 2
+// rows 39.4 (37.4), 4 rows 41.6 (37.9).  Up to 8 rows the 134 MB of weights (20 us at copy speed); beyond that the multiplier, 55 % busy (20 rows: 33 us at
 // 512 multiply-adds a cycle), with the latencies of a step (load, split, chain of six) behind four warps per scheduler.
 // Tried: persistent CTAs whose ring runs on across tiles (79 us at 20 rows: 3.5 tiles per CTA are dealt worse than by the
 // hardware), tiles of 16 columns with three CTAs per SM (71), all loads of a step ahead of its products (68).
@@ -37,6 +38,8 @@ constexpr int kPmCols = 32;            // columns j per CTA
 constexpr int kPmThreads = 256;
 constexpr int kPmTerms = 8;            // values of r per ring stage = depth of a matrix instruction
 constexpr int kPmStages = 3;
+// PM_SPLIT: two tf32 parts, three products; PM_FULL: four products; PM_FMA: FP32 multiply-adds (rule: permode.cu)
+enum PmProducts { PM_SPLIT, PM_FULL, PM_FMA };
 constexpr int kPmSumTile = 64;         // gradient of shared weights: rows i and columns j per CTA
 constexpr int kPmSumTerms = 4;         // and r per ring stage (each eight modes deep)
 
@@ -90,19 +93,38 @@ __device__ __forceinline__ PmFragP pm_negated(const PmFragP& f) {
     for (int i = 0; i < 2; ++i) { n.hi[i] = f.hi[i] ^ 0x80000000u; n.lo[i] = f.lo[i] ^ 0x80000000u; }
     return n;
 }
-// sum += P conj?(Q) over eight terms, the small products first
+// sum += P conj?(Q) over eight terms, the small products first.
+// FULL: lo*lo too, and hi*hi of the two parts apart from the rest, so that what the tensor cores truncate is small or exact.
 struct PmSum { float2 re[2], im[2]; };             // a fragment of results: lane 4 g + t holds columns 2 t, 2 t + 1 of rows g, g + 8
-template <bool CONJ_Q>
+template <bool CONJ_Q, bool FULL>
 __device__ __forceinline__ void pm_step(PmSum& sum, const PmFragQ& qr, const PmFragQ& qi, const PmFragP& pr, const PmFragP& pi, const PmFragP& n) {
     // Q: re = Pr Qr - Pi Qi, im = Pi Qr + Pr Qi, n = -Pi;  conj(Q): re = Pr Qr + Pi Qi, im = Pi Qr - Pr Qi, n = -Pr
     const PmFragP &re2 = CONJ_Q ? pi : n, &im2 = CONJ_Q ? n : pr;
     float a[4], b[4];
-    pm_mma_first(a, qr.lo, pr.hi);  pm_mma_first(b, qr.lo, pi.hi);
+    if constexpr (FULL) {
+        pm_mma_first(a, qr.lo, pr.lo); pm_mma_first(b, qr.lo, pi.lo);
+        pm_mma(a, qi.lo, re2.lo); pm_mma(b, qi.lo, im2.lo);
+        pm_mma(a, qr.lo, pr.hi);  pm_mma(b, qr.lo, pi.hi);
+    } else {
+        pm_mma_first(a, qr.lo, pr.hi); pm_mma_first(b, qr.lo, pi.hi);
+    }
     pm_mma(a, qi.lo, re2.hi); pm_mma(b, qi.lo, im2.hi);
     pm_mma(a, qr.hi, pr.lo);  pm_mma(b, qr.hi, pi.lo);
     pm_mma(a, qi.hi, re2.lo); pm_mma(b, qi.hi, im2.lo);
-    pm_mma(a, qr.hi, pr.hi);  pm_mma(b, qr.hi, pi.hi);
-    pm_mma(a, qi.hi, re2.hi); pm_mma(b, qi.hi, im2.hi);
+    if constexpr (FULL) {
+        float c[4], d[4], e[4], f[4];
+        pm_mma_first(c, qr.hi, pr.hi);  pm_mma_first(d, qr.hi, pi.hi);
+        pm_mma_first(e, qi.hi, re2.hi); pm_mma_first(f, qi.hi, im2.hi);
+#pragma unroll
+        for (int h = 0; h < 4; h += 2) {
+            const float2 re = __fadd2_rn(__fadd2_rn(make_float2(c[h], c[h + 1]), make_float2(e[h], e[h + 1])), make_float2(a[h], a[h + 1]));
+            const float2 im = __fadd2_rn(__fadd2_rn(make_float2(d[h], d[h + 1]), make_float2(f[h], f[h + 1])), make_float2(b[h], b[h + 1]));
+            a[h] = re.x; a[h + 1] = re.y; b[h] = im.x; b[h + 1] = im.y;
+        }
+    } else {
+        pm_mma(a, qr.hi, pr.hi);  pm_mma(b, qr.hi, pi.hi);
+        pm_mma(a, qi.hi, re2.hi); pm_mma(b, qi.hi, im2.hi);
+    }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         sum.re[h] = __fadd2_rn(sum.re[h], make_float2(a[2 * h], a[2 * h + 1]));
@@ -116,7 +138,8 @@ __device__ __forceinline__ void pm_step(PmSum& sum, const PmFragQ& qr, const PmF
 // sixteen lanes of a half-warp (four lines, four r) meet two by two.  The results leave through shared memory, as whole
 // 64-byte lines.
 // CONJ_Q: Q enters conjugated.  CONJ_O: the sum is conjugated before it is scaled (conj(P) Q = conj(P conj(Q))).
-template <int NT, bool CONJ_Q, bool CONJ_O>
+// MODE: how the products are made (see PmProducts).
+template <int NT, bool CONJ_Q, bool CONJ_O, PmProducts MODE>
 __global__ void __launch_bounds__(kPmThreads, NT == 1 ? 3 : 2) cgemm_permode_kernel(PerModeParams p) {
     constexpr int ROWS = 8 * NT, LINES = ROWS + kPmCols, STAGE = pm_stage_bytes<NT>(), MT = kPmCols / 16;
     static_assert(ROWS * kPmCols * 64 <= pm_smem_bytes<NT>(), "the results pass through the ring");
@@ -168,9 +191,17 @@ __global__ void __launch_bounds__(kPmThreads, NT == 1 ? 3 : 2) cgemm_permode_ker
     const int g = lane >> 2, t = lane & 3;
     const uint32_t frag = ring + (uint32_t)((t * LINES + g) * 64 + (((warp >> 1) ^ t) << 4) + (warp & 1) * 8);
     constexpr uint32_t HALF = 4 * LINES * 64;                    // terms t + 4
-    PmSum acc[NT][MT];
+    PmSum acc[MODE == PM_FMA ? 1 : NT][MT];
+    // PM_FMA: a lane has one mode, rows row + 4 a (adjacent lines of a half-warp cover all banks) and four columns
+    const int mode = lane & 7, row = lane >> 3, col = 4 * warp;
+    float2 sum[MODE == PM_FMA ? 2 * NT : 1][4];
+    if constexpr (MODE == PM_FMA) {
 #pragma unroll
-    for (int i = 0; i < NT * MT; ++i) (&acc[0][0])[i] = PmSum{};
+        for (int i = 0; i < 8 * NT; ++i) (&sum[0][0])[i] = make_float2(0.f, 0.f);
+    } else {
+#pragma unroll
+        for (int i = 0; i < NT * MT; ++i) (&acc[0][0])[i] = PmSum{};
+    }
     follow_previous_kernel();
     admit_next_kernel();
 #pragma unroll
@@ -180,28 +211,50 @@ __global__ void __launch_bounds__(kPmThreads, NT == 1 ? 3 : 2) cgemm_permode_ker
         asm volatile("cp.async.wait_group %0;" ::"n"(kPmStages - 2) : "memory");
         __syncthreads();                          // this stage has arrived; everybody has left the one refilled next
         fetch(step + kPmStages - 1);
-        const uint32_t st = frag + (uint32_t)(step % kPmStages) * STAGE;
-        PmFragQ qr[MT], qi[MT];
+        if constexpr (MODE == PM_FMA) {
+            const int last = terms - step * kPmTerms < kPmTerms ? terms - step * kPmTerms : kPmTerms;
+            const uint32_t st = ring + (uint32_t)(step % kPmStages) * STAGE + (uint32_t)(mode & 1) * 8;
+#pragma unroll 1
+            for (int r = 0; r < last; ++r) {
+                const uint32_t at = st + (uint32_t)(r * LINES * 64 + (((mode >> 1) ^ (r & 3)) << 4));
+                float2 q[4];
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
+                for (int b = 0; b < 4; ++b) q[b] = pm_load8(at + (uint32_t)(ROWS + col + b) * 64);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float2 v = pm_load8(st + (ROWS + 16 * mt + 8 * (i & 1)) * 64 + (i >> 1) * HALF);
-                pm_split(v.x, qr[mt].hi[i], qr[mt].lo[i]);
-                pm_split(v.y, qi[mt].hi[i], qi[mt].lo[i]);
+                for (int a = 0; a < 2 * NT; ++a) {
+                    const float2 v = pm_load8(at + (uint32_t)(row + 4 * a) * 64);
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) {
+                        float2& s = sum[a][b];
+                        s.x = fmaf(CONJ_Q ? v.y : -v.y, q[b].y, fmaf(v.x, q[b].x, s.x));
+                        s.y = fmaf(CONJ_Q ? -v.x : v.x, q[b].y, fmaf(v.y, q[b].x, s.y));
+                    }
+                }
             }
+        } else {
+            const uint32_t st = frag + (uint32_t)(step % kPmStages) * STAGE;
+            PmFragQ qr[MT], qi[MT];
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            PmFragP pr, pi;
+            for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const float2 v = pm_load8(st + nt * 512 + i * HALF);
-                pm_split(v.x, pr.hi[i], pr.lo[i]);
-                pm_split(v.y, pi.hi[i], pi.lo[i]);
+                for (int i = 0; i < 4; ++i) {
+                    const float2 v = pm_load8(st + (ROWS + 16 * mt + 8 * (i & 1)) * 64 + (i >> 1) * HALF);
+                    pm_split(v.x, qr[mt].hi[i], qr[mt].lo[i]);
+                    pm_split(v.y, qi[mt].hi[i], qi[mt].lo[i]);
+                }
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                PmFragP pr, pi;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const float2 v = pm_load8(st + nt * 512 + i * HALF);
+                    pm_split(v.x, pr.hi[i], pr.lo[i]);
+                    pm_split(v.y, pi.hi[i], pi.lo[i]);
+                }
+                const PmFragP n = pm_negated(CONJ_Q ? pr : pi);
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) pm_step<CONJ_Q, MODE == PM_FULL>(acc[nt][mt], qr[mt], qi[mt], pr, pi, n);
             }
-            const PmFragP n = pm_negated(CONJ_Q ? pr : pi);
-#pragma unroll
-            for (int mt = 0; mt < MT; ++mt) pm_step<CONJ_Q>(acc[nt][mt], qr[mt], qi[mt], pr, pi, n);
         }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -211,17 +264,27 @@ __global__ void __launch_bounds__(kPmThreads, NT == 1 ? 3 : 2) cgemm_permode_ker
     // pairs of i) covers all banks
     auto key = [](int i, int j) { return ((j >> 1) & 1) | (((i >> 1) & 3) << 1); };
     float2* out = reinterpret_cast<float2*>(smem_raw);
+    if constexpr (MODE == PM_FMA) {
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
+        for (int a = 0; a < 2 * NT; ++a)
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int i = 8 * nt + 2 * t + (e & 1), j = 16 * mt + g + 8 * (e >> 1);
-                const PmSum& s = acc[nt][mt];
-                const float re = (e & 1) ? s.re[e >> 1].y : s.re[e >> 1].x, im = (e & 1) ? s.im[e >> 1].y : s.im[e >> 1].x;
-                out[(i * kPmCols + j) * kPmModes + (warp ^ key(i, j))] = make_float2(re, CONJ_O ? -im : im);
+            for (int b = 0; b < 4; ++b) {
+                const int i = row + 4 * a, j = col + b;
+                out[(i * kPmCols + j) * kPmModes + (mode ^ key(i, j))] = make_float2(sum[a][b].x, CONJ_O ? -sum[a][b].y : sum[a][b].y);
             }
+    } else {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int i = 8 * nt + 2 * t + (e & 1), j = 16 * mt + g + 8 * (e >> 1);
+                    const PmSum& s = acc[nt][mt];
+                    const float re = (e & 1) ? s.re[e >> 1].y : s.re[e >> 1].x, im = (e & 1) ? s.im[e >> 1].y : s.im[e >> 1].x;
+                    out[(i * kPmCols + j) * kPmModes + (warp ^ key(i, j))] = make_float2(re, CONJ_O ? -im : im);
+                }
+    }
     __syncthreads();
     const long long m = m0 + 2 * (tid & 3);
     const float2 s0 = (m & 63) ? p.alpha : p.alpha0, s1 = p.alpha;       // m is even: m + 1 is no multiple of 64
@@ -249,6 +312,7 @@ __global__ void __launch_bounds__(kPmThreads, NT == 1 ? 3 : 2) cgemm_permode_ker
 // its line (any assignment of modes to terms serves, as long as P and Q share it).  64 x 64 results per CTA, a warp
 // 16 columns j by 32 rows i; the 64-byte pieces of odd lines change places in pairs, so that two adjacent lines at
 // the same r cover all banks.
+template <bool FULL>
 __global__ void __launch_bounds__(kPmThreads, 2) cgemm_modesum_kernel(PerModeParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -317,7 +381,7 @@ __global__ void __launch_bounds__(kPmThreads, 2) cgemm_modesum_kernel(PerModePar
                 pm_split(v.y, pi.hi[0], pi.lo[0]);
                 pm_split(v.z, pr.hi[1], pr.lo[1]);
                 pm_split(v.w, pi.hi[1], pi.lo[1]);
-                pm_step<true>(acc[nt], qr, qi, pr, pi, pm_negated(pr));
+                pm_step<true, FULL>(acc[nt], qr, qi, pr, pi, pm_negated(pr));
             }
         }
     }
@@ -349,7 +413,7 @@ __global__ void __launch_bounds__(256) permode_reduce_kernel(PerModeParams p) {
         p.o[(ij / p.J) * p.o_si + (ij % p.J) * p.o_sj + m * p.o_sm] = make_float2(s.x * v.x - s.y * v.y, s.x * v.y + s.y * v.x);
     }
 }
-// The same for shared weights: few results (K x N) of many splits, so eight threads share a result (a fixed order again).
+// The same for shared weights: few results (K x N) of many splits, so 32 threads share a result (a fixed order again).
 constexpr int kPmSumReducers = 32;
 __global__ void __launch_bounds__(32 * kPmSumReducers) modesum_reduce_kernel(PerModeParams p) {
     __shared__ float2 part[kPmSumReducers][32];

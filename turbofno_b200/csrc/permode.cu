@@ -9,7 +9,7 @@ bool is_grad(PermodeKind kind) { return kind == PERMODE_GRAD || kind == PERMODE_
 long long blocks_per_split(const PerModeParams& p, int nt) {
     return (p.modes / kPmModes) * (p.J / kPmCols) * ((p.I + 8LL * nt - 1) / (8 * nt));
 }
-// at least four ring stages of terms per CTA
+// splits of about four ring stages of terms (33 terms are split in two)
 long long most_splits(const PerModeParams& p, PermodeKind kind) { return kind == PERMODE_GRAD ? (p.red + 4 * kPmTerms - 1) / (4 * kPmTerms) : 1; }
 
 // Eights of rows i per CTA: as few blocks as 32 rows allow (each reads and splits Q again), padded least: 40 rows of 4096 modes
@@ -36,9 +36,20 @@ int grad_splits(const DeviceInfo& dev, const PerModeParams& p, PermodeKind kind)
     return splits < 1 ? 1 : (int)splits;
 }
 
+// How the products are made, by the number of terms of a sum.  The error of a short sum is that of its products, of which two tf32
+// parts hold fewer bits than FP32; the error of a long one is that of its additions, of which the tensor cores leave one for
+// eight terms.  Gradient of per-mode weights, 64 -> 64 channels, relative error against 64 bits in 1e-7, FP32 / four products / three:
+// 1 term 1.39 / 1.48 / 1.74, 8 terms 1.54 / 1.67 / 1.81, 12 1.63 / 1.68 / 1.83, 16 1.70 / 1.69 / 1.84, 20 1.78 / 1.70 / 1.85, 24
+// 1.85 / 1.71 / 1.85, 32 1.98 / - / 1.86, 1024 2.97 / - / 2.05 (1.33 of it is the transforms').  Gradients of a layer of real
+// 128 x 128 images, us, as chosen / with three products always: 1 item 94.5 / 100.4, 4 items 122 / 119, 7 155 / 145, 16 220 / 216, 20 272 / 259.
+// Gradient of shared weights, blocks of eight modes: 8 blocks 1.62 / 1.78 / 1.92, 16 1.77 / 1.79 / 1.93, 32 2.04 / 1.85 / 1.97, 8192
+// 3.44 / - / 2.39; four products take 2 us more of 32.
+constexpr long long kPmFmaTerms = 15, kPmFullTerms = 23, kPmSumFullBlocks = 16;
 template <int NT, bool CONJ_Q, bool CONJ_O>
 int launch_inst(const DeviceInfo& dev, const PerModeParams& p, cudaStream_t st) {
-    auto kernel = cgemm_permode_kernel<NT, CONJ_Q, CONJ_O>;
+    auto kernel = p.red <= kPmFmaTerms    ? cgemm_permode_kernel<NT, CONJ_Q, CONJ_O, PM_FMA>
+                  : p.red <= kPmFullTerms ? cgemm_permode_kernel<NT, CONJ_Q, CONJ_O, PM_FULL>
+                                          : cgemm_permode_kernel<NT, CONJ_Q, CONJ_O, PM_SPLIT>;
     constexpr size_t smem = pm_smem_bytes<NT>();
     int occ = 0;
     const int rc = prepare_kernel(kernel, smem, dev, &occ, kPmThreads);
@@ -59,10 +70,11 @@ int launch_rows(const DeviceInfo& dev, const PerModeParams& p, PermodeKind kind,
 
 int launch_modesum(const DeviceInfo& dev, const PerModeParams& p, cudaStream_t st) {
     int occ = 0;
-    const int rc = prepare_kernel(cgemm_modesum_kernel, kPmSumSmemBytes, dev, &occ, kPmThreads);
+    auto kernel = p.red <= kPmSumFullBlocks ? cgemm_modesum_kernel<true> : cgemm_modesum_kernel<false>;
+    const int rc = prepare_kernel(kernel, kPmSumSmemBytes, dev, &occ, kPmThreads);
     if (rc != TFNO_OK) return rc;
     const unsigned grid = (unsigned)((p.I + kPmSumTile - 1) / kPmSumTile) * (unsigned)(p.J / kPmSumTile) * (unsigned)p.splits;
-    return launch_chained(cgemm_modesum_kernel, dim3(grid), kPmThreads, kPmSumSmemBytes, st, true, 1, p);
+    return launch_chained(kernel, dim3(grid), kPmThreads, kPmSumSmemBytes, st, true, 1, p);
 }
 
 }  // namespace
