@@ -371,27 +371,10 @@ TFNO_D void store_decimated(const float2 (&v)[64], float2* __restrict__ sig, lon
 }
 
 // The same for contiguous, 16-byte aligned signals whose R lanes are ADJACENT lanes of a warp: a
-// lane and its neighbour (lane ^ 1) want samples that alternate in memory (R*n + r and
-// R*n + r + 1), so each of them moves 16 bytes (two samples, one its own and one the
-// neighbour's) for every second n and they swap the foreign halves with one shuffle.  Half as
-// many load / store instructions, each touching 64 instead of 32 contiguous bytes per signal.
-template <int R>
-TFNO_D void load_decimated_paired(float2 (&v)[64], const float2* __restrict__ sig, int r) {
-    const bool odd = (r & 1) != 0;
-    const float2* base = sig + (odd ? R : 0) + (r & ~1);
-#pragma unroll
-    for (int n2 = 0; n2 < 32; ++n2) {
-        const float4 q = load_global(reinterpret_cast<const float4*>(base + 2 * R * n2));   // samples R*(2*n2 + odd) + (r & ~1), +1
-        const float2 mine = odd ? make_float2(q.z, q.w) : make_float2(q.x, q.y);
-        const float2 send = odd ? make_float2(q.x, q.y) : make_float2(q.z, q.w);
-        float2 got;
-        got.x = __shfl_xor_sync(0xffffffffu, send.x, 1);
-        got.y = __shfl_xor_sync(0xffffffffu, send.y, 1);
-        v[2 * n2] = odd ? got : mine;          // even lane: its sample of n = 2*n2; odd lane: received
-        v[2 * n2 + 1] = odd ? mine : got;
-    }
-}
-
+// lane and its neighbour (lane ^ 1) own samples that alternate in memory (R*j2 + j1 and
+// R*j2 + j1 + 1), so each of them writes 16 bytes (two samples, one its own and one the
+// neighbour's) for every second j2 and they swap the foreign halves with one shuffle.  Half as
+// many store instructions, each touching 64 instead of 32 contiguous bytes per signal.
 template <int R>
 TFNO_D void store_decimated_paired(const float2 (&v)[64], float2* __restrict__ sig, int j1, bool live = true) {
     const bool odd = (j1 & 1) != 0;
