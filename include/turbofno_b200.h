@@ -137,7 +137,7 @@ int tfno_exec(const tfno_plan* plan, const void* x, const void* w, void* y,
 
 /* Scratch a plan can do without but runs faster with, or 0.  Not 0 for 1D variant D plans with shared weights, DY >= 512
  * and K <= 128 whose batch has at least one row (bs*dimX) per SM with N > 64, or four rows per SM with N = 64 and
- * K > 96 (at DY = 1024: K >= 64): given this much they run as three kernels, 1.1 to 1.9 times faster.
+ * K > 96 (at DY = 1024: K >= 64): given this much they run as three kernels, 1.1 to 2 times faster.
  * tfno_exec_scratch is tfno_exec with the size of the workspace: it uses the scratch when there is enough (and runs as
  * tfno_exec when there is less); the rule for one workspace and several streams or threads is the same. */
 size_t tfno_optional_workspace_bytes(const tfno_plan* plan);

@@ -110,10 +110,11 @@ Workspace carve(const tfno_plan_s& pl) {
 // every launch; its long transforms (DY = 512, 1024: chunks of eight and four channels) also use the tensor cores
 // least.  Three kernels over the compact spectra (which are 64/DY of the data) read x once.  Measured, fused against
 // three kernels, us:
-//   DY = 512   K=N=128 at 150 / 600 / 1024 rows 135 / 382 / 531 against 112 / 243 / 355; K=32 N=128 62 / 151 / 204 against 54 / 120 / 177
-//              K=128 N=64 at 600 / 2048 rows 192 / 513 against 161 / 466;  K=N=64 at 1024 rows 142 against 149: stays fused
-//   DY = 1024  K=N=128 at 150 / 1024 rows 191 / 1015 against 140 / 532;  K=N=64 at 600 / 2048 rows 174 / 467 against 153 / 425
-//   DY = 256   K=N=128 at 1024 / 2048 rows 295 / 536 against 274 / 556, K=64 N=128 151 / 269 against 153 / 261: stays fused
+//   DY = 512   K=N=128 at 150 / 600 / 1024 rows 124 / 371 / 520 against 106 / 217 / 320; K=32 N=128 58 / 145 / 198 against 51 / 114 / 172
+//              K=128 N=64 at 600 / 2048 rows 185 / 501 against 145 / 397;  K=N=64 at 1024 rows 149 against 148: stays fused
+//   DY = 1024  K=N=128 at 150 / 1024 rows 184 / 1009 against 137 / 507;  K=N=64 at 600 / 2048 rows 178 / 462 against 153 / 430
+//   DY = 256   K=64 N=128 at 1024 / 2048 rows 154 / 263 against 150 / 257: stays fused.  K=N=128 303 / 529 against 235 / 431, since the
+//              second launch of the contraction loads C ahead: not part of the rule yet
 // Below one row per SM (wide) and four rows per SM (64 outputs) a call is short enough that one or two launches
 // without a workspace are kept.  The scratch is a separate offer (tfno_exec_scratch, with its size): tfno_exec of these
 // plans needs none and leaves a pointer it is given alone, so a plan may run on several streams at once.

@@ -22,9 +22,10 @@
 // field 2.9e-7 -> 2.6e-7).  Operands below 2^-115 lose the last bits of their low parts.
 //
 // What bounds it (2D, 4096 modes, K = N = 64; us, with the FP32 kernel before it): layer of 1 row 36 (36), 16 rows 51 (73), 20
-// rows 66 (94), 64 rows 172 (242).  1D, 64 modes: 16 rows 7 (21), 512 rows 28 (37).  Not always ahead: 40 -> 128 channels, 2
-// rows 39.4 (37.4), 4 rows 41.6 (37.9).  Up to 8 rows the 134 MB of weights (20 us at copy speed); beyond that the multiplier, 55 % busy (20 rows: 33 us at
-// 512 multiply-adds a cycle), with the latencies of a step (load, split, chain of six) behind four warps per scheduler.
+// rows 66 (94), 64 rows 172 (242).  1D, 64 modes: 16 rows 7 (21), 512 rows 28 (37).  Not ahead everywhere: 40 -> 128 channels, 2
+// rows 39.4 (37.4), 4 rows 41.6 (37.9).  Up to 8 rows the 134 MB of weights (20 us at copy speed); beyond that the multiplier,
+// 55 % busy (20 rows: 33 us at 512 multiply-adds a cycle), with the latencies of a step (load, split, chain of six) behind
+// four warps per scheduler.
 // Tried: persistent CTAs whose ring runs on across tiles (79 us at 20 rows: 3.5 tiles per CTA are dealt worse than by the
 // hardware), tiles of 16 columns with three CTAs per SM (71), all loads of a step ahead of its products (68).
 #pragma once

@@ -171,19 +171,22 @@ int launch_permode(const DeviceInfo& dev, PerModeParams p, PermodeKind kind, cud
 
 #if defined(__CUDACC__)
 // Programmatic dependent launch.  A kernel launched `early` may have CTAs resident while the previous kernel of the stream
-// is still finishing.  Every kernel of the library calls follow_previous_kernel() in all threads once it has prepared what
-// needs no global memory (tables, barriers, tensor memory); the call returns when the previous kernel has completed and
-// its writes are visible, so whoever waits for a kernel of the chain waits for all before it.  Only then may the next one be
-// prepared: admit_next_kernel() allows that once every CTA has called it or ended.
+// is still finishing.  Only a kernel whose threads ALL call follow_previous_kernel() before they touch global memory may be
+// launched so; the call returns when the previous kernel has completed and its writes are visible, so whoever waits for a
+// kernel of the chain waits for all before it.  (The copies around the library transforms and the self-test of the bounded
+// wait do not call it: they are launched in order.)  admit_next_kernel() may be called after that wait only; the next launch,
+// if it is an early one, begins once every CTA has called it or ended.
 //
-// Launches of one wave admit others early, and go early where no SM gets two of their CTAs (those that start as SMs become free
-// are stacked on the first of them: contraction of 64 x 128 CTAs that fit twice 53 -> 60 us for a whole 2D layer of 128 -> 128 channels), as do the fused kernel and the per-mode contractions at any length (their
-// operands bypass the L1 cache; training step of 7 x 64 images of 128 x 128 194 against 201 us).  Longer launches of the
-// transforms read through that cache and lose more than they gain when they start beside a kernel that has the shared
+// Early: launches of at most one CTA per SM, and the fused kernel, the per-mode contractions and the weight gradients at any
+// length, whose operands bypass the L1 cache (training step of 7 x 64 images of 128 x 128 194 against 201 us).  Longer launches
+// of the transforms read through that cache and lose more than they gain when they start beside a kernel that has the shared
 // memory: an SM that never drains keeps the division of the two.  1D layer of 1024 x 128 signals of 512 samples as three
-// kernels: all early 391 us, none 351; 2D layer of 128 x 64 images 2160 against 2040.  The contraction of shared weights in
-// several waves: 359 against 355.  Gains: three kernels of one image 27.7 -> 24.0 us, a row-tile kernel behind another 14.3 -> 12.7,
-// training step of 512 x 64 signals of 512 samples 256 -> 247.
+// kernels: 40 us more with all of them early; 2D layer of 128 x 64 images 2160 against 2040 us.  The contraction of shared weights
+// in several waves: 4 us more of 355.  Gains: three kernels of one image 27.7 -> 19.9 us, a row-tile kernel behind another 14.3 ->
+// 12.7, training step of 512 x 64 signals of 512 samples 256 -> 246.
+// Admitted at any length: by the fused kernel, the contractions and gradients, and the clusters of the forward images; by the other
+// transforms and the row-tile kernel in launches of one wave.
+//
 // Dynamic shared memory for a launch of `ctas`.  A CTA for every SM or fewer: each asks for more than half of an SM's, so that none
 // share one; launched early they would be stacked on the first SMs that become free.  2D layers of one batch item, us, each
 // launch in order / early and stacked / early and apart: 64 images of 256 x 256 39.0 / 41.0 / 34.9, 64 of 128 x 128 28.8 / 26.2 /

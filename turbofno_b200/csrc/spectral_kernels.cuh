@@ -72,7 +72,8 @@ TFNO_D void store_modes_to_tile(const float2 (&v)[32], float2* tile, int row, in
 // one row, and a signal on twice the lanes is transformed in half the time while there are lanes to spare (8 channels of 128
 // samples keep 32 of them busy, 32 channels of 256 all 256).  The inverse has N signals and stays on 64 samples per lane:
 // its table for twice the lanes would take shared memory from the widest layers.  The first weights travel beside the
-// forward transforms.  Calls back to back, us, with 64 samples per lane and now: 64 rows, 32 -> 128 channels, 256 samples 12.7 -> 12.0;
+// forward transforms.  Calls back to back, us, with 64 samples per lane and now: 64 rows, 32 -> 128 channels, 256 samples 12.7 -> 12.0
+// (where more channels leave no lanes to spare it can cost: 192 rows, 104 -> 64 channels 49.3 -> 50.3, of 512 samples 80.7 -> 73.9);
 // together with launches that start beside the previous one's tail: 140 rows, 72 -> 64 channels 22.6 -> 19.4, 1200 rows, 200 -> 128 659 -> 610.
 // The contraction alone (!FWD && !INV) of 64 output channels runs two CTAs per SM, which its 128 registers a thread just allow: 1024
 // rows, 192 -> 64 channels 171 us, with 130 registers and one CTA 227.  Its weights are plain loads, which the compiler places
